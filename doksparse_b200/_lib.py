@@ -78,6 +78,8 @@ def _declare(lib):
         "dok_launch_count": ([], I64),
         "dok_table_layout": ([I, I, I64, ctypes.POINTER(LayoutInfo)], I),
         "dok_map_init": ([TP, P], I),
+        "dok_map_init_state": ([TP, P, I, P], I),
+        "dok_next_prime": ([ctypes.c_uint64], ctypes.c_uint64),
         "dok_map_uuid": ([TP, HP, P, I64, P, P, P], I),
         "dok_map_get": ([TP, HP, P, I64, P, P, P, P, P], I),
         "dok_map_get_probe_stats": ([TP, HP, P, I64, P, P, P, P], I),
@@ -101,6 +103,7 @@ def _declare(lib):
         "dok_dok_zero_items": ([TP, HP, SP, P, P], I),
         "dok_dok_gather_insert": ([TP, HP, SP, TP, HP, P, P], I),
         "dok_dok_set_dense": ([TP, HP, SP, P, P, P, I64, P, P], I),
+        "dok_dok_assign": ([TP, HP, SP, P, P, P, I64, P, P, P], I),
         "dok_dense_count_nonzero": ([P, I64, I, I, P, P], I),
         "dok_dense_insert_nonzero": ([TP, HP, P, P, I64, I, P, P], I),
         "dok_partition_tiles": ([I64], I64),

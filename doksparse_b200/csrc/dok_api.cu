@@ -170,7 +170,7 @@ struct Rekey {
 template <int SB>
 __global__ void __launch_bounds__(DOK_TPB) k_rekey_insert(DevTable src, DevTable dst, DevHash hp, Rekey rk, ll_t *counters) {
   const ll_t stride = (ll_t)gridDim.x * DOK_TPB;
-  int claimed = 0, failed = 0;
+  int claimed = 0, failed = 0, found = 0;
   for (ll_t base = (ll_t)blockIdx.x * DOK_TPB; base < src.nb; base += stride) {       // uniform over the block
     const ll_t s = base + threadIdx.x;
     bool active = false;
@@ -217,10 +217,12 @@ __global__ void __launch_bounds__(DOK_TPB) k_rekey_insert(DevTable src, DevTable
     }
     claimed += outcome == DOK_OUT_CLAIMED_EMPTY || outcome == DOK_OUT_REUSED;
     failed += outcome == DOK_OUT_FAILED;
+    found += outcome == DOK_OUT_FOUND;
   }
   if (counters) {
     dok_warp_add(counters + DOK_CNT_CLAIMED_EMPTY, claimed);
     dok_warp_add(counters + DOK_CNT_FAILED, failed);
+    dok_warp_add(counters + DOK_CNT_HITS, found);
   }
 }
 
@@ -320,6 +322,12 @@ int dok_dok_zero_items(const dok_table *t, const dok_hash_params *hp, const dok_
 int dok_dok_set_dense(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel, const void *src,
                       const int64_t *src_strides, int64_t *slot_scratch, int64_t epoch, int64_t *counters,
                       void *stream) {
+  return dok_dok_assign(t, hp, sel, src, src_strides, slot_scratch, epoch, counters, nullptr, stream);
+}
+
+int dok_dok_assign(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel, const void *src,
+                   const int64_t *src_strides, int64_t *slot_scratch, int64_t epoch, int64_t *counters, int64_t *more,
+                   void *stream) {
   DevHash dh;
   DevTable dt;
   SelKeys sk;
@@ -333,7 +341,7 @@ int dok_dok_set_dense(const dok_table *t, const dok_hash_params *hp, const dok_s
     sv.sizes[j] = j < sel->selector_ndim ? sel->sizes[j] : 1;
     sv.strides[j] = j < sel->selector_ndim ? src_strides[j] : 0;
   }
-  return launch_set_general(dt, dh, sk, sv, slot_scratch, epoch, nullptr, counters, (cudaStream_t)stream);
+  return launch_set_general(dt, dh, sk, sv, slot_scratch, epoch, nullptr, counters, (cudaStream_t)stream, more);
 }
 
 int dok_dok_gather_insert(const dok_table *src, const dok_hash_params *src_hp, const dok_selectors *sel,

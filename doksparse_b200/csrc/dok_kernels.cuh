@@ -119,10 +119,14 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_set_unique(DevTable t, DevHash h
   }
 }
 
-// Stamp word of a slot during a general set: (epoch << 33) | (row << 1) | conflict.  The epoch of a call is
-// larger than every epoch used on the table before, so an atomicMax leaves the LAST row of this batch that
-// targets the slot; the low bit records that more than one row of the batch did.
-__device__ __forceinline__ ll_t dok_stamp(ll_t epoch, ll_t row) { return (epoch << 33) | (row << 1); }
+// Stamp word of a slot during a general set: (epoch << 34) | (row << 2) | fresh << 1 | conflict, unsigned.  The epoch of
+// a call is larger than every epoch used on the table before, so an atomicMax leaves the LAST row of this batch that
+// targets the slot; the lowest bit records that more than one row of the batch did, the next one (k_set_count only) that
+// such a slot was claimed by this batch.
+#define DOK_STAMP_CONFLICT 1ULL
+#define DOK_STAMP_FRESH 2ULL
+#define DOK_ROW_FRESH (1LL << 62)      // bit of a row's slot index: this row claimed the slot
+__device__ __forceinline__ ull_t dok_stamp(ll_t epoch, ll_t row) { return ((ull_t)epoch << 34) | ((ull_t)row << 2); }
 
 // First kernel of the general set.  Find or claim the slot, store the row there and raise the slot's stamp --
 // for a batch without equal uuids that is all there is to do.  A row that finds the slot already stamped in
@@ -130,7 +134,7 @@ __device__ __forceinline__ ll_t dok_stamp(ll_t epoch, ll_t row) { return (epoch 
 // launch); the second kernel then lets the slot's last row rewrite it.
 template <int SB, class Keys, class Values>
 __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp, Keys keys, Values values,
-                                                       ll_t *__restrict__ slot_out, ll_t epoch,
+                                                       ll_t *__restrict__ slot_out, ll_t epoch, int mark_fresh,
                                                        uint8_t *__restrict__ out_stored, ll_t *counters) {
   __shared__ BlockTally tally;
   if (keys.idle()) return;
@@ -143,17 +147,20 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
   int outcome = -1, dup = 0;
   const ll_t slot = dok_find_or_claim<SB>(t, kh, active, &outcome);
   if (active) {
-    slot_out[e] = slot;
+    const bool fresh = outcome == DOK_OUT_CLAIMED_EMPTY || outcome == DOK_OUT_REUSED;
+    slot_out[e] = mark_fresh && fresh ? slot | DOK_ROW_FRESH : slot;
     if (slot >= 0) {
       // the row is stored without waiting for the stamp's answer: the two requests travel together.  If the slot
       // turns out to be shared, whatever the racing stores left is rewritten by the second kernel.
       ll_t *stamp = dok_stamp_ptr(t, slot);
       dok_write_row(t, hp, keys, values, e, slot, outcome != DOK_OUT_FOUND || hp.dtype >= DOK_F16);
-      const ll_t old = (ll_t)atomicMax(stamp, dok_stamp(epoch, e));
-      if ((old >> 33) == epoch) {
-        atomicOr((ull_t *)stamp, 1ULL);
+      const ull_t old = atomicMax((ull_t *)stamp, dok_stamp(epoch, e));
+      if ((old >> 34) == (ull_t)epoch) {
+        atomicOr((ull_t *)stamp, DOK_STAMP_CONFLICT);
         dup = 1;
       }
+    } else {
+      dup = mark_fresh;               // a row without a place is counted by k_set_count too
     }
     if (out_stored) out_stored[e] = (uint8_t)(slot >= 0);
   }
@@ -182,31 +189,61 @@ __global__ void __launch_bounds__(DOK_TPB) k_set_resolve(DevTable t, DevHash hp,
   for (ll_t j = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x; j < span; j += stride) {
     ll_t e;
     if (!keys.at(j, e)) continue;
-    const ll_t slot = slot_in[e];
+    ll_t slot = slot_in[e];
     if (slot < 0) continue;
+    const bool fresh = (slot & DOK_ROW_FRESH) != 0;
+    slot &= ~DOK_ROW_FRESH;
     if (t.win_hi != 0) {                         // windowed passes: by the slot's own group (each slot has one pass)
       const ll_t g = slot / t.spg;
       if (g < t.win_lo || g >= t.win_hi) continue;
     }
-    if (__ldcg(dok_stamp_ptr(t, slot)) != (dok_stamp(epoch, e) | 1)) continue;
+    const ull_t stamp = (ull_t)__ldcg(dok_stamp_ptr(t, slot));
+    if (!(stamp & DOK_STAMP_CONFLICT)) continue;
+    if (fresh) atomicOr((ull_t *)dok_stamp_ptr(t, slot), DOK_STAMP_FRESH);
+    if ((stamp & ~DOK_STAMP_FRESH) != (dok_stamp(epoch, e) | DOK_STAMP_CONFLICT)) continue;
     dok_write_row(t, hp, keys, values, e, slot, true);
   }
+}
+
+// Third kernel, for callers that count like the reference's DOK assignment does (sparse_dok_tensor_impl.py:461-474): every
+// row whose key was not stored before the batch, its repetitions too.  The claims are counted already; this adds the
+// other rows of the slots that the batch claimed, and rows that found the table full.  Counting the stored keys in a pass
+// of its own before the set, as the reference does, costs a walk per row: 145 of the 800 us of a 4 M-row assignment.
+template <class Keys>
+__global__ void __launch_bounds__(DOK_TPB) k_set_count(DevTable t, Keys keys, const ll_t *__restrict__ slot_in, ll_t epoch,
+                                                       ll_t *__restrict__ more) {
+  if (slot_in[keys.count()] == 0) return;
+  const ll_t span = keys.span(), stride = (ll_t)gridDim.x * DOK_TPB;
+  int c = 0;
+  for (ll_t j = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x; j < span; j += stride) {
+    ll_t e;
+    if (!keys.at(j, e)) continue;
+    const ll_t slot = slot_in[e];
+    if (slot < 0) { c++; continue; }
+    if (slot & DOK_ROW_FRESH) continue;
+    const ull_t stamp = (ull_t)__ldcg(dok_stamp_ptr(t, slot));
+    c += (stamp >> 34) == (ull_t)epoch && (stamp & DOK_STAMP_FRESH) != 0;
+  }
+  dok_warp_add(more, c);
 }
 
 // contiguous value rows [n, value_bytes]
 template <class Keys, class Values>
 inline int launch_set_general(const DevTable &t, const DevHash &hp, const Keys &keys, const Values &values,
-                              int64_t *slot_scratch, int64_t epoch, uint8_t *out_stored, int64_t *counters, cudaStream_t st) {
+                              int64_t *slot_scratch, int64_t epoch, uint8_t *out_stored, int64_t *counters, cudaStream_t st,
+                              int64_t *more = nullptr) {
   if (cudaMemsetAsync(slot_scratch + keys.n, 0, sizeof(int64_t), st) != cudaSuccess) return dok_check_launch();
   const dim3 grid = dok_grid(keys);
   int rc = DOK_OK;
   DOK_DISPATCH_SB(t, DOK_FOR_WINDOWS(t, rc, (k_set_claim<SB><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, (ll_t *)slot_scratch,
-                                                                                       (ll_t)epoch, out_stored, (ll_t *)counters))));
+                                                                                       (ll_t)epoch, more != nullptr, out_stored, (ll_t *)counters))));
   if (rc != DOK_OK) return rc;
   dim3 few = grid;
   if (few.x > 148 * 8) few.x = 148 * 8;
   DOK_FOR_WINDOWS(t, rc, (k_set_resolve<<<few, DOK_TPB, 0, st>>>(wt, hp, keys, values, (const ll_t *)slot_scratch, (ll_t)epoch)));
-  return rc;
+  if (rc != DOK_OK || more == nullptr) return rc;
+  k_set_count<<<few, DOK_TPB, 0, st>>>(t, keys, (const ll_t *)slot_scratch, (ll_t)epoch, (ll_t *)more);
+  return dok_check_launch();
 }
 
 inline int launch_set(const DevTable &t, const DevHash &hp, const RowKeys &keys, const char *values, int64_t *slot_scratch,
@@ -308,7 +345,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_count_new(DevTable t, DevHash hp, K
 template <int SB>
 __global__ void __launch_bounds__(DOK_TPB) k_reinsert(DevTable src, DevTable dst, DevHash hp, ll_t *counters) {
   const ll_t stride = (ll_t)gridDim.x * DOK_TPB;
-  int claimed = 0, failed = 0;
+  int claimed = 0, failed = 0, found = 0;
   for (ll_t base = (ll_t)blockIdx.x * DOK_TPB; base < src.nb; base += stride) {       // uniform over the block
     const ll_t s = base + threadIdx.x;
     bool active = false;
@@ -339,10 +376,12 @@ __global__ void __launch_bounds__(DOK_TPB) k_reinsert(DevTable src, DevTable dst
     }
     claimed += outcome == DOK_OUT_CLAIMED_EMPTY || outcome == DOK_OUT_REUSED;
     failed += outcome == DOK_OUT_FAILED;
+    found += outcome == DOK_OUT_FOUND;
   }
   if (counters) {
     dok_warp_add(counters + DOK_CNT_CLAIMED_EMPTY, claimed);
     dok_warp_add(counters + DOK_CNT_FAILED, failed);
+    dok_warp_add(counters + DOK_CNT_HITS, found);
   }
 }
 
@@ -350,8 +389,9 @@ __global__ void __launch_bounds__(DOK_TPB) k_reinsert(DevTable src, DevTable dst
 // init / uuid
 // ---------------------------------------------------------------------------------------------------------
 
-static __global__ void k_init(DevTable t) {
+static __global__ void k_init(DevTable t, ll_t *state, int state_words) {
   const ll_t stride = (ll_t)gridDim.x * blockDim.x;
+  if (blockIdx.x == 0 && threadIdx.x < state_words) state[threadIdx.x] = 0;
   for (ll_t i = (ll_t)blockIdx.x * blockDim.x + threadIdx.x; i < t.n_slots; i += stride) {
     *dok_tag_ptr(t, i) = i < t.nb ? DOK_EMPTY : DOK_BLOCKED;
     if (t.stamp_off >= 0 || t.stamp) *dok_stamp_ptr(t, i) = 0;

@@ -28,11 +28,13 @@ int dok_table_layout(int value_bytes, int key_bytes, int64_t n_buckets, dok_layo
   return DOK_OK;
 }
 
-int dok_map_init(const dok_table *t, void *stream) {
+int dok_map_init(const dok_table *t, void *stream) { return dok_map_init_state(t, nullptr, 0, stream); }
+
+int dok_map_init_state(const dok_table *t, int64_t *state, int state_words, void *stream) {
   DevTable dt;
-  if (!dok_make_table(t, &dt)) return DOK_BAD_ARG;
+  if (!dok_make_table(t, &dt) || state_words < 0 || state_words > 256 || (state_words > 0 && !state)) return DOK_BAD_ARG;
   const ll_t blocks = (dt.n_slots + 255) / 256;
-  k_init<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, (cudaStream_t)stream>>>(dt);
+  k_init<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, (cudaStream_t)stream>>>(dt, (ll_t *)state, state_words);
   return dok_check_launch();
 }
 

@@ -17,6 +17,7 @@ What is different (the slot layout is not part of the contract)
   * duplicates inside one `set` batch resolve deterministically to the last row.
 """
 import ctypes
+import threading
 
 import numpy as np
 import torch
@@ -24,6 +25,61 @@ from torch import Tensor
 
 from . import _lib as L
 from .util import next_prime
+
+_PARAM_NAMES = ("prime1", "prime2", "alpha1", "alpha2", "beta1", "beta2")
+
+# The counters of a table, one device int64 array (`_state`): kernels add to a block of L.N_COUNTERS each, and what the
+# map reports is a sum over them, so no operation needs counters of its own, their zeroing, or kernels that add them up.
+_STATE_WORDS = 32
+_BY_SET, _BY_REMOVE, _BY_ROWS, _BY_BULK = 0, 8, 16, 24      # set | remove | distinct new rows of float keys | bulk inserts
+_ADJUST = 7              # what n_elements differs by from the slots in use (the reference's DOK assignments over-count)
+_COUNTED_NEW = 23        # result of the exact count of a set that may have to grow the table
+
+
+class _PinnedRings:
+    """Pinned landing places for copies of the counters, 8 per table, cut from chunks that serve 64 tables: pinning memory
+    takes milliseconds (33 ms once the process has mapped a few GB), more than anything else a new table does.  A table
+    gives its ring back when it goes; at most 256 are kept."""
+
+    def __init__(self):
+        self._lock, self._free = threading.Lock(), []
+
+    def take(self):
+        with self._lock:
+            if not self._free:
+                chunk = torch.zeros(64, 8, _STATE_WORDS, dtype=torch.long, pin_memory=True)
+                self._free = [(chunk[i], None) for i in range(64)]
+            ring, last_copy = self._free.pop()
+        if last_copy is not None:
+            last_copy.synchronize()             # the previous owner's copies have landed: nothing writes here any more
+        return ring
+
+    def give(self, ring, last_copy):
+        with self._lock:
+            if len(self._free) < 256:
+                self._free.append((ring, last_copy))
+
+
+_rings = _PinnedRings()
+
+
+class _Shared:
+    """What shallow clones (views) must see together: the duplicate-resolution stamps with their epoch, and the host-side
+    upper bound of n_elements that lets `set` skip a device synchronisation."""
+    __slots__ = ("stamp", "epoch", "bound", "base", "snapshots", "ring", "last_copy")
+
+    def __init__(self, stamp=None, epoch=0, bound=0):
+        self.stamp, self.epoch, self.bound, self.base = stamp, epoch, bound, bound
+        self.snapshots, self.ring, self.last_copy = [], None, None
+
+    def __del__(self):
+        if self.ring is not None:
+            _rings.give(self.ring, self.last_copy)
+
+    def exact(self, n):
+        """n_elements is known to be n, and nothing enqueued later has been counted in."""
+        self.snapshots.clear()
+        self.bound = self.base = n
 
 
 class CudaClosedHashmap:
@@ -49,28 +105,26 @@ class CudaClosedHashmap:
         self.device = torch.device(device)
         if self.device.type != "cuda":
             raise L.DokError("CudaClosedHashmap needs a CUDA device: there is no CPU path")
+        if not torch.cuda.is_initialized():
+            torch.cuda.init()
         L.lib()  # fail loudly now if the extension is missing
         # before the first `set` only the tags exist (cuda_closed_hashmap.py:40)
         self._slots = None           # uint8 storage of the slot array
         self._key_shape = None
         self._key_dtype = None
-        self._uuid_only = torch.full((self._n_buckets,), self._empty_marker, device=self.device, dtype=torch.long)
-        # state that shallow clones (views) must see together: the duplicate-resolution stamps with their epoch,
-        # and the host-side upper bound of n_elements that lets `set` skip a device synchronisation
-        self._shared = {"stamp": None, "epoch": 0, "bound": 0, "snapshots": []}
+        self._shared = _Shared()
         self._value_shape = None
         self._value_dtype = None
 
         self._key_size = key_size
-        as_param = lambda v: v if v is None or isinstance(v, Tensor) else self._as_param(np.asarray(v).reshape(-1).tolist())
-        self._prime1, self._prime2 = as_param(prime1), as_param(prime2)
-        self._alpha1, self._alpha2 = as_param(alpha1), as_param(alpha2)
-        self._beta1, self._beta2 = as_param(beta1), as_param(beta2)
-        self._n_elements = torch.zeros(size=(), device=self.device, dtype=torch.long)
-        # rows that a set could not store because the table was full (the reference drops them silently,
-        # closed_hashmap_impl_class.cu:426; here they are counted on the device and reported at the next point where
-        # the host synchronises anyway: n_elements, state_dict, the exact-count path of set)
-        self._n_failed = torch.zeros(size=(), device=self.device, dtype=torch.long)
+        # hash parameters: host integers (`_host`) and, where the caller asks for them, device tensors (`_on_device`)
+        self._host, self._on_device = {}, {}
+        for name, given in zip(_PARAM_NAMES, (prime1, prime2, alpha1, alpha2, beta1, beta2)):
+            if isinstance(given, Tensor):
+                self._on_device[name] = given
+            elif given is not None:
+                self._host[name] = [int(v) for v in np.asarray(given).reshape(-1).tolist()]
+        self._counters_of_table = None
         self._rehash_factor = rehash_factor
         self._rehash_threshold = rehash_threshold
         # Tombstone-aware maintenance (no counterpart in the reference, whose rehash looks at live items only,
@@ -81,14 +135,14 @@ class CudaClosedHashmap:
         # "auto" (the default): t = 0.95, and only once the tombstones are worth a rebuild (2 % of the buckets).
         # None: never (the reference's behaviour).  A number: that t, for any number of tombstones.
         self._tombstone_threshold = tombstone_threshold
-        self._n_tombstones = torch.zeros(size=(), device=self.device, dtype=torch.long)   # upper bound, on the device
-        self._tombstone_host_bound = 0                                                  # looser bound, on the host
+        self._tombstone_host_bound = 0          # upper bound on the host of what `tombstone_bound` counts on the device
 
         self._key_perm = None
         if key_perm is not None:
             if not isinstance(key_perm, Tensor):
                 key_perm = torch.tensor(key_perm, dtype=torch.long, device=self.device)
             self._key_perm = key_perm.to(device=self.device, dtype=torch.long)
+        self._host_perm = None
         self._hp = None       # cached ctypes dok_hash_params
         self._table = None
 
@@ -99,49 +153,53 @@ class CudaClosedHashmap:
             return int(np.prod(self._key_shape))
         return int(self._key_size)
 
-    def _as_param(self, values):
-        return torch.tensor([int(v) for v in values], device=self.device, dtype=torch.long)
+    def _draw(self, name):
+        """A parameter that the caller did not give, drawn with the reference's calls (:66-113)."""
+        ks = self._current_key_size()
+        if name == "prime1":
+            raw = [np.random.randint(self.n_buckets, self.n_buckets * 2) for _ in range(ks)]
+            return [next_prime(r) for r in raw]
+        if name == "prime2":
+            raw = [np.random.randint(0, 2 ** 60, dtype="int64") for _ in range(ks)]
+            return [next_prime(r) for r in raw]
+        return [int(np.random.randint(p)) - 1 for p in self._host_param("prime1")]
+
+    def _host_param(self, name):
+        values = self._host.get(name)
+        if values is None:
+            given = self._on_device.get(name)
+            values = self._host[name] = self._draw(name) if given is None else given.cpu().tolist()
+        return values
+
+    def _param(self, name):
+        t = self._on_device.get(name)
+        if t is None:
+            t = self._on_device[name] = torch.tensor(self._host_param(name), device=self.device, dtype=torch.long)
+        return t
 
     @property
     def prime1(self):
-        if self._prime1 is None:
-            raw = [np.random.randint(self.n_buckets, self.n_buckets * 2) for _ in range(self._current_key_size())]
-            self._prime1 = self._as_param(next_prime(r) for r in raw)
-        return self._prime1
+        return self._param("prime1")
 
     @property
     def prime2(self):
-        if self._prime2 is None:
-            raw = [np.random.randint(0, 2 ** 60, dtype="int64") for _ in range(self._current_key_size())]
-            self._prime2 = self._as_param(next_prime(r) for r in raw)
-        return self._prime2
-
-    def _draw_below_prime1(self):
-        return self._as_param(np.random.randint(int(p)) - 1 for p in self.prime1.cpu())
+        return self._param("prime2")
 
     @property
     def alpha1(self):
-        if self._alpha1 is None:
-            self._alpha1 = self._draw_below_prime1()
-        return self._alpha1
+        return self._param("alpha1")
 
     @property
     def alpha2(self):
-        if self._alpha2 is None:
-            self._alpha2 = self._draw_below_prime1()
-        return self._alpha2
+        return self._param("alpha2")
 
     @property
     def beta1(self):
-        if self._beta1 is None:
-            self._beta1 = self._draw_below_prime1()
-        return self._beta1
+        return self._param("beta1")
 
     @property
     def beta2(self):
-        if self._beta2 is None:
-            self._beta2 = self._draw_below_prime1()
-        return self._beta2
+        return self._param("beta2")
 
     @property
     def key_perm(self):
@@ -159,11 +217,47 @@ class CudaClosedHashmap:
         new = new.to(device=self.device, dtype=torch.long)
         assert new.shape == self.key_perm.shape
         self._key_perm = new
+        self._host_perm = None
         self._hp = None
+
+    def _perm(self):
+        """key_perm as host integers."""
+        if self._host_perm is None:
+            n = int(np.prod(self.key_shape))
+            self._host_perm = list(range(n)) if self._key_perm is None else self._key_perm.cpu().tolist()
+            assert len(self._host_perm) == n
+        return self._host_perm
 
     def _materialise_parameters(self):
         # evaluation order of the reference's kernel call (cuda_closed_hashmap.py:350-357)
-        return (self.prime1, self.prime2, self.alpha1, self.alpha2, self.beta1, self.beta2, self.key_perm)
+        for name in _PARAM_NAMES:
+            self._host_param(name)
+
+    # ------------------------------------------------------------------ counters
+    @property
+    def _state(self):
+        if self._counters_of_table is None:
+            self._counters_of_table = torch.zeros(_STATE_WORDS, device=self.device, dtype=torch.long)
+        return self._counters_of_table
+
+    def _adjust(self, by):
+        """n_elements += by (a number or a device scalar) without a change of the slots in use."""
+        self._state[_ADJUST] += by
+        self._shared.bound += by if isinstance(by, int) else 0
+
+    def _counter_block(self, block):
+        return ctypes.c_void_p(self._state.data_ptr() + 8 * block)
+
+    def _sizes(self, state=None):
+        """(n_elements, live slots, tombstones, failed rows) from one read of the counters."""
+        c = self._state.tolist() if state is None else state
+        bulk = c[_BY_BULK] + c[_BY_BULK + 1]
+        removed = c[_BY_REMOVE + L.CNT_HITS]
+        live = c[0] + c[1] + bulk - removed
+        # float keys are counted by rows, because their value cast makes different rows share a slot
+        inserted = c[_BY_ROWS] if self._key_dtype in L.FLOAT_DTYPES else c[0] + c[1]
+        n = inserted + bulk + c[_BY_BULK + L.CNT_HITS] - removed + c[_ADJUST]
+        return n, live, removed - c[1], c[L.CNT_FAILED] + c[_BY_BULK + L.CNT_FAILED]
 
     # ------------------------------------------------------------------ storage
     def _allocate(self, key_shape, key_dtype, value_shape, value_dtype):
@@ -183,16 +277,19 @@ class CudaClosedHashmap:
         self._value_shape, self._value_dtype = torch.Size(value_shape), value_dtype
         self._key_shape, self._key_dtype = torch.Size(key_shape), key_dtype
         self._slots = torch.empty(lay.total_bytes, device=self.device, dtype=torch.uint8)
-        self._uuid_only = None
-        self._shared["stamp"] = None
+        self._shared.stamp = None
         self._hp = None
+        if self._counters_of_table is None:
+            self._counters_of_table = torch.empty(_STATE_WORDS, device=self.device, dtype=torch.long)
         with torch.cuda.device(self.device):
-            L.check(L.lib().dok_map_init(self._c_table(), L.stream_ptr(self.device)), "dok_map_init")
+            L.check(L.lib().dok_map_init_state(self._c_table(), self._counter_block(0), _STATE_WORDS,
+                                               L.stream_ptr(self.device)), "dok_map_init_state")
 
     def _begin_bulk_insert(self, key_shape, key_dtype, value_shape, value_dtype, n_new):
         """What `set` does to a never-used map before its kernel runs, for a batch known to hold `n_new` pairwise
         different new keys: allocate, draw the parameters, grow if the reference's trigger fires (which re-draws them,
-        cuda_closed_hashmap.py:365-366, 456-468), account for the new elements.  The caller then inserts the rows."""
+        cuda_closed_hashmap.py:365-366, 456-468).  The caller then inserts the rows with a kernel that counts into
+        `_counter_block(_BY_BULK)`."""
         assert self._slots is None
         self._allocate(key_shape, key_dtype, value_shape, value_dtype)
         if n_new == 0:
@@ -204,8 +301,7 @@ class CudaClosedHashmap:
                           tombstone_threshold=self._tombstone_threshold)
             self._allocate(key_shape, key_dtype, value_shape, value_dtype)
             self._materialise_parameters()
-        self._n_elements += n_new
-        self._shared["bound"] = n_new
+        self._shared.exact(n_new)
 
     def _slot_view(self, dtype, inner_shape, byte_offset):
         """[n_buckets, *inner_shape] strided view of one field of the slot array."""
@@ -221,7 +317,7 @@ class CudaClosedHashmap:
     def _uuid(self):
         """[n_buckets] int64 tags: uuid, -1 empty, -3 removed (a strided view of the slot array)."""
         if self._slots is None:
-            return self._uuid_only
+            return torch.full((self._n_buckets,), self._empty_marker, device=self.device, dtype=torch.long)
         return self._slot_view(torch.int64, (), 0)
 
     @property
@@ -242,17 +338,17 @@ class CudaClosedHashmap:
         """Epoch of the next general set: larger than every epoch stamped on this table before.  The stamps live in
         the slots when the layout has room for them, else in a separate array allocated on first use."""
         sh = self._shared
-        if self._layout.stamp_offset < 0 and sh["stamp"] is None:
-            sh["stamp"] = torch.zeros(self._layout.n_slots, device=self.device, dtype=torch.long)
-        if sh["epoch"] >= L.MAX_EPOCH - 1:
+        if self._layout.stamp_offset < 0 and sh.stamp is None:
+            sh.stamp = torch.zeros(self._layout.n_slots, device=self.device, dtype=torch.long)
+        if sh.epoch >= L.MAX_EPOCH - 1:
             raise L.DokError("stamp epochs exhausted: rehash() the map to start over")
-        sh["epoch"] += 1
-        return sh["epoch"]
+        sh.epoch += 1
+        return sh.epoch
 
     def _c_table(self):
         t = L.Table()
         t.slots = self._slots.data_ptr()
-        stamp = self._shared["stamp"]
+        stamp = self._shared.stamp
         t.stamp = stamp.data_ptr() if stamp is not None else None
         t.n_buckets = self._n_buckets
         t.slot_bytes = self._layout.slot_bytes
@@ -268,17 +364,12 @@ class CudaClosedHashmap:
             ks = int(np.prod(self.key_shape))
             hp.key_size = ks
             hp.key_dtype = L.DTYPE_CODES[self._key_dtype]
-            names = ("alpha2", "beta2", "prime2", "alpha1", "beta1", "prime1")
-            host = {name: getattr(self, name).cpu().tolist() for name in names}
-            perm = self.key_perm.cpu().tolist()
-            assert all(len(v) == ks for v in host.values()) and len(perm) == ks
-            for name in names:
-                arr = getattr(hp, name)
-                for i in range(ks):
-                    arr[i] = host[name][i]
-            for i in range(ks):
-                hp.key_perm[i] = perm[i]
-                assert abs(host["prime1"][i]) >= 2 and abs(host["prime2"][i]) >= 2, "primes must have magnitude >= 2"
+            host, perm = {name: self._host_param(name) for name in _PARAM_NAMES}, self._perm()
+            assert all(len(v) == ks for v in host.values())
+            for name in _PARAM_NAMES:
+                getattr(hp, name)[:ks] = host[name]
+            hp.key_perm[:ks] = perm
+            assert all(abs(p) >= 2 for p in host["prime1"] + host["prime2"]), "primes must have magnitude >= 2"
             if 0 in host["alpha2"]:
                 import warnings
                 warnings.warn("alpha2 contains 0: the uuid ignores that key element, so keys differing only there "
@@ -290,44 +381,51 @@ class CudaClosedHashmap:
         return torch.zeros(L.N_COUNTERS, device=self.device, dtype=torch.long)
 
     # The rehash decision of `set` needs n_elements on the host, which the reference gets with a blocking .item()
-    # per call.  Here the host keeps an UPPER BOUND instead: after every mutation the device count is copied to
-    # pinned memory without waiting, and the bound is the newest copy that has landed plus the sizes of the set
-    # batches enqueued after it.  Only when that bound crosses the threshold is the exact value fetched.
+    # per call.  Here the host keeps an UPPER BOUND instead: every set adds its rows to it, and now and then the device
+    # counters are copied to pinned memory without waiting; the bound is then the newest copy that has landed plus the
+    # sizes of the batches enqueued after it.  Only when the bound crosses the threshold is the exact value fetched.
+    # A copy costs more than a small set, so one is made when the bound has used up a quarter of the room that was left at
+    # the last one.
     def _after_mutation(self, added):
         sh = self._shared
-        sh["bound"] += added
-        snaps = sh["snapshots"]
-        for s in snaps:
+        sh.bound += added
+        for s in sh.snapshots:
             s[2] += added                       # rows that may have been inserted after that snapshot was taken
-        ring = sh.get("ring")
-        if ring is None:
-            ring = sh["ring"] = torch.zeros(8, dtype=torch.long, pin_memory=True)
-        free = set(range(ring.numel())) - {s[1] for s in snaps}
+        room = int(self._rehash_threshold * self._n_buckets) - sh.base
+        if 4 * (sh.bound - sh.base) < room:
+            return
+        if sh.ring is None:
+            sh.ring = _rings.take()
+        free = set(range(sh.ring.shape[0])) - {s[1] for s in sh.snapshots}
         if not free:
             return                              # eight copies still in flight: skip this one, the bound stays valid
         slot = free.pop()
         with torch.cuda.device(self.device):
-            ring[slot:slot + 1].copy_(self._n_elements.reshape(1), non_blocking=True)
+            sh.ring[slot].copy_(self._state, non_blocking=True)
             event = torch.cuda.Event()
             event.record()
-        snaps.append([event, slot, 0])
+        sh.snapshots.append([event, slot, 0])
+        sh.last_copy = event
+        sh.base = sh.bound
 
     def _element_bound(self):
         sh = self._shared
-        snaps = sh["snapshots"]
         newest = None
-        while snaps and snaps[0][0].query():
-            newest = snaps.pop(0)
+        while sh.snapshots and sh.snapshots[0][0].query():
+            newest = sh.snapshots.pop(0)
         if newest is not None:
-            sh["bound"] = min(sh["bound"], int(sh["ring"][newest[1]]) + newest[2])
-        return sh["bound"]
+            n = self._sizes(sh.ring[newest[1]].tolist())[0]
+            sh.bound = min(sh.bound, n + newest[2])
+            if not sh.snapshots:
+                sh.base = min(sh.base, n)
+        return sh.bound
 
     def _room_for(self, rows, limit):
         """bound + rows <= limit?  When the bound is too high only because the host runs ahead of the device, wait
         for the count copies still in flight to land -- oldest first, each an event on the stream -- instead of for the
         whole stream: the device keeps the work that is queued behind them."""
         bound = self._element_bound()
-        snaps = self._shared["snapshots"]
+        snaps = self._shared.snapshots
         while bound + rows > limit and snaps:
             snaps[0][0].synchronize()
             bound = self._element_bound()
@@ -360,16 +458,8 @@ class CudaClosedHashmap:
         return k, v, u
 
     def count_live(self):
-        """Live slots, counted by the compaction's first pass (one read of the tags, tile sums, one scan) instead of
-        a mask tensor plus a reduction."""
-        if self._slots is None:
-            return 0
-        lib = L.lib()
-        with torch.cuda.device(self.device):
-            tiles = lib.dok_compact_tiles(self._n_buckets)
-            offsets = torch.empty(tiles + 1, device=self.device, dtype=torch.long)
-            L.check(lib.dok_map_compact_count(self._c_table(), L.ptr(offsets), L.stream_ptr(self.device)), "dok_map_compact_count")
-            return int(offsets[-1].item())
+        """Live slots, from the counters that every kernel keeps."""
+        return 0 if self._slots is None else self._sizes()[1]
 
     @property
     def nonempty_mask(self):
@@ -387,7 +477,7 @@ class CudaClosedHashmap:
 
     def uuid(self):
         if self._slots is None:
-            return self._uuid_only[:0]
+            return torch.empty(0, device=self.device, dtype=torch.long)
         return self.items(keys=False, values=False)[2]
 
     def set_values(self, selectors, new_values):
@@ -402,37 +492,31 @@ class CudaClosedHashmap:
         assert len(set(ordering)) == len(ordering), "duplicates are not allowed"
         self._materialise_parameters()
         self._keys.copy_(self._keys[:, ordering].clone())
-        for name in ("_alpha1", "_alpha2", "_beta1", "_beta2", "_prime1", "_prime2"):
-            setattr(self, name, getattr(self, name)[ordering])
+        self._host = {name: [self._host_param(name)[i] for i in ordering] for name in _PARAM_NAMES}
+        self._on_device = {}
         self._hp = None
 
     def clone(self, deepclone=False):
         self._materialise_parameters()
         cp = (lambda x: x.clone()) if deepclone else (lambda x: x)
         new = CudaClosedHashmap(
-            n_buckets=self.n_buckets, device=self.device,
-            prime1=cp(self.prime1), prime2=cp(self.prime2), alpha1=cp(self.alpha1), alpha2=cp(self.alpha2),
-            beta1=cp(self.beta1), beta2=cp(self.beta2), key_perm=cp(self._key_perm),
+            n_buckets=self.n_buckets, device=self.device, **{name: list(self._host_param(name)) for name in _PARAM_NAMES},
+            key_perm=None if self._key_perm is None else cp(self._key_perm),
             rehash_factor=self._rehash_factor, rehash_threshold=self._rehash_threshold,
             tombstone_threshold=self._tombstone_threshold,
         )
-        new._n_tombstones = cp(self._n_tombstones)
         new._tombstone_host_bound = self._tombstone_host_bound
         if self._slots is not None:
             new._slots = cp(self._slots)
-            new._uuid_only = None
             new._layout = self._layout
             new._value_bytes, new._key_bytes = self._value_bytes, self._key_bytes
             new._value_shape, new._value_dtype = self._value_shape, self._value_dtype
             new._key_shape, new._key_dtype = self._key_shape, self._key_dtype
-        else:
-            new._uuid_only = cp(self._uuid_only)
-        new._n_elements = cp(self._n_elements)
-        new._n_failed = cp(self._n_failed)
+        new._counters_of_table = cp(self._state)
         if deepclone:
             # in-slot stamps were copied with the slots: continue their epochs; a separate array is copied too
-            new._shared = {"stamp": None if self._shared["stamp"] is None else self._shared["stamp"].clone(),
-                           "epoch": self._shared["epoch"], "bound": self._shared["bound"], "snapshots": []}
+            sh = self._shared
+            new._shared = _Shared(None if sh.stamp is None else sh.stamp.clone(), sh.epoch, sh.bound)
         else:
             new._shared = self._shared   # a view writes the same slots: same stamps, epoch and bound
         return new
@@ -440,19 +524,24 @@ class CudaClosedHashmap:
     # ------------------------------------------------------------------ sizes
     @property
     def n_elements(self):
-        n, failed = torch.stack([self._n_elements, self._n_failed]).tolist()      # one synchronisation for both
-        self._shared["snapshots"].clear()
-        self._shared["bound"] = n
+        state = self._state.tolist()
+        n, _, _, failed = self._sizes(state)
+        self._shared.exact(n)
         if failed:
-            self._n_failed.zero_()
+            # rows that a set could not store because the table was full (the reference drops them silently,
+            # closed_hashmap_impl_class.cu:426; here they are counted and reported where the host synchronises anyway)
+            self._state[L.CNT_FAILED] = self._state[_BY_BULK + L.CNT_FAILED] = 0
             raise L.DokError(f"{failed} rows of earlier set calls were not stored: the table was full "
                              f"({self._n_buckets} buckets); rehash() to a larger size and set them again")
         return n
 
+    def _size_on_device(self):
+        return torch.tensor(self._sizes()[0], device=self.device)
+
     @property
     def last_set_failed(self):
         """Rows that set calls could not store so far (table full); reading it synchronises."""
-        return int(self._n_failed.item())
+        return self._sizes()[3]
 
     @property
     def n_buckets(self):
@@ -539,38 +628,36 @@ class CudaClosedHashmap:
     def _launch_set(self, keys, values, assume_unique):
         lib = L.lib()
         n = keys.shape[0]
-        cnt = self._counters()
+        cnt = self._counter_block(_BY_SET)
         with torch.cuda.device(self.device):
             st = L.stream_ptr(self.device)
             if assume_unique:
                 L.check(lib.dok_map_set_unique(self._c_table(), self._c_hash(), L.ptr(keys), L.ptr(values), n, None,
-                                               L.ptr(cnt), st), "dok_map_set_unique")
+                                               cnt, st), "dok_map_set_unique")
             else:
                 epoch = self._next_epoch()
                 scratch = torch.empty(n + 1, device=self.device, dtype=torch.long)
                 L.check(lib.dok_map_set(self._c_table(), self._c_hash(), L.ptr(keys), L.ptr(values), n, L.ptr(scratch),
-                                        epoch, None, L.ptr(cnt), st), "dok_map_set")
-        return cnt
+                                        epoch, None, cnt, st), "dok_map_set")
 
-    def _count_new(self, keys):
-        """Number of distinct new keys of a batch (cuda_closed_hashmap.py:350-363).  Integer keys: distinct absent
-        uuids, counted on the device with a scratch tag set.  Floating keys: distinct absent ROWS like the
-        reference, because the value cast makes different rows share a uuid."""
+    def _count_new(self, keys, block):
+        """Adds the number of distinct new keys of a batch (cuda_closed_hashmap.py:350-363) to CNT_CLAIMED_EMPTY of a
+        counter block.  Integer keys: distinct absent uuids, counted with a scratch tag set.  Floating keys: distinct
+        absent ROWS like the reference, because the value cast makes different rows share a uuid."""
         lib = L.lib()
         n = keys.shape[0]
-        cnt = self._counters()
         with torch.cuda.device(self.device):
             st = L.stream_ptr(self.device)
             if keys.dtype in L.FLOAT_DTYPES:
                 found = torch.empty(n, device=self.device, dtype=torch.bool)
                 L.check(lib.dok_map_count_exists(self._c_table(), self._c_hash(), L.ptr(keys), n, L.ptr(found),
-                                                 L.ptr(cnt), st), "dok_map_count_exists")
-                return int(keys[~found].unique(dim=0).shape[0])
+                                                 None, st), "dok_map_count_exists")
+                self._state[block] += int(keys[~found].unique(dim=0).shape[0])
+                return
             slots = 2 * n
             scratch = torch.empty(slots, device=self.device, dtype=torch.long)
             L.check(lib.dok_map_count_new(self._c_table(), self._c_hash(), L.ptr(keys), n, L.ptr(scratch), slots,
-                                          L.ptr(cnt), st), "dok_map_count_new")
-        return int(cnt[L.CNT_CLAIMED_EMPTY].item())
+                                          self._counter_block(block), st), "dok_map_count_new")
 
     def set(self, new_keys, new_values, assume_unique=False):
         """Insert-or-assign a batch.  `assume_unique=True` promises pairwise different keys and runs one kernel
@@ -594,26 +681,26 @@ class CudaClosedHashmap:
         self._materialise_parameters()
         limit = int(self._rehash_threshold * self.n_buckets)
         row_counted = new_keys.dtype in L.FLOAT_DTYPES
-        fast = not row_counted and self._room_for(n, limit)
-        if not fast and not row_counted:
-            # the bound may only be stale (the host runs ahead of the device): fetch the exact count before paying
-            # for a pass that counts the distinct new keys
-            fast = self.n_elements + n <= limit
-        if fast:
+        # the bound may only be stale (the host runs ahead of the device): fetch the exact count before paying for a pass
+        # that counts the distinct new keys
+        if self._room_for(n, limit) or self.n_elements + n <= limit:
             # whatever the number of new keys is, the reference would not rehash: insert and count on the device
-            cnt = self._launch_set(new_keys, new_values, assume_unique)
-            self._account_set(cnt, n)
+            if row_counted:
+                self._count_new(new_keys, _BY_ROWS)
+            self._launch_set(new_keys, new_values, assume_unique)
+            self._after_mutation(n)
             return
-        n_new = self._count_new(new_keys)
-        n_elements = self.n_elements
+        self._state[_COUNTED_NEW] = 0
+        self._count_new(new_keys, _COUNTED_NEW)
+        state = self._state.tolist()
+        n_elements, live = self._sizes(state)[:2]
+        n_new = state[_COUNTED_NEW]
         if n_elements + n_new > limit:
-            self.rehash(int((n_elements + n_new) * self._rehash_factor))
-        cnt = self._launch_set(new_keys, new_values, assume_unique)
-        self._n_tombstones -= cnt[L.CNT_REUSED_REMOVED]
-        self._n_failed += cnt[L.CNT_FAILED]
-        self._n_elements += n_new
-        self._shared["snapshots"].clear()
-        self._shared["bound"] = n_elements + n_new
+            self.rehash(int((n_elements + n_new) * self._rehash_factor), live)
+        self._launch_set(new_keys, new_values, assume_unique)
+        if row_counted:
+            self._state[_BY_ROWS] += n_new
+        self._shared.exact(n_elements + n_new)
 
     def set_rows(self, keys, values, assume_unique=False):
         """Kernel only, like `remove_rows`: insert-or-assign without the reference's bookkeeping around it -- no count
@@ -627,15 +714,15 @@ class CudaClosedHashmap:
         if keys.shape[0] == 0:
             return
         self._materialise_parameters()
-        cnt = self._launch_set(keys.contiguous(), values.contiguous(), assume_unique)
-        self._account_set(cnt, keys.shape[0])
+        before = self._slots_claimed()
+        self._launch_set(keys.contiguous(), values.contiguous(), assume_unique)
+        if keys.dtype in L.FLOAT_DTYPES:
+            self._state[_BY_ROWS] += self._slots_claimed() - before
+        self._after_mutation(keys.shape[0])
 
-    def _account_set(self, cnt, rows):
-        """Device-side bookkeeping after a set launch that cannot have triggered a rehash."""
-        self._n_elements += cnt[L.CNT_CLAIMED_EMPTY] + cnt[L.CNT_REUSED_REMOVED]
-        self._n_tombstones -= cnt[L.CNT_REUSED_REMOVED]
-        self._n_failed += cnt[L.CNT_FAILED]
-        self._after_mutation(rows)
+    def _slots_claimed(self):
+        """For sets that count the new SLOTS of float keys where `set` counts rows: the slots claimed so far."""
+        return self._state[:2].sum() if self._key_dtype in L.FLOAT_DTYPES else None
 
     # ------------------------------------------------------------------ sliced batches (the inbox of a sharded map)
     # keys / values / outputs hold n_slices * slice_rows rows; only the first counts[s] rows of slice s are in use, and
@@ -657,13 +744,11 @@ class CudaClosedHashmap:
 
     def remove_sliced(self, keys, n_slices, slice_rows, counts, abort, is_removed):
         self._sliced_check(keys, n_slices, slice_rows, counts)
-        cnt = self._counters()
+        cnt = self._counter_block(_BY_REMOVE)
         with torch.cuda.device(self.device):
             L.check(L.lib().dok_map_remove_sliced(self._c_table(), self._c_hash(), L.ptr(keys), n_slices, slice_rows,
-                                                  L.ptr(counts), L.ptr(abort), L.ptr(is_removed), L.ptr(cnt),
+                                                  L.ptr(counts), L.ptr(abort), L.ptr(is_removed), cnt,
                                                   L.stream_ptr(self.device)), "dok_map_remove_sliced")
-        self._n_elements -= cnt[L.CNT_HITS]
-        self._n_tombstones += cnt[L.CNT_HITS]
         self._tombstone_host_bound += n_slices * slice_rows
         self._after_mutation(0)
 
@@ -677,22 +762,19 @@ class CudaClosedHashmap:
         self._materialise_parameters()
         rows = n_slices * slice_rows
         limit = int(self._rehash_threshold * self.n_buckets)
-        fast = self._room_for(rows, limit)
-        if not fast:
-            torch.cuda.current_stream(self.device).synchronize()
-            fast = self.n_elements + rows <= limit
-        if fast:
-            cnt = self._counters()
+        if self._room_for(rows, limit) or self.n_elements + rows <= limit:
             with torch.cuda.device(self.device):
-                epoch, scratch = 0, None
+                epoch, scratch, before = 0, None, self._slots_claimed()
                 if not assume_unique:
                     epoch = self._next_epoch()
                     scratch = torch.empty(rows + 1, device=self.device, dtype=torch.long)
                 L.check(L.lib().dok_map_set_sliced(self._c_table(), self._c_hash(), L.ptr(keys), L.ptr(values), n_slices,
                                                    slice_rows, L.ptr(counts), L.ptr(abort), L.ptr(scratch), epoch,
-                                                   int(bool(assume_unique)), L.ptr(cnt), L.stream_ptr(self.device)),
-                        "dok_map_set_sliced")
-            self._account_set(cnt, rows)
+                                                   int(bool(assume_unique)), self._counter_block(_BY_SET),
+                                                   L.stream_ptr(self.device)), "dok_map_set_sliced")
+                if before is not None:
+                    self._state[_BY_ROWS] += self._slots_claimed() - before
+            self._after_mutation(rows)
             return
         if abort is not None and int(abort.item()) != 0:
             return
@@ -761,12 +843,9 @@ class CudaClosedHashmap:
             is_removed = torch.empty(n, device=self.device, dtype=torch.bool)
         else:
             assert is_removed.dtype == torch.bool and is_removed.shape == (n,) and is_removed.is_contiguous()
-        cnt = self._counters()
         with torch.cuda.device(self.device):
-            L.check(L.lib().dok_map_remove(self._c_table(), self._c_hash(), L.ptr(keys), n, L.ptr(is_removed), L.ptr(cnt),
-                                           L.stream_ptr(self.device)), "dok_map_remove")
-        self._n_elements -= cnt[L.CNT_HITS]
-        self._n_tombstones += cnt[L.CNT_HITS]
+            L.check(L.lib().dok_map_remove(self._c_table(), self._c_hash(), L.ptr(keys), n, L.ptr(is_removed),
+                                           self._counter_block(_BY_REMOVE), L.stream_ptr(self.device)), "dok_map_remove")
         self._tombstone_host_bound += n
         self._after_mutation(0)
         self._maintain()
@@ -782,9 +861,9 @@ class CudaClosedHashmap:
         least = max(1, int(0.02 * self.n_buckets)) if auto else 1
         if self._tombstone_host_bound < least or self._element_bound() + self._tombstone_host_bound <= limit:
             return
-        tombstones = int(self._n_tombstones.item())
+        n, _, tombstones, _ = self._sizes()
         self._tombstone_host_bound = tombstones
-        if tombstones >= least and self.n_elements + tombstones > limit:
+        if tombstones >= least and n + tombstones > limit:
             try:
                 self.rebuild()
             except torch.OutOfMemoryError:
@@ -799,7 +878,7 @@ class CudaClosedHashmap:
         shallow clones made before keep the old slot array (as after a rehash in the reference)."""
         if self._slots is None:
             return
-        old_slots, old_stamp = self._slots, self._shared["stamp"]
+        old_slots, old_stamp = self._slots, self._shared.stamp
         source = L.Table()
         source.slots = old_slots.data_ptr()
         source.stamp = old_stamp.data_ptr() if old_stamp is not None else None
@@ -808,23 +887,25 @@ class CudaClosedHashmap:
         source.value_bytes, source.key_bytes = self._value_bytes, self._key_bytes
         fresh = torch.empty(self._layout.total_bytes, device=self.device, dtype=torch.uint8)     # may raise: nothing changed yet
         self._slots = fresh
-        self._shared["stamp"] = None
-        self._shared["epoch"] = 0
-        cnt = self._counters()
+        self._shared.stamp = None
+        self._shared.epoch = 0
+        state = self._state.clone()
         with torch.cuda.device(self.device):
             st = L.stream_ptr(self.device)
             L.check(L.lib().dok_map_init(self._c_table(), st), "dok_map_init")
-            L.check(L.lib().dok_map_reinsert(ctypes.byref(source), self._c_table(), self._c_hash(), L.ptr(cnt), st),
+            L.check(L.lib().dok_map_reinsert(ctypes.byref(source), self._c_table(), self._c_hash(), None, st),
                     "dok_map_reinsert")
         old_slots.record_stream(torch.cuda.current_stream(self.device))
-        self._n_failed += cnt[L.CNT_FAILED]
-        self._n_tombstones.zero_()
+        # the sizes are those of before; only the tombstones are gone: reused = removed
+        gone = state[_BY_REMOVE + L.CNT_HITS] - state[L.CNT_REUSED_REMOVED]
+        self._state[L.CNT_CLAIMED_EMPTY] -= gone
+        self._state[L.CNT_REUSED_REMOVED] += gone
         self._tombstone_host_bound = 0
 
     @property
     def tombstone_bound(self):
         """Upper bound of the tombstone slots, from the device counters (exact unless DOK assignments reused some)."""
-        return int(self._n_tombstones.item())
+        return self._sizes()[2]
 
     def remove(self, keys):
         if self._slots is None:
@@ -843,7 +924,7 @@ class CudaClosedHashmap:
         return self.remove_rows(unique_keys)
 
     # ------------------------------------------------------------------ rehash
-    def rehash(self, n_buckets):
+    def rehash(self, n_buckets, live=None):
         """New table of `n_buckets` with new random parameters holding the live items (cuda_closed_hashmap.py:456-468).
         One kernel walks the old slots and inserts every live one into the new table (dok_map_reinsert): no
         compaction, no pre-get, no unique.  Like the reference's recursive `set`, a table that the live items fill
@@ -853,8 +934,9 @@ class CudaClosedHashmap:
                           rehash_factor=self._rehash_factor, rehash_threshold=self._rehash_threshold,
                           tombstone_threshold=self._tombstone_threshold)
             return
-        live = self.count_live()
-        old_slots, old_stamp = self._slots, self._shared["stamp"]          # kept alive until the kernel has run
+        if live is None:
+            live = self.count_live()
+        old_slots, old_stamp = self._slots, self._shared.stamp          # kept alive until the kernel has run
         source = L.Table()
         source.slots = old_slots.data_ptr()
         source.stamp = old_stamp.data_ptr() if old_stamp is not None else None
@@ -869,10 +951,9 @@ class CudaClosedHashmap:
         )
         self._begin_bulk_insert(*geometry, live)
         if live:
-            cnt = self._counters()
             with torch.cuda.device(self.device):
-                L.check(L.lib().dok_map_reinsert(ctypes.byref(source), self._c_table(), self._c_hash(), L.ptr(cnt),
-                                                 L.stream_ptr(self.device)), "dok_map_reinsert")
+                L.check(L.lib().dok_map_reinsert(ctypes.byref(source), self._c_table(), self._c_hash(),
+                                                 self._counter_block(_BY_BULK), L.stream_ptr(self.device)), "dok_map_reinsert")
             old_slots.record_stream(torch.cuda.current_stream(self.device))
 
     # ------------------------------------------------------------------ persistence
@@ -885,9 +966,9 @@ class CudaClosedHashmap:
         state = {"format": 1, "n_buckets": self.n_buckets, "rehash_factor": self._rehash_factor,
                  "rehash_threshold": self._rehash_threshold, "tombstone_threshold": self._tombstone_threshold,
                  "key_perm": None if self._key_perm is None else self._key_perm.cpu(), "keys": None, "values": None}
-        for name in ("prime1", "prime2", "alpha1", "alpha2", "beta1", "beta2"):
-            v = getattr(self, "_" + name)
-            state[name] = None if v is None else v.cpu()
+        for name in _PARAM_NAMES:
+            drawn = name in self._host or name in self._on_device
+            state[name] = torch.tensor(self._host_param(name), dtype=torch.long) if drawn else None
         if self._slots is not None:
             keys, values, _ = self.items(uuid=False)
             state["keys"] = keys.reshape((-1,) + tuple(self.key_shape)).cpu()
@@ -901,16 +982,14 @@ class CudaClosedHashmap:
         table = cls(n_buckets=state["n_buckets"], device=device, rehash_factor=state["rehash_factor"],
                     rehash_threshold=state["rehash_threshold"], tombstone_threshold=state.get("tombstone_threshold"),
                     key_perm=state["key_perm"],
-                    **{name: state[name] for name in ("prime1", "prime2", "alpha1", "alpha2", "beta1", "beta2")})
+                    **{name: None if state[name] is None else state[name].tolist() for name in _PARAM_NAMES})
         if state["keys"] is not None:
             keys, values = state["keys"].to(table.device), state["values"].to(table.device)
             if keys.shape[0]:      # items() gives key columns in the caller's order, like rehash relies on
                 table.set(keys, values, assume_unique=True)
             else:
                 table._allocate(keys.shape[1:], keys.dtype, values.shape[1:], values.dtype)
-            table._n_elements.fill_(int(state["n_elements"]))
-            table._shared["bound"] = int(state["n_elements"])
-            table._shared["snapshots"].clear()
+            table._adjust(int(state["n_elements"]) - table.n_elements)
         return table
 
     def __getitem__(self, keys):

@@ -472,7 +472,7 @@ class CudaShardOps:
             self._in_flight = []
 
     def local_n_elements(self):
-        return self.local._n_elements
+        return self.local._size_on_device()
 
     def to_host(self, words):
         """Small int64 device tensor -> list of ints on the host, through a kernel store into pinned memory (a copy

@@ -15,6 +15,7 @@ from torch import Tensor
 
 from . import _lib as L
 from . import util
+from . import cuda_closed_hashmap as M
 from .cuda_closed_hashmap import CudaClosedHashmap
 from .selectors import normalise_selectors
 from .util import next_power_of_2, str2dtype
@@ -106,10 +107,10 @@ class SparseDOKTensor(object):
         hashmap._begin_bulk_insert((dense.ndim,), torch.long, (1,), dense.dtype, nnz)
         if nnz:
             sizes = (ctypes.c_int64 * dense.ndim)(*dense.shape)
-            cnt = hashmap._counters()
             with torch.cuda.device(device):
                 L.check(lib.dok_dense_insert_nonzero(hashmap._c_table(), hashmap._c_hash(), L.ptr(dense), sizes,
-                                                     dense.numel(), is_float, L.ptr(cnt), L.stream_ptr(device)),
+                                                     dense.numel(), is_float, hashmap._counter_block(M._BY_BULK),
+                                                     L.stream_ptr(device)),
                         "dok_dense_insert_nonzero")
         return new
 
@@ -286,9 +287,11 @@ class SparseDOKTensor(object):
             hits = found.nonzero().flatten()
             keys = torch.stack(torch.unravel_index(hits, shape), dim=1)
             out.set_rows(keys.contiguous(), values[hits][:, None].contiguous(), assume_unique=True)
-            out._n_elements.fill_(n)
+            out._adjust(n - out.n_elements)
         else:
             L.check(rc, "dok_dok_gather_insert")
+            out._state[M._BY_SET] += cnt[L.CNT_CLAIMED_EMPTY]
+            out._adjust(n - cnt[L.CNT_CLAIMED_EMPTY])
         return SparseDOKTensor.from_storage(out, size=shape)
 
     def _set_items_sparse(self, src, selectors):
@@ -315,12 +318,11 @@ class SparseDOKTensor(object):
             first_key = torch.stack([s[first] for s in selectors], dim=0)[None]
             hashmap.set(first_key, torch.zeros(1, 1, device=self.device, dtype=self.dtype))
         if selectors[0].numel():
-            cnt = hashmap._counters()
             sel = _selectors_struct(selectors)
             with torch.cuda.device(self.device):
-                L.check(L.lib().dok_dok_zero_items(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(cnt),
-                                                   L.stream_ptr(self.device)), "dok_dok_zero_items")
-            hashmap._n_elements -= cnt[L.CNT_HITS]
+                L.check(L.lib().dok_dok_zero_items(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel),
+                                                   hashmap._counter_block(M._BY_REMOVE), L.stream_ptr(self.device)),
+                        "dok_dok_zero_items")
             hashmap._after_mutation(0)
         n_src = int(src_values.shape[0])
         hashmap.rehash(math.ceil((hashmap.n_elements + n_src) * hashmap._rehash_factor * 2))
@@ -331,7 +333,7 @@ class SparseDOKTensor(object):
             before = hashmap.n_elements
             hashmap.set(dest_keys, src_values[:, None].contiguous())
             # the reference adds nnz(src) whatever was new (:340)
-            hashmap._n_elements += n_src - (hashmap.n_elements - before)
+            hashmap._adjust(n_src - (hashmap.n_elements - before))
             hashmap._after_mutation(n_src)
 
     def __setitem__(self, selectors, values):
@@ -374,7 +376,6 @@ class SparseDOKTensor(object):
             # the reference seeds an empty map with the first element before counting (:413-416)
             first_key = torch.stack([s[first] for s in selectors], dim=0)[None]
             hashmap.set(first_key, src[first].reshape(1, 1))
-        n_existing = self._count_existing(selectors)          # device scalar, no sync
         # rehash decision of the reference (:461-462) depends on n_elements and the batch size only
         if hashmap._element_bound() + n_sel > hashmap.n_buckets * hashmap._rehash_threshold:
             n_elements = hashmap.n_elements
@@ -385,10 +386,10 @@ class SparseDOKTensor(object):
         epoch = hashmap._next_epoch()
         scratch = torch.empty(n_sel + 1, device=self.device, dtype=torch.long)
         with torch.cuda.device(self.device):
-            L.check(L.lib().dok_dok_set_dense(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(src),
-                                              src_strides, L.ptr(scratch), epoch, None, L.stream_ptr(self.device)),
-                    "dok_dok_set_dense")
-        hashmap._n_elements += n_sel - n_existing             # duplicates over-count, like the reference (:474)
+            # n_elements grows by the selected positions that were not stored; duplicates over-count, like the reference (:474)
+            L.check(L.lib().dok_dok_assign(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(src),
+                                           src_strides, L.ptr(scratch), epoch, hashmap._counter_block(M._BY_SET),
+                                           hashmap._counter_block(M._ADJUST), L.stream_ptr(self.device)), "dok_dok_assign")
         hashmap._after_mutation(n_sel)
 
     def zero_items(self, selectors):
@@ -402,7 +403,7 @@ class SparseDOKTensor(object):
         with torch.cuda.device(self.device):
             L.check(L.lib().dok_dok_zero_items(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(cnt),
                                                L.stream_ptr(self.device)), "dok_dok_zero_items")
-        hashmap._n_elements -= cnt[L.CNT_HITS]
+        hashmap._state[M._BY_REMOVE + L.CNT_HITS] += cnt[L.CNT_HITS]
         hashmap._after_mutation(0)
         return int(cnt[L.CNT_HITS].item())
 
@@ -451,12 +452,12 @@ class SparseDOKTensor(object):
         out = CudaClosedHashmap(n_buckets=next_power_of_2(live), device=self.device)
         out._begin_bulk_insert((len(new_shape),), torch.long, (1,), self.dtype, live)
         if live:
-            cnt = out._counters()
             old_sizes = (ctypes.c_int64 * len(self.shape))(*[int(x) for x in self.shape])
             new_sizes = (ctypes.c_int64 * len(new_shape))(*new_shape)
             with torch.cuda.device(self.device):
                 L.check(L.lib().dok_dok_rekey_insert(hashmap._c_table(), hashmap._c_hash(), old_sizes, out._c_table(),
-                                                     out._c_hash(), new_sizes, L.ptr(cnt), L.stream_ptr(self.device)),
+                                                     out._c_hash(), new_sizes, out._counter_block(M._BY_BULK),
+                                                     L.stream_ptr(self.device)),
                         "dok_dok_rekey_insert")
         return SparseDOKTensor.from_storage(out, size=new_shape)
 

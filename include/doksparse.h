@@ -130,6 +130,11 @@ int dok_table_layout(int value_bytes, int key_bytes, int64_t n_buckets, dok_layo
 /* Fills the tags (DOK_TAG_EMPTY, blocked for padding slots; values untouched) and zeroes the stamps.
  * Replaces `torch.zeros(n_buckets) + empty_marker`, cuda_closed_hashmap.py:40. */
 int dok_map_init(const dok_table *t, void *stream);
+/* the same, and zeroes `state_words` int64 counters at `state` (a caller's bookkeeping, in the launch it needs anyway) */
+int dok_map_init_state(const dok_table *t, int64_t *state, int state_words, void *stream);
+
+/* smallest prime above n (host); the reference uses sympy.nextprime for its hash parameters (cuda_closed_hashmap.py:76, 88) */
+uint64_t dok_next_prime(uint64_t n);
 
 /* uuid (and this library's start slot) of each key row.  uuid_out / slot_out may be NULL; t may be NULL when
  * slot_out is.
@@ -257,6 +262,12 @@ int dok_dok_count_exists(const dok_table *t, const dok_hash_params *hp, const do
 int dok_dok_set_dense(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel,
                       const void *src, const int64_t *src_strides, int64_t *slot_scratch, int64_t epoch,
                       int64_t *counters, void *stream);
+/* The same with the reference's element count (sparse_dok_tensor_impl.py:461-474), which adds every selected position that
+ * was not stored before, repetitions included: the sum of counters[CLAIMED_EMPTY], counters[REUSED_REMOVED] and *more
+ * (device, ADDED to) grows by that number.  more may be NULL. */
+int dok_dok_assign(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel,
+                   const void *src, const int64_t *src_strides, int64_t *slot_scratch, int64_t epoch,
+                   int64_t *counters, int64_t *more, void *stream);
 
 /* Tombstones every selected element that is present; counters[DOK_CNT_HITS] += removed.
  * Replaces sparse_dok_zero_items (sparse_dok_tensor_impl.cu:58-108). */

@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+from tests.helpers import dev, host
 from tests.test_map_gpu import Pair
 
 pytestmark = pytest.mark.gpu
@@ -31,3 +32,23 @@ def test_chains_of_a_full_table(n_buckets, key_size, value_cols):
     pair.get(rows(0, n_buckets + 50)[0])
     pair.set(*rows(n_buckets, n_buckets + gone))
     pair.get(rows(0, n_buckets + gone + 50)[0])
+
+
+@pytest.mark.parametrize("n", [1, 31, 300, 5000, 70000])
+def test_assignment_counts_repeated_new_positions(n):
+    """n_elements grows by every selected position that was not stored, repetitions included; the last one's value stays."""
+    from doksparse_b200 import SparseDOKTensor
+    rng = np.random.default_rng(n)
+    np.random.seed(1)
+    t = SparseDOKTensor((3000, 3000), dev(rng.integers(0, 3000, (2, 50000))), dev(rng.standard_normal(50000)))
+    for _ in range(2):
+        i, j = rng.integers(0, 3000, (2, max(1, n // 3)))
+        pick = rng.integers(0, len(i), n)
+        i, j, v = i[pick], j[pick], rng.standard_normal(n)
+        dense = host(t.to_dense())
+        stored, before, live, buckets = t.count_items((dev(i), dev(j))), t._nnz(), t.values().numel(), t.storage().n_buckets
+        t[dev(i), dev(j)] = dev(v)
+        dense[i, j] = v
+        before = before if t.storage().n_buckets == buckets else live        # a rehash counts again
+        assert t._nnz() == before + n - stored
+        np.testing.assert_array_equal(host(t.to_dense()), dense)
