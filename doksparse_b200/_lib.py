@@ -58,6 +58,7 @@ class Selectors(ctypes.Structure):
         ("sizes", ctypes.c_int64 * MAX_SELECTOR_NDIM),
         ("ptr", ctypes.c_void_p * MAX_KEY_SIZE),
         ("strides", (ctypes.c_int64 * MAX_SELECTOR_NDIM) * MAX_KEY_SIZE),
+        ("base", ctypes.c_int64 * MAX_KEY_SIZE),
     ]
 
 
@@ -139,6 +140,7 @@ def _declare(lib):
 
 
 EXPORTED = None
+_plan_type = None
 
 
 def lib():
@@ -153,6 +155,20 @@ def lib():
         EXPORTED = sorted(_declare(loaded))
         _lib = loaded
     return _lib
+
+
+def plan_type():
+    """Plan of the _native module, which is built with the library: the hot calls on one table, without the ctypes way."""
+    global _plan_type
+    if _plan_type is None:
+        lib()
+        try:
+            from ._native import Plan
+        except ImportError as e:
+            raise DokError(f"doksparse_b200._native cannot be loaded ({e}): build it with "
+                           "`python -c 'import doksparse_b200.build as b; b.build()'`") from e
+        _plan_type = Plan
+    return _plan_type
 
 
 def check(status, what):

@@ -1,0 +1,404 @@
+// _native: the map's and the DOK tensor's hot calls from Python in one step each.
+//
+// A call of the C ABI through ctypes spends more time around the launch than in it: checking the tensors, allocating the
+// outputs, packing the structs and entering the device took 14 us of a 16 us lookup of 1000 rows.  A Plan holds what does
+// not change between calls on one table (the packed structs, the expected shapes and types) and does the rest in C++.
+// Every method answers None for arguments that it does not take as they are (another device, a view that is not
+// contiguous, a type to convert, ...); the Python methods then go their general way, which raises the documented errors.
+#define PY_SSIZE_T_CLEAN
+#include <ATen/Functions.h>
+#include <ATen/core/Tensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/doksparse.h"
+
+namespace {
+
+struct Plan {
+  PyObject_HEAD
+  dok_table table;
+  dok_hash_params hash;
+  int64_t *state;              // counter blocks of the table (device)
+  int device;
+  int key_ndim, value_ndim;    // dims of one row
+  int64_t key_shape[8], value_shape[8];
+  at::ScalarType key_type, value_type;
+};
+
+enum { STATE_SET = 0, STATE_REMOVE = 8, STATE_ADJUST = 7 };   // int64 offsets of the counter blocks
+
+PyObject *dok_error = nullptr;
+
+// -> true, or sets DokError with the wording of the ctypes path
+bool check(int status, const char *what) {
+  if (status == DOK_OK) return true;
+  const char *name = status == DOK_BAD_ARG ? "DOK_BAD_ARG" : status == DOK_CUDA_ERROR ? "DOK_CUDA_ERROR" : "DOK_TOO_LARGE";
+  if (status == DOK_CUDA_ERROR) PyErr_Format(dok_error, "%s failed: %s (cudaError %d)", what, name, dok_last_cuda_error());
+  else PyErr_Format(dok_error, "%s failed: %s", what, name);
+  return false;
+}
+
+bool rows_match(const at::Tensor &t, int device, at::ScalarType type, int ndim, const int64_t *shape) {
+  if (!t.is_cuda() || t.scalar_type() != type || t.layout() != at::kStrided || t.get_device() != device) return false;
+  const auto sizes = t.sizes();
+  if ((int)sizes.size() != ndim + 1) return false;
+  for (int i = 0; i < ndim; i++) if (sizes[i + 1] != shape[i]) return false;
+  return t.is_contiguous();
+}
+
+const at::Tensor *tensor_of(PyObject *o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+at::TensorOptions on_device(const Plan *p, at::ScalarType type) {
+  return at::TensorOptions().dtype(type).device(at::Device(at::kCUDA, (c10::DeviceIndex)p->device));
+}
+
+// C++ exceptions (out of memory, most of all) become Python's
+template <class F>
+PyObject *guarded(F f) {
+  HANDLE_TH_ERRORS
+  return f();
+  END_HANDLE_TH_ERRORS
+}
+
+int shape_from(PyObject *tuple, int64_t *out) {
+  if (!PyTuple_Check(tuple) || PyTuple_GET_SIZE(tuple) > 7) return -1;
+  const int n = (int)PyTuple_GET_SIZE(tuple);
+  for (int i = 0; i < n; i++) {
+    out[i] = PyLong_AsLongLong(PyTuple_GET_ITEM(tuple, i));
+    if (out[i] == -1 && PyErr_Occurred()) return -1;
+  }
+  return n;
+}
+
+// Plan(table: bytes, hash: bytes, state address, device index, key shape, key dtype, value shape, value dtype)
+int plan_init(Plan *self, PyObject *args, PyObject *) {
+  const char *table, *hash;
+  Py_ssize_t table_bytes, hash_bytes;
+  unsigned long long state;
+  int device;
+  PyObject *key_shape, *key_type, *value_shape, *value_type;
+  if (!PyArg_ParseTuple(args, "y#y#KiOOOO", &table, &table_bytes, &hash, &hash_bytes, &state, &device, &key_shape, &key_type,
+                        &value_shape, &value_type))
+    return -1;
+  self->key_ndim = shape_from(key_shape, self->key_shape);
+  self->value_ndim = shape_from(value_shape, self->value_shape);
+  if (table_bytes != sizeof(dok_table) || hash_bytes != sizeof(dok_hash_params) || self->key_ndim < 0 || self->value_ndim < 0 ||
+      !THPDtype_Check(key_type) || !THPDtype_Check(value_type)) {
+    PyErr_SetString(PyExc_ValueError, "Plan: bad arguments");
+    return -1;
+  }
+  memcpy(&self->table, table, sizeof(dok_table));
+  memcpy(&self->hash, hash, sizeof(dok_hash_params));
+  self->state = (int64_t *)state;
+  self->device = device;
+  self->key_type = reinterpret_cast<THPDtype *>(key_type)->scalar_type;
+  self->value_type = reinterpret_cast<THPDtype *>(value_type)->scalar_type;
+  return 0;
+}
+
+// ---- the map ------------------------------------------------------------------------------------------------
+
+// get(keys) -> (values, is_found) or None
+PyObject *plan_get(Plan *self, PyObject *arg) {
+  return guarded([&]() -> PyObject * {
+    const at::Tensor *keys = tensor_of(arg);
+    if (!keys || !rows_match(*keys, self->device, self->key_type, self->key_ndim, self->key_shape)) Py_RETURN_NONE;
+    const int64_t n = keys->size(0);
+    if (n == 0) Py_RETURN_NONE;
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
+    int64_t shape[8] = {n};
+    for (int i = 0; i < self->value_ndim; i++) shape[i + 1] = self->value_shape[i];
+    at::Tensor values = at::empty(at::IntArrayRef(shape, self->value_ndim + 1), on_device(self, self->value_type));
+    at::Tensor found = at::empty({n}, on_device(self, at::kBool));
+    if (!check(dok_map_get(&self->table, &self->hash, keys->data_ptr(), n, values.data_ptr(), (uint8_t *)found.data_ptr(), nullptr,
+                           nullptr, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()),
+               "dok_map_get"))
+      return nullptr;
+    PyObject *v = THPVariable_Wrap(std::move(values)), *f = THPVariable_Wrap(std::move(found));
+    PyObject *out = v && f ? PyTuple_Pack(2, v, f) : nullptr;
+    Py_XDECREF(v);
+    Py_XDECREF(f);
+    return out;
+  });
+}
+
+// set(keys, values, assume_unique, epoch, stamp address) -> the number of rows, or None
+PyObject *plan_set(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
+  return guarded([&]() -> PyObject * {
+    if (nargs != 5) { PyErr_SetString(PyExc_TypeError, "set takes 5 arguments"); return nullptr; }
+    const at::Tensor *keys = tensor_of(args[0]), *values = tensor_of(args[1]);
+    if (!keys || !values || !rows_match(*keys, self->device, self->key_type, self->key_ndim, self->key_shape) ||
+        !rows_match(*values, self->device, self->value_type, self->value_ndim, self->value_shape) || keys->size(0) != values->size(0) ||
+        keys->size(0) == 0)
+      Py_RETURN_NONE;
+    const int64_t n = keys->size(0);
+    const int unique = PyObject_IsTrue(args[2]);
+    const int64_t epoch = PyLong_AsLongLong(args[3]);
+    dok_table table = self->table;
+    table.stamp = (int64_t *)PyLong_AsVoidPtr(args[4]);
+    if (unique < 0 || PyErr_Occurred()) return nullptr;
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
+    void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream();
+    if (unique) {
+      if (!check(dok_map_set_unique(&table, &self->hash, keys->data_ptr(), values->data_ptr(), n, nullptr, self->state + STATE_SET, stream),
+                 "dok_map_set_unique"))
+        return nullptr;
+    } else {
+      at::Tensor scratch = at::empty({n + 1}, on_device(self, at::kLong));
+      if (!check(dok_map_set(&table, &self->hash, keys->data_ptr(), values->data_ptr(), n, (int64_t *)scratch.data_ptr(), epoch, nullptr,
+                             self->state + STATE_SET, stream),
+                 "dok_map_set"))
+        return nullptr;
+    }
+    return PyLong_FromLongLong(n);
+  });
+}
+
+// remove_rows(keys) -> is_removed or None
+PyObject *plan_remove_rows(Plan *self, PyObject *arg) {
+  return guarded([&]() -> PyObject * {
+    const at::Tensor *keys = tensor_of(arg);
+    if (!keys || !rows_match(*keys, self->device, self->key_type, self->key_ndim, self->key_shape)) Py_RETURN_NONE;
+    const int64_t n = keys->size(0);
+    if (n == 0) Py_RETURN_NONE;
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
+    at::Tensor removed = at::empty({n}, on_device(self, at::kBool));
+    if (!check(dok_map_remove(&self->table, &self->hash, keys->data_ptr(), n, (uint8_t *)removed.data_ptr(), self->state + STATE_REMOVE,
+                              c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()),
+               "dok_map_remove"))
+      return nullptr;
+    return THPVariable_Wrap(std::move(removed));
+  });
+}
+
+// ---- selectors of a DOK tensor ------------------------------------------------------------------------------
+
+struct Selection {
+  dok_selectors sel;
+  int64_t n;                          // selected positions
+  c10::SmallVector<int64_t, 8> shape; // their common shape
+  int scalars[DOK_MAX_KEY_SIZE];      // positions of the scalar selectors
+  int n_scalars;
+  c10::SmallVector<at::Tensor, 4> keep;
+};
+
+struct One { bool slice; int64_t start, stop; const at::Tensor *tensor; };   // tensor null and not a slice: the scalar `start`
+
+// integer member of a slice, or its default; false for anything but None and int
+bool bound_of(PyObject *o, int64_t size, int64_t none, int64_t *out) {
+  if (o == Py_None) { *out = none; return true; }
+  if (!PyLong_CheckExact(o)) return false;
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) { PyErr_Clear(); return false; }
+  *out = v < 0 ? std::max<int64_t>(v + size, 0) : v;
+  return true;
+}
+
+// What selectors.normalise_selectors computes, for ints, slices and index or mask tensors on the table's device, without
+// an index tensor for a slice or a scalar.  false: leave it to the general way.
+bool parse_selection(PyObject *selectors, const int64_t *size, int ndim, int device, Selection *out) {
+  One list[DOK_MAX_KEY_SIZE];
+  int count = 0;
+  const bool many = PyTuple_Check(selectors);
+  const Py_ssize_t given = many ? PyTuple_GET_SIZE(selectors) : 1;
+  out->keep.reserve(2 * DOK_MAX_KEY_SIZE);                     // `list` points into it
+  for (Py_ssize_t i = 0; i < given; i++) {
+    PyObject *o = many ? PyTuple_GET_ITEM(selectors, i) : selectors;
+    if (count >= ndim) return false;
+    if (PyLong_CheckExact(o)) {
+      const long long v = PyLong_AsLongLong(o);
+      if (v == -1 && PyErr_Occurred()) { PyErr_Clear(); return false; }
+      list[count++] = One{false, v, 0, nullptr};
+    } else if (PySlice_Check(o)) {
+      const PySliceObject *s = (const PySliceObject *)o;
+      int64_t start, stop;
+      if (!bound_of(s->start, size[count], 0, &start) || !bound_of(s->stop, size[count], size[count], &stop)) return false;
+      list[count++] = One{true, start, std::max(std::min(stop, size[count]), start), nullptr};
+    } else if (const at::Tensor *t = tensor_of(o)) {
+      if (!t->is_cuda() || t->get_device() != device || t->layout() != at::kStrided) return false;
+      if (t->scalar_type() == at::kLong) {
+        out->keep.push_back(*t);
+        list[count++] = One{false, 0, 0, &out->keep.back()};
+      } else if (t->scalar_type() == at::kBool && t->dim() > 0) {
+        if (count + t->dim() > ndim) return false;
+        const at::Tensor where = at::nonzero(*t);
+        for (int64_t d = 0; d < t->dim(); d++) {
+          out->keep.push_back(where.select(1, d));
+          list[count++] = One{false, 0, 0, &out->keep.back()};
+        }
+      } else {
+        return false;
+      }
+    } else {
+      return false;
+    }
+  }
+  for (; count < ndim; count++) list[count] = One{true, 0, size[count], nullptr};
+
+  // the broadcast block of the tensors, and where it sits among the slices
+  int64_t block[DOK_MAX_SELECTOR_NDIM];
+  int block_ndim = 0, n_slices = 0, first = -1;
+  for (int i = 0; i < ndim; i++) {
+    if (list[i].slice) { n_slices++; continue; }
+    if (first < 0) first = i;
+    if (list[i].tensor) block_ndim = std::max<int>(block_ndim, (int)list[i].tensor->dim());
+  }
+  if (block_ndim + n_slices > DOK_MAX_SELECTOR_NDIM) return false;
+  for (int j = 0; j < block_ndim; j++) block[j] = 1;
+  for (int i = 0; i < ndim; i++) {
+    if (!list[i].tensor) continue;
+    const auto sizes = list[i].tensor->sizes();
+    const int off = block_ndim - (int)sizes.size();
+    for (int j = 0; j < (int)sizes.size(); j++) {
+      if (sizes[j] == 1 || sizes[j] == block[off + j]) continue;
+      if (block[off + j] != 1) return false;
+      block[off + j] = sizes[j];
+    }
+  }
+  dok_selectors &sel = out->sel;
+  memset(&sel, 0, sizeof(sel));
+  sel.ndim = ndim;
+  sel.selector_ndim = block_ndim + n_slices;
+  out->n_scalars = 0;
+  int axis = 0;
+  for (int i = 0; i < ndim; i++) {
+    if (list[i].slice) {
+      sel.sizes[axis] = list[i].stop - list[i].start;
+      sel.strides[i][axis] = 1;
+      sel.base[i] = list[i].start;
+      axis++;
+      continue;
+    }
+    if (i == first) {
+      for (int j = 0; j < block_ndim; j++) sel.sizes[first + j] = block[j];
+      axis += block_ndim;
+    }
+    if (const at::Tensor *t = list[i].tensor) {
+      sel.ptr[i] = (const int64_t *)t->data_ptr();
+      const int off = block_ndim - (int)t->dim();
+      for (int j = 0; j < (int)t->dim(); j++)
+        if (t->size(j) != 1) sel.strides[i][first + off + j] = t->stride(j);
+    } else {
+      sel.base[i] = list[i].start;
+    }
+    if (!list[i].tensor || list[i].tensor->dim() == 0) out->scalars[out->n_scalars++] = i;
+  }
+  out->n = 1;
+  for (int j = 0; j < sel.selector_ndim; j++) {
+    out->shape.push_back(sel.sizes[j]);
+    out->n *= sel.sizes[j];
+  }
+  return true;
+}
+
+// index(selectors, size) -> the dense gather, or None
+PyObject *plan_index(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
+  return guarded([&]() -> PyObject * {
+    if (nargs != 2) { PyErr_SetString(PyExc_TypeError, "index takes 2 arguments"); return nullptr; }
+    int64_t size[8];
+    const int ndim = shape_from(args[1], size);
+    if (ndim < 1 || ndim > DOK_MAX_KEY_SIZE || ndim != self->hash.key_size || self->value_ndim != 1 || self->value_shape[0] != 1) {
+      PyErr_Clear();
+      Py_RETURN_NONE;
+    }
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
+    Selection s;
+    if (!parse_selection(args[0], size, ndim, self->device, &s)) Py_RETURN_NONE;
+    at::Tensor values = at::empty(s.shape, on_device(self, self->value_type));
+    if (s.n > 0 &&
+        !check(dok_dok_get(&self->table, &self->hash, &s.sel, values.data_ptr(), nullptr, nullptr, nullptr,
+                           c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()),
+               "dok_dok_get"))
+      return nullptr;
+    for (int k = s.n_scalars - 1; k >= 0; k--) {
+      const int i = s.scalars[k];
+      if (i < values.dim() && values.size(i) == 1) values = values.squeeze(i);
+    }
+    return THPVariable_Wrap(std::move(values));
+  });
+}
+
+// assign(selectors, size, values, room, epoch, stamp address) -> the number of positions, or None (`room`: more positions
+// than this may make the table grow)
+PyObject *plan_assign(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
+  return guarded([&]() -> PyObject * {
+    if (nargs != 6) { PyErr_SetString(PyExc_TypeError, "assign takes 6 arguments"); return nullptr; }
+    int64_t size[8];
+    const int ndim = shape_from(args[1], size);
+    const at::Tensor *given = tensor_of(args[2]);
+    const bool number = PyFloat_CheckExact(args[2]) ? at::isFloatingType(self->value_type)
+                                                    : PyLong_CheckExact(args[2]) && (at::isFloatingType(self->value_type) || self->value_type == at::kLong);
+    if (ndim < 1 || ndim > DOK_MAX_KEY_SIZE || ndim != self->hash.key_size || self->value_ndim != 1 || self->value_shape[0] != 1 ||
+        (given ? given->layout() != at::kStrided || !given->is_cuda() || given->get_device() != self->device ||
+                     given->scalar_type() != self->value_type
+               : !number)) {
+      PyErr_Clear();
+      Py_RETURN_NONE;
+    }
+    const double room = PyFloat_AsDouble(args[3]);
+    const int64_t epoch = PyLong_AsLongLong(args[4]);
+    dok_table table = self->table;
+    table.stamp = (int64_t *)PyLong_AsVoidPtr(args[5]);
+    if (PyErr_Occurred()) return nullptr;
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
+    Selection s;
+    if (!parse_selection(args[0], size, ndim, self->device, &s) || (double)s.n > room) Py_RETURN_NONE;
+    at::Tensor values;
+    if (given) {
+      values = given->expand(s.shape);
+    } else {
+      at::Scalar value;
+      if (PyFloat_CheckExact(args[2])) value = PyFloat_AS_DOUBLE(args[2]);
+      else {
+        const long long v = PyLong_AsLongLong(args[2]);
+        if (v == -1 && PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
+        value = (int64_t)v;
+      }
+      values = at::full({}, value, on_device(self, self->value_type)).expand(s.shape);
+    }
+    if (s.n > 0) {
+      at::Tensor scratch = at::empty({s.n + 1}, on_device(self, at::kLong));
+      if (!check(dok_dok_assign(&table, &self->hash, &s.sel, values.data_ptr(), values.strides().data(), (int64_t *)scratch.data_ptr(),
+                                epoch, self->state + STATE_SET, self->state + STATE_ADJUST,
+                                c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()),
+                 "dok_dok_assign"))
+        return nullptr;
+    }
+    return PyLong_FromLongLong(s.n);
+  });
+}
+
+PyMethodDef plan_methods[] = {
+    {"get", (PyCFunction)plan_get, METH_O, nullptr},
+    {"set", (PyCFunction)(void *)plan_set, METH_FASTCALL, nullptr},
+    {"remove_rows", (PyCFunction)plan_remove_rows, METH_O, nullptr},
+    {"index", (PyCFunction)(void *)plan_index, METH_FASTCALL, nullptr},
+    {"assign", (PyCFunction)(void *)plan_assign, METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyTypeObject plan_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, nullptr, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) {
+  plan_type.tp_name = "doksparse_b200._native.Plan";
+  plan_type.tp_basicsize = sizeof(Plan);
+  plan_type.tp_flags = Py_TPFLAGS_DEFAULT;
+  plan_type.tp_new = PyType_GenericNew;
+  plan_type.tp_init = (initproc)plan_init;
+  plan_type.tp_methods = plan_methods;
+  if (PyType_Ready(&plan_type) < 0) return nullptr;
+  PyObject *lib = PyImport_ImportModule("doksparse_b200._lib");
+  if (!lib) return nullptr;
+  dok_error = PyObject_GetAttrString(lib, "DokError");
+  Py_DECREF(lib);
+  PyObject *m = dok_error ? PyModule_Create(&module) : nullptr;
+  if (m && PyModule_AddObjectRef(m, "Plan", (PyObject *)&plan_type) < 0) { Py_DECREF(m); return nullptr; }
+  return m;
+}

@@ -37,7 +37,6 @@ static bool make_sel(const dok_selectors *sel, const DevHash &dh, SelKeys *out) 
     if (sel->sizes[j] < 0) return false;
     n *= sel->sizes[j];
   }
-  for (int d = 0; d < sel->ndim; d++) if (n > 0 && !sel->ptr[d]) return false;
   out->s = *sel;
   out->n = n;
   return n <= DOK_MAX_BATCH;

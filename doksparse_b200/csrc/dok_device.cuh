@@ -231,7 +231,7 @@ struct RowKeys {          // contiguous [n, ks] rows of the key dtype (closed_ha
   }
 };
 
-// ndim int64 index tensors broadcast to one shape; element e of the row-major linearisation of `sizes`.
+// ndim int64 index tensors (or affine index functions) broadcast to one shape; element e of the row-major linearisation of `sizes`.
 // Replaces StrictTensorAccessor::get_index_from_offset + get (tensor_accessor.cu:70-87) as used by
 // sparse_dok_tensor_impl.cu:36-42.
 struct SelKeys {
@@ -242,6 +242,7 @@ struct SelKeys {
   __device__ __forceinline__ bool at(ll_t j, ll_t &e) const { e = j; return j < n; }
   __device__ __forceinline__ ll_t span() const { return n; }
   __device__ __forceinline__ bool idle() const { return false; }
+  __device__ __forceinline__ ll_t index(int d, ll_t off) const { return s.ptr[d] ? s.ptr[d][off] : s.base[d] + off; }
   // element offsets of batch element e into each of the ndim index tensors (fully unrolled over the
   // maximum ndim with predication, so `off` stays in registers)
   __device__ __forceinline__ void offsets(ll_t e, ll_t (&off)[DOK_MAX_KEY_SIZE]) const {
@@ -272,13 +273,13 @@ struct SelKeys {
   __device__ __forceinline__ KeyHash hash(const DevHash &hp, ll_t e) const {
     ll_t off[DOK_MAX_KEY_SIZE];
     offsets(e, off);
-    ll_t k = s.ptr[0][off[0]];
+    ll_t k = index(0, off[0]);
     ll_t u = dok_uuid_term(k, hp.a[0], hp.b[0], hp.p[0], hp.m[0]);
     ull_t h = (ull_t)k * (ull_t)hp.a1[0] + (ull_t)hp.b1[0];
 #pragma unroll
     for (int d = 1; d < DOK_MAX_KEY_SIZE; d++)
       if (d < s.ndim) {
-        k = s.ptr[d][off[d]];
+        k = index(d, off[d]);
         u = (ll_t)((ull_t)u * (ull_t)dok_uuid_term(k, hp.a[d], hp.b[d], hp.p[d], hp.m[d]));
         h *= (ull_t)k * (ull_t)hp.a1[d] + (ull_t)hp.b1[d];
       }
@@ -289,7 +290,7 @@ struct SelKeys {
     offsets(e, off);
 #pragma unroll
     for (int d = 0; d < DOK_MAX_KEY_SIZE; d++)
-      if (d < s.ndim) ((ll_t *)dst_row)[hp.perm[d]] = s.ptr[d][off[d]];
+      if (d < s.ndim) ((ll_t *)dst_row)[hp.perm[d]] = index(d, off[d]);
   }
 };
 

@@ -144,6 +144,7 @@ class CudaClosedHashmap:
             self._key_perm = key_perm.to(device=self.device, dtype=torch.long)
         self._host_perm = None
         self._hp = None       # cached ctypes dok_hash_params
+        self._plan = None     # what the native calls need to know of this table (_native_plan)
         self._table = None
 
     # ------------------------------------------------------------------ parameters (lazy, reference order)
@@ -218,7 +219,7 @@ class CudaClosedHashmap:
         assert new.shape == self.key_perm.shape
         self._key_perm = new
         self._host_perm = None
-        self._hp = None
+        self._hp = self._plan = None
 
     def _perm(self):
         """key_perm as host integers."""
@@ -278,7 +279,7 @@ class CudaClosedHashmap:
         self._key_shape, self._key_dtype = torch.Size(key_shape), key_dtype
         self._slots = torch.empty(lay.total_bytes, device=self.device, dtype=torch.uint8)
         self._shared.stamp = None
-        self._hp = None
+        self._hp = self._plan = None
         if self._counters_of_table is None:
             self._counters_of_table = torch.empty(_STATE_WORDS, device=self.device, dtype=torch.long)
         with torch.cuda.device(self.device):
@@ -376,6 +377,22 @@ class CudaClosedHashmap:
                               "are told apart only by their first hash (the reference draws alpha2 from [-1, prime1-2])")
             self._hp = hp
         return ctypes.byref(self._hp)
+
+    def _native_plan(self):
+        """The native form of this table, or None where only the general calls serve it."""
+        if self._plan is None and self._slots is not None and self.device.index is not None:
+            self._c_hash()
+            self._c_table()
+            self._plan = L.plan_type()(bytes(self._table), bytes(self._hp), self._state.data_ptr(), self.device.index,
+                                       tuple(self._key_shape), self._key_dtype, tuple(self._value_shape), self._value_dtype)
+        return self._plan
+
+    def _stamp_address(self):
+        """Address of the separate stamp array (0: the stamps are in the slots), None while it has yet to be made."""
+        if self._layout.stamp_offset >= 0:
+            return 0
+        stamp = self._shared.stamp
+        return None if stamp is None else stamp.data_ptr()
 
     def _counters(self):
         return torch.zeros(L.N_COUNTERS, device=self.device, dtype=torch.long)
@@ -494,7 +511,7 @@ class CudaClosedHashmap:
         self._keys.copy_(self._keys[:, ordering].clone())
         self._host = {name: [self._host_param(name)[i] for i in ordering] for name in _PARAM_NAMES}
         self._on_device = {}
-        self._hp = None
+        self._hp = self._plan = None
 
     def clone(self, deepclone=False):
         self._materialise_parameters()
@@ -662,6 +679,15 @@ class CudaClosedHashmap:
     def set(self, new_keys, new_values, assume_unique=False):
         """Insert-or-assign a batch.  `assume_unique=True` promises pairwise different keys and runs one kernel
         instead of two.  Returns None like the reference."""
+        plan, sh = self._plan, self._shared
+        if plan is not None and self._key_dtype not in L.FLOAT_DTYPES and sh.epoch < L.MAX_EPOCH - 1 \
+                and self._room_for(new_keys.shape[0], int(self._rehash_threshold * self._n_buckets)):
+            stamp = self._stamp_address()
+            rows = None if stamp is None else plan.set(new_keys, new_values, assume_unique, sh.epoch + 1, stamp)
+            if rows is not None:
+                sh.epoch += 1
+                self._after_mutation(rows)
+                return
         assert new_keys.shape[0] == new_values.shape[0]
         if self._slots is None:
             assert new_keys.device == new_values.device == self.device
@@ -689,6 +715,7 @@ class CudaClosedHashmap:
                 self._count_new(new_keys, _BY_ROWS)
             self._launch_set(new_keys, new_values, assume_unique)
             self._after_mutation(n)
+            self._native_plan()
             return
         self._state[_COUNTED_NEW] = 0
         self._count_new(new_keys, _COUNTED_NEW)
@@ -796,6 +823,11 @@ class CudaClosedHashmap:
     def get(self, keys, fallback_value=None, values=None, is_found=None):
         """`values` / `is_found`: optional preallocated outputs (contiguous, [n, *value_shape] and bool [n]), like the
         `values=` argument of the reference launcher (closed_hashmap_impl.py:63)."""
+        if values is None and is_found is None and fallback_value is None:
+            plan = self._plan or self._native_plan()
+            out = None if plan is None else plan.get(keys)
+            if out is not None:
+                return out
         if self._slots is None:
             raise RuntimeError("store something first")
         if keys.shape[0] == 0:
@@ -837,6 +869,12 @@ class CudaClosedHashmap:
     def remove_rows(self, keys, is_removed=None):
         """Kernel only: flags aligned to the rows given (no dedup, no sort).  Equal rows report once.
         `is_removed`: optional preallocated bool[n] output."""
+        if is_removed is None:
+            plan = self._plan or self._native_plan()
+            out = None if plan is None else plan.remove_rows(keys)
+            if out is not None:
+                self._account_removal(out.shape[0])
+                return out
         keys = keys.contiguous()
         n = keys.shape[0]
         if is_removed is None:
@@ -846,10 +884,13 @@ class CudaClosedHashmap:
         with torch.cuda.device(self.device):
             L.check(L.lib().dok_map_remove(self._c_table(), self._c_hash(), L.ptr(keys), n, L.ptr(is_removed),
                                            self._counter_block(_BY_REMOVE), L.stream_ptr(self.device)), "dok_map_remove")
-        self._tombstone_host_bound += n
+        self._account_removal(n)
+        return is_removed
+
+    def _account_removal(self, rows):
+        self._tombstone_host_bound += rows
         self._after_mutation(0)
         self._maintain()
-        return is_removed
 
     def _maintain(self):
         """Rebuild in place when live + tombstone slots exceed the tombstone threshold.  The host first looks at its
@@ -887,6 +928,7 @@ class CudaClosedHashmap:
         source.value_bytes, source.key_bytes = self._value_bytes, self._key_bytes
         fresh = torch.empty(self._layout.total_bytes, device=self.device, dtype=torch.uint8)     # may raise: nothing changed yet
         self._slots = fresh
+        self._plan = None
         self._shared.stamp = None
         self._shared.epoch = 0
         state = self._state.clone()

@@ -230,6 +230,12 @@ class SparseDOKTensor(object):
 
     def __getitem__(self, selectors):
         """Dense gather with zero fill (sparse_dok_tensor.py:302-315)."""
+        hashmap = self._hashmap
+        plan = hashmap._plan or hashmap._native_plan()
+        if plan is not None and hashmap._value_dtype == self._dtype:
+            out = plan.index(selectors, self._size)
+            if out is not None:
+                return out
         selectors, scalar_positions = self._handle_selectors(selectors)
         shape = tuple(selectors[0].shape)
         values = torch.empty(shape, device=self.device, dtype=self.dtype)
@@ -339,6 +345,18 @@ class SparseDOKTensor(object):
     def __setitem__(self, selectors, values):
         """Dense assignment (sparse_dok_tensor.py:317-327 -> sparse_dok_tensor_impl.py:412-474).  A Python scalar is
         treated like a 0-dim tensor, as the reference's README documents."""
+        hashmap = self._hashmap
+        plan, sh = hashmap._plan or hashmap._native_plan(), hashmap._shared
+        if plan is not None and hashmap._value_dtype == self._dtype and sh.epoch < L.MAX_EPOCH - 1:
+            stamp = hashmap._stamp_address()
+            if stamp is not None:
+                room = hashmap.n_buckets * hashmap._rehash_threshold - hashmap._element_bound()
+                n = plan.assign(selectors, self._size, values, room, sh.epoch + 1, stamp)
+                if n is not None:
+                    if n:
+                        sh.epoch += 1
+                        hashmap._after_mutation(n)
+                    return
         selectors, _ = self._handle_selectors(selectors)
         shape = selectors[0].shape
         if isinstance(values, SparseDOKTensor) or (isinstance(values, Tensor) and values.is_sparse):

@@ -111,14 +111,16 @@ enum {
 /* Selector view for the fused DOK kernels: ndim index tensors broadcast to one shape
  * (sparse_dok_tensor.py:220-300 produces them; sparse_dok/util.py:295-310 and
  * tensor_accessor.cu:1-121 are the reference's packing and accessor).  Strides in ELEMENTS, 0 for a
- * broadcast dim.  Element e of the row-major linearisation of `sizes` addresses
- * ptr[d][ sum_j idx_j * strides[d][j] ]. */
+ * broadcast dim.  Element e of the row-major linearisation of `sizes` takes the index
+ * ptr[d][ sum_j idx_j * strides[d][j] ], or where ptr[d] is NULL base[d] + sum_j idx_j * strides[d][j]: a slice is its
+ * start with stride 1 along its dim, a scalar its value, and neither needs a tensor. */
 typedef struct dok_selectors {
   int32_t ndim;            /* number of index tensors = key_size of the DOK map */
   int32_t selector_ndim;   /* dims of the common shape, 0..DOK_MAX_SELECTOR_NDIM */
   int64_t sizes[DOK_MAX_SELECTOR_NDIM];
   const int64_t *ptr[DOK_MAX_KEY_SIZE];
   int64_t strides[DOK_MAX_KEY_SIZE][DOK_MAX_SELECTOR_NDIM];
+  int64_t base[DOK_MAX_KEY_SIZE];
 } dok_selectors;
 
 int dok_version(void);
