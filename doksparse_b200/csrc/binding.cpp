@@ -175,6 +175,45 @@ PyObject *plan_remove_rows(Plan *self, PyObject *arg) {
   });
 }
 
+// A word of pinned memory per thread, for a count that a call has to wait for.
+int64_t *count_word() {
+  static thread_local at::Tensor word;
+  if (!word.defined()) word = at::empty({8}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
+  return (int64_t *)word.data_ptr();
+}
+
+void wait_for(const c10::cuda::CUDAStream &stream) {           // other Python threads run meanwhile
+  struct Released {
+    PyThreadState *state = PyEval_SaveThread();
+    ~Released() { PyEval_RestoreThread(state); }
+  } released;
+  stream.synchronize();
+}
+
+// remove(keys) -> flags of the sorted unique rows, or None
+PyObject *plan_remove(Plan *self, PyObject *arg) {
+  return guarded([&]() -> PyObject * {
+    const at::Tensor *keys = tensor_of(arg);
+    if (!keys || !rows_match(*keys, self->device, self->key_type, self->key_ndim, self->key_shape)) Py_RETURN_NONE;
+    const int64_t n = keys->size(0), bytes = n ? dok_map_remove_unique_bytes(n) : -1;
+    if (bytes < 0) Py_RETURN_NONE;
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
+    const auto stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device);
+    at::Tensor removed = at::empty({n}, on_device(self, at::kBool)), work;
+    if (bytes) work = at::empty({bytes}, on_device(self, at::kByte));
+    volatile int64_t *count = count_word();
+    *count = -2;
+    const int status = dok_map_remove_unique(&self->table, &self->hash, keys->data_ptr(), n, (uint8_t *)removed.data_ptr(),
+                                             bytes ? work.data_ptr() : nullptr, (int64_t *)count, self->state + STATE_REMOVE, stream.stream());
+    if (status == DOK_TOO_LARGE) Py_RETURN_NONE;
+    if (!check(status, "dok_map_remove_unique")) return nullptr;
+    wait_for(stream);
+    if (*count == -1) Py_RETURN_NONE;
+    if (*count < 0) { PyErr_SetString(dok_error, "dok_map_remove_unique: a wait between blocks ran out"); return nullptr; }
+    return THPVariable_Wrap(removed.narrow(0, 0, *count));
+  });
+}
+
 // ---- selectors of a DOK tensor ------------------------------------------------------------------------------
 
 struct Selection {
@@ -376,6 +415,7 @@ PyMethodDef plan_methods[] = {
     {"get", (PyCFunction)plan_get, METH_O, nullptr},
     {"set", (PyCFunction)(void *)plan_set, METH_FASTCALL, nullptr},
     {"remove_rows", (PyCFunction)plan_remove_rows, METH_O, nullptr},
+    {"remove", (PyCFunction)plan_remove, METH_O, nullptr},
     {"index", (PyCFunction)(void *)plan_index, METH_FASTCALL, nullptr},
     {"assign", (PyCFunction)(void *)plan_assign, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};

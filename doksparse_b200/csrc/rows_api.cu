@@ -1,0 +1,628 @@
+// Row-wise passes that the reference leaves to `unique(dim=0)`: the count of the distinct new rows of a float-key set
+// (cuda_closed_hashmap.py:350-363) and the removal of a batch's sorted unique rows (:438-454).
+#include "dok_kernels.cuh"
+
+// ---------------------------------------------------------------------------------------------------------
+// element order and row comparison
+// ---------------------------------------------------------------------------------------------------------
+
+// Element as an unsigned number of the type's width that sorts like the element: the sign bit flipped for signed
+// integers, all bits for negative floats.  The two float zeros compare equal, so they get one image; *nan is set for a
+// NaN, which compares with nothing.
+__device__ __forceinline__ ull_t dok_ordered(const void *keys, int dtype, ll_t idx, bool *nan) {
+  switch (dtype) {
+    case DOK_I64: return ((const ull_t *)keys)[idx] ^ 0x8000000000000000ULL;
+    case DOK_I32: return ((const unsigned *)keys)[idx] ^ 0x80000000u;
+    case DOK_I16: return (unsigned)(((const unsigned short *)keys)[idx] ^ 0x8000u);
+    case DOK_I8: return (unsigned)(((const unsigned char *)keys)[idx] ^ 0x80u);
+    case DOK_U8: return ((const unsigned char *)keys)[idx];
+    case DOK_F64: {
+      ull_t b = ((const ull_t *)keys)[idx];
+      if ((b << 1) == 0) b = 0;
+      *nan |= (b << 1) > 0xffe0000000000000ULL;
+      return (b >> 63) ? ~b : b | 0x8000000000000000ULL;
+    }
+    case DOK_F32: {
+      unsigned b = ((const unsigned *)keys)[idx];
+      if ((b << 1) == 0) b = 0;
+      *nan |= (b << 1) > 0xff000000u;
+      return (b >> 31) ? (unsigned)~b : b | 0x80000000u;
+    }
+    default: {
+      unsigned b = ((const unsigned short *)keys)[idx];
+      if ((b & 0x7fffu) == 0) b = 0;
+      *nan |= (b & 0x7fffu) > (dtype == DOK_F16 ? 0x7c00u : 0x7f80u);
+      return (b >> 15) ? (~b & 0xffffu) : b | 0x8000u;
+    }
+  }
+}
+
+// rows a and b of the batch: < 0, 0, > 0 in lexicographic order
+__device__ __forceinline__ int dok_compare_rows(const void *keys, int dtype, int ks, ll_t a, ll_t b) {
+  bool nan = false;
+  for (int i = 0; i < ks; i++) {
+    const ull_t x = dok_ordered(keys, dtype, a * ks + i, &nan), y = dok_ordered(keys, dtype, b * ks + i, &nan);
+    if (x != y) return x < y ? -1 : 1;
+  }
+  return 0;
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// distinct absent rows
+// ---------------------------------------------------------------------------------------------------------
+
+// k_count_new for keys whose identity is the ROW, not the uuid (float keys: the value cast gives many rows one uuid).  The
+// scratch set holds {32 bits of the row's hash | row index}; a row that meets its hash there compares the rows.  A row with
+// a NaN equals none, not even itself, and counts each time.  Replaces a boolean gather and a sort of the absent rows:
+// 1 M rows of three floats took 0.5 ms of it.
+template <int SB>
+__global__ void __launch_bounds__(DOK_TPB) k_count_new_rows(DevTable t, DevHash hp, RowKeys keys, ull_t *__restrict__ scratch,
+                                                            ll_t scratch_slots, ll_t *counters) {
+  __shared__ BlockTally tally;
+  dok_tally_begin(tally);
+  ll_t e;
+  bool active = keys.row(e);
+  KeyHash kh{0, 0};
+  if (active) kh = keys.hash(hp, e);
+  active = dok_in_window(t, kh, active);
+  const Located loc = dok_locate<SB, 1, false>(t, kh, e, active, nullptr, NoEmit());
+  int claimed = 0;
+  if (active && loc.found < 0) {
+    bool nan = false;
+    ull_t h = 0x5851f42d4c957f2dULL;
+    for (int i = 0; i < hp.ks; i++) h = dok_mix64(h ^ dok_ordered(keys.keys, hp.dtype, e * hp.ks + i, &nan)) + 0x9e3779b97f4a7c15ULL;
+    const ull_t mine = (h << 32) | (ull_t)e;
+    ll_t slot = (ll_t)__umul64hi(h, (ull_t)scratch_slots);
+    claimed = nan;
+    for (ll_t i = 0; i < scratch_slots && !nan; i++) {
+      ull_t other = __ldcg(&scratch[slot]);
+      if (other == ~0ULL) {
+        other = atomicCAS(&scratch[slot], ~0ULL, mine);
+        if (other == ~0ULL) { claimed = 1; break; }
+      }
+      if ((other >> 32) == (mine >> 32) && dok_compare_rows(keys.keys, hp.dtype, hp.ks, e, (ll_t)(other & 0xffffffffULL)) == 0) break;
+      if (++slot == scratch_slots) slot = 0;
+    }
+  }
+  dok_tally_add(tally, DOK_CNT_CLAIMED_EMPTY, claimed);
+  dok_tally_flush(tally, counters, nullptr);
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// removal of the sorted unique rows: up to DOK_SMALL_ROWS rows in one block
+// ---------------------------------------------------------------------------------------------------------
+
+// A batch that one block holds in shared memory is sorted (bitonic network over the first 8 bytes of the rows' images,
+// equal prefixes compared by row), made unique and removed by ONE kernel.  Such a batch is all latency: the library's
+// sort, select and fill kernels, the removal kernel and their launches took 110 us for 200 rows.
+#define DOK_SMALL_ROWS 4096
+#define DOK_SMALL_TPB 1024
+
+struct SmallRows {
+  ull_t key[DOK_SMALL_ROWS];
+  unsigned short row[DOK_SMALL_ROWS];        // 0xffff: padding, behind every row
+};
+
+template <int SB>
+__global__ void __launch_bounds__(DOK_SMALL_TPB) k_remove_unique_small(DevTable t, DevHash hp, RowKeys keys, int padded,
+                                                                       uint8_t *__restrict__ out_removed,
+                                                                       ll_t *__restrict__ out_count, ll_t *counters) {
+  __shared__ SmallRows s;
+  __shared__ int warp_sums[DOK_SMALL_TPB / 32], removed;
+  const int n = (int)keys.n, tid = (int)threadIdx.x;
+  const int per = min(hp.ks, 8 / hp.elem_bytes);                 // columns in the prefix
+  const bool whole = per == hp.ks;
+  bool nan = false;
+  for (int i = tid; i < padded; i += DOK_SMALL_TPB) {
+    ull_t k = ~0ULL;
+    if (i < n) {
+      k = 0;
+      for (int c = 0; c < hp.ks; c++) {
+        const ull_t v = dok_ordered(keys.keys, hp.dtype, (ll_t)i * hp.ks + c, &nan);
+        if (c < per) k = hp.elem_bytes == 8 ? v : (k << (8 * hp.elem_bytes)) | v;
+      }
+    }
+    s.key[i] = k;
+    s.row[i] = i < n ? (unsigned short)i : (unsigned short)0xffff;
+  }
+  if (tid == 0) removed = 0;
+  if (__syncthreads_or(nan)) {                                   // rows that compare with nothing: the caller's way
+    if (tid == 0) *out_count = -1;
+    return;
+  }
+  auto before = [&](int a, int b) {                              // element a sorts before element b
+    const ull_t x = s.key[a], y = s.key[b];
+    if (x != y) return x < y;
+    const unsigned short p = s.row[a], q = s.row[b];
+    if (p == 0xffff || q == 0xffff) return p != 0xffff && q == 0xffff;
+    return !whole && dok_compare_rows(keys.keys, hp.dtype, hp.ks, p, q) < 0;
+  };
+  for (int size = 2; size <= padded; size <<= 1)
+    for (int step = size >> 1; step > 0; step >>= 1) {
+      for (int i = tid; i < padded / 2; i += DOK_SMALL_TPB) {
+        const int a = 2 * i - (i & (step - 1)), b = a + step;
+        const bool up = (a & size) == 0;
+        if (up ? before(b, a) : before(a, b)) {
+          const ull_t k = s.key[a];
+          s.key[a] = s.key[b];
+          s.key[b] = k;
+          const unsigned short r = s.row[a];
+          s.row[a] = s.row[b];
+          s.row[b] = r;
+        }
+      }
+      __syncthreads();
+    }
+  // the first row of each run of equal rows, compacted in order into s.row (a row never moves up, so the last row of a
+  // chunk stays in place for the comparison with the next chunk's first)
+  int count = 0;
+  for (int base = 0; base < n; base += DOK_SMALL_TPB) {
+    const int i = base + tid;
+    const unsigned short row = i < n ? s.row[i] : (unsigned short)0xffff;
+    bool head = i < n;
+    if (head && i > 0 && s.key[i] == s.key[i - 1])
+      head = !whole && dok_compare_rows(keys.keys, hp.dtype, hp.ks, row, s.row[i - 1]) != 0;
+    const unsigned votes = __ballot_sync(0xffffffffu, head);
+    if ((tid & 31) == 0) warp_sums[tid >> 5] = __popc(votes);
+    __syncthreads();
+    int at = count, total = 0;
+    for (int w = 0; w < DOK_SMALL_TPB / 32; w++) {
+      if (w < (tid >> 5)) at += warp_sums[w];
+      total += warp_sums[w];
+    }
+    at += __popc(votes & ((1u << (tid & 31)) - 1u));
+    if (head && at != i) s.row[at] = row;
+    count += total;
+    __syncthreads();
+  }
+  for (int base = 0; base < count; base += DOK_SMALL_TPB) {
+    const int i = base + tid;
+    const bool active = i < count;
+    const ll_t e = active ? s.row[i] : 0;
+    KeyHash kh{0, 0};
+    if (active) kh = keys.hash(hp, e);
+    const Located loc = dok_locate<SB, 1, false>(t, kh, 0, active, nullptr, NoEmit());
+    int hit = active && loc.found >= 0;
+    if (hit) hit = dok_cas_tag(t, loc.found, kh.uuid, DOK_REMOVED) == kh.uuid;
+    if (active) out_removed[i] = (uint8_t)hit;
+    const unsigned votes = __ballot_sync(0xffffffffu, hit);
+    if ((tid & 31) == 0 && votes) atomicAdd(&removed, __popc(votes));
+  }
+  __syncthreads();
+  if (tid == 0) {
+    *out_count = count;
+    if (removed && counters) atomicAdd((ull_t *)counters + DOK_CNT_HITS, (ull_t)removed);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// the same for larger batches: radix sort of 32-bit prefixes, ties by row
+// ---------------------------------------------------------------------------------------------------------
+
+// A row's columns are packed, first column on top, each in as many bits as the batch's smallest and largest value differ
+// by; the leading 32 bits of that are the prefix, and four passes of a single-pass-per-digit radix sort (D. Merrill and
+// M. Garland, "Single-pass parallel prefix scan with decoupled look-back", 2016; A. Adinets and D. Merrill, "Onesweep",
+// 2022) bring the row numbers into prefix order.  Where the packed columns have more than 32 bits, runs of equal prefixes
+// that hold different rows -- a handful for scattered keys -- are put in order by one thread each.  Half the passes of a
+// 64-bit sort, and rows of any number of columns at the price of one; a comparison sort of rows took 0.37 ms for 250 k
+// rows of three floats.  Digits that all rows share are skipped.
+#define DOK_SORT_TPB 256
+#define DOK_SORT_ITEMS 16
+#define DOK_SORT_TILE (DOK_SORT_TPB * DOK_SORT_ITEMS)
+#define DOK_SORT_MAX_ROWS (1LL << 30)      // counts travel in 30 bits beside two flags
+#define DOK_SORT_SPINS (1 << 22)           // bound of every wait for another block; far beyond what one takes
+#define DOK_MAX_RUN 64                     // longest run of equal prefixes with different rows that one thread sorts
+#define DOK_UNIQUE_ROUNDS 4
+#define DOK_UNIQUE_TILE (DOK_TPB * DOK_UNIQUE_ROUNDS)
+
+// zeroed before the first kernel
+struct SortControl {
+  ull_t not_min[DOK_MAX_KEY_SIZE], max[DOK_MAX_KEY_SIZE];     // of the ordered images, ~min so that 0 is neutral
+  unsigned hist[4][256];
+  unsigned ticket[5];                                         // next tile of each pass, and of the removal
+  unsigned refused;       // 1: a NaN, a long mixed run, or a wait that ran out in the sort; 2: a wait in the removal
+  unsigned n_mixed;
+  unsigned skip[4], from_b[4], final_b;                       // plan of the passes
+};
+
+__device__ __forceinline__ int dok_column_bits(const SortControl *c, int i) {
+  const ull_t span = c->max[i] - ~c->not_min[i];
+  return span ? 64 - __clzll(span) : 0;
+}
+// the leading 32 bits of the packed row (all of it when there are no more)
+__device__ __forceinline__ unsigned dok_row_prefix(const SortControl *c, const void *keys, int dtype, int ks, ll_t e) {
+  bool nan = false;
+  ull_t acc = 0;
+  int left = 32;
+  for (int i = 0; i < ks && left > 0; i++) {
+    const int w = dok_column_bits(c, i);
+    const ull_t v = dok_ordered(keys, dtype, e * ks + i, &nan) - ~c->not_min[i];
+    if (w <= left) { acc = (acc << w) | v; left -= w; }
+    else { acc = (acc << left) | (v >> (w - left)); left = 0; }
+  }
+  return (unsigned)acc;
+}
+__device__ __forceinline__ bool dok_prefix_is_row(const SortControl *c, int ks) {
+  int bits = 0;
+  for (int i = 0; i < ks; i++) bits += dok_column_bits(c, i);
+  return bits <= 32;
+}
+
+__global__ void __launch_bounds__(DOK_TPB) k_row_range(RowKeys keys, int dtype, int ks, SortControl *c) {
+  __shared__ ull_t lo_hi[2 * DOK_MAX_KEY_SIZE];
+  if (threadIdx.x < 2 * DOK_MAX_KEY_SIZE) lo_hi[threadIdx.x] = 0;
+  __syncthreads();
+  bool nan = false;
+  const ll_t stride = (ll_t)gridDim.x * DOK_TPB;
+  for (int i = 0; i < ks; i++) {
+    ull_t not_min = 0, max = 0;
+    for (ll_t e = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x; e < keys.n; e += stride) {
+      const ull_t v = dok_ordered(keys.keys, dtype, e * ks + i, &nan);
+      not_min = ~v > not_min ? ~v : not_min;
+      max = v > max ? v : max;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const ull_t a = __shfl_xor_sync(0xffffffffu, not_min, o), b = __shfl_xor_sync(0xffffffffu, max, o);
+      not_min = a > not_min ? a : not_min;
+      max = b > max ? b : max;
+    }
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(&lo_hi[2 * i], not_min);
+      atomicMax(&lo_hi[2 * i + 1], max);
+    }
+  }
+  nan = __syncthreads_or(nan);
+  if (threadIdx.x < ks) {
+    atomicMax(&c->not_min[threadIdx.x], lo_hi[2 * threadIdx.x]);
+    atomicMax(&c->max[threadIdx.x], lo_hi[2 * threadIdx.x + 1]);
+  }
+  if (threadIdx.x == 0 && nan) c->refused = 1;
+}
+
+__global__ void __launch_bounds__(DOK_TPB) k_row_prefix(RowKeys keys, int dtype, int ks, SortControl *c, unsigned *prefix, unsigned *row) {
+  __shared__ unsigned hist[4][256];
+  for (int i = threadIdx.x; i < 1024; i += DOK_TPB) ((unsigned *)hist)[i] = 0;
+  __syncthreads();
+  const ll_t stride = (ll_t)gridDim.x * DOK_TPB;
+  for (ll_t e = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x; e < keys.n; e += stride) {
+    const unsigned p = dok_row_prefix(c, keys.keys, dtype, ks, e);
+    prefix[e] = p;
+    row[e] = (unsigned)e;
+#pragma unroll
+    for (int d = 0; d < 4; d++) atomicAdd(&hist[d][(p >> (8 * d)) & 255u], 1u);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 1024; i += DOK_TPB)
+    if (((unsigned *)hist)[i]) atomicAdd((unsigned *)c->hist + i, ((unsigned *)hist)[i]);
+}
+
+// digit counts -> exclusive offsets; which passes move anything, and from which buffer each one reads
+__global__ void __launch_bounds__(256) k_sort_plan(SortControl *c, unsigned n) {
+  __shared__ unsigned sums[8];
+  unsigned in_b = 0;
+  for (int d = 0; d < 4; d++) {
+    const unsigned own = c->hist[d][threadIdx.x];
+    unsigned v = own;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned u = __shfl_up_sync(0xffffffffu, v, o);
+      if ((threadIdx.x & 31) >= o) v += u;
+    }
+    if ((threadIdx.x & 31) == 31) sums[threadIdx.x >> 5] = v;
+    const bool same = __syncthreads_or(own == n);
+    for (int w = 0; w < (int)(threadIdx.x >> 5); w++) v += sums[w];
+    c->hist[d][threadIdx.x] = v - own;
+    if (threadIdx.x == 0) { c->skip[d] = same; c->from_b[d] = in_b; }
+    if (!same) in_b ^= 1;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) c->final_b = in_b;
+}
+
+#define DOK_LB_LOCAL 0x40000000u           // a tile's own count
+#define DOK_LB_TOTAL 0x80000000u           // the count up to and including the tile
+#define DOK_LB_VALUE 0x3fffffffu
+
+__device__ __forceinline__ unsigned dok_peek(const unsigned *p) { return *(const volatile unsigned *)p; }
+__device__ __forceinline__ void dok_post(unsigned *p, unsigned v) { *(volatile unsigned *)p = v; }
+
+// One digit.  A tile of 4096 (prefix, row) pairs is ranked by digit with warp votes, its digit counts are posted, the counts
+// of the tiles before it are summed up by looking back (tiles are handed out in order, so all of them have started), and
+// the pairs leave through shared memory in digit order, a run of the output at a time.
+__global__ void __launch_bounds__(DOK_SORT_TPB) k_sort_pass(SortControl *c, int digit, unsigned n, unsigned *key_a, unsigned *row_a,
+                                                            unsigned *key_b, unsigned *row_b, unsigned *look) {
+  if (c->skip[digit]) return;
+  __shared__ unsigned keys[DOK_SORT_TILE], rows[DOK_SORT_TILE];
+  __shared__ unsigned counts[DOK_SORT_TPB / 32][256];
+  __shared__ unsigned start[256], shift_by[256], sums[8], tile_id;
+  const bool b = c->from_b[digit];
+  const unsigned *key_in = b ? key_b : key_a, *row_in = b ? row_b : row_a;
+  unsigned *key_out = b ? key_a : key_b, *row_out = b ? row_a : row_b;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, shift = 8 * digit;
+  if (tid == 0) tile_id = atomicAdd(&c->ticket[digit], 1u);
+  for (int i = tid; i < (DOK_SORT_TPB / 32) * 256; i += DOK_SORT_TPB) ((unsigned *)counts)[i] = 0;
+  __syncthreads();
+  const unsigned tile = tile_id;
+  const unsigned first = tile * DOK_SORT_TILE, size = min((unsigned)DOK_SORT_TILE, n - first);
+  unsigned key[DOK_SORT_ITEMS], row[DOK_SORT_ITEMS], rank[DOK_SORT_ITEMS];
+#pragma unroll
+  for (int k = 0; k < DOK_SORT_ITEMS; k++) {
+    const unsigned i = warp * 32 * DOK_SORT_ITEMS + k * 32 + lane;
+    key[k] = i < size ? key_in[first + i] : 0;
+    row[k] = i < size ? row_in[first + i] : 0;
+  }
+#pragma unroll
+  for (int k = 0; k < DOK_SORT_ITEMS; k++) {
+    const unsigned i = warp * 32 * DOK_SORT_ITEMS + k * 32 + lane;
+    const unsigned digit_of = i < size ? (key[k] >> shift) & 255u : 256u;
+    const unsigned peers = __match_any_sync(0xffffffffu, digit_of);
+    unsigned base = 0;
+    if (lane == __ffs(peers) - 1 && i < size) { base = counts[warp][digit_of]; counts[warp][digit_of] = base + __popc(peers); }
+    base = __shfl_sync(0xffffffffu, base, __ffs(peers) - 1);
+    rank[k] = base + __popc(peers & ((1u << lane) - 1u));
+    __syncwarp();
+  }
+  __syncthreads();
+  // thread d owns digit d
+  unsigned total = 0;
+  for (int w = 0; w < DOK_SORT_TPB / 32; w++) {
+    const unsigned v = counts[w][tid];
+    counts[w][tid] = total;
+    total += v;
+  }
+  dok_post(look + (size_t)tile * 256 + tid, (tile == 0 ? DOK_LB_TOTAL : DOK_LB_LOCAL) | total);
+  unsigned v = total;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  if (lane == 31) sums[warp] = v;
+  __syncthreads();
+  for (int w = 0; w < warp; w++) v += sums[w];
+  start[tid] = v - total;
+  unsigned before = 0;
+  int spins = 0;
+  for (unsigned p = tile; p > 0;) {
+    const unsigned s = dok_peek(look + (size_t)(p - 1) * 256 + tid);
+    if (s == 0) {
+      if (++spins < DOK_SORT_SPINS) continue;
+      c->refused = 1;
+      break;
+    }
+    before += s & DOK_LB_VALUE;
+    if (s & DOK_LB_TOTAL) break;
+    p--;
+  }
+  if (tile > 0) dok_post(look + (size_t)tile * 256 + tid, DOK_LB_TOTAL | (before + total));
+  shift_by[tid] = c->hist[digit][tid] + before - (v - total);
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < DOK_SORT_ITEMS; k++) {
+    const unsigned i = warp * 32 * DOK_SORT_ITEMS + k * 32 + lane;
+    if (i < size) {
+      const unsigned d = (key[k] >> shift) & 255u, at = start[d] + counts[warp][d] + rank[k];
+      keys[at] = key[k];
+      rows[at] = row[k];
+    }
+  }
+  __syncthreads();
+  for (unsigned i = tid; i < size; i += DOK_SORT_TPB) {
+    const unsigned k = keys[i], to = i + shift_by[(k >> shift) & 255u];
+    if (to < n) { key_out[to] = k; row_out[to] = rows[i]; }
+  }
+}
+
+// Runs of equal prefixes that hold different rows.  LIST: the first place where two neighbours of such a run differ lists
+// the run's start (nothing is written to the rows meanwhile); otherwise: one thread per listed run sorts it by insertion.
+template <bool LIST>
+__global__ void __launch_bounds__(DOK_TPB) k_sort_ties(SortControl *c, RowKeys keys, int dtype, int ks, unsigned *key_a, unsigned *row_a,
+                                                       unsigned *key_b, unsigned *row_b) {
+  const unsigned n = (unsigned)keys.n;
+  if (c->refused || dok_prefix_is_row(c, ks)) return;
+  const unsigned *key = c->final_b ? key_b : key_a;
+  unsigned *row = c->final_b ? row_b : row_a, *list = c->final_b ? key_a : key_b;
+  const unsigned stride = gridDim.x * DOK_TPB;
+  if (LIST) {
+    for (unsigned i = blockIdx.x * DOK_TPB + threadIdx.x; i + 1 < n; i += stride) {
+      if (key[i] != key[i + 1] || dok_compare_rows(keys.keys, dtype, ks, row[i], row[i + 1]) == 0) continue;
+      unsigned lo = i;
+      int steps = 0;
+      bool first = true;
+      while (lo > 0 && key[lo - 1] == key[i] && first && steps < DOK_MAX_RUN) {
+        first = dok_compare_rows(keys.keys, dtype, ks, row[lo - 1], row[lo]) == 0;
+        lo--;
+        steps++;
+      }
+      if (!first) continue;                          // an earlier place lists the run
+      if (steps == DOK_MAX_RUN) { c->refused = 1; return; }
+      list[atomicAdd(&c->n_mixed, 1u)] = lo;
+    }
+  } else {
+    for (unsigned m = blockIdx.x * DOK_TPB + threadIdx.x; m < c->n_mixed; m += stride) {
+      const unsigned lo = list[m];
+      unsigned hi = lo + 1;
+      while (hi < n && hi - lo <= DOK_MAX_RUN && key[hi] == key[lo]) hi++;
+      if (hi - lo > DOK_MAX_RUN) { c->refused = 1; return; }
+      for (unsigned i = lo + 1; i < hi; i++) {
+        const unsigned r = row[i];
+        unsigned j = i;
+        for (; j > lo && dok_compare_rows(keys.keys, dtype, ks, r, row[j - 1]) < 0; j--) row[j] = row[j - 1];
+        row[j] = r;
+      }
+    }
+  }
+}
+
+// First row of each run of equal rows: looked up, its slot turned into a tombstone, its flag written at the run's number.
+// Runs are counted across tiles by looking back like in the sort, when the tile's own lookups are done.
+template <int SB>
+__global__ void __launch_bounds__(DOK_TPB) k_remove_unique(DevTable t, DevHash hp, RowKeys keys, SortControl *c, const unsigned *key_a,
+                                                           const unsigned *row_a, const unsigned *key_b, const unsigned *row_b,
+                                                           unsigned *look, unsigned tiles, uint8_t *__restrict__ out_removed,
+                                                           ll_t *__restrict__ out_count, ll_t *counters) {
+  __shared__ unsigned sums[DOK_UNIQUE_ROUNDS][DOK_TPB / 32], tile_id, base_of_tile;
+  __shared__ int removed;
+  const unsigned n = (unsigned)keys.n;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (c->refused == 1) {                           // set before this kernel: nothing has been removed
+    if (blockIdx.x == 0 && tid == 0) *out_count = -1;
+    return;
+  }
+  if (tid == 0) { tile_id = atomicAdd(&c->ticket[4], 1u); removed = 0; }
+  __syncthreads();
+  const unsigned tile = tile_id;
+  const unsigned *key = c->final_b ? key_b : key_a, *row = c->final_b ? row_b : row_a;
+  const bool whole = dok_prefix_is_row(c, hp.ks);
+  unsigned head_votes[DOK_UNIQUE_ROUNDS], flags = 0;
+  int hits = 0;
+#pragma unroll
+  for (int r = 0; r < DOK_UNIQUE_ROUNDS; r++) {
+    const unsigned i = tile * DOK_UNIQUE_TILE + r * DOK_TPB + tid;
+    bool head = i < n;
+    const unsigned e = i < n ? row[i] : 0;
+    if (head && i > 0 && key[i] == key[i - 1])
+      head = !whole && dok_compare_rows(keys.keys, hp.dtype, hp.ks, e, row[i - 1]) != 0;
+    head_votes[r] = __ballot_sync(0xffffffffu, head);
+    if (lane == 0) sums[r][warp] = __popc(head_votes[r]);
+    KeyHash kh{0, 0};
+    if (head) kh = keys.hash(hp, e);
+    const Located loc = dok_locate<SB, 1, false>(t, kh, 0, head, nullptr, NoEmit());
+    int hit = head && loc.found >= 0;
+    if (hit) hit = dok_cas_tag(t, loc.found, kh.uuid, DOK_REMOVED) == kh.uuid;
+    flags |= (unsigned)hit << r;
+    hits += hit;
+  }
+  for (int o = 16; o > 0; o >>= 1) hits += __shfl_xor_sync(0xffffffffu, hits, o);
+  if (lane == 0 && hits) atomicAdd(&removed, hits);
+  __syncthreads();
+  unsigned total = 0;
+  for (int r = 0; r < DOK_UNIQUE_ROUNDS; r++) for (int w = 0; w < DOK_TPB / 32; w++) total += sums[r][w];
+  if (warp == 0) {                                 // 32 predecessors at a time
+    if (lane == 0) dok_post(look + tile, (tile == 0 ? DOK_LB_TOTAL : DOK_LB_LOCAL) | total);
+    unsigned before = 0;
+    int spins = 0;
+    for (ll_t end = tile; end > 0;) {
+      const ll_t p = end - 1 - lane;
+      const unsigned s = p >= 0 ? dok_peek(look + p) : DOK_LB_TOTAL;
+      if (__any_sync(0xffffffffu, s == 0)) {
+        if (++spins < DOK_SORT_SPINS) continue;
+        if (lane == 0) c->refused = 2;
+        break;
+      }
+      const unsigned totals = __ballot_sync(0xffffffffu, (s & DOK_LB_TOTAL) != 0);
+      const int stop = totals ? __ffs(totals) - 1 : 31;
+      unsigned v = lane <= stop ? s & DOK_LB_VALUE : 0;
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      before += v;
+      if (totals) break;
+      end -= 32;
+    }
+    if (lane == 0) {
+      if (tile > 0) dok_post(look + tile, DOK_LB_TOTAL | (before + total));
+      base_of_tile = before;
+      if (tile == tiles - 1) *out_count = *(volatile unsigned *)&c->refused == 2 ? -2 : (ll_t)before + total;
+      if (removed && counters) atomicAdd((ull_t *)counters + DOK_CNT_HITS, (ull_t)removed);
+    }
+  }
+  __syncthreads();
+  unsigned at = base_of_tile;
+  for (int r = 0; r < DOK_UNIQUE_ROUNDS; r++) {
+    unsigned mine = at;
+    for (int w = 0; w < DOK_TPB / 32; w++) {
+      if (w < warp) mine += sums[r][w];
+      at += sums[r][w];
+    }
+    mine += __popc(head_votes[r] & ((1u << lane) - 1u));
+    if (((head_votes[r] >> lane) & 1u) && mine < n) out_removed[mine] = (uint8_t)((flags >> r) & 1u);
+  }
+}
+
+struct SortWork {
+  SortControl *control;
+  unsigned *look, *unique_look, *key_a, *row_a, *key_b, *row_b;
+  size_t zeroed, bytes;
+  unsigned tiles, unique_tiles;
+};
+
+static SortWork sort_work(void *base, ll_t n) {
+  SortWork w;
+  size_t at = 0;
+  const auto take = [&](size_t bytes) { const size_t from = at; at += (bytes + 255) / 256 * 256; return (char *)base + from; };
+  w.tiles = (unsigned)((n + DOK_SORT_TILE - 1) / DOK_SORT_TILE);
+  w.unique_tiles = (unsigned)((n + DOK_UNIQUE_TILE - 1) / DOK_UNIQUE_TILE);
+  w.control = (SortControl *)take(sizeof(SortControl));
+  w.look = (unsigned *)take((size_t)w.tiles * 256 * 4 * sizeof(unsigned));
+  w.unique_look = (unsigned *)take((size_t)w.unique_tiles * sizeof(unsigned));
+  w.zeroed = at;
+  w.key_a = (unsigned *)take((size_t)n * sizeof(unsigned));
+  w.row_a = (unsigned *)take((size_t)n * sizeof(unsigned));
+  w.key_b = (unsigned *)take((size_t)n * sizeof(unsigned));
+  w.row_b = (unsigned *)take((size_t)n * sizeof(unsigned));
+  w.bytes = at;
+  return w;
+}
+
+extern "C" {
+
+int dok_map_count_new_rows(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n,
+                           int64_t *scratch, int64_t scratch_slots, int64_t *counters, void *stream) {
+  DevHash dh;
+  DevTable dt;
+  if (!dok_make_hash(hp, &dh) || !dok_make_table(t, &dt) || dt.kb != dh.ks * dh.elem_bytes || n < 0 || n > DOK_MAX_BATCH) return DOK_BAD_ARG;
+  if (n == 0) return DOK_OK;
+  if (!keys || !scratch || !counters || scratch_slots < 2 * n) return DOK_BAD_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (cudaMemsetAsync(scratch, 0xff, (size_t)scratch_slots * 8, st) != cudaSuccess) return dok_check_launch();
+  RowKeys rk{keys, n};
+  int rc = DOK_OK;
+  DOK_DISPATCH_SB(dt, DOK_FOR_WINDOWS(dt, rc, (k_count_new_rows<SB><<<dok_grid(rk), DOK_TPB, 0, st>>>(
+                                                  wt, dh, rk, (ull_t *)scratch, scratch_slots, (ll_t *)counters))));
+  return rc;
+}
+
+int64_t dok_map_remove_unique_bytes(int64_t n) {
+  return n <= DOK_SMALL_ROWS ? 0 : n > DOK_SORT_MAX_ROWS ? -1 : (int64_t)sort_work(nullptr, n).bytes;
+}
+
+int dok_map_remove_unique(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n, uint8_t *out_removed,
+                          void *work, int64_t *out_count, int64_t *counters, void *stream) {
+  DevHash dh;
+  DevTable dt;
+  if (!dok_make_hash(hp, &dh) || !dok_make_table(t, &dt) || dt.kb != dh.ks * dh.elem_bytes || n < 1 || !keys || !out_removed || !out_count)
+    return DOK_BAD_ARG;
+  if (n > DOK_SORT_MAX_ROWS || dok_window_passes(dt) > 1) return DOK_TOO_LARGE;
+  cudaStream_t st = (cudaStream_t)stream;
+  RowKeys rk{keys, n};
+  if (n <= DOK_SMALL_ROWS) {
+    int padded = 1;
+    while (padded < n) padded *= 2;
+    DOK_DISPATCH_SB(dt, (k_remove_unique_small<SB><<<1, DOK_SMALL_TPB, 0, st>>>(dt, dh, rk, padded, out_removed, (ll_t *)out_count, (ll_t *)counters)));
+    return dok_check_launch();
+  }
+  if (!work) return DOK_BAD_ARG;
+  const SortWork w = sort_work(work, n);
+  if (cudaMemsetAsync(work, 0, w.zeroed, st) != cudaSuccess) return dok_check_launch();
+  const ll_t blocks = (n + DOK_TPB - 1) / DOK_TPB;
+  const unsigned grid = (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8);
+  int rc;
+  k_row_range<<<grid, DOK_TPB, 0, st>>>(rk, dh.dtype, dh.ks, w.control);
+  if ((rc = dok_check_launch()) != DOK_OK) return rc;
+  k_row_prefix<<<grid, DOK_TPB, 0, st>>>(rk, dh.dtype, dh.ks, w.control, w.key_a, w.row_a);
+  if ((rc = dok_check_launch()) != DOK_OK) return rc;
+  k_sort_plan<<<1, 256, 0, st>>>(w.control, (unsigned)n);
+  if ((rc = dok_check_launch()) != DOK_OK) return rc;
+  for (int d = 0; d < 4; d++) {
+    k_sort_pass<<<w.tiles, DOK_SORT_TPB, 0, st>>>(w.control, d, (unsigned)n, w.key_a, w.row_a, w.key_b, w.row_b,
+                                                  w.look + (size_t)d * w.tiles * 256);
+    if ((rc = dok_check_launch()) != DOK_OK) return rc;
+  }
+  k_sort_ties<true><<<grid, DOK_TPB, 0, st>>>(w.control, rk, dh.dtype, dh.ks, w.key_a, w.row_a, w.key_b, w.row_b);
+  if ((rc = dok_check_launch()) != DOK_OK) return rc;
+  k_sort_ties<false><<<grid < 148 ? grid : 148, DOK_TPB, 0, st>>>(w.control, rk, dh.dtype, dh.ks, w.key_a, w.row_a, w.key_b, w.row_b);
+  if ((rc = dok_check_launch()) != DOK_OK) return rc;
+  DOK_DISPATCH_SB(dt, (k_remove_unique<SB><<<w.unique_tiles, DOK_TPB, 0, st>>>(dt, dh, rk, w.control, w.key_a, w.row_a, w.key_b, w.row_b,
+                                                                               w.unique_look, w.unique_tiles, out_removed,
+                                                                               (ll_t *)out_count, (ll_t *)counters)));
+  return dok_check_launch();
+}
+
+}  // extern "C"

@@ -665,16 +665,11 @@ class CudaClosedHashmap:
         n = keys.shape[0]
         with torch.cuda.device(self.device):
             st = L.stream_ptr(self.device)
-            if keys.dtype in L.FLOAT_DTYPES:
-                found = torch.empty(n, device=self.device, dtype=torch.bool)
-                L.check(lib.dok_map_count_exists(self._c_table(), self._c_hash(), L.ptr(keys), n, L.ptr(found),
-                                                 None, st), "dok_map_count_exists")
-                self._state[block] += int(keys[~found].unique(dim=0).shape[0])
-                return
             slots = 2 * n
             scratch = torch.empty(slots, device=self.device, dtype=torch.long)
-            L.check(lib.dok_map_count_new(self._c_table(), self._c_hash(), L.ptr(keys), n, L.ptr(scratch), slots,
-                                          self._counter_block(block), st), "dok_map_count_new")
+            count = lib.dok_map_count_new_rows if keys.dtype in L.FLOAT_DTYPES else lib.dok_map_count_new
+            L.check(count(self._c_table(), self._c_hash(), L.ptr(keys), n, L.ptr(scratch), slots,
+                          self._counter_block(block), st), "dok_map_count_new")
 
     def set(self, new_keys, new_values, assume_unique=False):
         """Insert-or-assign a batch.  `assume_unique=True` promises pairwise different keys and runs one kernel
@@ -950,6 +945,11 @@ class CudaClosedHashmap:
         return self._sizes()[2]
 
     def remove(self, keys):
+        plan = self._plan or self._native_plan()
+        out = None if plan is None else plan.remove(keys)
+        if out is not None:
+            self._account_removal(out.shape[0])
+            return out
         if self._slots is None:
             raise RuntimeError("store something first")
         if keys.shape[0] == 0:

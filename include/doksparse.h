@@ -204,6 +204,20 @@ int64_t dok_static_scratch_max_rows(void);
 int dok_map_count_new_static(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n,
                              int64_t *counters, void *stream);
 
+/* The same for keys whose identity is the row, as the reference counts every key type (:363): distinct absent ROWS, by
+ * value (float keys, where the value cast gives different rows one uuid; a row with a NaN counts each time). */
+int dok_map_count_new_rows(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n,
+                           int64_t *scratch, int64_t scratch_slots, int64_t *counters, void *stream);
+
+/* CudaClosedHashmap.remove (cuda_closed_hashmap.py:438-454): removes the batch's unique rows and writes their flags in
+ * sorted order to out_removed (room for n), their number to *out_count, which may be pinned host memory and has to hold
+ * -2 before the call.  -1: a row holds a NaN, or many rows differ only in their last bits; nothing was removed, and the
+ * rows have to be made unique another way.  -2 afterwards: a wait inside the kernels ran out.
+ * work: dok_map_remove_unique_bytes(n) bytes of device memory (0: none needed, -1: n is too large). */
+int64_t dok_map_remove_unique_bytes(int64_t n);
+int dok_map_remove_unique(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n, uint8_t *out_removed,
+                          void *work, int64_t *out_count, int64_t *counters, void *stream);
+
 /* ---- sliced batches -------------------------------------------------------------------------------------
  * The same three operations on a batch that arrives as n_slices slices of slice_rows rows each (keys / values /
  * outputs are [n_slices * slice_rows] rows, slice s at row s * slice_rows), of which only the first

@@ -1,6 +1,7 @@
 """Kernels at the sizes where they can go wrong: edges of tiles, remainders, the smallest and the largest of a range."""
 import numpy as np
 import pytest
+import torch
 
 from tests.helpers import dev, host
 from tests.test_map_gpu import Pair
@@ -52,3 +53,58 @@ def test_assignment_counts_repeated_new_positions(n):
         before = before if t.storage().n_buckets == buckets else live        # a rehash counts again
         assert t._nnz() == before + n - stored
         np.testing.assert_array_equal(host(t.to_dense()), dense)
+
+
+def _rows(rng, kind, n):
+    if kind == "i64":
+        return rng.integers(-2 ** 62, 2 ** 62, (n, 1))
+    if kind == "i64 close":                       # equal leading bits, runs that need a look at the whole row
+        return (rng.integers(-2 ** 30, 2 ** 30, (n, 1)) << 24) + rng.integers(0, 3, (n, 1))
+    if kind == "i64 clustered":                   # thousands of different rows with equal leading bits
+        return (rng.integers(0, 2, (n, 1)) << 60) + rng.integers(0, 4 * n, (n, 1))
+    if kind == "i64x3":
+        return rng.integers(-5, 40, (n, 3))
+    if kind == "i32x4":
+        return rng.integers(-2 ** 31, 2 ** 31, (n, 4)).astype(np.int32)
+    if kind == "u8x5":
+        return rng.integers(0, 8, (n, 5)).astype(np.uint8)
+    if kind == "one":
+        return np.full((n, 2), 7, np.int16)
+    return np.round(rng.uniform(-3000, 3000, (n, 3))).astype(np.float32)
+
+
+@pytest.mark.parametrize("kind", ["i64", "i64 close", "i64 clustered", "i64x3", "i32x4", "u8x5", "one", "f32x3"])
+@pytest.mark.parametrize("n", [1, 2, 33, 1024, 1025, 4096, 4097, 8193, 70001])
+def test_removal_of_sorted_unique_rows(kind, n):
+    """One block up to 4096 rows, radix passes over tiles of 4096 and 1024 rows beyond; half of the rows are stored."""
+    rng = np.random.default_rng(n)
+    stored = _rows(rng, kind, n)
+    pair = Pair(seed=n, n_buckets=1 << 18)
+    pair.set(stored, rng.standard_normal((n, 1)))
+    batch = np.concatenate([stored[rng.integers(0, n, n - n // 2)], _rows(rng, kind, n)[:n // 2]])
+    flags = pair.remove(batch)
+    assert flags.shape[0] == np.unique(batch, axis=0).shape[0]
+    pair.get(stored)
+
+
+@pytest.mark.parametrize("n", [100, 6000])
+def test_removal_of_rows_with_nans(n):
+    from doksparse_b200 import CudaClosedHashmap
+    np.random.seed(1)
+    t = CudaClosedHashmap(n_buckets=1 << 16)
+    keys = torch.arange(2 * n, device="cuda").reshape(n, 2).float()
+    t.set(keys, torch.ones(n, 1, device="cuda"))
+    keys[n // 2, 1] = float("nan")
+    before = t.n_elements
+    assert t.remove(keys).shape[0] == n and t.n_elements < before
+
+
+@pytest.mark.parametrize("dtype", [np.float16, np.float32, np.float64])
+def test_distinct_new_rows_of_float_keys(dtype):
+    """-0.0 equals 0.0, a stored row is not new, rows that share a uuid count each."""
+    pair = Pair(seed=2, n_buckets=1 << 16)
+    rng = np.random.default_rng(0)
+    first = (rng.integers(-40, 40, (3000, 2)) / 4).astype(dtype)
+    pair.set(first, rng.standard_normal((3000, 1)))
+    second = np.concatenate([-first[:500], first[500:1500] * 0, (rng.integers(-60, 60, (5000, 2)) / 4).astype(dtype)])
+    pair.set(second, rng.standard_normal((len(second), 1)))
