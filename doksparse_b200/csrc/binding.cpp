@@ -254,9 +254,10 @@ bool parse_selection(PyObject *selectors, const int64_t *size, int ndim, int dev
       list[count++] = One{false, v, 0, nullptr};
     } else if (PySlice_Check(o)) {
       const PySliceObject *s = (const PySliceObject *)o;
+      const int64_t extent = size[count];
       int64_t start, stop;
-      if (!bound_of(s->start, size[count], 0, &start) || !bound_of(s->stop, size[count], size[count], &stop)) return false;
-      list[count++] = One{true, start, std::max(std::min(stop, size[count]), start), nullptr};
+      if (!bound_of(s->start, extent, 0, &start) || !bound_of(s->stop, extent, extent, &stop)) return false;
+      list[count++] = One{true, start, std::max(std::min(stop, extent), start), nullptr};
     } else if (const at::Tensor *t = tensor_of(o)) {
       if (!t->is_cuda() || t->get_device() != device || t->layout() != at::kStrided) return false;
       if (t->scalar_type() == at::kLong) {

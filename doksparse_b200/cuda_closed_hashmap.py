@@ -73,7 +73,7 @@ class _Shared:
         self.snapshots, self.ring, self.last_copy = [], None, None
 
     def __del__(self):
-        if self.ring is not None:
+        if self.ring is not None and _rings is not None:         # (None: the interpreter is going down)
             _rings.give(self.ring, self.last_copy)
 
     def exact(self, n):

@@ -108,3 +108,35 @@ def test_distinct_new_rows_of_float_keys(dtype):
     pair.set(first, rng.standard_normal((3000, 1)))
     second = np.concatenate([-first[:500], first[500:1500] * 0, (rng.integers(-60, 60, (5000, 2)) / 4).astype(dtype)])
     pair.set(second, rng.standard_normal((len(second), 1)))
+
+
+_SELECTORS = {"int": (3,), "negative slice": (slice(-3, None), slice(2, -2)), "column": (slice(None), 257), "last": (slice(None), slice(None), 2),
+              "all ints": (6, 299, 4), "pairs": (np.arange(7), np.arange(7) * 40), "outer": (np.arange(3)[:, None], slice(5, 9), np.arange(4)[None]),
+              "mask": (slice(1, 3), np.arange(300) % 7 == 0), "mask 2-d": (np.arange(2100).reshape(7, 300) % 11 == 0, slice(0, 2)),
+              "empty slice": (slice(5, 2),), "beyond": (slice(4, 100), 3), "0-d": (np.int64(2), slice(0, 4)), "bare slice": slice(1, 4)}
+
+
+@pytest.mark.parametrize("name", sorted(_SELECTORS))
+def test_native_selectors_agree_with_the_general_ones(name):
+    """Extents that differ in every dim; the same selection through normalise_selectors is the oracle."""
+    from doksparse_b200 import SparseDOKTensor
+    from doksparse_b200.selectors import normalise_selectors
+    shape = (7, 300, 5)
+    np.random.seed(1)
+    rng = np.random.default_rng(0)
+    dense = torch.from_numpy((rng.random(shape) < 0.4) * rng.standard_normal(shape)).cuda()
+    selectors = _SELECTORS[name]
+    on_device = lambda s: torch.from_numpy(np.asarray(s)).cuda() if isinstance(s, (np.ndarray, np.integer)) else s
+    selectors = on_device(selectors) if not isinstance(selectors, tuple) else tuple(on_device(s) for s in selectors)
+    t = SparseDOKTensor.from_dense(dense)
+    index, scalars = normalise_selectors(selectors, shape, torch.device("cuda:0"))
+    expected = dense[tuple(index)]
+    squeezed = expected
+    for i in reversed(scalars):
+        squeezed = squeezed.squeeze(i) if i < squeezed.ndim and squeezed.shape[i] == 1 else squeezed
+    got = t[selectors]
+    assert got.shape == squeezed.shape and torch.equal(got, squeezed)
+    for values in (torch.randn(expected.shape, device="cuda", dtype=torch.float64), 2.5):
+        t[selectors] = values
+        dense[tuple(index)] = values
+        assert torch.equal(t.to_dense(), dense)
