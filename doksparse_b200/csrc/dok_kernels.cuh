@@ -128,6 +128,50 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_set_unique(DevTable t, DevHash h
 #define DOK_ROW_FRESH (1LL << 62)      // bit of a row's slot index: this row claimed the slot
 __device__ __forceinline__ ull_t dok_stamp(ll_t epoch, ll_t row) { return ((ull_t)epoch << 34) | ((ull_t)row << 2); }
 
+// The rows of a block that hold the same key, found in shared memory before the table is touched: only the last of them,
+// which is the one whose value stays, goes on.  In a Zipf batch the most popular key is 4 % of the rows, and every one of
+// them read, stored and stamped the same line, which the L2 serves one after the other: 12.8 M such rows took 20 ms.
+// Same key: same uuid and same chain, so that the rows would have met in one slot.  The set is keyed by the chain's hash;
+// rows that share it by chance have different uuids and go on by themselves.
+#define DOK_TWIN_SLOTS (2 * DOK_TPB)
+struct BlockTwins {
+  ll_t chain[DOK_TWIN_SLOTS];              // 55 bits of the chain's hash | 8 bits: thread of the key's last row so far
+  ll_t uuid[DOK_TPB], slot[DOK_TPB];       // by thread; inactive rows have no uuid
+  uint8_t more[DOK_TPB * 2];               // by place: more than one row
+};
+struct Twins { int last; bool more; };     // thread of the key's last row; whether there are others
+
+// every thread of the block must call
+__device__ __forceinline__ Twins dok_find_twins(BlockTwins &b, const KeyHash &kh, bool active) {
+#pragma unroll
+  for (int i = threadIdx.x; i < DOK_TWIN_SLOTS; i += DOK_TPB) { b.chain[i] = DOK_EMPTY; b.more[i] = 0; }
+  b.uuid[threadIdx.x] = active ? kh.uuid : DOK_EMPTY;
+  __syncthreads();
+  int at = 0;
+  if (active) {
+    const ll_t mine = ((ll_t)dok_chain_hash(kh) & 0x7fffffffffffff00LL) | threadIdx.x;
+    at = (int)(mine >> 8) & (DOK_TWIN_SLOTS - 1);
+    for (;;) {                             // at most DOK_TPB of the DOK_TWIN_SLOTS places are ever taken
+      const ll_t old = (ll_t)atomicCAS((ull_t *)&b.chain[at], (ull_t)DOK_EMPTY, (ull_t)mine);
+      if (old == DOK_EMPTY) break;
+      if (((old ^ mine) >> 8) == 0) {
+        atomicMax(&b.chain[at], mine);
+        b.more[at] = 1;
+        break;
+      }
+      at = (at + 1) & (DOK_TWIN_SLOTS - 1);
+    }
+  }
+  __syncthreads();
+  Twins w{(int)threadIdx.x, false};
+  if (active) {
+    const int last = (int)(b.chain[at] & 255);
+    if (b.uuid[last] == kh.uuid) w.last = last;
+    w.more = b.more[at] != 0;
+  }
+  return w;
+}
+
 // First kernel of the general set.  Find or claim the slot, store the row there and raise the slot's stamp --
 // for a batch without equal uuids that is all there is to do.  A row that finds the slot already stamped in
 // this epoch sets the conflict bit and counts a duplicate (in slot_out[n], zeroed by the host before the
@@ -137,6 +181,7 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
                                                        ll_t *__restrict__ slot_out, ll_t epoch, int mark_fresh,
                                                        uint8_t *__restrict__ out_stored, ll_t *counters) {
   __shared__ BlockTally tally;
+  __shared__ BlockTwins twins;
   if (keys.idle()) return;
   dok_tally_begin(tally);
   ll_t e;
@@ -144,33 +189,53 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
   KeyHash kh{0, 0};
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
-  int outcome = -1, dup = 0;
-  const ll_t slot = dok_find_or_claim<SB>(t, kh, active, &outcome);
-  if (active) {
+  const Twins same = dok_find_twins(twins, kh, active);
+  const bool last = active && same.last == (int)threadIdx.x;
+  int outcome = -1, conflict = 0;
+  ll_t slot = dok_find_or_claim<SB>(t, kh, last, &outcome);
+  if (last) {
     const bool fresh = outcome == DOK_OUT_CLAIMED_EMPTY || outcome == DOK_OUT_REUSED;
     slot_out[e] = mark_fresh && fresh ? slot | DOK_ROW_FRESH : slot;
     if (slot >= 0) {
       // the row is stored without waiting for the stamp's answer: the two requests travel together.  If the slot
       // turns out to be shared, whatever the racing stores left is rewritten by the second kernel.
       ll_t *stamp = dok_stamp_ptr(t, slot);
-      dok_write_row(t, hp, keys, values, e, slot, outcome != DOK_OUT_FOUND || hp.dtype >= DOK_F16);
+      dok_write_row(t, hp, keys, values, e, slot, fresh || hp.dtype >= DOK_F16);
       const ull_t old = atomicMax((ull_t *)stamp, dok_stamp(epoch, e));
-      if ((old >> 34) == (ull_t)epoch) {
+      if ((old >> 34) == (ull_t)epoch || (mark_fresh && same.more)) {
         atomicOr((ull_t *)stamp, DOK_STAMP_CONFLICT);
-        dup = 1;
+        conflict = 1;
       }
     } else {
-      dup = mark_fresh;               // a row without a place is counted by k_set_count too
+      conflict = mark_fresh;          // a row without a place is counted by k_set_count too
     }
     if (out_stored) out_stored[e] = (uint8_t)(slot >= 0);
+    if (slot < 0 && same.more && counters) {                        // a full table: its twins, counted as found below,
+      ll_t others = -1;                                             // have no place either
+      for (int i = 0; i < DOK_TPB; i++) others += twins.uuid[i] == kh.uuid;
+      atomicAdd((ull_t *)counters + DOK_CNT_FAILED, (ull_t)others);
+      atomicAdd((ull_t *)counters + DOK_CNT_HITS, (ull_t)-others);
+    }
   }
-  dok_tally_add(tally, DOK_TALLY_EXTRA, dup);
+  if (out_stored || mark_fresh) {                                   // uniform over the launch
+    if (last) twins.slot[threadIdx.x] = slot;
+    __syncthreads();
+    if (active && !last) {
+      slot = twins.slot[same.last];
+      slot_out[e] = slot;
+      if (out_stored) out_stored[e] = (uint8_t)(slot >= 0);
+    }
+  } else if (active && !last) {
+    slot_out[e] = -1;                                               // nothing to rewrite: a later row of the block may
+  }
+  dok_tally_add(tally, DOK_TALLY_EXTRA, conflict);
   if (counters) {
+    const bool twin = active && !last;
     dok_tally_add(tally, DOK_CNT_CLAIMED_EMPTY, outcome == DOK_OUT_CLAIMED_EMPTY);
     dok_tally_add(tally, DOK_CNT_REUSED_REMOVED, outcome == DOK_OUT_REUSED);
     dok_tally_add(tally, DOK_CNT_FAILED, outcome == DOK_OUT_FAILED);
-    dok_tally_add(tally, DOK_CNT_HITS, outcome == DOK_OUT_FOUND);
-    dok_tally_add(tally, DOK_CNT_DUPLICATES, dup);
+    dok_tally_add(tally, DOK_CNT_HITS, twin || outcome == DOK_OUT_FOUND);
+    dok_tally_add(tally, DOK_CNT_DUPLICATES, twin || (conflict && slot >= 0));
   }
   dok_tally_flush(tally, counters, slot_out + keys.count());
 }
