@@ -292,16 +292,17 @@ class CudaClosedHashmap:
         cuda_closed_hashmap.py:365-366, 456-468).  The caller then inserts the rows with a kernel that counts into
         `_counter_block(_BY_BULK)`."""
         assert self._slots is None
-        self._allocate(key_shape, key_dtype, value_shape, value_dtype)
         if n_new == 0:
+            self._allocate(key_shape, key_dtype, value_shape, value_dtype)
             return
+        self._key_size = int(np.prod(key_shape))
         self._materialise_parameters()
         if n_new > int(self._rehash_threshold * self.n_buckets):
             self.__init__(n_buckets=int(n_new * self._rehash_factor), device=self.device, key_perm=self._key_perm,
                           rehash_factor=self._rehash_factor, rehash_threshold=self._rehash_threshold,
                           tombstone_threshold=self._tombstone_threshold)
-            self._allocate(key_shape, key_dtype, value_shape, value_dtype)
-            self._materialise_parameters()
+        self._allocate(key_shape, key_dtype, value_shape, value_dtype)
+        self._materialise_parameters()
         self._shared.exact(n_new)
 
     def _slot_view(self, dtype, inner_shape, byte_offset):

@@ -101,9 +101,8 @@ class SparseDOKTensor(object):
             L.check(lib.dok_dense_count_nonzero(L.ptr(dense), dense.numel(), es, is_float, L.ptr(count), st),
                     "dok_dense_count_nonzero")
             nnz = int(count.item())
-        new = cls(size=tuple(dense.shape), device=device, dtype=dense.dtype)
         hashmap = CudaClosedHashmap(n_buckets=next_power_of_2(nnz), device=device)
-        new._hashmap = hashmap
+        new = cls(size=tuple(dense.shape), dtype=dense.dtype, storage=hashmap)
         hashmap._begin_bulk_insert((dense.ndim,), torch.long, (1,), dense.dtype, nnz)
         if nnz:
             sizes = (ctypes.c_int64 * dense.ndim)(*dense.shape)
@@ -222,7 +221,18 @@ class SparseDOKTensor(object):
         return self.to_sparse_coo().to_sparse_csr()
 
     def to_dense(self):
-        return self.to_sparse_coo().to_dense()
+        """Same result as to_sparse_coo().to_dense() (sparse_dok_tensor.py:209-211), from one pass over the slots."""
+        hashmap = self._hashmap
+        if hashmap._slots is None or hashmap._value_dtype != self._dtype or hashmap._value_bytes not in (1, 2, 4, 8) \
+                or self._dtype.is_complex or len(hashmap._key_shape) != 1:
+            return self.to_sparse_coo().to_dense()
+        dense = torch.zeros(tuple(self._size), device=self.device, dtype=self._dtype)
+        if dense.numel():
+            sizes = (ctypes.c_int64 * self.ndim)(*self._size)
+            with torch.cuda.device(self.device):
+                L.check(L.lib().dok_dok_to_dense(hashmap._c_table(), hashmap._c_hash(), sizes, L.ptr(dense),
+                                                 L.stream_ptr(self.device)), "dok_dok_to_dense")
+        return dense
 
     # ------------------------------------------------------------------ indexing
     def _handle_selectors(self, selectors, return_slice_as_tensor=True):

@@ -285,6 +285,11 @@ int dok_dok_assign(const dok_table *t, const dok_hash_params *hp, const dok_sele
                    const void *src, const int64_t *src_strides, int64_t *slot_scratch, int64_t epoch,
                    int64_t *counters, int64_t *more, void *stream);
 
+/* Value of every stored element to its position of a dense row-major tensor of the given sizes (HOST int64[key_size]; one
+ * value element of 1, 2, 4 or 8 bytes), which the caller has zeroed.  Positions outside the sizes are left out.  Replaces
+ * to_sparse_coo().to_dense() (sparse_dok_tensor.py:195-215). */
+int dok_dok_to_dense(const dok_table *t, const dok_hash_params *hp, const int64_t *sizes, void *dense, void *stream);
+
 /* Tombstones every selected element that is present; counters[DOK_CNT_HITS] += removed.
  * Replaces sparse_dok_zero_items (sparse_dok_tensor_impl.cu:58-108). */
 int dok_dok_zero_items(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel,

@@ -140,3 +140,18 @@ def test_native_selectors_agree_with_the_general_ones(name):
         t[selectors] = values
         dense[tuple(index)] = values
         assert torch.equal(t.to_dense(), dense)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.uint8, torch.float64])
+@pytest.mark.parametrize("shape,density", [((1,), 1.0), ((2047,), 0.5), ((2048, 3), 1.0), ((129, 17, 5), 0.02), ((700, 1500), 0.001), ((1300, 1000), 0.4)])
+def test_dense_round_trip(dtype, shape, density):
+    """Spans of 2048 elements whose non-zeros are inserted 256 at a time: few, exactly full and many per span."""
+    from doksparse_b200 import SparseDOKTensor
+    np.random.seed(2)
+    rng = np.random.default_rng(1)
+    dense = torch.from_numpy((rng.random(shape) < density) * rng.integers(1, 100, shape)).cuda().to(dtype)
+    t = SparseDOKTensor.from_dense(dense)
+    assert t._nnz() == int((dense != 0).sum())
+    assert torch.equal(t.to_dense(), dense) and torch.equal(t.to_sparse_coo().to_dense(), dense)
+    if len(shape) > 1:
+        assert torch.equal(t.transpose(0, 1).to_dense(), dense.transpose(0, 1))
