@@ -9,7 +9,9 @@
 #include <ATen/Functions.h>
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAStream.h>
+#include <cuda_runtime_api.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -29,7 +31,7 @@ struct Plan {
   at::ScalarType key_type, value_type;
 };
 
-enum { STATE_SET = 0, STATE_REMOVE = 8, STATE_ADJUST = 7 };   // int64 offsets of the counter blocks
+enum { STATE_SET = 0, STATE_REMOVE = 8, STATE_BULK = 24, STATE_ADJUST = 7, STATE_WORDS = 32 };   // int64 offsets of the counter blocks
 
 PyObject *dok_error = nullptr;
 
@@ -175,11 +177,11 @@ PyObject *plan_remove_rows(Plan *self, PyObject *arg) {
   });
 }
 
-// A word of pinned memory per thread, for a count that a call has to wait for.
-int64_t *count_word() {
-  static thread_local at::Tensor word;
-  if (!word.defined()) word = at::empty({8}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
-  return (int64_t *)word.data_ptr();
+// A few words of pinned memory per thread, for counts that a call has to wait for.
+int64_t *pinned_words() {
+  static thread_local at::Tensor words;
+  if (!words.defined()) words = at::empty({STATE_WORDS}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
+  return (int64_t *)words.data_ptr();
 }
 
 void wait_for(const c10::cuda::CUDAStream &stream) {           // other Python threads run meanwhile
@@ -188,6 +190,76 @@ void wait_for(const c10::cuda::CUDAStream &stream) {           // other Python t
     ~Released() { PyEval_RestoreThread(state); }
   } released;
   stream.synchronize();
+}
+
+PyObject *read_state(Plan *self, const c10::cuda::CUDAStream &stream) {
+  int64_t *words = pinned_words();
+  C10_CUDA_CHECK(cudaMemcpyAsync(words, self->state, STATE_WORDS * sizeof(int64_t), cudaMemcpyDeviceToHost, stream.stream()));
+  wait_for(stream);
+  PyObject *list = PyList_New(STATE_WORDS);
+  for (int i = 0; list && i < STATE_WORDS; i++) PyList_SET_ITEM(list, i, PyLong_FromLongLong(words[i]));
+  return list;
+}
+
+// read() -> the counters of the table
+PyObject *plan_read(Plan *self, PyObject *) {
+  return guarded([&]() -> PyObject * {
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
+    return read_state(self, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device));
+  });
+}
+
+// count_new(keys, word, exact): adds the number of distinct new keys to the counter `word`; exact: sets it, and answers
+// the counters
+PyObject *plan_count_new(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
+  return guarded([&]() -> PyObject * {
+    if (nargs != 3) { PyErr_SetString(PyExc_TypeError, "count_new takes 3 arguments"); return nullptr; }
+    const at::Tensor *keys = tensor_of(args[0]);
+    const long word = PyLong_AsLong(args[1]);
+    const int exact = PyObject_IsTrue(args[2]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!keys || word < 0 || word >= STATE_WORDS || !rows_match(*keys, self->device, self->key_type, self->key_ndim, self->key_shape)) {
+      PyErr_SetString(PyExc_ValueError, "count_new: not a batch of this table");
+      return nullptr;
+    }
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
+    const auto stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device);
+    const int64_t n = keys->size(0);
+    at::Tensor scratch = at::empty({2 * n}, on_device(self, at::kLong));
+    if (exact) C10_CUDA_CHECK(cudaMemsetAsync(self->state + word, 0, sizeof(int64_t), stream.stream()));
+    const auto count = at::isFloatingType(self->key_type) ? dok_map_count_new_rows : dok_map_count_new;
+    if (!check(count(&self->table, &self->hash, keys->data_ptr(), n, (int64_t *)scratch.data_ptr(), 2 * n, self->state + word, stream.stream()),
+               "dok_map_count_new"))
+      return nullptr;
+    if (exact) return read_state(self, stream);
+    Py_RETURN_NONE;
+  });
+}
+
+// init(): empty tags, zero counters
+PyObject *plan_init_table(Plan *self, PyObject *) {
+  return guarded([&]() -> PyObject * {
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
+    if (!check(dok_map_init_state(&self->table, self->state, STATE_WORDS, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()),
+               "dok_map_init_state"))
+      return nullptr;
+    Py_RETURN_NONE;
+  });
+}
+
+extern PyTypeObject plan_type;
+
+// reinsert(plan): the live rows of another table of the same row shape
+PyObject *plan_reinsert(Plan *self, PyObject *arg) {
+  return guarded([&]() -> PyObject * {
+    if (Py_TYPE(arg) != &plan_type) { PyErr_SetString(PyExc_TypeError, "reinsert takes a Plan"); return nullptr; }
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
+    if (!check(dok_map_reinsert(&((Plan *)arg)->table, &self->table, &self->hash, self->state + STATE_BULK,
+                                c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()),
+               "dok_map_reinsert"))
+      return nullptr;
+    Py_RETURN_NONE;
+  });
 }
 
 // remove(keys) -> flags of the sorted unique rows, or None
@@ -201,7 +273,7 @@ PyObject *plan_remove(Plan *self, PyObject *arg) {
     const auto stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device);
     at::Tensor removed = at::empty({n}, on_device(self, at::kBool)), work;
     if (bytes) work = at::empty({bytes}, on_device(self, at::kByte));
-    volatile int64_t *count = count_word();
+    volatile int64_t *count = pinned_words();
     *count = -2;
     const int status = dok_map_remove_unique(&self->table, &self->hash, keys->data_ptr(), n, (uint8_t *)removed.data_ptr(),
                                              bytes ? work.data_ptr() : nullptr, (int64_t *)count, self->state + STATE_REMOVE, stream.stream());
@@ -417,11 +489,16 @@ PyMethodDef plan_methods[] = {
     {"set", (PyCFunction)(void *)plan_set, METH_FASTCALL, nullptr},
     {"remove_rows", (PyCFunction)plan_remove_rows, METH_O, nullptr},
     {"remove", (PyCFunction)plan_remove, METH_O, nullptr},
+    {"read", (PyCFunction)plan_read, METH_NOARGS, nullptr},
+    {"count_new", (PyCFunction)(void *)plan_count_new, METH_FASTCALL, nullptr},
+    {"init", (PyCFunction)plan_init_table, METH_NOARGS, nullptr},
+    {"reinsert", (PyCFunction)plan_reinsert, METH_O, nullptr},
     {"index", (PyCFunction)(void *)plan_index, METH_FASTCALL, nullptr},
     {"assign", (PyCFunction)(void *)plan_assign, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 
-PyTypeObject plan_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+PyTypeObject plan_type = {  // filled in below
+    PyVarObject_HEAD_INIT(nullptr, 0)};
 
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, nullptr, nullptr, nullptr, nullptr, nullptr};
 

@@ -17,6 +17,7 @@ What is different (the slot layout is not part of the contract)
   * duplicates inside one `set` batch resolve deterministically to the last row.
 """
 import ctypes
+import math
 import threading
 
 import numpy as np
@@ -151,7 +152,7 @@ class CudaClosedHashmap:
     def _current_key_size(self):
         assert self._slots is not None or self._key_size is not None
         if self._slots is not None:
-            return int(np.prod(self._key_shape))
+            return math.prod(self._key_shape)
         return int(self._key_size)
 
     def _draw(self, name):
@@ -206,7 +207,7 @@ class CudaClosedHashmap:
     def key_perm(self):
         if self._key_perm is None:
             assert self._slots is not None
-            self._key_perm = torch.arange(int(np.prod(self.key_shape)), device=self.device)
+            self._key_perm = torch.arange(math.prod(self._key_shape), device=self.device)
         else:
             assert self._key_perm.shape[0] == np.prod(self.key_shape)
         return self._key_perm
@@ -224,13 +225,20 @@ class CudaClosedHashmap:
     def _perm(self):
         """key_perm as host integers."""
         if self._host_perm is None:
-            n = int(np.prod(self.key_shape))
+            n = math.prod(self._key_shape)
             self._host_perm = list(range(n)) if self._key_perm is None else self._key_perm.cpu().tolist()
             assert len(self._host_perm) == n
         return self._host_perm
 
     def _materialise_parameters(self):
         # evaluation order of the reference's kernel call (cuda_closed_hashmap.py:350-357)
+        if not self._host and not self._on_device:
+            # all of them: the four groups below prime1 in one call, which consumes the random state like single ones do
+            p = self._host_param("prime1")
+            self._host_param("prime2")
+            drawn = (np.random.randint(p[0], size=4) if len(p) == 1 else np.random.randint(np.array(p * 4))) - 1
+            for i, name in enumerate(_PARAM_NAMES[2:]):
+                self._host[name] = drawn[i * len(p):(i + 1) * len(p)].tolist()
         for name in _PARAM_NAMES:
             self._host_param(name)
 
@@ -249,9 +257,12 @@ class CudaClosedHashmap:
     def _counter_block(self, block):
         return ctypes.c_void_p(self._state.data_ptr() + 8 * block)
 
+    def _read_state(self):
+        return self._state.tolist() if self._plan is None else self._plan.read()
+
     def _sizes(self, state=None):
         """(n_elements, live slots, tombstones, failed rows) from one read of the counters."""
-        c = self._state.tolist() if state is None else state
+        c = self._read_state() if state is None else state
         bulk = c[_BY_BULK] + c[_BY_BULK + 1]
         removed = c[_BY_REMOVE + L.CNT_HITS]
         live = c[0] + c[1] + bulk - removed
@@ -262,15 +273,15 @@ class CudaClosedHashmap:
 
     # ------------------------------------------------------------------ storage
     def _allocate(self, key_shape, key_dtype, value_shape, value_dtype):
-        value_bytes = int(np.prod(value_shape, dtype=np.int64)) * torch.empty((), dtype=value_dtype).element_size()
-        key_size = int(np.prod(key_shape, dtype=np.int64))
+        value_bytes = math.prod(value_shape) * value_dtype.itemsize
+        key_size = math.prod(key_shape)
         if key_dtype not in L.DTYPE_CODES:
             raise L.DokError(f"unsupported key dtype {key_dtype}")
         if not (1 <= key_size <= L.MAX_KEY_SIZE):
             raise L.DokError(f"keys may have 1..{L.MAX_KEY_SIZE} elements, got {key_size}")
         if not (1 <= value_bytes <= L.MAX_VALUE_BYTES):
             raise L.DokError(f"value rows may have 1..{L.MAX_VALUE_BYTES} bytes, got {value_bytes}")
-        key_bytes = key_size * torch.empty((), dtype=key_dtype).element_size()
+        key_bytes = key_size * key_dtype.itemsize
         lay = L.LayoutInfo()
         L.check(L.lib().dok_table_layout(value_bytes, key_bytes, self._n_buckets, ctypes.byref(lay)), "dok_table_layout")
         self._layout = lay
@@ -282,7 +293,7 @@ class CudaClosedHashmap:
         self._hp = self._plan = None
         if self._counters_of_table is None:
             self._counters_of_table = torch.empty(_STATE_WORDS, device=self.device, dtype=torch.long)
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             L.check(L.lib().dok_map_init_state(self._c_table(), self._counter_block(0), _STATE_WORDS,
                                                L.stream_ptr(self.device)), "dok_map_init_state")
 
@@ -295,7 +306,7 @@ class CudaClosedHashmap:
         if n_new == 0:
             self._allocate(key_shape, key_dtype, value_shape, value_dtype)
             return
-        self._key_size = int(np.prod(key_shape))
+        self._key_size = math.prod(key_shape)
         self._materialise_parameters()
         if n_new > int(self._rehash_threshold * self.n_buckets):
             self.__init__(n_buckets=int(n_new * self._rehash_factor), device=self.device, key_perm=self._key_perm,
@@ -307,7 +318,7 @@ class CudaClosedHashmap:
 
     def _slot_view(self, dtype, inner_shape, byte_offset):
         """[n_buckets, *inner_shape] strided view of one field of the slot array."""
-        es = torch.empty((), dtype=dtype).element_size()
+        es = dtype.itemsize
         strides, acc = [], 1
         for extent in reversed(tuple(inner_shape)):
             strides.append(acc)
@@ -363,7 +374,7 @@ class CudaClosedHashmap:
         if self._hp is None:
             self._materialise_parameters()
             hp = L.HashParams()
-            ks = int(np.prod(self.key_shape))
+            ks = math.prod(self._key_shape)
             hp.key_size = ks
             hp.key_dtype = L.DTYPE_CODES[self._key_dtype]
             host, perm = {name: self._host_param(name) for name in _PARAM_NAMES}, self._perm()
@@ -381,10 +392,10 @@ class CudaClosedHashmap:
 
     def _native_plan(self):
         """The native form of this table, or None where only the general calls serve it."""
-        if self._plan is None and self._slots is not None and self.device.index is not None:
+        if self._plan is None and self._slots is not None:
             self._c_hash()
             self._c_table()
-            self._plan = L.plan_type()(bytes(self._table), bytes(self._hp), self._state.data_ptr(), self.device.index,
+            self._plan = L.plan_type()(bytes(self._table), bytes(self._hp), self._state.data_ptr(), self._slots.device.index,
                                        tuple(self._key_shape), self._key_dtype, tuple(self._value_shape), self._value_dtype)
         return self._plan
 
@@ -418,7 +429,7 @@ class CudaClosedHashmap:
         if not free:
             return                              # eight copies still in flight: skip this one, the bound stays valid
         slot = free.pop()
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             sh.ring[slot].copy_(self._state, non_blocking=True)
             event = torch.cuda.Event()
             event.record()
@@ -454,13 +465,13 @@ class CudaClosedHashmap:
         """(keys, values, uuid) of the live slots in slot order, from one pass over the tags."""
         assert self._slots is not None
         lib = L.lib()
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             st = L.stream_ptr(self.device)
             tiles = lib.dok_compact_tiles(self._n_buckets)
             offsets = torch.empty(tiles + 1, device=self.device, dtype=torch.long)
             L.check(lib.dok_map_compact_count(self._c_table(), L.ptr(offsets), st), "dok_map_compact_count")
             count = int(offsets[-1].item())
-            ks = int(np.prod(self.key_shape))
+            ks = math.prod(self._key_shape)
             k = v = u = None
             if keys:
                 shape = (ks, count) if transposed_keys else (count, ks)
@@ -542,7 +553,7 @@ class CudaClosedHashmap:
     # ------------------------------------------------------------------ sizes
     @property
     def n_elements(self):
-        state = self._state.tolist()
+        state = self._read_state()
         n, _, _, failed = self._sizes(state)
         self._shared.exact(n)
         if failed:
@@ -637,40 +648,16 @@ class CudaClosedHashmap:
         assert self._slots is not None
         keys = keys.contiguous()
         out = torch.empty(keys.shape[0], device=self.device, dtype=torch.long)
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             L.check(L.lib().dok_map_uuid(self._c_table(), self._c_hash(), L.ptr(keys), keys.shape[0], L.ptr(out), None,
                                          L.stream_ptr(self.device)), "dok_map_uuid")
         return out
 
     # ------------------------------------------------------------------ set
     def _launch_set(self, keys, values, assume_unique):
-        lib = L.lib()
-        n = keys.shape[0]
-        cnt = self._counter_block(_BY_SET)
-        with torch.cuda.device(self.device):
-            st = L.stream_ptr(self.device)
-            if assume_unique:
-                L.check(lib.dok_map_set_unique(self._c_table(), self._c_hash(), L.ptr(keys), L.ptr(values), n, None,
-                                               cnt, st), "dok_map_set_unique")
-            else:
-                epoch = self._next_epoch()
-                scratch = torch.empty(n + 1, device=self.device, dtype=torch.long)
-                L.check(lib.dok_map_set(self._c_table(), self._c_hash(), L.ptr(keys), L.ptr(values), n, L.ptr(scratch),
-                                        epoch, None, cnt, st), "dok_map_set")
-
-    def _count_new(self, keys, block):
-        """Adds the number of distinct new keys of a batch (cuda_closed_hashmap.py:350-363) to CNT_CLAIMED_EMPTY of a
-        counter block.  Integer keys: distinct absent uuids, counted with a scratch tag set.  Floating keys: distinct
-        absent ROWS like the reference, because the value cast makes different rows share a uuid."""
-        lib = L.lib()
-        n = keys.shape[0]
-        with torch.cuda.device(self.device):
-            st = L.stream_ptr(self.device)
-            slots = 2 * n
-            scratch = torch.empty(slots, device=self.device, dtype=torch.long)
-            count = lib.dok_map_count_new_rows if keys.dtype in L.FLOAT_DTYPES else lib.dok_map_count_new
-            L.check(count(self._c_table(), self._c_hash(), L.ptr(keys), n, L.ptr(scratch), slots,
-                          self._counter_block(block), st), "dok_map_count_new")
+        """The set kernels on contiguous rows of this table."""
+        epoch = self._shared.epoch if assume_unique else self._next_epoch()
+        self._native_plan().set(keys, values, assume_unique, epoch, self._stamp_address() or 0)
 
     def set(self, new_keys, new_values, assume_unique=False):
         """Insert-or-assign a batch.  `assume_unique=True` promises pairwise different keys and runs one kernel
@@ -705,17 +692,17 @@ class CudaClosedHashmap:
         row_counted = new_keys.dtype in L.FLOAT_DTYPES
         # the bound may only be stale (the host runs ahead of the device): fetch the exact count before paying for a pass
         # that counts the distinct new keys
+        # The distinct new keys (cuda_closed_hashmap.py:350-363) are counted with a scratch set on the device: uuids of
+        # integer keys, ROWS of floating ones like in the reference, because the value cast makes many rows share a uuid.
+        plan = self._native_plan()
         if self._room_for(n, limit) or self.n_elements + n <= limit:
             # whatever the number of new keys is, the reference would not rehash: insert and count on the device
             if row_counted:
-                self._count_new(new_keys, _BY_ROWS)
+                plan.count_new(new_keys, _BY_ROWS, False)
             self._launch_set(new_keys, new_values, assume_unique)
             self._after_mutation(n)
-            self._native_plan()
             return
-        self._state[_COUNTED_NEW] = 0
-        self._count_new(new_keys, _COUNTED_NEW)
-        state = self._state.tolist()
+        state = plan.count_new(new_keys, _COUNTED_NEW, True)
         n_elements, live = self._sizes(state)[:2]
         n_new = state[_COUNTED_NEW]
         if n_elements + n_new > limit:
@@ -760,7 +747,7 @@ class CudaClosedHashmap:
     def get_sliced(self, keys, n_slices, slice_rows, counts, abort, fallback_value, values, is_found):
         self._sliced_check(keys, n_slices, slice_rows, counts)
         fb, _keep = self._fallback_ptr(fallback_value)
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             L.check(L.lib().dok_map_get_sliced(self._c_table(), self._c_hash(), L.ptr(keys), n_slices, slice_rows,
                                                L.ptr(counts), L.ptr(abort), L.ptr(values), L.ptr(is_found), fb, None,
                                                L.stream_ptr(self.device)), "dok_map_get_sliced")
@@ -768,7 +755,7 @@ class CudaClosedHashmap:
     def remove_sliced(self, keys, n_slices, slice_rows, counts, abort, is_removed):
         self._sliced_check(keys, n_slices, slice_rows, counts)
         cnt = self._counter_block(_BY_REMOVE)
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             L.check(L.lib().dok_map_remove_sliced(self._c_table(), self._c_hash(), L.ptr(keys), n_slices, slice_rows,
                                                   L.ptr(counts), L.ptr(abort), L.ptr(is_removed), cnt,
                                                   L.stream_ptr(self.device)), "dok_map_remove_sliced")
@@ -786,7 +773,7 @@ class CudaClosedHashmap:
         rows = n_slices * slice_rows
         limit = int(self._rehash_threshold * self.n_buckets)
         if self._room_for(rows, limit) or self.n_elements + rows <= limit:
-            with torch.cuda.device(self.device):
+            with L.on(self.device):
                 epoch, scratch, before = 0, None, self._slots_claimed()
                 if not assume_unique:
                     epoch = self._next_epoch()
@@ -844,7 +831,7 @@ class CudaClosedHashmap:
             is_found = torch.empty(n, device=self.device, dtype=torch.bool)
         else:
             assert is_found.dtype == torch.bool and is_found.shape == (n,) and is_found.is_contiguous()
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             L.check(L.lib().dok_map_get(self._c_table(), self._c_hash(), L.ptr(keys), n, L.ptr(values), L.ptr(is_found),
                                         fb, None, L.stream_ptr(self.device)), "dok_map_get")
         return values, is_found
@@ -855,7 +842,7 @@ class CudaClosedHashmap:
         n = keys.shape[0]
         values = torch.empty(n, *self.value_shape, device=self.device, dtype=self._value_dtype)
         cnt = self._counters()
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             L.check(L.lib().dok_map_get_probe_stats(self._c_table(), self._c_hash(), L.ptr(keys), n, L.ptr(values), None,
                                                     L.ptr(cnt), L.stream_ptr(self.device)), "dok_map_get_probe_stats")
         cnt = cnt.cpu()
@@ -877,7 +864,7 @@ class CudaClosedHashmap:
             is_removed = torch.empty(n, device=self.device, dtype=torch.bool)
         else:
             assert is_removed.dtype == torch.bool and is_removed.shape == (n,) and is_removed.is_contiguous()
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             L.check(L.lib().dok_map_remove(self._c_table(), self._c_hash(), L.ptr(keys), n, L.ptr(is_removed),
                                            self._counter_block(_BY_REMOVE), L.stream_ptr(self.device)), "dok_map_remove")
         self._account_removal(n)
@@ -928,7 +915,7 @@ class CudaClosedHashmap:
         self._shared.stamp = None
         self._shared.epoch = 0
         state = self._state.clone()
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             st = L.stream_ptr(self.device)
             L.check(L.lib().dok_map_init(self._c_table(), st), "dok_map_init")
             L.check(L.lib().dok_map_reinsert(ctypes.byref(source), self._c_table(), self._c_hash(), None, st),
@@ -958,7 +945,7 @@ class CudaClosedHashmap:
         assert keys.dtype == self._key_dtype
         assert keys.device == self.device
         assert keys.shape[1:] == self.key_shape
-        if int(np.prod(self._key_shape)) == 1 and keys.dtype not in L.FLOAT_DTYPES:
+        if math.prod(self._key_shape) == 1 and keys.dtype not in L.FLOAT_DTYPES:
             # one integer column: a flat radix-sort unique gives the rows of `unique(dim=0)` in the same (sorted) order
             # without the lexicographic row sort
             unique_keys = torch.unique(keys.reshape(-1)).reshape((-1,) + tuple(self._key_shape))
@@ -979,13 +966,7 @@ class CudaClosedHashmap:
             return
         if live is None:
             live = self.count_live()
-        old_slots, old_stamp = self._slots, self._shared.stamp          # kept alive until the kernel has run
-        source = L.Table()
-        source.slots = old_slots.data_ptr()
-        source.stamp = old_stamp.data_ptr() if old_stamp is not None else None
-        source.n_buckets = self._n_buckets
-        source.slot_bytes = self._layout.slot_bytes
-        source.value_bytes, source.key_bytes = self._value_bytes, self._key_bytes
+        old_slots, source = self._slots, self._native_plan() if live else None          # kept alive until the kernel has run
         geometry = (self._key_shape, self._key_dtype, self._value_shape, self._value_dtype)
         self.__init__(
             n_buckets=n_buckets, device=self.device, key_perm=self._key_perm,
@@ -994,9 +975,7 @@ class CudaClosedHashmap:
         )
         self._begin_bulk_insert(*geometry, live)
         if live:
-            with torch.cuda.device(self.device):
-                L.check(L.lib().dok_map_reinsert(ctypes.byref(source), self._c_table(), self._c_hash(),
-                                                 self._counter_block(_BY_BULK), L.stream_ptr(self.device)), "dok_map_reinsert")
+            self._native_plan().reinsert(source)
             old_slots.record_stream(torch.cuda.current_stream(self.device))
 
     # ------------------------------------------------------------------ persistence

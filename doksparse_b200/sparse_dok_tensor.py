@@ -95,7 +95,7 @@ class SparseDOKTensor(object):
         device = dense.device
         es = dense.element_size()
         is_float = int(dense.dtype.is_floating_point)
-        with torch.cuda.device(device):
+        with L.on(device):
             st = L.stream_ptr(device)
             count = torch.zeros(1, device=device, dtype=torch.long)
             L.check(lib.dok_dense_count_nonzero(L.ptr(dense), dense.numel(), es, is_float, L.ptr(count), st),
@@ -106,7 +106,7 @@ class SparseDOKTensor(object):
         hashmap._begin_bulk_insert((dense.ndim,), torch.long, (1,), dense.dtype, nnz)
         if nnz:
             sizes = (ctypes.c_int64 * dense.ndim)(*dense.shape)
-            with torch.cuda.device(device):
+            with L.on(device):
                 L.check(lib.dok_dense_insert_nonzero(hashmap._c_table(), hashmap._c_hash(), L.ptr(dense), sizes,
                                                      dense.numel(), is_float, hashmap._counter_block(M._BY_BULK),
                                                      L.stream_ptr(device)),
@@ -229,7 +229,7 @@ class SparseDOKTensor(object):
         dense = torch.zeros(tuple(self._size), device=self.device, dtype=self._dtype)
         if dense.numel():
             sizes = (ctypes.c_int64 * self.ndim)(*self._size)
-            with torch.cuda.device(self.device):
+            with L.on(self.device):
                 L.check(L.lib().dok_dok_to_dense(hashmap._c_table(), hashmap._c_hash(), sizes, L.ptr(dense),
                                                  L.stream_ptr(self.device)), "dok_dok_to_dense")
         return dense
@@ -254,7 +254,7 @@ class SparseDOKTensor(object):
             values.zero_()
         elif values.numel():
             sel = _selectors_struct(selectors)
-            with torch.cuda.device(self.device):
+            with L.on(self.device):
                 L.check(L.lib().dok_dok_get(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(values), None,
                                             None, None, L.stream_ptr(self.device)), "dok_dok_get")
         for i in reversed(scalar_positions):
@@ -279,7 +279,7 @@ class SparseDOKTensor(object):
         lib = L.lib()
         # pass 1: how many selected positions are stored (sizes the new map like the reference: int(2 * hits) buckets)
         cnt = hashmap._counters()
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             L.check(lib.dok_dok_count_exists(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(cnt),
                                              L.stream_ptr(self.device)), "dok_dok_count_exists")
         n = int(cnt[L.CNT_HITS].item())
@@ -291,13 +291,13 @@ class SparseDOKTensor(object):
         out._begin_bulk_insert((len(shape),), torch.long, (1,), self.dtype, n)
         # pass 2: lookup and insert in ONE kernel (positions in the selection are the new keys)
         cnt = hashmap._counters()
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             rc = lib.dok_dok_gather_insert(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), out._c_table(),
                                            out._c_hash(), L.ptr(cnt), L.stream_ptr(self.device))
         if rc == 3:                                            # a table served in passes: lookup, then insert
             values = torch.empty(n_sel, device=self.device, dtype=self.dtype)
             found = torch.empty(n_sel, device=self.device, dtype=torch.bool)
-            with torch.cuda.device(self.device):
+            with L.on(self.device):
                 L.check(lib.dok_dok_get(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(values),
                                         L.ptr(found), None, None, L.stream_ptr(self.device)), "dok_dok_get")
             hits = found.nonzero().flatten()
@@ -335,7 +335,7 @@ class SparseDOKTensor(object):
             hashmap.set(first_key, torch.zeros(1, 1, device=self.device, dtype=self.dtype))
         if selectors[0].numel():
             sel = _selectors_struct(selectors)
-            with torch.cuda.device(self.device):
+            with L.on(self.device):
                 L.check(L.lib().dok_dok_zero_items(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel),
                                                    hashmap._counter_block(M._BY_REMOVE), L.stream_ptr(self.device)),
                         "dok_dok_zero_items")
@@ -382,7 +382,7 @@ class SparseDOKTensor(object):
         hashmap = self._hashmap
         cnt = hashmap._counters()
         sel = _selectors_struct(selectors)
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             L.check(L.lib().dok_dok_count_exists(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(cnt),
                                                  L.stream_ptr(self.device)), "dok_dok_count_exists")
         return cnt[L.CNT_HITS]
@@ -413,7 +413,7 @@ class SparseDOKTensor(object):
         src_strides = (ctypes.c_int64 * L.MAX_SELECTOR_NDIM)(*src.stride())
         epoch = hashmap._next_epoch()
         scratch = torch.empty(n_sel + 1, device=self.device, dtype=torch.long)
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             # n_elements grows by the selected positions that were not stored; duplicates over-count, like the reference (:474)
             L.check(L.lib().dok_dok_assign(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(src),
                                            src_strides, L.ptr(scratch), epoch, hashmap._counter_block(M._BY_SET),
@@ -428,7 +428,7 @@ class SparseDOKTensor(object):
             return 0
         cnt = hashmap._counters()
         sel = _selectors_struct(selectors)
-        with torch.cuda.device(self.device):
+        with L.on(self.device):
             L.check(L.lib().dok_dok_zero_items(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(cnt),
                                                L.stream_ptr(self.device)), "dok_dok_zero_items")
         hashmap._state[M._BY_REMOVE + L.CNT_HITS] += cnt[L.CNT_HITS]
@@ -482,7 +482,7 @@ class SparseDOKTensor(object):
         if live:
             old_sizes = (ctypes.c_int64 * len(self.shape))(*[int(x) for x in self.shape])
             new_sizes = (ctypes.c_int64 * len(new_shape))(*new_shape)
-            with torch.cuda.device(self.device):
+            with L.on(self.device):
                 L.check(L.lib().dok_dok_rekey_insert(hashmap._c_table(), hashmap._c_hash(), old_sizes, out._c_table(),
                                                      out._c_hash(), new_sizes, out._counter_block(M._BY_BULK),
                                                      L.stream_ptr(self.device)),
