@@ -105,8 +105,8 @@ __device__ __forceinline__ ll_t dok_key_elem(const void *keys, int dtype, ll_t i
   }
 }
 
-// Mixer (the 64-bit finaliser of MurmurHash3); with a multiply-high range reduction any table size works
-// without a modulo.
+// Mixer (the 64-bit finaliser of MurmurHash3); with a multiply-high range reduction of its upper half (a table that fits
+// a GPU has fewer than 2^31 groups) any table size works without a modulo.
 __device__ __forceinline__ ull_t dok_mix64(ull_t h) {
   h ^= h >> 33; h *= 0xff51afd7ed558ccdULL;
   h ^= h >> 33; h *= 0xc4ceb9fe1a85ec53ULL;
@@ -123,7 +123,7 @@ __device__ __forceinline__ ull_t dok_chain_hash(const KeyHash &h) {
   return dok_mix64((ull_t)h.uuid ^ ((ull_t)h.hash1 * 0x9e3779b97f4a7c15ULL));
 }
 __device__ __forceinline__ ll_t dok_start_group(const KeyHash &h, const DevTable &t) {
-  return (ll_t)__umul64hi(dok_chain_hash(h), (ull_t)t.n_groups);
+  return (ll_t)__umulhi((unsigned)(dok_chain_hash(h) >> 32), (unsigned)t.n_groups);
 }
 // Order of a chain's groups.  Plain linear probing piles full groups up into long runs, and every miss walks its run to
 // the end: at load 0.9 with 4 slots per group a miss inspects 13.2 groups on average and 300 at most, a hit 2.0; at 0.745
@@ -195,6 +195,16 @@ struct RowKeys {          // contiguous [n, ks] rows of the key dtype (closed_ha
     return j < slice_rows && j < slice_counts[blockIdx.y];
   }
   __device__ __forceinline__ ll_t span() const { return slice_rows == 0 ? n : slice_rows; }
+  // rows in use (of slice blockIdx.y), and the batch element of one of them
+  __device__ __forceinline__ ll_t total() const {
+    if (slice_rows == 0) return n;
+    if (abort != nullptr && *abort != 0) return 0;
+    const ll_t used = slice_counts[blockIdx.y];
+    return used < slice_rows ? used : slice_rows;
+  }
+  __device__ __forceinline__ ll_t elem(unsigned row) const {
+    return slice_rows == 0 ? (ll_t)row : (ll_t)blockIdx.y * slice_rows + row;
+  }
   // block-uniform: nothing for this block to do
   __device__ __forceinline__ bool idle() const {
     if (slice_rows == 0) return false;
@@ -241,6 +251,8 @@ struct SelKeys {
   __device__ __forceinline__ bool row(ll_t &e) const { e = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x; return e < n; }
   __device__ __forceinline__ bool at(ll_t j, ll_t &e) const { e = j; return j < n; }
   __device__ __forceinline__ ll_t span() const { return n; }
+  __device__ __forceinline__ ll_t total() const { return n; }
+  __device__ __forceinline__ ll_t elem(unsigned row) const { return (ll_t)row; }
   __device__ __forceinline__ bool idle() const { return false; }
   __device__ __forceinline__ ll_t index(int d, ll_t off) const { return s.ptr[d] ? s.ptr[d][off] : s.base[d] + off; }
   // element offsets of batch element e into each of the ndim index tensors (fully unrolled over the
@@ -663,6 +675,10 @@ __device__ __forceinline__ void dok_tally_begin(BlockTally &b) {
 __device__ __forceinline__ void dok_tally_add(BlockTally &b, int slot, int pred) {
   const unsigned m = __ballot_sync(0xffffffffu, pred);
   if ((threadIdx.x & 31) == 0 && m) atomicAdd(&b.v[slot], __popc(m));
+}
+__device__ __forceinline__ void dok_tally_sum(BlockTally &b, int slot, int v) {     // a count per lane
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0 && v) atomicAdd(&b.v[slot], v);
 }
 __device__ __forceinline__ void dok_tally_flush(BlockTally &b, ll_t *counters, ll_t *extra) {
   __syncwarp();

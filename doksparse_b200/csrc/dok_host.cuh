@@ -112,6 +112,7 @@ inline bool dok_make_table(const dok_table *t, DevTable *out) {
   out->stamp_off = lay.stamp_off;
   out->vwords = (t->value_bytes + 7) / 8;
   out->win_lo = out->win_hi = 0;
+  if (out->n_groups >= 0x7fffffffLL) return false;                    // 256 GiB of slots and more
   if (lay.sb <= 128 && out->n_slots >= 0xffffffffLL) return false;    // the cooperative walk keeps slot indices in 32 bits
   return true;
 }

@@ -1,0 +1,133 @@
+// The walk of a large batch: a warp keeps 32 chains in flight and takes the next row whenever one of them ends.
+//
+// With one row per thread a warp walks until the longest of its 32 chains ends.  At load 0.6 one row in six needs a second
+// group, so nearly every warp made one to three more dependent round trips to DRAM for a handful of lanes: a row stayed on
+// its SM for 10 us, five times the latency of one access, and DRAM ran at 74 % of what a copy reaches.  Here a warp has a
+// share of the batch.  It hashes 32 rows at a time (coalesced) into a queue in shared memory; a lane whose chain has ended
+// takes the queue's next row; and every round of the loop inspects one group for each of the 32 lanes, the four lanes of a
+// quad reading the line of each of the quad's four keys together (dok_device.cuh).  Rows that belong to another window of a
+// windowed launch never enter the queue, so they cost their hash and nothing else.
+//
+// Small batches have one row per lane and no refill; the code is the same.
+#pragma once
+#include "dok_host.cuh"
+
+#define DOK_QUEUE 64                     // entries per warp: up to 31 waiting plus 32 new ones
+#define DOK_WARPS (DOK_TPB / 32)
+#define DOK_NONE 0xffffffffu
+
+struct WarpQueue { ulonglong2 entry[DOK_QUEUE]; };      // uuid | group, stride - 1 (6 bits), row of the share (26 bits)
+
+// What a lane works on.  row (of the warp's share) == DOK_NONE: nothing; its uuid then matches no tag, and the group it
+// reads is the one of its last row (or group 0).
+struct LaneRow {
+  ll_t uuid;
+  unsigned group, word, row;
+  __device__ __forceinline__ bool busy() const { return row != DOK_NONE; }
+  __device__ __forceinline__ void done() { row = DOK_NONE; uuid = -4; }
+};
+#define DOK_IDLE_LANE LaneRow{-4, 0, 0, DOK_NONE}
+
+// A warp's share of the batch (of the block's slice), handed out 32 rows at a time from its end to its beginning: when rows
+// with equal keys meet in one warp, the later one, whose value stays, comes first.
+struct WarpShare {
+  unsigned first, left;                  // rows first .. first + left - 1 are still to be hashed
+  unsigned head, waiting;                // queue position, entries
+};
+
+__device__ __forceinline__ WarpShare dok_share(ll_t total) {
+  const ll_t warps = (ll_t)gridDim.x * DOK_WARPS, w = (ll_t)blockIdx.x * DOK_WARPS + (threadIdx.x >> 5);
+  ll_t per = (total + warps - 1) / warps;
+  if (per < 32) per = 32;                // a short batch: whole warps first
+  ll_t first = w * per, end = first + per;
+  if (end > total) end = total;
+  if (first > end) first = end;
+  return WarpShare{(unsigned)first, (unsigned)(end - first), 0, 0};
+}
+
+// Fills the queue until 32 rows wait or the share is used up.  `admit(row, KeyHash, enter)` may keep a row out of it.
+template <class Keys, class Admit>
+__device__ __forceinline__ void dok_fill_queue(WarpQueue &q, WarpShare &s, const DevTable &t, const DevHash &hp, const Keys &keys,
+                                               const Admit &admit) {
+  const unsigned lane = threadIdx.x & 31u;
+  while (s.waiting < 32 && s.left > 0) {
+    const unsigned take = s.left < 32 ? s.left : 32;
+    s.left -= take;
+    const unsigned row = s.left + lane;
+    KeyHash kh{0, 0};
+    bool enter = lane < take;
+    if (enter) {
+      kh = keys.hash(hp, keys.elem(s.first + row));
+      enter = dok_in_window(t, kh, true);
+    }
+    enter = admit(s.first + row, kh, enter);
+    const unsigned votes = __ballot_sync(0xffffffffu, enter);
+    if (enter) {
+      const ull_t h = dok_chain_hash(kh);
+      const unsigned group = __umulhi((unsigned)(h >> 32), (unsigned)t.n_groups);
+      const unsigned at = (s.head + s.waiting + __popc(votes & ((1u << lane) - 1u))) & (DOK_QUEUE - 1);
+      q.entry[at] = make_ulonglong2((ull_t)kh.uuid, (ull_t)group << 32 | (row << 6 | ((unsigned)h & 63u)));
+    }
+    s.waiting += __popc(votes);
+  }
+  __syncwarp();
+}
+
+// Lanes without a row take the next ones; false when no lane of the warp has a row.
+__device__ __forceinline__ bool dok_refill(const WarpQueue &q, WarpShare &s, LaneRow &r, const DevTable &t) {
+  const unsigned idle = __ballot_sync(0xffffffffu, !r.busy());
+  if (idle == 0) return true;
+  const unsigned rank = __popc(idle & ((1u << (threadIdx.x & 31u)) - 1u));
+  if (!r.busy() && rank < s.waiting) {
+    const ulonglong2 e = q.entry[(s.head + rank) & (DOK_QUEUE - 1)];
+    r.uuid = (ll_t)e.x;
+    r.group = (unsigned)(e.y >> 32);
+    r.word = t.n_groups > 64 ? (unsigned)e.y & 63u : DOK_CHAIN_LINEAR;
+    r.row = (unsigned)e.y >> 6;
+  }
+  const unsigned n = __popc(idle), taken = n < s.waiting ? n : s.waiting;
+  s.head += taken;
+  s.waiting -= taken;
+  __syncwarp();
+  return n < 32 || taken > 0;
+}
+
+// One group for each lane.  m / me / tb: match, match-or-empty and tombstone bits of the lane's own group by LANE of the quad:
+// the slot at lane position p of a group is p * 32 / SB.  `seen(words of the quad's four lines, match and empty votes of the
+// warp for each of the four keys, me)` runs on all lanes while they hold the lines.
+template <int SB, int LW, bool TOMB, class Seen>
+__device__ __forceinline__ void dok_pass(const DevTable &t, const LaneRow &lr, unsigned &m, unsigned &me, unsigned &tb, const Seen &seen) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const unsigned l = threadIdx.x & 3u, base = threadIdx.x & 28u;
+  const bool has_tag = ((32u * l) % SB) == 0;
+  const char *my_base = t.slots + 32 * l;
+  ull_t w[4][LW];
+#pragma unroll
+  for (unsigned r = 0; r < 4; r++)
+    dok_load_words<LW>(my_base + (ull_t)__shfl_sync(FULL, lr.group, base + r) * 128u, w[r]);
+  unsigned match[4], empty[4], own_m = 0, own_e = 0, own_t = 0;
+#pragma unroll
+  for (unsigned r = 0; r < 4; r++) {
+    const ll_t uuid_r = __shfl_sync(FULL, lr.uuid, base + r), tag = (ll_t)w[r][0];
+    match[r] = __ballot_sync(FULL, has_tag && tag == uuid_r);
+    empty[r] = __ballot_sync(FULL, has_tag && tag == DOK_EMPTY);
+    if (l == r) { own_m = match[r]; own_e = empty[r]; }
+    if (TOMB) {
+      const unsigned tombs = __ballot_sync(FULL, has_tag && tag == DOK_REMOVED);
+      if (l == r) own_t = tombs;
+    }
+  }
+  m = (own_m >> base) & 0xfu;
+  me = ((own_m | own_e) >> base) & 0xfu;
+  tb = TOMB ? (own_t >> base) & 0xfu : 0u;
+  seen(w, match, empty, me);
+}
+
+struct NoLines {
+  template <int LW>
+  __device__ __forceinline__ void operator()(const ull_t (&)[4][LW], const unsigned (&)[4], const unsigned (&)[4], unsigned) const {}
+};
+struct AdmitAll {
+  __device__ __forceinline__ bool operator()(unsigned, const KeyHash &, bool enter) const { return enter; }
+};
+
