@@ -11,11 +11,11 @@ struct StridedValues {
   ll_t sizes[DOK_MAX_SELECTOR_NDIM];
   ll_t strides[DOK_MAX_SELECTOR_NDIM];
   __device__ __forceinline__ const char *row(const DevTable &t, ll_t e) const {
-    ull_t rem = (ull_t)e;
+    unsigned rem = (unsigned)e;        // batches have fewer than 2^32 elements
     ll_t off = 0;
     for (int j = selector_ndim - 1; j >= 0; j--) {
-      const ull_t size = (ull_t)sizes[j];
-      const ull_t q = rem / size;
+      const unsigned size = (unsigned)sizes[j];
+      const unsigned q = j > 0 ? rem / size : 0;
       off += (ll_t)(rem - q * size) * strides[j];
       rem = q;
     }

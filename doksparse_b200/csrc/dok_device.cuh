@@ -260,26 +260,14 @@ struct SelKeys {
   __device__ __forceinline__ void offsets(ll_t e, ll_t (&off)[DOK_MAX_KEY_SIZE]) const {
 #pragma unroll
     for (int d = 0; d < DOK_MAX_KEY_SIZE; d++) off[d] = 0;
-    if (n <= 0xffffffffLL) {           // 32-bit index arithmetic: the common case, far cheaper than 64-bit division
-      unsigned rem = (unsigned)e;
-      for (int j = s.selector_ndim - 1; j >= 0; j--) {
-        const unsigned size = (unsigned)s.sizes[j];
-        const unsigned q = rem / size;
-        const ll_t idx = (ll_t)(rem - q * size);
-        rem = q;
+    unsigned rem = (unsigned)e;        // batches have fewer than 2^32 elements; the outermost index is what is left
+    for (int j = s.selector_ndim - 1; j >= 0; j--) {
+      const unsigned size = (unsigned)s.sizes[j];
+      const unsigned q = j > 0 ? rem / size : 0;
+      const ll_t idx = (ll_t)(rem - q * size);
+      rem = q;
 #pragma unroll
-        for (int d = 0; d < DOK_MAX_KEY_SIZE; d++) if (d < s.ndim) off[d] += idx * s.strides[d][j];
-      }
-    } else {
-      ull_t rem = (ull_t)e;
-      for (int j = s.selector_ndim - 1; j >= 0; j--) {
-        const ull_t size = (ull_t)s.sizes[j];
-        const ull_t q = rem / size;
-        const ll_t idx = (ll_t)(rem - q * size);
-        rem = q;
-#pragma unroll
-        for (int d = 0; d < DOK_MAX_KEY_SIZE; d++) if (d < s.ndim) off[d] += idx * s.strides[d][j];
-      }
+      for (int d = 0; d < DOK_MAX_KEY_SIZE; d++) if (d < s.ndim) off[d] += idx * s.strides[d][j];
     }
   }
   __device__ __forceinline__ KeyHash hash(const DevHash &hp, ll_t e) const {
@@ -675,10 +663,6 @@ __device__ __forceinline__ void dok_tally_begin(BlockTally &b) {
 __device__ __forceinline__ void dok_tally_add(BlockTally &b, int slot, int pred) {
   const unsigned m = __ballot_sync(0xffffffffu, pred);
   if ((threadIdx.x & 31) == 0 && m) atomicAdd(&b.v[slot], __popc(m));
-}
-__device__ __forceinline__ void dok_tally_sum(BlockTally &b, int slot, int v) {     // a count per lane
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0 && v) atomicAdd(&b.v[slot], v);
 }
 __device__ __forceinline__ void dok_tally_flush(BlockTally &b, ll_t *counters, ll_t *extra) {
   __syncwarp();

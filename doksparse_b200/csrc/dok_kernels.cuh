@@ -8,15 +8,19 @@
 //
 // No thread of a warp returns early: the cooperative walk needs all 32 lanes.
 #pragma once
+#include <type_traits>
 #include "dok_stream.cuh"
 
 // ---------------------------------------------------------------------------------------------------------
 // get
 // ---------------------------------------------------------------------------------------------------------
-// Slots wider than a line: one row per thread, walked by its own lane.
-template <class Keys>
-__global__ void __launch_bounds__(DOK_TPB) k_get_wide(DevTable t, DevHash hp, Keys keys, char *__restrict__ out_values,
-                                                      uint8_t *__restrict__ out_found, Fallback fb, ll_t *counters, int count_probes) {
+// One row per thread: for 32-byte slots with values of at most 8 bytes, whose walk fits 32 registers, so that 64 warps are
+// resident (8.4 M lookups at load 0.6: 251 us; the form below, with half the instructions but 32 warps: 291), and for slots
+// wider than a line, which a lane walks by itself.
+template <int SB, int LW, class Keys>
+__global__ void __launch_bounds__(DOK_TPB, SB == 32 ? 8 : 1) k_get_row(DevTable t, DevHash hp, Keys keys, char *__restrict__ out_values,
+                                                    uint8_t *__restrict__ out_found, Fallback fb, ll_t *counters,
+                                                    int count_probes) {
   __shared__ BlockTally tally;
   if (keys.idle()) return;
   if (counters) dok_tally_begin(tally);
@@ -26,15 +30,15 @@ __global__ void __launch_bounds__(DOK_TPB) k_get_wide(DevTable t, DevHash hp, Ke
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
   int probes = 0;
-  Located loc{-1, -1, -1};
-  if (active) loc = dok_locate_serial(t, kh, &probes);
+  // on a hit the quad writes the value from the registers that hold the line
+  const Located loc = dok_locate<SB, LW, false>(t, kh, e, active, &probes, EmitValue<(SB == 0 ? 32 : SB), LW>{t, out_values});
   const int hit = active && loc.found >= 0;
   if (active) {
     char *dst = out_values + e * (ll_t)t.vb;
-    if (hit) dok_load_value(t, loc.found, dst);
-    else dok_store_fallback(t, fb, dst);
-    if (out_found) out_found[e] = (uint8_t)hit;
+    if (SB == 0 && hit) dok_load_value(t, loc.found, dst);
+    if (!hit) dok_store_fallback(t, fb, dst);
   }
+  if (active && out_found) out_found[e] = (uint8_t)hit;
   if (counters) {
     dok_tally_add(tally, DOK_CNT_HITS, hit);
     dok_tally_flush(tally, counters, nullptr);
@@ -42,6 +46,10 @@ __global__ void __launch_bounds__(DOK_TPB) k_get_wide(DevTable t, DevHash hp, Ke
   }
 }
 
+// A warp's share of the batch (dok_stream.cuh): for everything else.  Wider values need the registers of whole lines (3
+// blocks of 256 per SM in either form), and where a line holds fewer slots the chains are longer, so that a warp that waits
+// for its longest chain leaves most of its lanes idle: 8.4 M lookups of 16-byte values 544 -> 354 us, 8.4 M misses in
+// 64-byte slots at load 0.69 750 -> 595, selections of 32-byte slots 153 -> 141.
 // Values of at most 8 bytes lie behind the tag in the word pair that a lane has loaded: the key's own lane fetches it from
 // the lane of the slot that matched, and stores value (or fallback) and flag of its row -- one store for 32 rows of which
 // most are neighbours.  Wider values are written by the quad from the registers that hold the line.  Either way a hit needs
@@ -52,58 +60,50 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, De
                                                                   int count_probes) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ WarpQueue queues[DOK_WARPS];
-  WarpQueue &queue = queues[threadIdx.x >> 5];
-  WarpShare share = dok_share(keys.total());
-  LaneRow lr = DOK_IDLE_LANE;
   int hits = 0, probes = 0;
-  for (;;) {
-    dok_fill_queue(queue, share, t, hp, keys, AdmitAll());
-    if (!dok_refill(queue, share, lr, t)) break;
-    unsigned m, me, tb;
+  dok_walk_share<LW>(queues[threadIdx.x >> 5], t, hp, keys, [&](LaneRow &lr, const Lines<LW> &f, const WarpShare &share) {
+    unsigned m, me, match[4], empty[4];
+    dok_inspect<SB, LW>(lr, f, m, me, match, empty);
+    const unsigned l = threadIdx.x & 3u, base = threadIdx.x & 28u;
     ull_t value = 0;
-    dok_pass<SB, LW, false>(t, lr, m, me, tb, [&](const ull_t (&w)[4][LW], const unsigned (&match)[4], const unsigned (&empty)[4],
-                                                  unsigned me_own) {
-      const unsigned l = threadIdx.x & 3u, base = threadIdx.x & 28u;
-      if constexpr (LW == 2) {
-        const unsigned from = base + (me_own ? (unsigned)(__ffs(me_own) - 1) : 0u);
+    if constexpr (LW == 2) {
+      const unsigned from = base + (me ? (unsigned)(__ffs(me) - 1) : 0u);
 #pragma unroll
-        for (unsigned r = 0; r < 4; r++) {
-          const ull_t v = __shfl_sync(FULL, w[r][1], from);
-          if (l == r) value = v;
-        }
-      } else {
-        const EmitValue<SB, LW> emit{t, out_values};
-#pragma unroll
-        for (unsigned r = 0; r < 4; r++) {
-          const unsigned row_r = __shfl_sync(FULL, lr.row, base + r);
-          const unsigned m_r = (match[r] >> base) & 0xfu, me_r = m_r | ((empty[r] >> base) & 0xfu);
-          if (me_r) {
-            const int lane = __ffs(me_r) - 1, pos = lane * 32 / SB;
-            if ((m_r >> lane) & 1u) emit(keys.elem(share.first + row_r), pos, w[r]);
-          }
-        }
+      for (unsigned r = 0; r < 4; r++) {
+        const ull_t v = __shfl_sync(FULL, f.w[r][1], from);
+        if (l == r) value = v;
       }
-    });
-    if (lr.busy()) {
-      const bool hit = me && ((m >> (__ffs(me) - 1)) & 1u);
-      probes++;
-      if (me || !dok_next_group<unsigned>(lr.group, lr.word, (unsigned)t.n_groups)) {
-        const ll_t e = keys.elem(share.first + lr.row);
-        char *dst = out_values + e * (ll_t)t.vb;
-        if constexpr (LW == 2) {
-          if (!hit) value = fb.w[0];
-          if (t.vb == 8) *(ull_t *)dst = value;
-          else if (t.vb == 4) *(unsigned *)dst = (unsigned)value;
-          else dok_store_word(dst, value, t.vb, t.vb & -t.vb);
-        } else {
-          if (!hit) dok_store_fallback(t, fb, dst);
+    } else {
+      const EmitValue<SB, LW> emit{t, out_values};
+#pragma unroll
+      for (unsigned r = 0; r < 4; r++) {
+        const unsigned row_r = __shfl_sync(FULL, lr.row, base + r);
+        const unsigned m_r = (match[r] >> base) & 0xfu, me_r = m_r | ((empty[r] >> base) & 0xfu);
+        if (me_r) {
+          const int lane = __ffs(me_r) - 1, pos = lane * 32 / SB;
+          if ((m_r >> lane) & 1u) emit(keys.elem(share.first + row_r), pos, f.w[r]);
         }
-        if (out_found) out_found[e] = (uint8_t)hit;
-        hits += hit;
-        lr.done();
       }
     }
-  }
+    if (!lr.busy()) return;
+    const bool hit = me && ((m >> (__ffs(me) - 1)) & 1u);
+    probes++;
+    if (me || !dok_next_group<unsigned>(lr.group, lr.word, (unsigned)t.n_groups)) {
+      const ll_t e = keys.elem(share.first + lr.row);
+      char *dst = out_values + e * (ll_t)t.vb;
+      if constexpr (LW == 2) {
+        if (!hit) value = fb.w[0];
+        if (t.vb == 8) *(ull_t *)dst = value;
+        else if (t.vb == 4) *(unsigned *)dst = (unsigned)value;
+        else dok_store_word(dst, value, t.vb, t.vb & -t.vb);
+      } else {
+        if (!hit) dok_store_fallback(t, fb, dst);
+      }
+      if (out_found) out_found[e] = (uint8_t)hit;
+      hits += hit;
+      lr.done();
+    }
+  });
   if (counters) {
     dok_warp_add(counters + DOK_CNT_HITS, hits);
     if (count_probes) dok_warp_add(counters + DOK_CNT_PROBES, probes);
@@ -156,10 +156,13 @@ inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, vo
   ll_t *cnt = (ll_t *)counters;
   // tag and value fit the first 16 bytes of the slot: half the load width
   const bool narrow = t.vb <= 8;
+  constexpr bool ROWS = std::is_same<Keys, RowKeys>::value;
   switch (t.sb) {
     case 32:
-      if (narrow) DOK_STREAM(t, rc, st, keys, (k_get<32, 2, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
-      else DOK_STREAM(t, rc, st, keys, (k_get<32, 4, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
+      if (!narrow) DOK_STREAM(t, rc, st, keys, (k_get<32, 4, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
+      else if constexpr (ROWS)
+        DOK_FOR_WINDOWS(t, rc, (k_get_row<32, 2, Keys><<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, values, out_found, fb, cnt, count_probes)));
+      else DOK_STREAM(t, rc, st, keys, (k_get<32, 2, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
       break;
     case 64:
       if (narrow) DOK_STREAM(t, rc, st, keys, (k_get<64, 2, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
@@ -170,7 +173,7 @@ inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, vo
       else DOK_STREAM(t, rc, st, keys, (k_get<128, 4, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
       break;
     default:
-      DOK_FOR_WINDOWS(t, rc, (k_get_wide<Keys><<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, values, out_found, fb, cnt, count_probes)));
+      DOK_FOR_WINDOWS(t, rc, (k_get_row<0, 4, Keys><<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, values, out_found, fb, cnt, count_probes)));
   }
   return rc;
 }
@@ -191,82 +194,9 @@ __device__ __forceinline__ void dok_write_row(const DevTable &t, const DevHash &
   dok_store_value(t, slot, values.row(t, e));
 }
 
-// Insert-or-find over a warp's share of the batch (LW = 1: the tags are all that a claim needs).  The lane whose chain has
-// ended claims the place the chain offers -- the first tombstone, else the first empty slot -- with one CAS.  Losing it to
-// the same uuid means that a twin row has claimed it: join.  Losing it to another one is rare; the lane then redoes the
-// operation by itself.  `done(batch element, slot or -1, outcome)` runs on that lane.
-template <int SB, class Keys, class Admit, class Done>
-__device__ __forceinline__ void dok_claim_share(WarpQueue &queue, const DevTable &t, const DevHash &hp, const Keys &keys, const Admit &admit,
-                                                const Done &done) {
-  constexpr unsigned SPG = 128 / SB;
-  WarpShare share = dok_share(keys.total());
-  LaneRow lr = DOK_IDLE_LANE;
-  unsigned tomb = DOK_NONE;
-  for (;;) {
-    dok_fill_queue(queue, share, t, hp, keys, admit);
-    if (!dok_refill(queue, share, lr, t)) break;
-    unsigned m, me, tb;
-    dok_pass<SB, 1, true>(t, lr, m, me, tb, NoLines());
-    if (lr.busy()) {
-      const unsigned pos = me ? (unsigned)__ffs(me) - 1 : 0, here = lr.group * SPG;
-      if (tomb == DOK_NONE) {
-        const unsigned before = me ? tb & ((1u << pos) - 1u) : tb;
-        if (before) tomb = here + ((unsigned)__ffs(before) - 1) * 32 / SB;
-      }
-      if (me || !dok_next_group<unsigned>(lr.group, lr.word, (unsigned)t.n_groups)) {
-        const ll_t e = keys.elem(share.first + lr.row);
-        ll_t slot = -1;
-        int outcome = DOK_OUT_FAILED;         // no match, no tombstone, no empty slot: the table is full
-        if (me && ((m >> pos) & 1u)) {
-          slot = here + pos * 32 / SB;
-          outcome = DOK_OUT_FOUND;
-        } else if (me || tomb != DOK_NONE) {
-          const bool reuse = tomb != DOK_NONE;
-          const ll_t expect = reuse ? DOK_REMOVED : DOK_EMPTY;
-          slot = reuse ? (ll_t)tomb : (ll_t)(here + pos * 32 / SB);
-          const ll_t old = dok_cas_tag(t, slot, expect, lr.uuid);
-          if (old == expect) outcome = reuse ? DOK_OUT_REUSED : DOK_OUT_CLAIMED_EMPTY;
-          else if (old == lr.uuid) outcome = DOK_OUT_FOUND;
-          else slot = dok_find_or_claim_serial(t, keys.hash(hp, e), &outcome);
-        }
-        done(e, slot, outcome);
-        tomb = DOK_NONE;
-        lr.done();
-      }
-    }
-  }
-}
-
-__device__ __forceinline__ void dok_tally_outcome(BlockTally &b, int claimed, int reused, int failed, int hits) {
-  dok_tally_sum(b, DOK_CNT_CLAIMED_EMPTY, claimed);
-  dok_tally_sum(b, DOK_CNT_REUSED_REMOVED, reused);
-  dok_tally_sum(b, DOK_CNT_FAILED, failed);
-  dok_tally_sum(b, DOK_CNT_HITS, hits);
-}
-
 // One kernel, for batches whose rows have pairwise different uuids.
 template <int SB, class Keys, class Values>
 __global__ void __launch_bounds__(DOK_TPB, 4) k_set_unique(DevTable t, DevHash hp, Keys keys, Values values,
-                                                        uint8_t *__restrict__ out_stored, ll_t *counters) {
-  __shared__ BlockTally tally;
-  __shared__ WarpQueue queues[DOK_WARPS];
-  dok_tally_begin(tally);
-  int claimed = 0, reused = 0, failed = 0, hits = 0;
-  dok_claim_share<SB>(queues[threadIdx.x >> 5], t, hp, keys, AdmitAll(), [&](ll_t e, ll_t slot, int outcome) {
-    if (slot >= 0) dok_write_row(t, hp, keys, values, e, slot, outcome != DOK_OUT_FOUND || hp.dtype >= DOK_F16);
-    if (out_stored) out_stored[e] = (uint8_t)(slot >= 0);
-    claimed += outcome == DOK_OUT_CLAIMED_EMPTY;
-    reused += outcome == DOK_OUT_REUSED;
-    failed += outcome == DOK_OUT_FAILED;
-    hits += outcome == DOK_OUT_FOUND;
-  });
-  dok_tally_outcome(tally, claimed, reused, failed, hits);
-  dok_tally_flush(tally, counters, nullptr);
-}
-
-// The same for slots wider than a line: one row per thread.
-template <class Keys, class Values>
-__global__ void __launch_bounds__(DOK_TPB) k_set_unique_wide(DevTable t, DevHash hp, Keys keys, Values values,
                                                         uint8_t *__restrict__ out_stored, ll_t *counters) {
   __shared__ BlockTally tally;
   if (keys.idle()) return;
@@ -277,7 +207,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_set_unique_wide(DevTable t, DevHash
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
   int outcome = -1;
-  const ll_t slot = dok_find_or_claim<0>(t, kh, active, &outcome);
+  const ll_t slot = dok_find_or_claim<SB>(t, kh, active, &outcome);
   if (active) {
     if (slot >= 0) dok_write_row(t, hp, keys, values, e, slot, outcome != DOK_OUT_FOUND || hp.dtype >= DOK_F16);
     if (out_stored) out_stored[e] = (uint8_t)(slot >= 0);
@@ -300,52 +230,72 @@ __global__ void __launch_bounds__(DOK_TPB) k_set_unique_wide(DevTable t, DevHash
 #define DOK_ROW_FRESH (1LL << 62)      // bit of a row's slot index: this row claimed the slot
 __device__ __forceinline__ ull_t dok_stamp(ll_t epoch, ll_t row) { return ((ull_t)epoch << 34) | ((ull_t)row << 2); }
 
-// Rows that a block has met last, by key (1024 places by the chain's hash: 32 more bits of it | row of the slice).  A share
-// is worked through from its end, so a row whose key was met before has a later row that overrides it and need not go to
-// the table at all -- if the keys are really the same, which is checked against the row named here: same uuid and same
-// chain, so that both rows would have met in one slot.  In a Zipf batch the most popular key is 4 % of the rows; every one
-// of them read, stored and stamped the same line, which the L2 serves one after the other: 12.8 M such rows took 20 ms, and
-// 5.8 ms with the equal keys of each 256 rows found first.  A batch without equal keys pays a read and a write of shared
-// memory per row.
-#define DOK_MET 1024
-struct BlockMet { ull_t place[DOK_MET]; };
+// The rows of a block that hold the same key, found in shared memory before the table is touched: only the last of them,
+// which is the one whose value stays, goes on.  In a Zipf batch the most popular key is 4 % of the rows, and every one of
+// them read, stored and stamped the same line, which the L2 serves one after the other: 12.8 M such rows took 20 ms.
+// Same key: same uuid and same chain, so that the rows would have met in one slot.  The set is keyed by the chain's hash;
+// rows that share it by chance have different uuids and go on by themselves.
+#define DOK_TWIN_SLOTS (2 * DOK_TPB)
+struct BlockTwins {
+  ll_t chain[DOK_TWIN_SLOTS];              // 55 bits of the chain's hash | 8 bits: thread of the key's last row so far
+  ll_t uuid[DOK_TPB], slot[DOK_TPB];       // by thread; inactive rows have no uuid
+  uint8_t more[DOK_TPB * 2];               // by place: more than one row
+};
+struct Twins { int last; bool more; };     // thread of the key's last row; whether there are others
+
+// every thread of the block must call
+__device__ __forceinline__ Twins dok_find_twins(BlockTwins &b, const KeyHash &kh, bool active) {
+#pragma unroll
+  for (int i = threadIdx.x; i < DOK_TWIN_SLOTS; i += DOK_TPB) { b.chain[i] = DOK_EMPTY; b.more[i] = 0; }
+  b.uuid[threadIdx.x] = active ? kh.uuid : DOK_EMPTY;
+  __syncthreads();
+  int at = 0;
+  if (active) {
+    const ll_t mine = ((ll_t)dok_chain_hash(kh) & 0x7fffffffffffff00LL) | threadIdx.x;
+    at = (int)(mine >> 8) & (DOK_TWIN_SLOTS - 1);
+    for (;;) {                             // at most DOK_TPB of the DOK_TWIN_SLOTS places are ever taken
+      const ll_t old = (ll_t)atomicCAS((ull_t *)&b.chain[at], (ull_t)DOK_EMPTY, (ull_t)mine);
+      if (old == DOK_EMPTY) break;
+      if (((old ^ mine) >> 8) == 0) {
+        atomicMax(&b.chain[at], mine);
+        b.more[at] = 1;
+        break;
+      }
+      at = (at + 1) & (DOK_TWIN_SLOTS - 1);
+    }
+  }
+  __syncthreads();
+  Twins w{(int)threadIdx.x, false};
+  if (active) {
+    const int last = (int)(b.chain[at] & 255);
+    if (b.uuid[last] == kh.uuid) w.last = last;
+    w.more = b.more[at] != 0;
+  }
+  return w;
+}
 
 // First kernel of the general set.  Find or claim the slot, store the row there and raise the slot's stamp --
 // for a batch without equal uuids that is all there is to do.  A row that finds the slot already stamped in
 // this epoch sets the conflict bit and counts a duplicate (in slot_out[n], zeroed by the host before the
 // launch); the second kernel then lets the slot's last row rewrite it.
-// slot_out of a row: its slot, -1 without a place, -2 - f when the later row f of the batch stands for it.
 template <int SB, class Keys, class Values>
-__global__ void __launch_bounds__(DOK_TPB, 4) k_set_claim(DevTable t, DevHash hp, Keys keys, Values values,
+__global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp, Keys keys, Values values,
                                                        ll_t *__restrict__ slot_out, ll_t epoch, int mark_fresh,
                                                        uint8_t *__restrict__ out_stored, ll_t *counters) {
   __shared__ BlockTally tally;
-  __shared__ WarpQueue queues[DOK_WARPS];
-  __shared__ BlockMet met;
-  for (int i = threadIdx.x; i < DOK_MET; i += DOK_TPB) met.place[i] = 0;
+  __shared__ BlockTwins twins;
+  if (keys.idle()) return;
   dok_tally_begin(tally);
-  int claimed = 0, reused = 0, failed = 0, hits = 0, dups = 0, conflicts = 0;
-  const auto admit = [&](unsigned row, const KeyHash &kh, bool enter) {
-    if (enter && !out_stored) {                          // (flags are wanted for every row: each goes to the table)
-      const ull_t h = dok_chain_hash(kh), mine = (h | 1ULL << 32) >> 32 << 32 | row;
-      volatile ull_t *place = &met.place[(unsigned)h >> 8 & (DOK_MET - 1)];
-      const ull_t old = *place;
-      if ((old ^ mine) >> 32 == 0 && (unsigned)old > row) {
-        const ll_t later = keys.elem((unsigned)old);
-        const KeyHash other = keys.hash(hp, later);
-        if (other.uuid == kh.uuid && other.hash1 == kh.hash1) {
-          slot_out[keys.elem(row)] = -2 - later;
-          hits++;
-          dups++;
-          conflicts += mark_fresh;
-          return false;
-        }
-      }
-      *place = mine;
-    }
-    return enter;
-  };
-  dok_claim_share<SB>(queues[threadIdx.x >> 5], t, hp, keys, admit, [&](ll_t e, ll_t slot, int outcome) {
+  ll_t e;
+  bool active = keys.row(e);
+  KeyHash kh{0, 0};
+  if (active) kh = keys.hash(hp, e);
+  active = dok_in_window(t, kh, active);
+  const Twins same = dok_find_twins(twins, kh, active);
+  const bool last = active && same.last == (int)threadIdx.x;
+  int outcome = -1, conflict = 0;
+  ll_t slot = dok_find_or_claim<SB>(t, kh, last, &outcome);
+  if (last) {
     const bool fresh = outcome == DOK_OUT_CLAIMED_EMPTY || outcome == DOK_OUT_REUSED;
     slot_out[e] = mark_fresh && fresh ? slot | DOK_ROW_FRESH : slot;
     if (slot >= 0) {
@@ -354,72 +304,42 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_set_claim(DevTable t, DevHash hp
       ll_t *stamp = dok_stamp_ptr(t, slot);
       dok_write_row(t, hp, keys, values, e, slot, fresh || hp.dtype >= DOK_F16);
       const ull_t old = atomicMax((ull_t *)stamp, dok_stamp(epoch, e));
-      if ((old >> 34) == (ull_t)epoch) {
+      if ((old >> 34) == (ull_t)epoch || (mark_fresh && same.more)) {
         atomicOr((ull_t *)stamp, DOK_STAMP_CONFLICT);
-        dups++;
-        conflicts++;
+        conflict = 1;
       }
     } else {
-      conflicts++;                    // rows that it stands for have no place either: the second kernel counts them
+      conflict = mark_fresh;          // a row without a place is counted by k_set_count too
     }
     if (out_stored) out_stored[e] = (uint8_t)(slot >= 0);
-    claimed += outcome == DOK_OUT_CLAIMED_EMPTY;
-    reused += outcome == DOK_OUT_REUSED;
-    failed += outcome == DOK_OUT_FAILED;
-    hits += outcome == DOK_OUT_FOUND;
-  });
-  dok_tally_outcome(tally, claimed, reused, failed, hits);
-  dok_tally_sum(tally, DOK_CNT_DUPLICATES, dups);
-  dok_tally_sum(tally, DOK_TALLY_EXTRA, conflicts);
-  dok_tally_flush(tally, counters, slot_out + keys.count());
-}
-
-// The same for slots wider than a line: one row per thread, every row goes to the table.
-template <class Keys, class Values>
-__global__ void __launch_bounds__(DOK_TPB) k_set_claim_wide(DevTable t, DevHash hp, Keys keys, Values values,
-                                                            ll_t *__restrict__ slot_out, ll_t epoch, int mark_fresh,
-                                                            uint8_t *__restrict__ out_stored, ll_t *counters) {
-  __shared__ BlockTally tally;
-  if (keys.idle()) return;
-  dok_tally_begin(tally);
-  ll_t e;
-  bool active = keys.row(e);
-  KeyHash kh{0, 0};
-  if (active) kh = keys.hash(hp, e);
-  active = dok_in_window(t, kh, active);
-  int outcome = -1, dup = 0, conflict = 0;
-  const ll_t slot = dok_find_or_claim<0>(t, kh, active, &outcome);
-  if (active) {
-    const bool fresh = outcome == DOK_OUT_CLAIMED_EMPTY || outcome == DOK_OUT_REUSED;
-    slot_out[e] = mark_fresh && fresh ? slot | DOK_ROW_FRESH : slot;
-    if (slot >= 0) {
-      ll_t *stamp = dok_stamp_ptr(t, slot);
-      dok_write_row(t, hp, keys, values, e, slot, fresh || hp.dtype >= DOK_F16);
-      const ull_t old = atomicMax((ull_t *)stamp, dok_stamp(epoch, e));
-      if ((old >> 34) == (ull_t)epoch) {
-        atomicOr((ull_t *)stamp, DOK_STAMP_CONFLICT);
-        dup = conflict = 1;
-      }
-    } else {
-      conflict = mark_fresh;
+    if (slot < 0 && same.more && counters) {                        // a full table: its twins, counted as found below,
+      ll_t others = -1;                                             // have no place either
+      for (int i = 0; i < DOK_TPB; i++) others += twins.uuid[i] == kh.uuid;
+      atomicAdd((ull_t *)counters + DOK_CNT_FAILED, (ull_t)others);
+      atomicAdd((ull_t *)counters + DOK_CNT_HITS, (ull_t)-others);
     }
-    if (out_stored) out_stored[e] = (uint8_t)(slot >= 0);
+  }
+  if (out_stored || mark_fresh) {                                   // uniform over the launch
+    if (last) twins.slot[threadIdx.x] = slot;
+    __syncthreads();
+    if (active && !last) {
+      slot = twins.slot[same.last];
+      slot_out[e] = slot;
+      if (out_stored) out_stored[e] = (uint8_t)(slot >= 0);
+    }
+  } else if (active && !last) {
+    slot_out[e] = -1;                                               // nothing to rewrite: a later row of the block may
   }
   dok_tally_add(tally, DOK_TALLY_EXTRA, conflict);
   if (counters) {
+    const bool twin = active && !last;
     dok_tally_add(tally, DOK_CNT_CLAIMED_EMPTY, outcome == DOK_OUT_CLAIMED_EMPTY);
     dok_tally_add(tally, DOK_CNT_REUSED_REMOVED, outcome == DOK_OUT_REUSED);
     dok_tally_add(tally, DOK_CNT_FAILED, outcome == DOK_OUT_FAILED);
-    dok_tally_add(tally, DOK_CNT_HITS, outcome == DOK_OUT_FOUND);
-    dok_tally_add(tally, DOK_CNT_DUPLICATES, dup);
+    dok_tally_add(tally, DOK_CNT_HITS, twin || outcome == DOK_OUT_FOUND);
+    dok_tally_add(tally, DOK_CNT_DUPLICATES, twin || (conflict && slot >= 0));
   }
   dok_tally_flush(tally, counters, slot_out + keys.count());
-}
-
-// What stands in slot_in for the row that represents row e in the end (rows refer to later ones, so this terminates).
-__device__ __forceinline__ ll_t dok_final_slot(const ll_t *slot_in, ll_t slot) {
-  while (slot <= -2) slot = slot_in[-2 - slot];
-  return slot;
 }
 
 // Second kernel: does nothing unless the first one counted duplicates.  Then the row that owns a conflicted
@@ -427,7 +347,7 @@ __device__ __forceinline__ ll_t dok_final_slot(const ll_t *slot_in, ll_t slot) {
 // every first-kernel write has completed, so rows cannot tear and the last row wins.
 template <class Keys, class Values>
 __global__ void __launch_bounds__(DOK_TPB) k_set_resolve(DevTable t, DevHash hp, Keys keys, Values values,
-                                                         const ll_t *__restrict__ slot_in, ll_t epoch, ll_t *counters) {
+                                                         const ll_t *__restrict__ slot_in, ll_t epoch) {
   if (slot_in[keys.count()] == 0) return;        // the first kernel met no duplicate: every row is already in place
   if (keys.idle()) return;
   // a few blocks per SM stride over the rows: the usual launch has nothing to do, and a grid of one block per 256
@@ -437,13 +357,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_set_resolve(DevTable t, DevHash hp,
     ll_t e;
     if (!keys.at(j, e)) continue;
     ll_t slot = slot_in[e];
-    if (slot < 0) {
-      if (slot <= -2 && counters && t.win_lo == 0 && dok_final_slot(slot_in, slot) == -1) {   // represented by a row that found no place
-        atomicAdd((ull_t *)counters + DOK_CNT_FAILED, 1ULL);
-        atomicAdd((ull_t *)counters + DOK_CNT_HITS, ~0ULL);
-      }
-      continue;
-    }
+    if (slot < 0) continue;
     const bool fresh = (slot & DOK_ROW_FRESH) != 0;
     slot &= ~DOK_ROW_FRESH;
     if (t.win_hi != 0) {                         // windowed passes: by the slot's own group (each slot has one pass)
@@ -471,9 +385,9 @@ __global__ void __launch_bounds__(DOK_TPB) k_set_count(DevTable t, Keys keys, co
   for (ll_t j = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x; j < span; j += stride) {
     ll_t e;
     if (!keys.at(j, e)) continue;
-    const ll_t own = slot_in[e], slot = dok_final_slot(slot_in, own);
+    const ll_t slot = slot_in[e];
     if (slot < 0) { c++; continue; }
-    if (slot & DOK_ROW_FRESH) { c += own != slot; continue; }
+    if (slot & DOK_ROW_FRESH) continue;
     const ull_t stamp = (ull_t)__ldcg(dok_stamp_ptr(t, slot));
     c += (stamp >> 34) == (ull_t)epoch && (stamp & DOK_STAMP_FRESH) != 0;
   }
@@ -488,19 +402,12 @@ inline int launch_set_general(const DevTable &t, const DevHash &hp, const Keys &
   if (cudaMemsetAsync(slot_scratch + keys.n, 0, sizeof(int64_t), st) != cudaSuccess) return dok_check_launch();
   const dim3 grid = dok_grid(keys);
   int rc = DOK_OK;
-  ll_t *slots = (ll_t *)slot_scratch, *cnt = (ll_t *)counters;
-  const int fresh = more != nullptr;
-  switch (t.sb) {
-    case 32: DOK_STREAM(t, rc, st, keys, (k_set_claim<32, Keys, Values>), hp, keys, values, slots, (ll_t)epoch, fresh, out_stored, cnt); break;
-    case 64: DOK_STREAM(t, rc, st, keys, (k_set_claim<64, Keys, Values>), hp, keys, values, slots, (ll_t)epoch, fresh, out_stored, cnt); break;
-    case 128: DOK_STREAM(t, rc, st, keys, (k_set_claim<128, Keys, Values>), hp, keys, values, slots, (ll_t)epoch, fresh, out_stored, cnt); break;
-    default:
-      DOK_FOR_WINDOWS(t, rc, (k_set_claim_wide<<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, slots, (ll_t)epoch, fresh, out_stored, cnt)));
-  }
+  DOK_DISPATCH_SB(t, DOK_FOR_WINDOWS(t, rc, (k_set_claim<SB><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, (ll_t *)slot_scratch,
+                                                                                       (ll_t)epoch, more != nullptr, out_stored, (ll_t *)counters))));
   if (rc != DOK_OK) return rc;
   dim3 few = grid;
   if (few.x > 148 * 8) few.x = 148 * 8;
-  DOK_FOR_WINDOWS(t, rc, (k_set_resolve<<<few, DOK_TPB, 0, st>>>(wt, hp, keys, values, slots, (ll_t)epoch, cnt)));
+  DOK_FOR_WINDOWS(t, rc, (k_set_resolve<<<few, DOK_TPB, 0, st>>>(wt, hp, keys, values, (const ll_t *)slot_scratch, (ll_t)epoch)));
   if (rc != DOK_OK || more == nullptr) return rc;
   k_set_count<<<few, DOK_TPB, 0, st>>>(t, keys, (const ll_t *)slot_scratch, (ll_t)epoch, (ll_t *)more);
   return dok_check_launch();
@@ -515,15 +422,9 @@ inline int launch_set(const DevTable &t, const DevHash &hp, const RowKeys &keys,
 inline int launch_set_unique(const DevTable &t, const DevHash &hp, const RowKeys &keys, const char *values,
                              uint8_t *out_stored, int64_t *counters, cudaStream_t st) {
   RowValues rv{values};
+  const dim3 grid = dok_grid(keys);
   int rc = DOK_OK;
-  ll_t *cnt = (ll_t *)counters;
-  switch (t.sb) {
-    case 32: DOK_STREAM(t, rc, st, keys, (k_set_unique<32, RowKeys, RowValues>), hp, keys, rv, out_stored, cnt); break;
-    case 64: DOK_STREAM(t, rc, st, keys, (k_set_unique<64, RowKeys, RowValues>), hp, keys, rv, out_stored, cnt); break;
-    case 128: DOK_STREAM(t, rc, st, keys, (k_set_unique<128, RowKeys, RowValues>), hp, keys, rv, out_stored, cnt); break;
-    default:
-      DOK_FOR_WINDOWS(t, rc, (k_set_unique_wide<<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, rv, out_stored, cnt)));
-  }
+  DOK_DISPATCH_SB(t, DOK_FOR_WINDOWS(t, rc, (k_set_unique<SB><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, rv, out_stored, (ll_t *)counters))));
   return rc;
 }
 
@@ -534,39 +435,7 @@ inline int launch_set_unique(const DevTable &t, const DevHash &hp, const RowKeys
 // REMOVE = 1: the tag is swapped to the tombstone by CAS so that equal uuids in one batch report exactly once
 // (ClosedHashmap::remove, closed_hashmap_impl_class.cu:459-484, stores it non-atomically).
 template <int SB, int REMOVE, class Keys>
-__global__ void __launch_bounds__(DOK_TPB, 4) k_find(DevTable t, DevHash hp, Keys keys, uint8_t *__restrict__ out_flags,
-                                                     ll_t *counters) {
-  __shared__ BlockTally tally;
-  __shared__ WarpQueue queues[DOK_WARPS];
-  dok_tally_begin(tally);
-  WarpQueue &queue = queues[threadIdx.x >> 5];
-  WarpShare share = dok_share(keys.total());
-  LaneRow lr = DOK_IDLE_LANE;
-  int hits = 0;
-  for (;;) {
-    dok_fill_queue(queue, share, t, hp, keys, AdmitAll());
-    if (!dok_refill(queue, share, lr, t)) break;
-    unsigned m, me, tb;
-    dok_pass<SB, 1, false>(t, lr, m, me, tb, NoLines());
-    if (lr.busy()) {
-      const unsigned pos = me ? (unsigned)__ffs(me) - 1 : 0;
-      const unsigned slot = lr.group * (128 / SB) + pos * 32 / SB;
-      if (me || !dok_next_group<unsigned>(lr.group, lr.word, (unsigned)t.n_groups)) {
-        int hit = (m >> pos) & 1u;
-        if (REMOVE && hit) hit = dok_cas_tag(t, slot, lr.uuid, DOK_REMOVED) == lr.uuid;
-        if (out_flags) out_flags[keys.elem(share.first + lr.row)] = (uint8_t)hit;
-        hits += hit;
-        lr.done();
-      }
-    }
-  }
-  dok_tally_sum(tally, DOK_CNT_HITS, hits);
-  dok_tally_flush(tally, counters, nullptr);
-}
-
-// The same for slots wider than a line: one row per thread.
-template <int REMOVE, class Keys>
-__global__ void __launch_bounds__(DOK_TPB) k_find_wide(DevTable t, DevHash hp, Keys keys, uint8_t *__restrict__ out_flags,
+__global__ void __launch_bounds__(DOK_TPB) k_find(DevTable t, DevHash hp, Keys keys, uint8_t *__restrict__ out_flags,
                                                   ll_t *counters) {
   __shared__ BlockTally tally;
   if (keys.idle()) return;
@@ -576,7 +445,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_find_wide(DevTable t, DevHash hp, K
   KeyHash kh{0, 0};
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
-  const Located loc = dok_locate<0, 1, false>(t, kh, e, active, nullptr, NoEmit());
+  const Located loc = dok_locate<SB, 1, false>(t, kh, e, active, nullptr, NoEmit());
   int hit = active && loc.found >= 0;
   if (REMOVE && hit) hit = dok_cas_tag(t, loc.found, kh.uuid, DOK_REMOVED) == kh.uuid;
   if (active && out_flags) out_flags[e] = (uint8_t)hit;
@@ -589,15 +458,9 @@ __global__ void __launch_bounds__(DOK_TPB) k_find_wide(DevTable t, DevHash hp, K
 template <int REMOVE, class Keys>
 inline int launch_find(const DevTable &t, const DevHash &hp, const Keys &keys, uint8_t *out_flags, int64_t *counters,
                        cudaStream_t st) {
+  const dim3 grid = dok_grid(keys);
   int rc = DOK_OK;
-  ll_t *cnt = (ll_t *)counters;
-  switch (t.sb) {
-    case 32: DOK_STREAM(t, rc, st, keys, (k_find<32, REMOVE, Keys>), hp, keys, out_flags, cnt); break;
-    case 64: DOK_STREAM(t, rc, st, keys, (k_find<64, REMOVE, Keys>), hp, keys, out_flags, cnt); break;
-    case 128: DOK_STREAM(t, rc, st, keys, (k_find<128, REMOVE, Keys>), hp, keys, out_flags, cnt); break;
-    default:
-      DOK_FOR_WINDOWS(t, rc, (k_find_wide<REMOVE><<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, out_flags, cnt)));
-  }
+  DOK_DISPATCH_SB(t, DOK_FOR_WINDOWS(t, rc, (k_find<SB, REMOVE><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, out_flags, (ll_t *)counters))));
   return rc;
 }
 

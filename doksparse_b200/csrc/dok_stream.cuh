@@ -16,7 +16,7 @@
 #define DOK_WARPS (DOK_TPB / 32)
 #define DOK_NONE 0xffffffffu
 
-struct WarpQueue { ulonglong2 entry[DOK_QUEUE]; };      // uuid | group, stride - 1 (6 bits), row of the share (26 bits)
+struct WarpQueue { ulonglong2 entry[DOK_QUEUE]; };      // uuid | group, row of the share (26 bits), stride - 1 (6 bits)
 
 // What a lane works on.  row (of the warp's share) == DOK_NONE: nothing; its uuid then matches no tag, and the group it
 // reads is the one of its last row (or group 0).
@@ -28,10 +28,10 @@ struct LaneRow {
 };
 #define DOK_IDLE_LANE LaneRow{-4, 0, 0, DOK_NONE}
 
-// A warp's share of the batch (of the block's slice), handed out 32 rows at a time from its end to its beginning: when rows
-// with equal keys meet in one warp, the later one, whose value stays, comes first.
+// A warp's share of the batch (of the block's slice): one range of rows.  (Every warp taking each so-many-th piece of 32
+// rows, so that the grid works on neighbouring rows, was 3 % slower.)
 struct WarpShare {
-  unsigned first, left;                  // rows first .. first + left - 1 are still to be hashed
+  unsigned first, rows, next;            // range; row of it that is hashed next
   unsigned head, waiting;                // queue position, entries
 };
 
@@ -42,31 +42,28 @@ __device__ __forceinline__ WarpShare dok_share(ll_t total) {
   ll_t first = w * per, end = first + per;
   if (end > total) end = total;
   if (first > end) first = end;
-  return WarpShare{(unsigned)first, (unsigned)(end - first), 0, 0};
+  return WarpShare{(unsigned)first, (unsigned)(end - first), 0, 0, 0};
 }
 
-// Fills the queue until 32 rows wait or the share is used up.  `admit(row, KeyHash, enter)` may keep a row out of it.
-template <class Keys, class Admit>
-__device__ __forceinline__ void dok_fill_queue(WarpQueue &q, WarpShare &s, const DevTable &t, const DevHash &hp, const Keys &keys,
-                                               const Admit &admit) {
+// Fills the queue until 32 rows wait or the share is used up.
+template <class Keys>
+__device__ __forceinline__ void dok_fill_queue(WarpQueue &q, WarpShare &s, const DevTable &t, const DevHash &hp, const Keys &keys) {
   const unsigned lane = threadIdx.x & 31u;
-  while (s.waiting < 32 && s.left > 0) {
-    const unsigned take = s.left < 32 ? s.left : 32;
-    s.left -= take;
-    const unsigned row = s.left + lane;
+  while (s.waiting < 32 && s.next < s.rows) {
+    const unsigned k = s.next + lane;
+    s.next += 32;
     KeyHash kh{0, 0};
-    bool enter = lane < take;
+    bool enter = k < s.rows;
     if (enter) {
-      kh = keys.hash(hp, keys.elem(s.first + row));
+      kh = keys.hash(hp, keys.elem(s.first + k));
       enter = dok_in_window(t, kh, true);
     }
-    enter = admit(s.first + row, kh, enter);
     const unsigned votes = __ballot_sync(0xffffffffu, enter);
     if (enter) {
       const ull_t h = dok_chain_hash(kh);
       const unsigned group = __umulhi((unsigned)(h >> 32), (unsigned)t.n_groups);
       const unsigned at = (s.head + s.waiting + __popc(votes & ((1u << lane) - 1u))) & (DOK_QUEUE - 1);
-      q.entry[at] = make_ulonglong2((ull_t)kh.uuid, (ull_t)group << 32 | (row << 6 | ((unsigned)h & 63u)));
+      q.entry[at] = make_ulonglong2((ull_t)kh.uuid, (ull_t)group << 32 | (k << 6 | ((unsigned)h & 63u)));
     }
     s.waiting += __popc(votes);
   }
@@ -92,42 +89,48 @@ __device__ __forceinline__ bool dok_refill(const WarpQueue &q, WarpShare &s, Lan
   return n < 32 || taken > 0;
 }
 
-// One group for each lane.  m / me / tb: match, match-or-empty and tombstone bits of the lane's own group by LANE of the quad:
-// the slot at lane position p of a group is p * 32 / SB.  `seen(words of the quad's four lines, match and empty votes of the
-// warp for each of the four keys, me)` runs on all lanes while they hold the lines.
-template <int SB, int LW, bool TOMB, class Seen>
-__device__ __forceinline__ void dok_pass(const DevTable &t, const LaneRow &lr, unsigned &m, unsigned &me, unsigned &tb, const Seen &seen) {
+// One group for each lane: four requests, each for the lines of a quad's key in its turn.
+template <int LW>
+struct Lines { ull_t w[4][LW]; };
+template <int LW>
+__device__ __forceinline__ void dok_request(const DevTable &t, const LaneRow &lr, Lines<LW> &f) {
+  const char *my_base = t.slots + 32 * (threadIdx.x & 3u);
+#pragma unroll
+  for (unsigned r = 0; r < 4; r++)
+    dok_load_words<LW>(my_base + (ull_t)__shfl_sync(0xffffffffu, lr.group, (threadIdx.x & 28u) + r) * 128u, f.w[r]);
+}
+
+// m / me: match and match-or-empty bits of the lane's own group by LANE of the quad (the slot at lane position p of a group
+// is p * 32 / SB); match, empty: the votes of the warp for each of the quads' four keys.
+template <int SB, int LW>
+__device__ __forceinline__ void dok_inspect(const LaneRow &lr, const Lines<LW> &f, unsigned &m, unsigned &me, unsigned (&match)[4],
+                                            unsigned (&empty)[4]) {
   constexpr unsigned FULL = 0xffffffffu;
   const unsigned l = threadIdx.x & 3u, base = threadIdx.x & 28u;
   const bool has_tag = ((32u * l) % SB) == 0;
-  const char *my_base = t.slots + 32 * l;
-  ull_t w[4][LW];
-#pragma unroll
-  for (unsigned r = 0; r < 4; r++)
-    dok_load_words<LW>(my_base + (ull_t)__shfl_sync(FULL, lr.group, base + r) * 128u, w[r]);
-  unsigned match[4], empty[4], own_m = 0, own_e = 0, own_t = 0;
+  unsigned own_m = 0, own_e = 0;
 #pragma unroll
   for (unsigned r = 0; r < 4; r++) {
-    const ll_t uuid_r = __shfl_sync(FULL, lr.uuid, base + r), tag = (ll_t)w[r][0];
+    const ll_t uuid_r = __shfl_sync(FULL, lr.uuid, base + r), tag = (ll_t)f.w[r][0];
     match[r] = __ballot_sync(FULL, has_tag && tag == uuid_r);
     empty[r] = __ballot_sync(FULL, has_tag && tag == DOK_EMPTY);
     if (l == r) { own_m = match[r]; own_e = empty[r]; }
-    if (TOMB) {
-      const unsigned tombs = __ballot_sync(FULL, has_tag && tag == DOK_REMOVED);
-      if (l == r) own_t = tombs;
-    }
   }
   m = (own_m >> base) & 0xfu;
   me = ((own_m | own_e) >> base) & 0xfu;
-  tb = TOMB ? (own_t >> base) & 0xfu : 0u;
-  seen(w, match, empty, me);
 }
 
-struct NoLines {
-  template <int LW>
-  __device__ __forceinline__ void operator()(const ull_t (&)[4][LW], const unsigned (&)[4], const unsigned (&)[4], unsigned) const {}
-};
-struct AdmitAll {
-  __device__ __forceinline__ bool operator()(unsigned, const KeyHash &, bool enter) const { return enter; }
-};
-
+// The loop.  `step(lane's row, lines, share)` inspects the lines, lets the row go to its next group (dok_next_group) or ends
+// it (done()).
+template <int LW, class Keys, class Step>
+__device__ __forceinline__ void dok_walk_share(WarpQueue &queue, const DevTable &t, const DevHash &hp, const Keys &keys, const Step &step) {
+  WarpShare share = dok_share(keys.total());
+  LaneRow lr = DOK_IDLE_LANE;
+  Lines<LW> lines;
+  for (;;) {
+    dok_fill_queue(queue, share, t, hp, keys);
+    if (!dok_refill(queue, share, lr, t)) break;
+    dok_request<LW>(t, lr, lines);
+    step(lr, lines, share);
+  }
+}

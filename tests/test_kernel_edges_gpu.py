@@ -155,3 +155,23 @@ def test_dense_round_trip(dtype, shape, density):
     assert torch.equal(t.to_dense(), dense) and torch.equal(t.to_sparse_coo().to_dense(), dense)
     if len(shape) > 1:
         assert torch.equal(t.transpose(0, 1).to_dense(), dense.transpose(0, 1))
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 257, 148 * 3 * 256 - 1, 148 * 4 * 256 + 33, 400_003])
+@pytest.mark.parametrize("key_cols,value_dtype,value_cols", [(1, torch.float32, 4), (4, torch.float32, 1), (3, torch.int64, 4), (1, torch.uint8, 11),
+                                                             (8, torch.float16, 3), (2, torch.float64, 12)])
+def test_lookups_over_warp_shares(n, key_cols, value_dtype, value_cols):
+    """Slots of 32, 64 and 128 bytes, values in and beyond the word behind the tag; one row per lane, and many."""
+    from doksparse_b200 import CudaClosedHashmap
+    np.random.seed(4)
+    stored = 50_000
+    table = CudaClosedHashmap(n_buckets=60_000, rehash_threshold=0.9)
+    of = lambda c: torch.stack([c * (2 * j + 3) + 10 ** 6 * j for j in range(key_cols)], dim=1).contiguous()
+    all_values = torch.randint(0, 200, (stored, value_cols), device="cuda").to(value_dtype)
+    table.set(of(torch.arange(stored, device="cuda")), all_values, assume_unique=True)
+    query = torch.randint(0, 2 * stored, (n,), device="cuda")
+    values, found = table.get(of(query))
+    assert torch.equal(found, query < stored)
+    assert torch.equal(values[found], all_values[query[found]]) and not values[~found].any()
+    values, _ = table.get(of(query), fallback_value=7)
+    assert (values[~found] == 7).all() and torch.equal(values[found], all_values[query[found]])
