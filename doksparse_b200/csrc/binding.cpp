@@ -150,10 +150,12 @@ PyObject *plan_set(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
                  "dok_map_set_unique"))
         return nullptr;
     } else {
-      at::Tensor scratch = at::empty({n + 1}, on_device(self, at::kLong));
-      if (!check(dok_map_set(&table, &self->hash, keys->data_ptr(), values->data_ptr(), n, (int64_t *)scratch.data_ptr(), epoch, nullptr,
-                             self->state + STATE_SET, stream),
-                 "dok_map_set"))
+      const int64_t words = dok_set_scratch_words(&table, n);
+      at::Tensor scratch;
+      if (words > 0) scratch = at::empty({words}, on_device(self, at::kLong));
+      if (!check(dok_map_set_with(&table, &self->hash, keys->data_ptr(), values->data_ptr(), n,
+                                  words > 0 ? (int64_t *)scratch.data_ptr() : nullptr, words, epoch, self->state + STATE_SET, stream),
+                 "dok_map_set_with"))
         return nullptr;
     }
     return PyLong_FromLongLong(n);
@@ -473,9 +475,11 @@ PyObject *plan_assign(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
       values = at::full({}, value, on_device(self, self->value_type)).expand(s.shape);
     }
     if (s.n > 0) {
-      at::Tensor scratch = at::empty({s.n + 1}, on_device(self, at::kLong));
-      if (!check(dok_dok_assign(&table, &self->hash, &s.sel, values.data_ptr(), values.strides().data(), (int64_t *)scratch.data_ptr(),
-                                epoch, self->state + STATE_SET, self->state + STATE_ADJUST,
+      const int64_t words = dok_set_scratch_words(&table, s.n);
+      at::Tensor scratch;
+      if (words > 0) scratch = at::empty({words}, on_device(self, at::kLong));
+      if (!check(dok_dok_assign(&table, &self->hash, &s.sel, values.data_ptr(), values.strides().data(),
+                                words > 0 ? (int64_t *)scratch.data_ptr() : nullptr, words, epoch, self->state + STATE_SET, self->state + STATE_ADJUST,
                                 c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()),
                  "dok_dok_assign"))
         return nullptr;

@@ -354,18 +354,22 @@ int dok_dok_zero_items(const dok_table *t, const dok_hash_params *hp, const dok_
 int dok_dok_set_dense(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel, const void *src,
                       const int64_t *src_strides, int64_t *slot_scratch, int64_t epoch, int64_t *counters,
                       void *stream) {
-  return dok_dok_assign(t, hp, sel, src, src_strides, slot_scratch, epoch, counters, nullptr, stream);
+  if (!slot_scratch) return DOK_BAD_ARG;
+  int64_t n = 1;
+  for (int j = 0; sel && j < sel->selector_ndim && j < DOK_MAX_SELECTOR_NDIM; j++) n *= sel->sizes[j];
+  return dok_dok_assign(t, hp, sel, src, src_strides, slot_scratch, n + 1, epoch, counters, nullptr, stream);
 }
 
 int dok_dok_assign(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel, const void *src,
-                   const int64_t *src_strides, int64_t *slot_scratch, int64_t epoch, int64_t *counters, int64_t *more,
-                   void *stream) {
+                   const int64_t *src_strides, int64_t *scratch, int64_t scratch_words, int64_t epoch, int64_t *counters,
+                   int64_t *more, void *stream) {
   DevHash dh;
   DevTable dt;
   SelKeys sk;
   if (!prepare(t, hp, &dt, &dh) || !make_sel(sel, dh, &sk)) return DOK_BAD_ARG;
   if (sk.n == 0) return DOK_OK;
-  if (!src || !src_strides || !slot_scratch || !dok_has_stamps(dt) || epoch < 1 || epoch > DOK_MAX_EPOCH) return DOK_BAD_ARG;
+  if (!dok_set_is_small(dt, sk.n) && (!scratch || scratch_words < sk.n + 1)) return DOK_BAD_ARG;
+  if (!src || !src_strides || !dok_has_stamps(dt) || epoch < 1 || epoch > DOK_MAX_EPOCH) return DOK_BAD_ARG;
   StridedValues sv;
   sv.src = (const char *)src;
   sv.selector_ndim = sel->selector_ndim;
@@ -373,7 +377,7 @@ int dok_dok_assign(const dok_table *t, const dok_hash_params *hp, const dok_sele
     sv.sizes[j] = j < sel->selector_ndim ? sel->sizes[j] : 1;
     sv.strides[j] = j < sel->selector_ndim ? src_strides[j] : 0;
   }
-  return launch_set_general(dt, dh, sk, sv, slot_scratch, epoch, nullptr, counters, (cudaStream_t)stream, more);
+  return launch_set_general(dt, dh, sk, sv, scratch, epoch, nullptr, counters, (cudaStream_t)stream, more, scratch_words);
 }
 
 int dok_dok_gather_insert(const dok_table *src, const dok_hash_params *src_hp, const dok_selectors *sel,

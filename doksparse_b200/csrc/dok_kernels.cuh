@@ -8,6 +8,7 @@
 //
 // No thread of a warp returns early: the cooperative walk needs all 32 lanes.
 #pragma once
+#include <cooperative_groups.h>
 #include <type_traits>
 #include "dok_stream.cuh"
 
@@ -227,6 +228,21 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_set_unique(DevTable t, DevHash h
 // such a slot was claimed by this batch.
 #define DOK_STAMP_CONFLICT 1ULL
 #define DOK_STAMP_FRESH 2ULL
+// Filter of the slots with a conflict (by 22 bits of a product of the slot index, so a set bit may be another slot's): a
+// batch of millions of rows with some repetitions would otherwise read a stamp at random for every row in the second and
+// third kernel, 151 us of a 4 M-row assignment; 512 KB that stay in L2 answer for most rows.
+#define DOK_FILTER_BITS 22
+#define DOK_FILTER_WORDS (1 << (DOK_FILTER_BITS - 6))                       // int64 words behind slot_out[n]
+#define DOK_FILTER_FROM 65536                                               // rows; below, clearing it costs more
+__device__ __forceinline__ unsigned dok_filter_bit(ll_t slot) { return ((unsigned)slot * 0x9e3779b1u) >> (32 - DOK_FILTER_BITS); }
+__device__ __forceinline__ void dok_filter_set(unsigned *filter, ll_t slot) {
+  const unsigned b = dok_filter_bit(slot);
+  if (filter) atomicOr(filter + (b >> 5), 1u << (b & 31u));
+}
+__device__ __forceinline__ bool dok_filter_has(const unsigned *filter, ll_t slot) {
+  const unsigned b = dok_filter_bit(slot);
+  return !filter || ((__ldcg(filter + (b >> 5)) >> (b & 31u)) & 1u);
+}
 #define DOK_ROW_FRESH (1LL << 62)      // bit of a row's slot index: this row claimed the slot
 __device__ __forceinline__ ull_t dok_stamp(ll_t epoch, ll_t row) { return ((ull_t)epoch << 34) | ((ull_t)row << 2); }
 
@@ -280,7 +296,7 @@ __device__ __forceinline__ Twins dok_find_twins(BlockTwins &b, const KeyHash &kh
 // launch); the second kernel then lets the slot's last row rewrite it.
 template <int SB, class Keys, class Values>
 __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp, Keys keys, Values values,
-                                                       ll_t *__restrict__ slot_out, ll_t epoch, int mark_fresh,
+                                                       ll_t *__restrict__ slot_out, unsigned *filter, ll_t epoch, int mark_fresh,
                                                        uint8_t *__restrict__ out_stored, ll_t *counters) {
   __shared__ BlockTally tally;
   __shared__ BlockTwins twins;
@@ -306,6 +322,7 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
       const ull_t old = atomicMax((ull_t *)stamp, dok_stamp(epoch, e));
       if ((old >> 34) == (ull_t)epoch || (mark_fresh && same.more)) {
         atomicOr((ull_t *)stamp, DOK_STAMP_CONFLICT);
+        dok_filter_set(filter, slot);
         conflict = 1;
       }
     } else {
@@ -347,7 +364,7 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
 // every first-kernel write has completed, so rows cannot tear and the last row wins.
 template <class Keys, class Values>
 __global__ void __launch_bounds__(DOK_TPB) k_set_resolve(DevTable t, DevHash hp, Keys keys, Values values,
-                                                         const ll_t *__restrict__ slot_in, ll_t epoch) {
+                                                         const ll_t *__restrict__ slot_in, const unsigned *filter, ll_t epoch) {
   if (slot_in[keys.count()] == 0) return;        // the first kernel met no duplicate: every row is already in place
   if (keys.idle()) return;
   // a few blocks per SM stride over the rows: the usual launch has nothing to do, and a grid of one block per 256
@@ -364,6 +381,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_set_resolve(DevTable t, DevHash hp,
       const ll_t g = slot / t.spg;
       if (g < t.win_lo || g >= t.win_hi) continue;
     }
+    if (!dok_filter_has(filter, slot)) continue;
     const ull_t stamp = (ull_t)__ldcg(dok_stamp_ptr(t, slot));
     if (!(stamp & DOK_STAMP_CONFLICT)) continue;
     if (fresh) atomicOr((ull_t *)dok_stamp_ptr(t, slot), DOK_STAMP_FRESH);
@@ -377,7 +395,8 @@ __global__ void __launch_bounds__(DOK_TPB) k_set_resolve(DevTable t, DevHash hp,
 // other rows of the slots that the batch claimed, and rows that found the table full.  Counting the stored keys in a pass
 // of its own before the set, as the reference does, costs a walk per row: 145 of the 800 us of a 4 M-row assignment.
 template <class Keys>
-__global__ void __launch_bounds__(DOK_TPB) k_set_count(DevTable t, Keys keys, const ll_t *__restrict__ slot_in, ll_t epoch,
+__global__ void __launch_bounds__(DOK_TPB) k_set_count(DevTable t, Keys keys, const ll_t *__restrict__ slot_in,
+                                                       const unsigned *filter, ll_t epoch,
                                                        ll_t *__restrict__ more) {
   if (slot_in[keys.count()] == 0) return;
   const ll_t span = keys.span(), stride = (ll_t)gridDim.x * DOK_TPB;
@@ -387,36 +406,123 @@ __global__ void __launch_bounds__(DOK_TPB) k_set_count(DevTable t, Keys keys, co
     if (!keys.at(j, e)) continue;
     const ll_t slot = slot_in[e];
     if (slot < 0) { c++; continue; }
-    if (slot & DOK_ROW_FRESH) continue;
+    if ((slot & DOK_ROW_FRESH) || !dok_filter_has(filter, slot)) continue;      // a slot with several rows has a conflict
     const ull_t stamp = (ull_t)__ldcg(dok_stamp_ptr(t, slot));
     c += (stamp >> 34) == (ull_t)epoch && (stamp & DOK_STAMP_FRESH) != 0;
   }
   dok_warp_add(more, c);
 }
 
+// The general set of a batch that one cluster holds, one row per thread: the three kernels above as three phases of one
+// launch.  Such a batch is all latency: a set of 400 rows was a clearing of the scratch, two or three launches and an
+// allocation, 16 us of which the table took 4.  The barrier is the cluster's (up to 8 blocks of 1024 threads), and slots
+// stay in registers, so there is no scratch.
+#define DOK_SMALL_SET_TPB 1024
+#define DOK_SMALL_SET_ROWS (8 * DOK_SMALL_SET_TPB)
+
+template <int SB, class Keys, class Values>
+__global__ void __launch_bounds__(DOK_SMALL_SET_TPB) k_set_small(DevTable t, DevHash hp, Keys keys, Values values, ll_t epoch,
+                                                                 ll_t *counters, ll_t *more) {
+  __shared__ BlockTally tally;
+  dok_tally_begin(tally);
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const ll_t e = (ll_t)blockIdx.x * DOK_SMALL_SET_TPB + threadIdx.x;
+  const bool active = e < keys.count();
+  KeyHash kh{0, 0};
+  if (active) kh = keys.hash(hp, e);
+  int outcome = -1, dup = 0, again = 0;
+  const ll_t slot = dok_find_or_claim<SB>(t, kh, active, &outcome);
+  const bool placed = active && slot >= 0, fresh = outcome == DOK_OUT_CLAIMED_EMPTY || outcome == DOK_OUT_REUSED;
+  ull_t *stamp = placed ? (ull_t *)dok_stamp_ptr(t, slot) : nullptr;
+  if (placed) {
+    dok_write_row(t, hp, keys, values, e, slot, fresh || hp.dtype >= DOK_F16);
+    if ((atomicMax(stamp, dok_stamp(epoch, e)) >> 34) == (ull_t)epoch) {
+      atomicOr(stamp, DOK_STAMP_CONFLICT);
+      dup = 1;
+    }
+  }
+  cluster.sync();
+  if (placed) {
+    const ull_t now = __ldcg(stamp);
+    if (now & DOK_STAMP_CONFLICT) {
+      if (more && fresh) atomicOr(stamp, DOK_STAMP_FRESH);
+      if ((now & ~DOK_STAMP_FRESH) == (dok_stamp(epoch, e) | DOK_STAMP_CONFLICT)) dok_write_row(t, hp, keys, values, e, slot, true);
+    }
+  }
+  if (more) {                                             // uniform over the launch
+    cluster.sync();
+    if (placed && !fresh) {
+      const ull_t now = __ldcg(stamp);
+      again = (now >> 34) == (ull_t)epoch && (now & DOK_STAMP_FRESH) != 0;
+    } else {
+      again = active && !placed;
+    }
+  }
+  dok_tally_add(tally, DOK_TALLY_EXTRA, again);
+  if (counters) {
+    dok_tally_add(tally, DOK_CNT_CLAIMED_EMPTY, outcome == DOK_OUT_CLAIMED_EMPTY);
+    dok_tally_add(tally, DOK_CNT_REUSED_REMOVED, outcome == DOK_OUT_REUSED);
+    dok_tally_add(tally, DOK_CNT_FAILED, outcome == DOK_OUT_FAILED);
+    dok_tally_add(tally, DOK_CNT_HITS, outcome == DOK_OUT_FOUND);
+    dok_tally_add(tally, DOK_CNT_DUPLICATES, dup);
+  }
+  dok_tally_flush(tally, counters, more);
+}
+
+template <int SB, class Keys, class Values>
+inline int launch_set_small(const DevTable &t, const DevHash &hp, const Keys &keys, const Values &values, ll_t epoch, ll_t *counters,
+                            ll_t *more, cudaStream_t st) {
+  unsigned blocks = 1;
+  while ((ll_t)blocks * DOK_SMALL_SET_TPB < keys.n) blocks *= 2;
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = blocks;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(blocks);
+  config.blockDim = dim3(DOK_SMALL_SET_TPB);
+  config.stream = st;
+  config.attrs = &cluster;
+  config.numAttrs = 1;
+  cudaLaunchKernelEx(&config, k_set_small<SB, Keys, Values>, t, hp, keys, values, epoch, counters, more);
+  return dok_check_launch();
+}
+
+inline bool dok_is_sliced(const RowKeys &k) { return k.slice_rows != 0; }
+inline bool dok_is_sliced(const SelKeys &) { return false; }
+inline bool dok_set_is_small(const DevTable &t, ll_t n) { return n <= DOK_SMALL_SET_ROWS && dok_window_passes(t) == 1; }
+
 // contiguous value rows [n, value_bytes]
 template <class Keys, class Values>
 inline int launch_set_general(const DevTable &t, const DevHash &hp, const Keys &keys, const Values &values,
                               int64_t *slot_scratch, int64_t epoch, uint8_t *out_stored, int64_t *counters, cudaStream_t st,
-                              int64_t *more = nullptr) {
-  if (cudaMemsetAsync(slot_scratch + keys.n, 0, sizeof(int64_t), st) != cudaSuccess) return dok_check_launch();
+                              int64_t *more = nullptr, int64_t scratch_words = 0) {
+  if (!out_stored && !dok_is_sliced(keys) && dok_set_is_small(t, keys.n)) {
+    int rc = DOK_OK;
+    DOK_DISPATCH_SB(t, (rc = launch_set_small<SB>(t, hp, keys, values, (ll_t)epoch, (ll_t *)counters, (ll_t *)more, st)));
+    return rc;
+  }
+  const bool filtered = keys.n >= DOK_FILTER_FROM && scratch_words >= keys.n + 1 + DOK_FILTER_WORDS;
+  unsigned *filter = filtered ? (unsigned *)(slot_scratch + keys.n + 1) : nullptr;
+  const size_t zeroed = sizeof(int64_t) * (filtered ? 1 + DOK_FILTER_WORDS : 1);
+  if (cudaMemsetAsync(slot_scratch + keys.n, 0, zeroed, st) != cudaSuccess) return dok_check_launch();
   const dim3 grid = dok_grid(keys);
   int rc = DOK_OK;
-  DOK_DISPATCH_SB(t, DOK_FOR_WINDOWS(t, rc, (k_set_claim<SB><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, (ll_t *)slot_scratch,
+  DOK_DISPATCH_SB(t, DOK_FOR_WINDOWS(t, rc, (k_set_claim<SB><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, (ll_t *)slot_scratch, filter,
                                                                                        (ll_t)epoch, more != nullptr, out_stored, (ll_t *)counters))));
   if (rc != DOK_OK) return rc;
   dim3 few = grid;
   if (few.x > 148 * 8) few.x = 148 * 8;
-  DOK_FOR_WINDOWS(t, rc, (k_set_resolve<<<few, DOK_TPB, 0, st>>>(wt, hp, keys, values, (const ll_t *)slot_scratch, (ll_t)epoch)));
+  DOK_FOR_WINDOWS(t, rc, (k_set_resolve<<<few, DOK_TPB, 0, st>>>(wt, hp, keys, values, (const ll_t *)slot_scratch, filter, (ll_t)epoch)));
   if (rc != DOK_OK || more == nullptr) return rc;
-  k_set_count<<<few, DOK_TPB, 0, st>>>(t, keys, (const ll_t *)slot_scratch, (ll_t)epoch, (ll_t *)more);
+  k_set_count<<<few, DOK_TPB, 0, st>>>(t, keys, (const ll_t *)slot_scratch, filter, (ll_t)epoch, (ll_t *)more);
   return dok_check_launch();
 }
 
 inline int launch_set(const DevTable &t, const DevHash &hp, const RowKeys &keys, const char *values, int64_t *slot_scratch,
-                      int64_t epoch, uint8_t *out_stored, int64_t *counters, cudaStream_t st) {
+                      int64_t epoch, uint8_t *out_stored, int64_t *counters, cudaStream_t st, int64_t scratch_words = 0) {
   RowValues rv{values};
-  return launch_set_general(t, hp, keys, rv, slot_scratch, epoch, out_stored, counters, st);
+  return launch_set_general(t, hp, keys, rv, slot_scratch, epoch, out_stored, counters, st, nullptr, scratch_words);
 }
 
 inline int launch_set_unique(const DevTable &t, const DevHash &hp, const RowKeys &keys, const char *values,

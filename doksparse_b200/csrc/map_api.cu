@@ -94,6 +94,25 @@ int dok_map_set(const dok_table *t, const dok_hash_params *hp, const void *keys,
   return launch_set(dt, dh, rk, (const char *)values, slot_scratch, epoch, out_stored, counters, (cudaStream_t)stream);
 }
 
+int64_t dok_set_scratch_words(const dok_table *t, int64_t n) {
+  DevTable dt;
+  if (!dok_make_table(t, &dt) || n < 0 || n > DOK_MAX_BATCH) return -1;
+  if (dok_set_is_small(dt, n)) return 0;
+  return n + 1 + (n >= DOK_FILTER_FROM ? DOK_FILTER_WORDS : 0);
+}
+
+int dok_map_set_with(const dok_table *t, const dok_hash_params *hp, const void *keys, const void *values, int64_t n,
+                     int64_t *scratch, int64_t scratch_words, int64_t epoch, int64_t *counters, void *stream) {
+  DevHash dh;
+  DevTable dt;
+  if (!prepare(t, hp, &dt, &dh) || n < 0 || n > DOK_MAX_BATCH) return DOK_BAD_ARG;
+  if (n == 0) return DOK_OK;
+  if (!keys || !values || !dok_has_stamps(dt) || epoch < 1 || epoch > DOK_MAX_EPOCH) return DOK_BAD_ARG;
+  if (!dok_set_is_small(dt, n) && (!scratch || scratch_words < n + 1)) return DOK_BAD_ARG;
+  RowKeys rk{keys, n};
+  return launch_set(dt, dh, rk, (const char *)values, scratch, epoch, nullptr, counters, (cudaStream_t)stream, scratch_words);
+}
+
 int dok_map_remove(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n, uint8_t *out_removed,
                    int64_t *counters, void *stream) {
   DevHash dh;

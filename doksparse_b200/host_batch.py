@@ -44,6 +44,7 @@ class HostBatch:
             self.s_in, self.s_run, self.s_out = (torch.cuda.Stream() for _ in range(3))
         self._rings = {}
         self._takes_outputs = hasattr(table, "_slots")      # a plain map writes straight into the staging buffers
+        self._staged_set_rows = 0                           # of set chunks whose kernels are not enqueued yet
         self.begin()
 
     # ------------------------------------------------------------------ stream plumbing
@@ -92,9 +93,22 @@ class HostBatch:
     # ------------------------------------------------------------------ chunk programs
     # A chunk is (inputs, body): inputs = [(tag, pinned host slice)], body(device views) runs on the kernel stream and
     # returns (pairs, rings) for the copy-out: [(host slice, device tensor)], [(ring, index)] of result buffers.
-    def _chunks(self, n):
-        for lo in range(0, n, self.chunk_rows):
-            yield lo, min(n, lo + self.chunk_rows)
+    # On a plain map a batch goes in at least four pieces: a batch of one piece is copied in, worked on and copied out one
+    # after the other.  A piece costs some 80 us of host time, which 2^18 rows hide.
+    def _chunks(self, n, divisible=True):
+        rows = self.chunk_rows
+        if divisible and self._takes_outputs:
+            rows = min(rows, max(1 << 18, -(-n // 4)))
+        for lo in range(0, n, rows):
+            yield lo, min(n, lo + rows)
+
+    def _set_is_divisible(self, keys_host):
+        """Whether the pieces of a set leave the table as the whole would: where it might have to grow, the size it grows
+        to depends on the batch that makes it grow."""
+        if not self._takes_outputs or self.table._slots is None or keys_host.dtype.is_floating_point:
+            return False
+        rows = self._staged_set_rows + keys_host.shape[0]
+        return self.table._element_bound() + rows <= int(self.table._rehash_threshold * self.table.n_buckets)
 
     def _get_chunks(self, keys_host, out_values_host, out_found_host, fallback_value=None):
         vr = self._ring("ov", out_values_host.shape[1:], out_values_host.dtype)
@@ -114,10 +128,12 @@ class HostBatch:
             yield [("k", keys_host[lo:hi])], body
 
     def _set_chunks(self, keys_host, values_host, assume_unique=False):
-        for lo, hi in self._chunks(keys_host.shape[0]):
+        for lo, hi in self._chunks(keys_host.shape[0], self._set_is_divisible(keys_host)):
             def body(keys, values):
                 self.table.set(keys, values, assume_unique=assume_unique)
+                self._staged_set_rows -= keys.shape[0]
                 return [], []
+            self._staged_set_rows += hi - lo
             yield [("k", keys_host[lo:hi]), ("v", values_host[lo:hi])], body
 
     def _remove_chunks(self, keys_host, out_flags_host=None):

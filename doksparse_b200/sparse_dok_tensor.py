@@ -412,11 +412,12 @@ class SparseDOKTensor(object):
         sel = _selectors_struct(selectors)
         src_strides = (ctypes.c_int64 * L.MAX_SELECTOR_NDIM)(*src.stride())
         epoch = hashmap._next_epoch()
-        scratch = torch.empty(n_sel + 1, device=self.device, dtype=torch.long)
+        words = L.lib().dok_set_scratch_words(hashmap._c_table(), n_sel)
+        scratch = torch.empty(words, device=self.device, dtype=torch.long)
         with L.on(self.device):
             # n_elements grows by the selected positions that were not stored; duplicates over-count, like the reference (:474)
             L.check(L.lib().dok_dok_assign(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(src),
-                                           src_strides, L.ptr(scratch), epoch, hashmap._counter_block(M._BY_SET),
+                                           src_strides, L.ptr(scratch), words, epoch, hashmap._counter_block(M._BY_SET),
                                            hashmap._counter_block(M._ADJUST), L.stream_ptr(self.device)), "dok_dok_assign")
         hashmap._after_mutation(n_sel)
 

@@ -204,6 +204,12 @@ int64_t dok_static_scratch_max_rows(void);
 int dok_map_count_new_static(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n,
                              int64_t *counters, void *stream);
 
+/* dok_map_set with as much scratch as it can use: dok_set_scratch_words(t, n) int64 words (0: none), at least n + 1
+ * otherwise.  Without flags per row. */
+int64_t dok_set_scratch_words(const dok_table *t, int64_t n);
+int dok_map_set_with(const dok_table *t, const dok_hash_params *hp, const void *keys, const void *values, int64_t n,
+                     int64_t *scratch, int64_t scratch_words, int64_t epoch, int64_t *counters, void *stream);
+
 /* The same for keys whose identity is the row, as the reference counts every key type (:363): distinct absent ROWS, by
  * value (float keys, where the value cast gives different rows one uuid; a row with a NaN counts each time). */
 int dok_map_count_new_rows(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n,
@@ -280,9 +286,9 @@ int dok_dok_set_dense(const dok_table *t, const dok_hash_params *hp, const dok_s
                       int64_t *counters, void *stream);
 /* The same with the reference's element count (sparse_dok_tensor_impl.py:461-474), which adds every selected position that
  * was not stored before, repetitions included: the sum of counters[CLAIMED_EMPTY], counters[REUSED_REMOVED] and *more
- * (device, ADDED to) grows by that number.  more may be NULL. */
+ * (device, ADDED to) grows by that number.  more may be NULL; scratch as for dok_map_set_with. */
 int dok_dok_assign(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel,
-                   const void *src, const int64_t *src_strides, int64_t *slot_scratch, int64_t epoch,
+                   const void *src, const int64_t *src_strides, int64_t *scratch, int64_t scratch_words, int64_t epoch,
                    int64_t *counters, int64_t *more, void *stream);
 
 /* Value of every stored element to its position of a dense row-major tensor of the given sizes (HOST int64[key_size]; one

@@ -175,3 +175,15 @@ def test_lookups_over_warp_shares(n, key_cols, value_dtype, value_cols):
     assert torch.equal(values[found], all_values[query[found]]) and not values[~found].any()
     values, _ = table.get(of(query), fallback_value=7)
     assert (values[~found] == 7).all() and torch.equal(values[found], all_values[query[found]])
+
+
+@pytest.mark.parametrize("n", [1, 2, 1024, 1025, 2049, 8192, 8193, 65535, 65537, 200_001])
+@pytest.mark.parametrize("value_cols", [2, 4, 31])              # stamps in the slot, in an array of their own, slots wider than a line
+def test_sets_with_repeated_keys(n, value_cols):
+    """One cluster up to 8192 rows, two kernels beyond; a filter of the conflicts from 65536 rows on."""
+    pair = Pair(seed=n, n_buckets=1 << 19, **params(1))
+    rng = np.random.default_rng(n)
+    for spread in (3 * n + 1, n // 50 + 1):
+        keys = rng.integers(0, spread, (n, 1))
+        pair.set(keys, rng.standard_normal((n, value_cols)))
+        pair.get(keys)
