@@ -211,14 +211,14 @@ PyObject *plan_read(Plan *self, PyObject *) {
   });
 }
 
-// count_new(keys, word, exact): adds the number of distinct new keys to the counter `word`; exact: sets it, and answers
+// count_new(keys, word, exact, empty table): adds the number of distinct new keys to the counter `word`; exact: sets it, and answers
 // the counters
 PyObject *plan_count_new(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
   return guarded([&]() -> PyObject * {
-    if (nargs != 3) { PyErr_SetString(PyExc_TypeError, "count_new takes 3 arguments"); return nullptr; }
+    if (nargs != 4) { PyErr_SetString(PyExc_TypeError, "count_new takes 4 arguments"); return nullptr; }
     const at::Tensor *keys = tensor_of(args[0]);
     const long word = PyLong_AsLong(args[1]);
-    const int exact = PyObject_IsTrue(args[2]);
+    const int exact = PyObject_IsTrue(args[2]), empty = PyObject_IsTrue(args[3]);
     if (PyErr_Occurred()) return nullptr;
     if (!keys || word < 0 || word >= STATE_WORDS || !rows_match(*keys, self->device, self->key_type, self->key_ndim, self->key_shape)) {
       PyErr_SetString(PyExc_ValueError, "count_new: not a batch of this table");
@@ -230,7 +230,7 @@ PyObject *plan_count_new(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
     at::Tensor scratch = at::empty({2 * n}, on_device(self, at::kLong));
     if (exact) C10_CUDA_CHECK(cudaMemsetAsync(self->state + word, 0, sizeof(int64_t), stream.stream()));
     const auto count = at::isFloatingType(self->key_type) ? dok_map_count_new_rows : dok_map_count_new;
-    if (!check(count(&self->table, &self->hash, keys->data_ptr(), n, (int64_t *)scratch.data_ptr(), 2 * n, self->state + word, stream.stream()),
+    if (!check(count(empty ? nullptr : &self->table, &self->hash, keys->data_ptr(), n, (int64_t *)scratch.data_ptr(), 2 * n, self->state + word, stream.stream()),
                "dok_map_count_new"))
       return nullptr;
     if (exact) return read_state(self, stream);

@@ -188,6 +188,7 @@ struct RowKeys {          // contiguous [n, ks] rows of the key dtype (closed_ha
     e = (ll_t)blockIdx.y * slice_rows + j;
     return j < slice_rows && j < slice_counts[blockIdx.y];
   }
+  __device__ __forceinline__ bool row(ll_t &e, unsigned block) const { return at((ll_t)block * DOK_TPB + threadIdx.x, e); }
   // the same for position j of the batch (of slice blockIdx.y), for kernels that stride over the rows
   __device__ __forceinline__ bool at(ll_t j, ll_t &e) const {
     if (slice_rows == 0) { e = j; return j < n; }
@@ -206,10 +207,11 @@ struct RowKeys {          // contiguous [n, ks] rows of the key dtype (closed_ha
     return slice_rows == 0 ? (ll_t)row : (ll_t)blockIdx.y * slice_rows + row;
   }
   // block-uniform: nothing for this block to do
-  __device__ __forceinline__ bool idle() const {
+  __device__ __forceinline__ bool idle() const { return idle(blockIdx.x); }
+  __device__ __forceinline__ bool idle(unsigned block) const {
     if (slice_rows == 0) return false;
     if (abort != nullptr && *abort != 0) return true;
-    return (ll_t)blockIdx.x * DOK_TPB >= slice_counts[blockIdx.y];
+    return (ll_t)block * DOK_TPB >= slice_counts[blockIdx.y];
   }
   // get_uuid of the reference (closed_hashmap_impl_class.cu:98-107) and the chain-decorrelating product, in one
   // pass over the key
@@ -253,7 +255,8 @@ struct SelKeys {
   __device__ __forceinline__ ll_t span() const { return n; }
   __device__ __forceinline__ ll_t total() const { return n; }
   __device__ __forceinline__ ll_t elem(unsigned row) const { return (ll_t)row; }
-  __device__ __forceinline__ bool idle() const { return false; }
+  __device__ __forceinline__ bool idle(unsigned = 0) const { return false; }
+  __device__ __forceinline__ bool row(ll_t &e, unsigned block) const { return at((ll_t)block * DOK_TPB + threadIdx.x, e); }
   __device__ __forceinline__ ll_t index(int d, ll_t off) const { return s.ptr[d] ? s.ptr[d][off] : s.base[d] + off; }
   // element offsets of batch element e into each of the ndim index tensors (fully unrolled over the
   // maximum ndim with predication, so `off` stays in registers)

@@ -300,16 +300,18 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
                                                        uint8_t *__restrict__ out_stored, ll_t *counters) {
   __shared__ BlockTally tally;
   __shared__ BlockTwins twins;
-  if (keys.idle()) return;
+  // from the end of the batch to its beginning, see below
+  const unsigned block = gridDim.x - 1 - blockIdx.x;
+  if (keys.idle(block)) return;
   dok_tally_begin(tally);
   ll_t e;
-  bool active = keys.row(e);
+  bool active = keys.row(e, block);
   KeyHash kh{0, 0};
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
   const Twins same = dok_find_twins(twins, kh, active);
   const bool last = active && same.last == (int)threadIdx.x;
-  int outcome = -1, conflict = 0;
+  int outcome = -1, conflict = 0, dup = 0;
   ll_t slot = dok_find_or_claim<SB>(t, kh, last, &outcome);
   if (last) {
     const bool fresh = outcome == DOK_OUT_CLAIMED_EMPTY || outcome == DOK_OUT_REUSED;
@@ -317,13 +319,21 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
     if (slot >= 0) {
       // the row is stored without waiting for the stamp's answer: the two requests travel together.  If the slot
       // turns out to be shared, whatever the racing stores left is rewritten by the second kernel.
-      ll_t *stamp = dok_stamp_ptr(t, slot);
-      dok_write_row(t, hp, keys, values, e, slot, fresh || hp.dtype >= DOK_F16);
-      const ull_t old = atomicMax((ull_t *)stamp, dok_stamp(epoch, e));
-      if ((old >> 34) == (ull_t)epoch || (mark_fresh && same.more)) {
-        atomicOr((ull_t *)stamp, DOK_STAMP_CONFLICT);
+      ull_t *stamp = (ull_t *)dok_stamp_ptr(t, slot);
+      // A key that the block holds several times is probably all over the batch.  If a later row has already stamped its
+      // slot -- blocks start from the batch's end, so one has unless it is still running -- this row has nothing to write,
+      // and a line that most of the blocks want is read, not written: writes to one line come 140 ns apart.
+      ull_t old = same.more && !fresh ? __ldcg(stamp) : 0;
+      const bool over = old > (dok_stamp(epoch, e) | 3);
+      dup = over;
+      if (!over) {
+        dok_write_row(t, hp, keys, values, e, slot, fresh || hp.dtype >= DOK_F16);
+        old = atomicMax(stamp, dok_stamp(epoch, e));
+      }
+      if (over ? mark_fresh && !(old & DOK_STAMP_CONFLICT) : (old >> 34) == (ull_t)epoch || (mark_fresh && same.more)) {
+        atomicOr(stamp, DOK_STAMP_CONFLICT);
         dok_filter_set(filter, slot);
-        conflict = 1;
+        conflict = dup = 1;
       }
     } else {
       conflict = mark_fresh;          // a row without a place is counted by k_set_count too
@@ -354,7 +364,7 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
     dok_tally_add(tally, DOK_CNT_REUSED_REMOVED, outcome == DOK_OUT_REUSED);
     dok_tally_add(tally, DOK_CNT_FAILED, outcome == DOK_OUT_FAILED);
     dok_tally_add(tally, DOK_CNT_HITS, twin || outcome == DOK_OUT_FOUND);
-    dok_tally_add(tally, DOK_CNT_DUPLICATES, twin || (conflict && slot >= 0));
+    dok_tally_add(tally, DOK_CNT_DUPLICATES, twin || dup);
   }
   dok_tally_flush(tally, counters, slot_out + keys.count());
 }
@@ -587,7 +597,8 @@ __global__ void __launch_bounds__(DOK_TPB) k_count_new(DevTable t, DevHash hp, K
   KeyHash kh{0, 0};
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
-  const Located loc = dok_locate<SB, 1, false>(t, kh, e, active, nullptr, NoEmit());
+  Located loc{-1, -1, -1};
+  if (t.n_groups > 0) loc = dok_locate<SB, 1, false>(t, kh, e, active, nullptr, NoEmit());      // (0: no table, every row is absent)
   int claimed = 0;
   if (active && loc.found < 0) {
     const ll_t uuid = kh.uuid;
@@ -662,12 +673,20 @@ __global__ void __launch_bounds__(DOK_TPB) k_reinsert(DevTable src, DevTable dst
 // init / uuid
 // ---------------------------------------------------------------------------------------------------------
 
+__device__ __forceinline__ void dok_store_sector(char *p, ll_t first) {
+  asm volatile("st.global.v4.u64 [%0], {%1, %2, %2, %2};" ::"l"(p), "l"(first), "l"(0LL) : "memory");
+}
+
 static __global__ void k_init(DevTable t, ll_t *state, int state_words) {
   const ll_t stride = (ll_t)gridDim.x * blockDim.x;
   if (blockIdx.x == 0 && threadIdx.x < state_words) state[threadIdx.x] = 0;
+  // whole 32-byte sectors, so that none of them has to be read to be completed: 2^21 64-byte slots 22 -> 14 us
+  const int stamp_sector = t.stamp_off & ~31;
   for (ll_t i = (ll_t)blockIdx.x * blockDim.x + threadIdx.x; i < t.n_slots; i += stride) {
-    *dok_tag_ptr(t, i) = i < t.nb ? DOK_EMPTY : DOK_BLOCKED;
-    if (t.stamp_off >= 0 || t.stamp) *dok_stamp_ptr(t, i) = 0;
+    char *slot = dok_slot_ptr(t, i);
+    dok_store_sector(slot, i < t.nb ? DOK_EMPTY : DOK_BLOCKED);
+    if (t.stamp_off >= 32) dok_store_sector(slot + stamp_sector, 0);
+    if (t.stamp_off < 0 && t.stamp) t.stamp[i] = 0;
   }
 }
 

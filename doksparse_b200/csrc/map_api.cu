@@ -139,7 +139,8 @@ int dok_map_count_new(const dok_table *t, const dok_hash_params *hp, const void 
                       int64_t *scratch_tags, int64_t scratch_slots, int64_t *counters, void *stream) {
   DevHash dh;
   DevTable dt;
-  if (!prepare(t, hp, &dt, &dh) || n < 0 || n > DOK_MAX_BATCH) return DOK_BAD_ARG;
+  memset(&dt, 0, sizeof(dt));
+  if (!(t ? prepare(t, hp, &dt, &dh) : dok_make_hash(hp, &dh)) || n < 0 || n > DOK_MAX_BATCH) return DOK_BAD_ARG;
   if (n == 0) return DOK_OK;
   if (!keys || !scratch_tags || !counters || scratch_slots < 2 * n) return DOK_BAD_ARG;
   const ll_t blocks = (scratch_slots + 255) / 256;

@@ -65,7 +65,8 @@ __global__ void __launch_bounds__(DOK_TPB) k_count_new_rows(DevTable t, DevHash 
   KeyHash kh{0, 0};
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
-  const Located loc = dok_locate<SB, 1, false>(t, kh, e, active, nullptr, NoEmit());
+  Located loc{-1, -1, -1};
+  if (t.n_groups > 0) loc = dok_locate<SB, 1, false>(t, kh, e, active, nullptr, NoEmit());      // (0: no table, every row is absent)
   int claimed = 0;
   if (active && loc.found < 0) {
     bool nan = false;
@@ -207,13 +208,13 @@ __global__ void __launch_bounds__(DOK_SMALL_TPB) k_remove_unique_small(DevTable 
 // 64-bit sort, and rows of any number of columns at the price of one; a comparison sort of rows took 0.37 ms for 250 k
 // rows of three floats.  Digits that all rows share are skipped.
 #define DOK_SORT_TPB 256
-#define DOK_SORT_ITEMS 16
-#define DOK_SORT_TILE (DOK_SORT_TPB * DOK_SORT_ITEMS)
+#define DOK_SORT_ITEMS 16                  // per thread; a quarter where that leaves SMs without a tile
+#define DOK_SORT_SMALL_ITEMS 4
+#define DOK_SORT_SMALL (148LL * DOK_SORT_TPB * DOK_SORT_ITEMS)
 #define DOK_SORT_MAX_ROWS (1LL << 30)      // counts travel in 30 bits beside two flags
 #define DOK_SORT_SPINS (1 << 22)           // bound of every wait for another block; far beyond what one takes
 #define DOK_MAX_RUN 64                     // longest run of equal prefixes with different rows that one thread sorts
-#define DOK_UNIQUE_ROUNDS 4
-#define DOK_UNIQUE_TILE (DOK_TPB * DOK_UNIQUE_ROUNDS)
+#define DOK_UNIQUE_ROUNDS 4                // rows per thread of the removal; one of them for small batches, likewise
 
 // zeroed before the first kernel
 struct SortControl {
@@ -325,13 +326,15 @@ __global__ void __launch_bounds__(256) k_sort_plan(SortControl *c, unsigned n) {
 __device__ __forceinline__ unsigned dok_peek(const unsigned *p) { return *(const volatile unsigned *)p; }
 __device__ __forceinline__ void dok_post(unsigned *p, unsigned v) { *(volatile unsigned *)p = v; }
 
-// One digit.  A tile of 4096 (prefix, row) pairs is ranked by digit with warp votes, its digit counts are posted, the counts
+// One digit.  A tile of 4096 or 1024 (prefix, row) pairs is ranked by digit with warp votes, its digit counts are posted, the counts
 // of the tiles before it are summed up by looking back (tiles are handed out in order, so all of them have started), and
 // the pairs leave through shared memory in digit order, a run of the output at a time.
+template <int ITEMS>
 __global__ void __launch_bounds__(DOK_SORT_TPB) k_sort_pass(SortControl *c, int digit, unsigned n, unsigned *key_a, unsigned *row_a,
                                                             unsigned *key_b, unsigned *row_b, unsigned *look) {
+  constexpr int TILE = DOK_SORT_TPB * ITEMS;
   if (c->skip[digit]) return;
-  __shared__ unsigned keys[DOK_SORT_TILE], rows[DOK_SORT_TILE];
+  __shared__ unsigned keys[TILE], rows[TILE];
   __shared__ unsigned counts[DOK_SORT_TPB / 32][256];
   __shared__ unsigned start[256], shift_by[256], sums[8], tile_id;
   const bool b = c->from_b[digit];
@@ -342,17 +345,17 @@ __global__ void __launch_bounds__(DOK_SORT_TPB) k_sort_pass(SortControl *c, int 
   for (int i = tid; i < (DOK_SORT_TPB / 32) * 256; i += DOK_SORT_TPB) ((unsigned *)counts)[i] = 0;
   __syncthreads();
   const unsigned tile = tile_id;
-  const unsigned first = tile * DOK_SORT_TILE, size = min((unsigned)DOK_SORT_TILE, n - first);
-  unsigned key[DOK_SORT_ITEMS], row[DOK_SORT_ITEMS], rank[DOK_SORT_ITEMS];
+  const unsigned first = tile * TILE, size = min((unsigned)TILE, n - first);
+  unsigned key[ITEMS], row[ITEMS], rank[ITEMS];
 #pragma unroll
-  for (int k = 0; k < DOK_SORT_ITEMS; k++) {
-    const unsigned i = warp * 32 * DOK_SORT_ITEMS + k * 32 + lane;
+  for (int k = 0; k < ITEMS; k++) {
+    const unsigned i = warp * 32 * ITEMS + k * 32 + lane;
     key[k] = i < size ? key_in[first + i] : 0;
     row[k] = i < size ? row_in[first + i] : 0;
   }
 #pragma unroll
-  for (int k = 0; k < DOK_SORT_ITEMS; k++) {
-    const unsigned i = warp * 32 * DOK_SORT_ITEMS + k * 32 + lane;
+  for (int k = 0; k < ITEMS; k++) {
+    const unsigned i = warp * 32 * ITEMS + k * 32 + lane;
     const unsigned digit_of = i < size ? (key[k] >> shift) & 255u : 256u;
     const unsigned peers = __match_any_sync(0xffffffffu, digit_of);
     unsigned base = 0;
@@ -396,8 +399,8 @@ __global__ void __launch_bounds__(DOK_SORT_TPB) k_sort_pass(SortControl *c, int 
   shift_by[tid] = c->hist[digit][tid] + before - (v - total);
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < DOK_SORT_ITEMS; k++) {
-    const unsigned i = warp * 32 * DOK_SORT_ITEMS + k * 32 + lane;
+  for (int k = 0; k < ITEMS; k++) {
+    const unsigned i = warp * 32 * ITEMS + k * 32 + lane;
     if (i < size) {
       const unsigned d = (key[k] >> shift) & 255u, at = start[d] + counts[warp][d] + rank[k];
       keys[at] = key[k];
@@ -454,12 +457,12 @@ __global__ void __launch_bounds__(DOK_TPB) k_sort_ties(SortControl *c, RowKeys k
 
 // First row of each run of equal rows: looked up, its slot turned into a tombstone, its flag written at the run's number.
 // Runs are counted across tiles by looking back like in the sort, when the tile's own lookups are done.
-template <int SB>
+template <int SB, int ROUNDS>
 __global__ void __launch_bounds__(DOK_TPB) k_remove_unique(DevTable t, DevHash hp, RowKeys keys, SortControl *c, const unsigned *key_a,
                                                            const unsigned *row_a, const unsigned *key_b, const unsigned *row_b,
                                                            unsigned *look, unsigned tiles, uint8_t *__restrict__ out_removed,
                                                            ll_t *__restrict__ out_count, ll_t *counters) {
-  __shared__ unsigned sums[DOK_UNIQUE_ROUNDS][DOK_TPB / 32], tile_id, base_of_tile;
+  __shared__ unsigned sums[ROUNDS][DOK_TPB / 32], tile_id, base_of_tile;
   __shared__ int removed;
   const unsigned n = (unsigned)keys.n;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -472,11 +475,11 @@ __global__ void __launch_bounds__(DOK_TPB) k_remove_unique(DevTable t, DevHash h
   const unsigned tile = tile_id;
   const unsigned *key = c->final_b ? key_b : key_a, *row = c->final_b ? row_b : row_a;
   const bool whole = dok_prefix_is_row(c, hp.ks);
-  unsigned head_votes[DOK_UNIQUE_ROUNDS], flags = 0;
+  unsigned head_votes[ROUNDS], flags = 0;
   int hits = 0;
 #pragma unroll
-  for (int r = 0; r < DOK_UNIQUE_ROUNDS; r++) {
-    const unsigned i = tile * DOK_UNIQUE_TILE + r * DOK_TPB + tid;
+  for (int r = 0; r < ROUNDS; r++) {
+    const unsigned i = tile * (DOK_TPB * ROUNDS) + r * DOK_TPB + tid;
     bool head = i < n;
     const unsigned e = i < n ? row[i] : 0;
     if (head && i > 0 && key[i] == key[i - 1])
@@ -495,7 +498,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_remove_unique(DevTable t, DevHash h
   if (lane == 0 && hits) atomicAdd(&removed, hits);
   __syncthreads();
   unsigned total = 0;
-  for (int r = 0; r < DOK_UNIQUE_ROUNDS; r++) for (int w = 0; w < DOK_TPB / 32; w++) total += sums[r][w];
+  for (int r = 0; r < ROUNDS; r++) for (int w = 0; w < DOK_TPB / 32; w++) total += sums[r][w];
   if (warp == 0) {                                 // 32 predecessors at a time
     if (lane == 0) dok_post(look + tile, (tile == 0 ? DOK_LB_TOTAL : DOK_LB_LOCAL) | total);
     unsigned before = 0;
@@ -525,7 +528,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_remove_unique(DevTable t, DevHash h
   }
   __syncthreads();
   unsigned at = base_of_tile;
-  for (int r = 0; r < DOK_UNIQUE_ROUNDS; r++) {
+  for (int r = 0; r < ROUNDS; r++) {
     unsigned mine = at;
     for (int w = 0; w < DOK_TPB / 32; w++) {
       if (w < warp) mine += sums[r][w];
@@ -541,14 +544,17 @@ struct SortWork {
   unsigned *look, *unique_look, *key_a, *row_a, *key_b, *row_b;
   size_t zeroed, bytes;
   unsigned tiles, unique_tiles;
+  bool small;
 };
 
 static SortWork sort_work(void *base, ll_t n) {
   SortWork w;
   size_t at = 0;
   const auto take = [&](size_t bytes) { const size_t from = at; at += (bytes + 255) / 256 * 256; return (char *)base + from; };
-  w.tiles = (unsigned)((n + DOK_SORT_TILE - 1) / DOK_SORT_TILE);
-  w.unique_tiles = (unsigned)((n + DOK_UNIQUE_TILE - 1) / DOK_UNIQUE_TILE);
+  w.small = n < DOK_SORT_SMALL;
+  const ll_t tile = DOK_SORT_TPB * (w.small ? DOK_SORT_SMALL_ITEMS : DOK_SORT_ITEMS), unique_tile = DOK_TPB * (w.small ? 1 : DOK_UNIQUE_ROUNDS);
+  w.tiles = (unsigned)((n + tile - 1) / tile);
+  w.unique_tiles = (unsigned)((n + unique_tile - 1) / unique_tile);
   w.control = (SortControl *)take(sizeof(SortControl));
   w.look = (unsigned *)take((size_t)w.tiles * 256 * 4 * sizeof(unsigned));
   w.unique_look = (unsigned *)take((size_t)w.unique_tiles * sizeof(unsigned));
@@ -567,7 +573,8 @@ int dok_map_count_new_rows(const dok_table *t, const dok_hash_params *hp, const 
                            int64_t *scratch, int64_t scratch_slots, int64_t *counters, void *stream) {
   DevHash dh;
   DevTable dt;
-  if (!dok_make_hash(hp, &dh) || !dok_make_table(t, &dt) || dt.kb != dh.ks * dh.elem_bytes || n < 0 || n > DOK_MAX_BATCH) return DOK_BAD_ARG;
+  memset(&dt, 0, sizeof(dt));
+  if (!dok_make_hash(hp, &dh) || (t && (!dok_make_table(t, &dt) || dt.kb != dh.ks * dh.elem_bytes)) || n < 0 || n > DOK_MAX_BATCH) return DOK_BAD_ARG;
   if (n == 0) return DOK_OK;
   if (!keys || !scratch || !counters || scratch_slots < 2 * n) return DOK_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
@@ -611,17 +618,20 @@ int dok_map_remove_unique(const dok_table *t, const dok_hash_params *hp, const v
   k_sort_plan<<<1, 256, 0, st>>>(w.control, (unsigned)n);
   if ((rc = dok_check_launch()) != DOK_OK) return rc;
   for (int d = 0; d < 4; d++) {
-    k_sort_pass<<<w.tiles, DOK_SORT_TPB, 0, st>>>(w.control, d, (unsigned)n, w.key_a, w.row_a, w.key_b, w.row_b,
-                                                  w.look + (size_t)d * w.tiles * 256);
+    const auto pass = w.small ? k_sort_pass<DOK_SORT_SMALL_ITEMS> : k_sort_pass<DOK_SORT_ITEMS>;
+    pass<<<w.tiles, DOK_SORT_TPB, 0, st>>>(w.control, d, (unsigned)n, w.key_a, w.row_a, w.key_b, w.row_b,
+                                           w.look + (size_t)d * w.tiles * 256);
     if ((rc = dok_check_launch()) != DOK_OK) return rc;
   }
   k_sort_ties<true><<<grid, DOK_TPB, 0, st>>>(w.control, rk, dh.dtype, dh.ks, w.key_a, w.row_a, w.key_b, w.row_b);
   if ((rc = dok_check_launch()) != DOK_OK) return rc;
   k_sort_ties<false><<<grid < 148 ? grid : 148, DOK_TPB, 0, st>>>(w.control, rk, dh.dtype, dh.ks, w.key_a, w.row_a, w.key_b, w.row_b);
   if ((rc = dok_check_launch()) != DOK_OK) return rc;
-  DOK_DISPATCH_SB(dt, (k_remove_unique<SB><<<w.unique_tiles, DOK_TPB, 0, st>>>(dt, dh, rk, w.control, w.key_a, w.row_a, w.key_b, w.row_b,
-                                                                               w.unique_look, w.unique_tiles, out_removed,
-                                                                               (ll_t *)out_count, (ll_t *)counters)));
+  const auto remove = [&](auto kernel) {
+    kernel<<<w.unique_tiles, DOK_TPB, 0, st>>>(dt, dh, rk, w.control, w.key_a, w.row_a, w.key_b, w.row_b, w.unique_look, w.unique_tiles,
+                                               out_removed, (ll_t *)out_count, (ll_t *)counters);
+  };
+  DOK_DISPATCH_SB(dt, (w.small ? remove(k_remove_unique<SB, 1>) : remove(k_remove_unique<SB, DOK_UNIQUE_ROUNDS>)));
   return dok_check_launch();
 }
 

@@ -698,11 +698,11 @@ class CudaClosedHashmap:
         if self._room_for(n, limit) or self.n_elements + n <= limit:
             # whatever the number of new keys is, the reference would not rehash: insert and count on the device
             if row_counted:
-                plan.count_new(new_keys, _BY_ROWS, False)
+                plan.count_new(new_keys, _BY_ROWS, False, self._shared.bound == 0)
             self._launch_set(new_keys, new_values, assume_unique)
             self._after_mutation(n)
             return
-        state = plan.count_new(new_keys, _COUNTED_NEW, True)
+        state = plan.count_new(new_keys, _COUNTED_NEW, True, self._shared.bound == 0)
         n_elements, live = self._sizes(state)[:2]
         n_new = state[_COUNTED_NEW]
         if n_elements + n_new > limit:

@@ -204,6 +204,8 @@ int64_t dok_static_scratch_max_rows(void);
 int dok_map_count_new_static(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n,
                              int64_t *counters, void *stream);
 
+/* Both counts take t == NULL for a table that is known to hold nothing. */
+
 /* dok_map_set with as much scratch as it can use: dok_set_scratch_words(t, n) int64 words (0: none), at least n + 1
  * otherwise.  Without flags per row. */
 int64_t dok_set_scratch_words(const dok_table *t, int64_t n);
