@@ -37,7 +37,7 @@ struct DevHash {
   int ks;                       // key elements per row
   int dtype;                    // dok_dtype of the key rows
   int elem_bytes;               // bytes of one key element
-  int pad_;
+  int in_order;                 // key_perm is the identity
   ll_t a[DOK_MAX_KEY_SIZE];     // alpha2[key_perm[i]]   -- second hash: the uuid (key identity)
   ll_t b[DOK_MAX_KEY_SIZE];     // beta2[key_perm[i]]
   ull_t p[DOK_MAX_KEY_SIZE];    // |prime2[key_perm[i]]|  (>= 2)
@@ -165,6 +165,17 @@ __device__ __forceinline__ int dok_owner_shard(ll_t uuid, int n_shards) {
   return (int)__umul64hi(dok_mix64((ull_t)uuid ^ DOK_SHARD_SALT), (ull_t)n_shards);
 }
 
+// `n` 8-byte words word(0), word(1), ... to `off` bytes (a multiple of 8) behind a slot's start, which is 32-byte aligned:
+// two at a time wherever that is 16-byte aligned.  Every store instruction to a table beyond L2 costs a request per lane,
+// so a 40-byte value goes in three instead of five.
+template <class Word>
+__device__ __forceinline__ void dok_store_words(char *slot, int off, int n, const Word &word) {
+  int i = 0;
+  if ((off & 8) && n > 0) { *(ull_t *)(slot + off) = word(0); i = 1; }
+  for (; i + 1 < n; i += 2) *(ulonglong2 *)(slot + off + 8 * i) = make_ulonglong2(word(i), word(i + 1));
+  if (i < n) *(ull_t *)(slot + off + 8 * i) = word(i);
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // Key sources.  A key source yields, for batch element e, the uuid of its key and can write the key's raw
 // bytes into a table key row.  Keys are never held in a register array (key_size is a run-time value):
@@ -232,8 +243,16 @@ struct RowKeys {          // contiguous [n, ks] rows of the key dtype (closed_ha
     return KeyHash{dok_llabs(u), (ll_t)h};
   }
   // set_key_permuted (closed_hashmap_impl_class.cu:144-150): storage column perm[i] <- key element i
-  __device__ __forceinline__ void store_key(const DevHash &hp, ll_t e, char *dst_row) const {
+  __device__ __forceinline__ void store_key(const DevTable &t, const DevHash &hp, ll_t e, char *slot) const {
     const char *src = (const char *)keys + e * (ll_t)hp.ks * hp.elem_bytes;
+    char *dst_row = slot + t.key_off;
+    if (hp.in_order && hp.elem_bytes >= 4) {
+      if (hp.elem_bytes == 8) { dok_store_words(slot, t.key_off, hp.ks, [&](int i) { return ((const ull_t *)src)[i]; }); return; }
+      const unsigned *s4 = (const unsigned *)src;
+      dok_store_words(slot, t.key_off, hp.ks >> 1, [&](int i) { return (ull_t)s4[2 * i] | (ull_t)s4[2 * i + 1] << 32; });
+      if (hp.ks & 1) ((unsigned *)dst_row)[hp.ks - 1] = s4[hp.ks - 1];
+      return;
+    }
     switch (hp.elem_bytes) {
       case 8: for (int i = 0; i < hp.ks; i++) ((ll_t *)dst_row)[hp.perm[i]] = ((const ll_t *)src)[i]; break;
       case 4: for (int i = 0; i < hp.ks; i++) ((int *)dst_row)[hp.perm[i]] = ((const int *)src)[i]; break;
@@ -288,9 +307,18 @@ struct SelKeys {
       }
     return KeyHash{dok_llabs(u), (ll_t)h};
   }
-  __device__ __forceinline__ void store_key(const DevHash &hp, ll_t e, char *dst_row) const {
+  __device__ __forceinline__ void store_key(const DevTable &t, const DevHash &hp, ll_t e, char *slot) const {
     ll_t off[DOK_MAX_KEY_SIZE];
     offsets(e, off);
+    char *dst_row = slot + t.key_off;
+    if (hp.in_order && (t.key_off & 8) == 0) {
+#pragma unroll
+      for (int d = 0; d < DOK_MAX_KEY_SIZE; d += 2) {
+        if (d + 1 < s.ndim) *(longlong2 *)(dst_row + 8 * d) = make_longlong2(index(d, off[d]), index(d + 1, off[d + 1]));
+        else if (d < s.ndim) *(ll_t *)(dst_row + 8 * d) = index(d, off[d]);
+      }
+      return;
+    }
 #pragma unroll
     for (int d = 0; d < DOK_MAX_KEY_SIZE; d++)
       if (d < s.ndim) ((ll_t *)dst_row)[hp.perm[d]] = index(d, off[d]);
@@ -597,20 +625,20 @@ __device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHa
 
 // value row (vb bytes at `src`, alignment of the widest power of two dividing vb, capped at 8) -> slot
 __device__ __forceinline__ void dok_store_value(const DevTable &t, ll_t slot, const char *src) {
-  ull_t *dst = (ull_t *)dok_value_ptr(t, slot);
-  if (t.vb == 8) { *dst = *(const ull_t *)src; return; }
+  char *dst = dok_value_ptr(t, slot);
+  if (t.vb == 8) { *(ull_t *)dst = *(const ull_t *)src; return; }
   if (t.vb == 4) { *(unsigned *)dst = *(const unsigned *)src; return; }
   if ((t.vb & 7) == 0) {
-    for (int w = 0; w < t.vwords; w++) dst[w] = ((const ull_t *)src)[w];
+    dok_store_words(dok_slot_ptr(t, slot), t.val_off, t.vwords, [&](int i) { return ((const ull_t *)src)[i]; });
   } else if ((t.vb & 3) == 0) {
-    unsigned *d32 = (unsigned *)dst;
-    for (int w = 0; w < (t.vb >> 2); w++) d32[w] = ((const unsigned *)src)[w];
+    const unsigned *s4 = (const unsigned *)src;
+    dok_store_words(dok_slot_ptr(t, slot), t.val_off, t.vb >> 3, [&](int i) { return (ull_t)s4[2 * i] | (ull_t)s4[2 * i + 1] << 32; });
+    ((unsigned *)dst)[(t.vb >> 2) - 1] = s4[(t.vb >> 2) - 1];
   } else if ((t.vb & 1) == 0) {
     unsigned short *d16 = (unsigned short *)dst;
     for (int w = 0; w < (t.vb >> 1); w++) d16[w] = ((const unsigned short *)src)[w];
   } else {
-    char *d8 = (char *)dst;
-    for (int w = 0; w < t.vb; w++) d8[w] = src[w];
+    for (int w = 0; w < t.vb; w++) dst[w] = src[w];
   }
 }
 

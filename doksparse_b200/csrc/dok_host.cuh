@@ -56,6 +56,7 @@ inline bool dok_make_hash(const dok_hash_params *hp, DevHash *out) {
   out->dtype = hp->key_dtype;
   out->elem_bytes = eb;
   unsigned seen = 0;
+  out->in_order = 1;
   for (int i = 0; i < hp->key_size; i++) {
     const int c = hp->key_perm[i];
     if (c < 0 || c >= hp->key_size || (seen >> c) & 1u) return false;
@@ -70,6 +71,7 @@ inline bool dok_make_hash(const dok_hash_params *hp, DevHash *out) {
     out->a1[i] = hp->alpha1[c] | 1;     // odd: the linear term is then injective in the key element
     out->b1[i] = hp->beta1[c];
     out->perm[i] = c;
+    if (c != i) out->in_order = 0;
   }
   return true;
 }

@@ -191,7 +191,7 @@ inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, vo
 template <class Keys, class Values>
 __device__ __forceinline__ void dok_write_row(const DevTable &t, const DevHash &hp, const Keys &keys, const Values &values,
                                               ll_t e, ll_t slot, bool with_key) {
-  if (with_key) keys.store_key(hp, e, dok_key_row(t, slot));
+  if (with_key) keys.store_key(t, hp, e, dok_slot_ptr(t, slot));
   dok_store_value(t, slot, values.row(t, e));
 }
 
