@@ -147,7 +147,7 @@ def _declare(lib):
 
 
 EXPORTED = None
-_plan_type = None
+_native = None
 
 
 def lib():
@@ -164,18 +164,18 @@ def lib():
     return _lib
 
 
-def plan_type():
-    """Plan of the _native module, which is built with the library: the hot calls on one table, without the ctypes way."""
-    global _plan_type
-    if _plan_type is None:
+def native():
+    """The _native module, which is built with the library: the hot calls on one table, without the ctypes way."""
+    global _native
+    if _native is None:
         lib()
         try:
-            from ._native import Plan
+            from . import _native as module
         except ImportError as e:
             raise DokError(f"doksparse_b200._native cannot be loaded ({e}): build it with "
                            "`python -c 'import doksparse_b200.build as b; b.build()'`") from e
-        _plan_type = Plan
-    return _plan_type
+        _native = module
+    return _native
 
 
 def check(status, what):

@@ -34,6 +34,7 @@ struct Plan {
 enum { STATE_SET = 0, STATE_REMOVE = 8, STATE_BULK = 24, STATE_ADJUST = 7, STATE_WORDS = 32 };   // int64 offsets of the counter blocks
 
 PyObject *dok_error = nullptr;
+extern PyTypeObject plan_type;
 
 // -> true, or sets DokError with the wording of the ctypes path
 bool check(int status, const char *what) {
@@ -100,6 +101,154 @@ int plan_init(Plan *self, PyObject *args, PyObject *) {
   self->key_type = reinterpret_cast<THPDtype *>(key_type)->scalar_type;
   self->value_type = reinterpret_cast<THPDtype *>(value_type)->scalar_type;
   return 0;
+}
+
+// allocate(device index, buckets, key shape, key dtype, value shape, value dtype, state tensor or None) ->
+// (plan without hash parameters, slots, state, layout): a new slot array with empty tags and zero counters
+PyObject *plan_allocate(PyObject *, PyObject *args) {
+  return guarded([&]() -> PyObject * {
+    int device;
+    long long buckets;
+    PyObject *key_shape, *key_type, *value_shape, *value_type, *given_state;
+    if (!PyArg_ParseTuple(args, "iLOOOOO", &device, &buckets, &key_shape, &key_type, &value_shape, &value_type, &given_state)) return nullptr;
+    Plan *p = PyObject_New(Plan, &plan_type);
+    if (!p) return nullptr;
+    struct Drop { Plan *p; ~Drop() { Py_XDECREF((PyObject *)p); } } drop{p};
+    memset(&p->table, 0, sizeof(p->table));
+    memset(&p->hash, 0, sizeof(p->hash));
+    p->device = device;
+    p->key_ndim = shape_from(key_shape, p->key_shape);
+    p->value_ndim = shape_from(value_shape, p->value_shape);
+    if (p->key_ndim < 0 || p->value_ndim < 0 || !THPDtype_Check(key_type) || !THPDtype_Check(value_type)) {
+      if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "allocate: bad arguments");
+      return nullptr;
+    }
+    p->key_type = reinterpret_cast<THPDtype *>(key_type)->scalar_type;
+    p->value_type = reinterpret_cast<THPDtype *>(value_type)->scalar_type;
+    int64_t key_bytes = c10::elementSize(p->key_type), value_bytes = c10::elementSize(p->value_type);
+    for (int i = 0; i < p->key_ndim; i++) key_bytes *= p->key_shape[i];
+    for (int i = 0; i < p->value_ndim; i++) value_bytes *= p->value_shape[i];
+    dok_layout_info lay;
+    if (!check(dok_table_layout((int)value_bytes, (int)key_bytes, buckets, &lay), "dok_table_layout")) return nullptr;
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+    at::Tensor slots = at::empty({lay.total_bytes}, on_device(p, at::kByte));
+    const at::Tensor *given = tensor_of(given_state);
+    at::Tensor state = given ? *given : at::empty({STATE_WORDS}, on_device(p, at::kLong));
+    p->table.slots = slots.data_ptr();
+    p->table.n_buckets = buckets;
+    p->table.slot_bytes = lay.slot_bytes;
+    p->table.value_bytes = (int32_t)value_bytes;
+    p->table.key_bytes = (int32_t)key_bytes;
+    p->state = (int64_t *)state.data_ptr();
+    if (!check(dok_map_init_state(&p->table, p->state, STATE_WORDS, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream()),
+               "dok_map_init_state"))
+      return nullptr;
+    drop.p = nullptr;
+    return Py_BuildValue("(NNN(iiiiiLL))", (PyObject *)p, THPVariable_Wrap(std::move(slots)), THPVariable_Wrap(std::move(state)), lay.slot_bytes,
+                         lay.slots_per_group, lay.value_offset, lay.key_offset, lay.stamp_offset, (long long)lay.n_slots,
+                         (long long)lay.total_bytes);
+  });
+}
+
+// set_hash(dtype code, alpha2, beta2, prime2, alpha1, beta1, prime1, key_perm): lists of one integer per key element
+PyObject *plan_set_hash(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
+  if (nargs != 8) { PyErr_SetString(PyExc_TypeError, "set_hash takes 8 arguments"); return nullptr; }
+  self->hash.key_dtype = (int32_t)PyLong_AsLong(args[0]);
+  const Py_ssize_t n = PyList_Check(args[1]) ? PyList_GET_SIZE(args[1]) : 0;
+  int64_t *to[6] = {self->hash.alpha2, self->hash.beta2, self->hash.prime2, self->hash.alpha1, self->hash.beta1, self->hash.prime1};
+  for (int k = 1; k < 8; k++) {
+    if (!PyList_Check(args[k]) || PyList_GET_SIZE(args[k]) != n || n < 1 || n > DOK_MAX_KEY_SIZE) {
+      PyErr_SetString(PyExc_ValueError, "set_hash: one value per key element");
+      return nullptr;
+    }
+    for (Py_ssize_t i = 0; i < n; i++) {
+      const long long v = PyLong_AsLongLong(PyList_GET_ITEM(args[k], i));
+      if (k < 7) to[k - 1][i] = v; else self->hash.key_perm[i] = (int32_t)v;
+    }
+  }
+  if (PyErr_Occurred()) return nullptr;
+  self->hash.key_size = (int32_t)n;
+  Py_RETURN_NONE;
+}
+
+// ---- counts that travel to the host by themselves -----------------------------------------------------------
+
+// Eight landing places for copies of a table's counters, in pinned memory that the caller provides, with an event each.
+struct Ring {
+  PyObject_HEAD
+  PyObject *memory;            // keeps the pinned words alive
+  int64_t *words;
+  int device;
+  cudaEvent_t events[8];
+  unsigned used;
+};
+
+// Ring(pinned int64 tensor of 8 * STATE_WORDS, device index)
+int ring_init(Ring *self, PyObject *args, PyObject *) {
+  PyObject *memory;
+  if (!PyArg_ParseTuple(args, "Oi", &memory, &self->device)) return -1;
+  const at::Tensor *t = tensor_of(memory);
+  if (!t || t->scalar_type() != at::kLong || t->numel() != 8 * STATE_WORDS || !t->is_contiguous()) {
+    PyErr_SetString(PyExc_ValueError, "Ring: pinned words expected");
+    return -1;
+  }
+  Py_INCREF(memory);
+  self->memory = memory;
+  self->words = (int64_t *)t->data_ptr();
+  return 0;
+}
+void ring_dealloc(Ring *self) {
+  for (int i = 0; i < 8; i++) if (self->events[i]) cudaEventDestroy(self->events[i]);
+  Py_XDECREF(self->memory);
+  Py_TYPE(self)->tp_free((PyObject *)self);
+}
+
+// copy(plan, place): enqueues a copy of the plan's counters
+PyObject *ring_copy(Ring *self, PyObject *const *args, Py_ssize_t nargs) {
+  return guarded([&]() -> PyObject * {
+    if (nargs != 2 || Py_TYPE(args[0]) != &plan_type) { PyErr_SetString(PyExc_TypeError, "copy takes a Plan and a place"); return nullptr; }
+    const Plan *plan = (const Plan *)args[0];
+    const long i = PyLong_AsLong(args[1]);
+    if (i < 0 || i > 7 || plan->device != self->device) { PyErr_SetString(PyExc_ValueError, "copy: no such place"); return nullptr; }
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
+    const auto stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device);
+    if (!self->events[i]) C10_CUDA_CHECK(cudaEventCreateWithFlags(&self->events[i], cudaEventDisableTiming));
+    C10_CUDA_CHECK(cudaMemcpyAsync(self->words + i * STATE_WORDS, plan->state, STATE_WORDS * sizeof(int64_t), cudaMemcpyDeviceToHost, stream.stream()));
+    C10_CUDA_CHECK(cudaEventRecord(self->events[i], stream.stream()));
+    self->used |= 1u << i;
+    Py_RETURN_NONE;
+  });
+}
+// landed(place) -> bool
+PyObject *ring_landed(Ring *self, PyObject *arg) {
+  return guarded([&]() -> PyObject * {
+    const long i = PyLong_AsLong(arg);
+    if (i < 0 || i > 7 || !self->events[i]) { PyErr_SetString(PyExc_ValueError, "landed: no such copy"); return nullptr; }
+    const cudaError_t e = cudaEventQuery(self->events[i]);
+    if (e == cudaErrorNotReady) { (void)cudaGetLastError(); Py_RETURN_FALSE; }
+    C10_CUDA_CHECK(e);
+    Py_RETURN_TRUE;
+  });
+}
+// wait(place), or wait(-1) for every copy so far
+PyObject *ring_wait(Ring *self, PyObject *arg) {
+  return guarded([&]() -> PyObject * {
+    const long i = PyLong_AsLong(arg);
+    cudaError_t e = cudaSuccess;
+    Py_BEGIN_ALLOW_THREADS
+    for (int k = 0; k < 8; k++) if ((i < 0 || i == k) && ((self->used >> k) & 1u) && e == cudaSuccess) e = cudaEventSynchronize(self->events[k]);
+    Py_END_ALLOW_THREADS
+    C10_CUDA_CHECK(e);
+    Py_RETURN_NONE;
+  });
+}
+// read(place) -> the counters
+PyObject *ring_read(Ring *self, PyObject *arg) {
+  const long i = PyLong_AsLong(arg);
+  if (i < 0 || i > 7) { PyErr_SetString(PyExc_ValueError, "read: no such place"); return nullptr; }
+  PyObject *list = PyList_New(STATE_WORDS);
+  for (int k = 0; list && k < STATE_WORDS; k++) PyList_SET_ITEM(list, k, PyLong_FromLongLong(self->words[i * STATE_WORDS + k]));
+  return list;
 }
 
 // ---- the map ------------------------------------------------------------------------------------------------
@@ -248,8 +397,6 @@ PyObject *plan_init_table(Plan *self, PyObject *) {
     Py_RETURN_NONE;
   });
 }
-
-extern PyTypeObject plan_type;
 
 // reinsert(plan): the live rows of another table of the same row shape
 PyObject *plan_reinsert(Plan *self, PyObject *arg) {
@@ -488,7 +635,19 @@ PyObject *plan_assign(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
   });
 }
 
+PyMethodDef ring_methods[] = {
+    {"copy", (PyCFunction)(void *)ring_copy, METH_FASTCALL, nullptr},
+    {"landed", (PyCFunction)ring_landed, METH_O, nullptr},
+    {"wait", (PyCFunction)ring_wait, METH_O, nullptr},
+    {"read", (PyCFunction)ring_read, METH_O, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyTypeObject ring_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+PyMethodDef module_methods[] = {{"allocate", (PyCFunction)plan_allocate, METH_VARARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
+
 PyMethodDef plan_methods[] = {
+    {"set_hash", (PyCFunction)(void *)plan_set_hash, METH_FASTCALL, nullptr},
     {"get", (PyCFunction)plan_get, METH_O, nullptr},
     {"set", (PyCFunction)(void *)plan_set, METH_FASTCALL, nullptr},
     {"remove_rows", (PyCFunction)plan_remove_rows, METH_O, nullptr},
@@ -504,7 +663,7 @@ PyMethodDef plan_methods[] = {
 PyTypeObject plan_type = {  // filled in below
     PyVarObject_HEAD_INIT(nullptr, 0)};
 
-PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, nullptr, nullptr, nullptr, nullptr, nullptr};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, module_methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 
@@ -515,12 +674,19 @@ PyMODINIT_FUNC PyInit__native(void) {
   plan_type.tp_new = PyType_GenericNew;
   plan_type.tp_init = (initproc)plan_init;
   plan_type.tp_methods = plan_methods;
-  if (PyType_Ready(&plan_type) < 0) return nullptr;
+  ring_type.tp_name = "doksparse_b200._native.Ring";
+  ring_type.tp_basicsize = sizeof(Ring);
+  ring_type.tp_flags = Py_TPFLAGS_DEFAULT;
+  ring_type.tp_new = PyType_GenericNew;
+  ring_type.tp_init = (initproc)ring_init;
+  ring_type.tp_dealloc = (destructor)ring_dealloc;
+  ring_type.tp_methods = ring_methods;
+  if (PyType_Ready(&plan_type) < 0 || PyType_Ready(&ring_type) < 0) return nullptr;
   PyObject *lib = PyImport_ImportModule("doksparse_b200._lib");
   if (!lib) return nullptr;
   dok_error = PyObject_GetAttrString(lib, "DokError");
   Py_DECREF(lib);
   PyObject *m = dok_error ? PyModule_Create(&module) : nullptr;
-  if (m && PyModule_AddObjectRef(m, "Plan", (PyObject *)&plan_type) < 0) { Py_DECREF(m); return nullptr; }
+  if (m && (PyModule_AddObjectRef(m, "Plan", (PyObject *)&plan_type) < 0 || PyModule_AddObjectRef(m, "Ring", (PyObject *)&ring_type) < 0)) { Py_DECREF(m); return nullptr; }
   return m;
 }

@@ -31,18 +31,16 @@ struct Mont {
 const uint16_t SMALL[] = {3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61, 67, 71, 73, 79, 83, 89, 97,
                           101, 103, 107, 109, 113, 127, 131, 137, 139, 149, 151, 157, 163, 167, 173, 179, 181, 191, 193};
 
-// Miller-Rabin; the first twelve primes as bases decide every n below 3.3e24 (J. Sorenson and J. Webster, "Strong
-// pseudoprimes to twelve prime bases", 2015), so this is exact for 64-bit numbers.
+// Miller-Rabin with the seven bases that J. Sinclair found to decide every 64-bit number (2011, verified against the list of
+// strong pseudoprimes to base 2 by J. Feitsma); n is odd and has no factor below 197.
 bool is_prime(uint64_t n) {
-  if (n < 2) return false;
-  if (n % 2 == 0) return n == 2;
-  for (uint16_t p : SMALL) if (n % p == 0) return n == p;
-  if (n < 193ull * 193ull) return true;
   const Mont m(n);
   const uint64_t minus_one = n - m.one;
   const int s = __builtin_ctzll(n - 1);
   const uint64_t d = (n - 1) >> s;
-  for (uint64_t base : {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37}) {
+  for (uint64_t base : {2ull, 325ull, 9375ull, 28178ull, 450775ull, 9780504ull, 1795265022ull}) {
+    base %= n;
+    if (base == 0) continue;
     const uint64_t b = m.mul(base, m.r2);
     uint64_t x = m.one;
     for (int i = 63 - __builtin_clzll(d); i >= 0; i--) {
@@ -64,6 +62,27 @@ bool is_prime(uint64_t n) {
 
 extern "C" uint64_t dok_next_prime(uint64_t n) {
   if (n < 2) return 2;
-  for (uint64_t c = (n + 1) | 1; c > n; c += 2) if (is_prime(c)) return c;
-  return 0;                                             // above the largest 64-bit prime
+  if (n < 193 * 193) {                                  // the small primes decide
+    for (uint64_t c = (n + 1) | 1;; c += 2) {
+      bool prime = true;
+      for (uint16_t p : SMALL) {
+        if ((uint32_t)p * p > c) break;
+        if (c % p == 0) { prime = false; break; }
+      }
+      if (prime) return c;
+    }
+  }
+  for (uint64_t first = (n + 1) | 1; first > n; first += 2 * 256) {       // 256 odd candidates, those with a small factor struck out
+    bool struck[256] = {};
+    for (uint16_t p : SMALL) {
+      // first + 2 i = 0 (mod p): i = -first / 2 = (p - first % p) * (p + 1) / 2
+      for (uint32_t i = (uint32_t)((p - first % p) % p * ((p + 1u) / 2) % p); i < 256; i += p) struck[i] = true;
+    }
+    for (uint32_t i = 0; i < 256; i++) {
+      const uint64_t c = first + 2 * i;
+      if (c < first) return 0;                          // above the largest 64-bit prime
+      if (!struck[i] && is_prime(c)) return c;
+    }
+  }
+  return 0;
 }

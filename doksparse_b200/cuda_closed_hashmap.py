@@ -19,6 +19,7 @@ What is different (the slot layout is not part of the contract)
 import ctypes
 import math
 import threading
+from collections import namedtuple
 
 import numpy as np
 import torch
@@ -43,22 +44,22 @@ class _PinnedRings:
     gives its ring back when it goes; at most 256 are kept."""
 
     def __init__(self):
-        self._lock, self._free = threading.Lock(), []
+        self._lock, self._free = threading.Lock(), {}
 
-    def take(self):
+    def take(self, device):
         with self._lock:
-            if not self._free:
-                chunk = torch.zeros(64, 8, _STATE_WORDS, dtype=torch.long, pin_memory=True)
-                self._free = [(chunk[i], None) for i in range(64)]
-            ring, last_copy = self._free.pop()
-        if last_copy is not None:
-            last_copy.synchronize()             # the previous owner's copies have landed: nothing writes here any more
+            free = self._free.setdefault(device, [])
+            if not free:
+                chunk = torch.zeros(64, 8 * _STATE_WORDS, dtype=torch.long, pin_memory=True)
+                free += [L.native().Ring(words, device) for words in chunk]
+            ring = free.pop()
+        ring.wait(-1)                   # the previous owner's copies have landed: nothing writes here any more
         return ring
 
-    def give(self, ring, last_copy):
+    def give(self, ring, device):
         with self._lock:
-            if len(self._free) < 256:
-                self._free.append((ring, last_copy))
+            if len(self._free[device]) < 256:
+                self._free[device].append(ring)
 
 
 _rings = _PinnedRings()
@@ -67,20 +68,23 @@ _rings = _PinnedRings()
 class _Shared:
     """What shallow clones (views) must see together: the duplicate-resolution stamps with their epoch, and the host-side
     upper bound of n_elements that lets `set` skip a device synchronisation."""
-    __slots__ = ("stamp", "epoch", "bound", "base", "snapshots", "ring", "last_copy")
+    __slots__ = ("stamp", "epoch", "bound", "base", "snapshots", "ring", "device")
 
     def __init__(self, stamp=None, epoch=0, bound=0):
         self.stamp, self.epoch, self.bound, self.base = stamp, epoch, bound, bound
-        self.snapshots, self.ring, self.last_copy = [], None, None
+        self.snapshots, self.ring, self.device = [], None, None
 
     def __del__(self):
         if self.ring is not None and _rings is not None:         # (None: the interpreter is going down)
-            _rings.give(self.ring, self.last_copy)
+            _rings.give(self.ring, self.device)
 
     def exact(self, n):
         """n_elements is known to be n, and nothing enqueued later has been counted in."""
         self.snapshots.clear()
         self.bound = self.base = n
+
+
+_Layout = namedtuple("_Layout", "slot_bytes slots_per_group value_offset key_offset stamp_offset n_slots total_bytes")
 
 
 class CudaClosedHashmap:
@@ -145,6 +149,7 @@ class CudaClosedHashmap:
             self._key_perm = key_perm.to(device=self.device, dtype=torch.long)
         self._host_perm = None
         self._hp = None       # cached ctypes dok_hash_params
+        self._bare_plan = None          # of the slot array that `_allocate` made, without hash parameters
         self._plan = None     # what the native calls need to know of this table (_native_plan)
         self._table = None
 
@@ -281,21 +286,15 @@ class CudaClosedHashmap:
             raise L.DokError(f"keys may have 1..{L.MAX_KEY_SIZE} elements, got {key_size}")
         if not (1 <= value_bytes <= L.MAX_VALUE_BYTES):
             raise L.DokError(f"value rows may have 1..{L.MAX_VALUE_BYTES} bytes, got {value_bytes}")
-        key_bytes = key_size * key_dtype.itemsize
-        lay = L.LayoutInfo()
-        L.check(L.lib().dok_table_layout(value_bytes, key_bytes, self._n_buckets, ctypes.byref(lay)), "dok_table_layout")
-        self._layout = lay
-        self._value_bytes, self._key_bytes = value_bytes, key_bytes
+        self._value_bytes, self._key_bytes = value_bytes, key_size * key_dtype.itemsize
         self._value_shape, self._value_dtype = torch.Size(value_shape), value_dtype
         self._key_shape, self._key_dtype = torch.Size(key_shape), key_dtype
-        self._slots = torch.empty(lay.total_bytes, device=self.device, dtype=torch.uint8)
         self._shared.stamp = None
         self._hp = self._plan = None
-        if self._counters_of_table is None:
-            self._counters_of_table = torch.empty(_STATE_WORDS, device=self.device, dtype=torch.long)
-        with L.on(self.device):
-            L.check(L.lib().dok_map_init_state(self._c_table(), self._counter_block(0), _STATE_WORDS,
-                                               L.stream_ptr(self.device)), "dok_map_init_state")
+        device = torch.cuda.current_device() if self.device.index is None else self.device.index
+        self._bare_plan, self._slots, self._counters_of_table, layout = L.native().allocate(
+            device, self._n_buckets, self._key_shape, key_dtype, self._value_shape, value_dtype, self._counters_of_table)
+        self._layout = _Layout(*layout)
 
     def _begin_bulk_insert(self, key_shape, key_dtype, value_shape, value_dtype, n_new):
         """What `set` does to a never-used map before its kernel runs, for a batch known to hold `n_new` pairwise
@@ -377,25 +376,36 @@ class CudaClosedHashmap:
             ks = math.prod(self._key_shape)
             hp.key_size = ks
             hp.key_dtype = L.DTYPE_CODES[self._key_dtype]
-            host, perm = {name: self._host_param(name) for name in _PARAM_NAMES}, self._perm()
-            assert all(len(v) == ks for v in host.values())
+            host = self._checked_params()
             for name in _PARAM_NAMES:
                 getattr(hp, name)[:ks] = host[name]
-            hp.key_perm[:ks] = perm
-            assert all(abs(p) >= 2 for p in host["prime1"] + host["prime2"]), "primes must have magnitude >= 2"
-            if 0 in host["alpha2"]:
-                import warnings
-                warnings.warn("alpha2 contains 0: the uuid ignores that key element, so keys differing only there "
-                              "are told apart only by their first hash (the reference draws alpha2 from [-1, prime1-2])")
+            hp.key_perm[:ks] = self._perm()
             self._hp = hp
         return ctypes.byref(self._hp)
 
+    def _checked_params(self):
+        ks = math.prod(self._key_shape)
+        host = {name: self._host_param(name) for name in _PARAM_NAMES}
+        assert all(len(v) == ks for v in host.values())
+        assert all(abs(p) >= 2 for p in host["prime1"] + host["prime2"]), "primes must have magnitude >= 2"
+        if 0 in host["alpha2"]:
+            import warnings
+            warnings.warn("alpha2 contains 0: the uuid ignores that key element, so keys differing only there "
+                          "are told apart only by their first hash (the reference draws alpha2 from [-1, prime1-2])")
+        return host
+
     def _native_plan(self):
         """The native form of this table, or None where only the general calls serve it."""
-        if self._plan is None and self._slots is not None:
+        if self._plan is None and self._bare_plan is not None:
+            self._materialise_parameters()
+            host = self._checked_params()
+            self._bare_plan.set_hash(L.DTYPE_CODES[self._key_dtype], host["alpha2"], host["beta2"], host["prime2"], host["alpha1"],
+                                     host["beta1"], host["prime1"], self._perm())
+            self._plan = self._bare_plan
+        elif self._plan is None and self._slots is not None:
             self._c_hash()
             self._c_table()
-            self._plan = L.plan_type()(bytes(self._table), bytes(self._hp), self._state.data_ptr(), self._slots.device.index,
+            self._plan = L.native().Plan(bytes(self._table), bytes(self._hp), self._state.data_ptr(), self._slots.device.index,
                                        tuple(self._key_shape), self._key_dtype, tuple(self._value_shape), self._value_dtype)
         return self._plan
 
@@ -419,32 +429,29 @@ class CudaClosedHashmap:
         sh = self._shared
         sh.bound += added
         for s in sh.snapshots:
-            s[2] += added                       # rows that may have been inserted after that snapshot was taken
+            s[1] += added                       # rows that may have been inserted after that snapshot was taken
         room = int(self._rehash_threshold * self._n_buckets) - sh.base
         if 4 * (sh.bound - sh.base) < room:
             return
         if sh.ring is None:
-            sh.ring = _rings.take()
-        free = set(range(sh.ring.shape[0])) - {s[1] for s in sh.snapshots}
-        if not free:
+            sh.device = self._slots.device.index
+            sh.ring = _rings.take(sh.device)
+        in_flight = [s[0] for s in sh.snapshots]
+        place = next((i for i in range(8) if i not in in_flight), None)
+        if place is None:
             return                              # eight copies still in flight: skip this one, the bound stays valid
-        slot = free.pop()
-        with L.on(self.device):
-            sh.ring[slot].copy_(self._state, non_blocking=True)
-            event = torch.cuda.Event()
-            event.record()
-        sh.snapshots.append([event, slot, 0])
-        sh.last_copy = event
+        sh.ring.copy(self._native_plan(), place)
+        sh.snapshots.append([place, 0])
         sh.base = sh.bound
 
     def _element_bound(self):
         sh = self._shared
         newest = None
-        while sh.snapshots and sh.snapshots[0][0].query():
+        while sh.snapshots and sh.ring.landed(sh.snapshots[0][0]):
             newest = sh.snapshots.pop(0)
         if newest is not None:
-            n = self._sizes(sh.ring[newest[1]].tolist())[0]
-            sh.bound = min(sh.bound, n + newest[2])
+            n = self._sizes(sh.ring.read(newest[0]))[0]
+            sh.bound = min(sh.bound, n + newest[1])
             if not sh.snapshots:
                 sh.base = min(sh.base, n)
         return sh.bound
@@ -456,7 +463,7 @@ class CudaClosedHashmap:
         bound = self._element_bound()
         snaps = self._shared.snapshots
         while bound + rows > limit and snaps:
-            snaps[0][0].synchronize()
+            self._shared.ring.wait(snaps[0][0])
             bound = self._element_bound()
         return bound + rows <= limit
 
@@ -911,7 +918,7 @@ class CudaClosedHashmap:
         source.value_bytes, source.key_bytes = self._value_bytes, self._key_bytes
         fresh = torch.empty(self._layout.total_bytes, device=self.device, dtype=torch.uint8)     # may raise: nothing changed yet
         self._slots = fresh
-        self._plan = None
+        self._plan = self._bare_plan = None
         self._shared.stamp = None
         self._shared.epoch = 0
         state = self._state.clone()
