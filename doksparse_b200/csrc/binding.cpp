@@ -583,8 +583,8 @@ PyObject *plan_index(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
   });
 }
 
-// assign(selectors, size, values, room, epoch, stamp address) -> the number of positions, or None (`room`: more positions
-// than this may make the table grow)
+// assign(selectors, size, values, room, epoch, stamp address) -> the number of positions, or None; its negative, and
+// nothing done, when it is more than `room`, so that the table might have to grow
 PyObject *plan_assign(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
   return guarded([&]() -> PyObject * {
     if (nargs != 6) { PyErr_SetString(PyExc_TypeError, "assign takes 6 arguments"); return nullptr; }
@@ -607,7 +607,8 @@ PyObject *plan_assign(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
     if (PyErr_Occurred()) return nullptr;
     const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
     Selection s;
-    if (!parse_selection(args[0], size, ndim, self->device, &s) || (double)s.n > room) Py_RETURN_NONE;
+    if (!parse_selection(args[0], size, ndim, self->device, &s)) Py_RETURN_NONE;
+    if ((double)s.n > room) return PyLong_FromLongLong(-s.n);
     at::Tensor values;
     if (given) {
       values = given->expand(s.shape);

@@ -360,9 +360,11 @@ class SparseDOKTensor(object):
         if plan is not None and hashmap._value_dtype == self._dtype and sh.epoch < L.MAX_EPOCH - 1:
             stamp = hashmap._stamp_address()
             if stamp is not None:
-                room = hashmap.n_buckets * hashmap._rehash_threshold - hashmap._element_bound()
-                n = plan.assign(selectors, self._size, values, room, sh.epoch + 1, stamp)
-                if n is not None:
+                limit = hashmap._n_buckets * hashmap._rehash_threshold
+                n = plan.assign(selectors, self._size, values, limit - hashmap._element_bound(), sh.epoch + 1, stamp)
+                if n is not None and n < 0 and hashmap._room_for(-n, limit):
+                    n = plan.assign(selectors, self._size, values, -n, sh.epoch + 1, stamp)
+                if n is not None and n >= 0:
                     if n:
                         sh.epoch += 1
                         hashmap._after_mutation(n)
