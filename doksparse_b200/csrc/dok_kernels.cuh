@@ -233,6 +233,15 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_set_unique(DevTable t, DevHash h
 // third kernel, 151 us of a 4 M-row assignment; 512 KB that stay in L2 answer for most rows.
 #define DOK_FILTER_BITS 22
 #define DOK_FILTER_WORDS (1 << (DOK_FILTER_BITS - 6))                       // int64 words behind slot_out[n]
+// One block in 16 adds up its rows whose slot another block has stamped, for the blocks that come later; a line of its own,
+// and a sample, because every block reads it (all of them adding to a word that all of them read: a 4 M-row assignment
+// 488 -> 700 us).
+#define DOK_FILTER_SIGNAL (2 * DOK_FILTER_WORDS + 32)                       // unsigned words behind the filter's start
+#define DOK_SIGNAL_SAMPLE 16
+__device__ __forceinline__ unsigned *dok_signal(unsigned *filter) {         // 16-byte aligned
+  return (unsigned *)(((uintptr_t)(filter + DOK_FILTER_SIGNAL) + 15) & ~(uintptr_t)15);
+}
+#define DOK_FILTER_ALL (DOK_FILTER_WORDS + 32)                              // int64 words, all zeroed
 #define DOK_FILTER_FROM 65536                                               // rows; below, clearing it costs more
 __device__ __forceinline__ unsigned dok_filter_bit(ll_t slot) { return ((unsigned)slot * 0x9e3779b1u) >> (32 - DOK_FILTER_BITS); }
 __device__ __forceinline__ void dok_filter_set(unsigned *filter, ll_t slot) {
@@ -256,6 +265,7 @@ struct BlockTwins {
   ll_t chain[DOK_TWIN_SLOTS];              // 55 bits of the chain's hash | 8 bits: thread of the key's last row so far
   ll_t uuid[DOK_TPB], slot[DOK_TPB];       // by thread; inactive rows have no uuid
   uint8_t more[DOK_TPB * 2];               // by place: more than one row
+  uint4 signal;                            // see dok_signal
 };
 struct Twins { int last; bool more; };     // thread of the key's last row; whether there are others
 
@@ -280,6 +290,7 @@ __device__ __forceinline__ Twins dok_find_twins(BlockTwins &b, const KeyHash &kh
       at = (at + 1) & (DOK_TWIN_SLOTS - 1);
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");              // (k_set_claim: the signal)
   __syncthreads();
   Twins w{(int)threadIdx.x, false};
   if (active) {
@@ -304,6 +315,9 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
   const unsigned block = gridDim.x - 1 - blockIdx.x;
   if (keys.idle(block)) return;
   dok_tally_begin(tally);
+  // on its way while the rows are hashed, and in no register
+  if (filter && threadIdx.x == 0)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(&twins.signal)), "l"(dok_signal(filter)) : "memory");
   ll_t e;
   bool active = keys.row(e, block);
   KeyHash kh{0, 0};
@@ -322,8 +336,11 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
       ull_t *stamp = (ull_t *)dok_stamp_ptr(t, slot);
       // A key that the block holds several times is probably all over the batch.  If a later row has already stamped its
       // slot -- blocks start from the batch's end, so one has unless it is still running -- this row has nothing to write,
-      // and a line that most of the blocks want is read, not written: writes to one line come 140 ns apart.
-      ull_t old = same.more && !fresh ? __ldcg(stamp) : 0;
+      // and a line that most of the blocks want is read, not written: writes to one line come 140 ns apart.  In a batch with
+      // many repetitions (one row in 16 so far, by a sample) the same goes for the keys that a block holds once: one in a thousand rows of a Zipf batch of 12.8 M
+      // is 12,800 writes to one line.  Elsewhere the look would cost every row a round trip for nothing.
+      const bool contended = filter && (ull_t)twins.signal.x * DOK_SIGNAL_SAMPLE * 16 > ((ull_t)blockIdx.y * gridDim.x + blockIdx.x) * DOK_TPB;
+      ull_t old = (same.more || contended) && !fresh ? __ldcg(stamp) : 0;
       const bool over = old > (dok_stamp(epoch, e) | 3);
       dup = over;
       if (!over) {
@@ -358,6 +375,10 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
     slot_out[e] = -1;                                               // nothing to rewrite: a later row of the block may
   }
   dok_tally_add(tally, DOK_TALLY_EXTRA, conflict);
+  if (filter && blockIdx.x % DOK_SIGNAL_SAMPLE == 0) {            // uniform over the block
+    const unsigned votes = __ballot_sync(0xffffffffu, dup);
+    if ((threadIdx.x & 31) == 0 && votes) atomicAdd(dok_signal(filter), __popc(votes));
+  }
   if (counters) {
     const bool twin = active && !last;
     dok_tally_add(tally, DOK_CNT_CLAIMED_EMPTY, outcome == DOK_OUT_CLAIMED_EMPTY);
@@ -490,7 +511,7 @@ inline int launch_set_small(const DevTable &t, const DevHash &hp, const Keys &ke
   cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(blocks);
-  config.blockDim = dim3(DOK_SMALL_SET_TPB);
+  config.blockDim = dim3(blocks > 1 ? DOK_SMALL_SET_TPB : (unsigned)((keys.n + 63) / 64 * 64));
   config.stream = st;
   config.attrs = &cluster;
   config.numAttrs = 1;
@@ -512,9 +533,9 @@ inline int launch_set_general(const DevTable &t, const DevHash &hp, const Keys &
     DOK_DISPATCH_SB(t, (rc = launch_set_small<SB>(t, hp, keys, values, (ll_t)epoch, (ll_t *)counters, (ll_t *)more, st)));
     return rc;
   }
-  const bool filtered = keys.n >= DOK_FILTER_FROM && scratch_words >= keys.n + 1 + DOK_FILTER_WORDS;
+  const bool filtered = keys.n >= DOK_FILTER_FROM && scratch_words >= keys.n + 1 + DOK_FILTER_ALL;
   unsigned *filter = filtered ? (unsigned *)(slot_scratch + keys.n + 1) : nullptr;
-  const size_t zeroed = sizeof(int64_t) * (filtered ? 1 + DOK_FILTER_WORDS : 1);
+  const size_t zeroed = sizeof(int64_t) * (filtered ? 1 + DOK_FILTER_ALL : 1);
   if (cudaMemsetAsync(slot_scratch + keys.n, 0, zeroed, st) != cudaSuccess) return dok_check_launch();
   const dim3 grid = dok_grid(keys);
   int rc = DOK_OK;

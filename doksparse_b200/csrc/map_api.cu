@@ -98,7 +98,7 @@ int64_t dok_set_scratch_words(const dok_table *t, int64_t n) {
   DevTable dt;
   if (!dok_make_table(t, &dt) || n < 0 || n > DOK_MAX_BATCH) return -1;
   if (dok_set_is_small(dt, n)) return 0;
-  return n + 1 + (n >= DOK_FILTER_FROM ? DOK_FILTER_WORDS : 0);
+  return n + 1 + (n >= DOK_FILTER_FROM ? DOK_FILTER_ALL : 0);
 }
 
 int dok_map_set_with(const dok_table *t, const dok_hash_params *hp, const void *keys, const void *values, int64_t n,

@@ -110,11 +110,11 @@ __global__ void __launch_bounds__(DOK_SMALL_TPB) k_remove_unique_small(DevTable 
                                                                        ll_t *__restrict__ out_count, ll_t *counters) {
   __shared__ SmallRows s;
   __shared__ int warp_sums[DOK_SMALL_TPB / 32], removed;
-  const int n = (int)keys.n, tid = (int)threadIdx.x;
+  const int n = (int)keys.n, tid = (int)threadIdx.x, threads = (int)blockDim.x;
   const int per = min(hp.ks, 8 / hp.elem_bytes);                 // columns in the prefix
   const bool whole = per == hp.ks;
   bool nan = false;
-  for (int i = tid; i < padded; i += DOK_SMALL_TPB) {
+  for (int i = tid; i < padded; i += threads) {
     ull_t k = ~0ULL;
     if (i < n) {
       k = 0;
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(DOK_SMALL_TPB) k_remove_unique_small(DevTable 
   };
   for (int size = 2; size <= padded; size <<= 1)
     for (int step = size >> 1; step > 0; step >>= 1) {
-      for (int i = tid; i < padded / 2; i += DOK_SMALL_TPB) {
+      for (int i = tid; i < padded / 2; i += threads) {
         const int a = 2 * i - (i & (step - 1)), b = a + step;
         const bool up = (a & size) == 0;
         if (up ? before(b, a) : before(a, b)) {
@@ -152,12 +152,14 @@ __global__ void __launch_bounds__(DOK_SMALL_TPB) k_remove_unique_small(DevTable 
           s.row[b] = r;
         }
       }
-      __syncthreads();
+      // up to a step of 32 each warp keeps to the same 64 elements
+      if (step > 32 || (step == 1 && size > 32)) __syncthreads(); else __syncwarp();
     }
+  __syncthreads();
   // the first row of each run of equal rows, compacted in order into s.row (a row never moves up, so the last row of a
   // chunk stays in place for the comparison with the next chunk's first)
   int count = 0;
-  for (int base = 0; base < n; base += DOK_SMALL_TPB) {
+  for (int base = 0; base < n; base += threads) {
     const int i = base + tid;
     const unsigned short row = i < n ? s.row[i] : (unsigned short)0xffff;
     bool head = i < n;
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(DOK_SMALL_TPB) k_remove_unique_small(DevTable 
     if ((tid & 31) == 0) warp_sums[tid >> 5] = __popc(votes);
     __syncthreads();
     int at = count, total = 0;
-    for (int w = 0; w < DOK_SMALL_TPB / 32; w++) {
+    for (int w = 0; w < threads / 32; w++) {
       if (w < (tid >> 5)) at += warp_sums[w];
       total += warp_sums[w];
     }
@@ -176,7 +178,7 @@ __global__ void __launch_bounds__(DOK_SMALL_TPB) k_remove_unique_small(DevTable 
     count += total;
     __syncthreads();
   }
-  for (int base = 0; base < count; base += DOK_SMALL_TPB) {
+  for (int base = 0; base < count; base += threads) {
     const int i = base + tid;
     const bool active = i < count;
     const ll_t e = active ? s.row[i] : 0;
@@ -602,7 +604,8 @@ int dok_map_remove_unique(const dok_table *t, const dok_hash_params *hp, const v
   if (n <= DOK_SMALL_ROWS) {
     int padded = 1;
     while (padded < n) padded *= 2;
-    DOK_DISPATCH_SB(dt, (k_remove_unique_small<SB><<<1, DOK_SMALL_TPB, 0, st>>>(dt, dh, rk, padded, out_removed, (ll_t *)out_count, (ll_t *)counters)));
+    const int threads = padded < 64 ? 64 : padded < DOK_SMALL_TPB ? padded : DOK_SMALL_TPB;      // fewer wait at the barriers
+    DOK_DISPATCH_SB(dt, (k_remove_unique_small<SB><<<1, threads, 0, st>>>(dt, dh, rk, padded, out_removed, (ll_t *)out_count, (ll_t *)counters)));
     return dok_check_launch();
   }
   if (!work) return DOK_BAD_ARG;
