@@ -69,7 +69,7 @@ struct DenseShape { int ndim; ll_t sizes[DOK_MAX_KEY_SIZE]; };
 #define DOK_DENSE_SPAN (DOK_TPB * DOK_DENSE_ROUNDS)
 
 template <int SB, typename T>
-__global__ void __launch_bounds__(DOK_TPB) k_dense_insert(DevTable t, DevHash hp, const T *__restrict__ dense, ll_t numel,
+__global__ void __launch_bounds__(DOK_TPB, 4) k_dense_insert(DevTable t, DevHash hp, const T *__restrict__ dense, ll_t numel,
                                                           int is_float, DenseShape shape, ll_t *counters) {
   __shared__ ll_t found_at[DOK_DENSE_SPAN + DOK_TPB];
   __shared__ T found_value[DOK_DENSE_SPAN + DOK_TPB];
@@ -78,25 +78,49 @@ __global__ void __launch_bounds__(DOK_TPB) k_dense_insert(DevTable t, DevHash hp
   int claimed = 0, reused = 0, failed = 0, hits = 0;
   if (threadIdx.x == 0) n_found = 0;
   __syncthreads();
-  for (ll_t base = (ll_t)blockIdx.x * DOK_DENSE_SPAN; base < numel; base += stride) {     // uniform over the block
-    T v[DOK_DENSE_ROUNDS];
+  const auto unravel = [&](auto rem, ll_t (&idx)[DOK_MAX_KEY_SIZE]) {          // a 64-bit division costs four of 32 bits
+    using U = decltype(rem);
+#pragma unroll
+    for (int d = DOK_MAX_KEY_SIZE - 1; d >= 0; d--) {
+      idx[d] = 0;
+      if (d < shape.ndim) {
+        const U size = (U)shape.sizes[d], q = rem / size;
+        idx[d] = (ll_t)(rem - q * size);
+        rem = q;
+      }
+    }
+  };
+  // the next span's elements are on their way while this one's are collected and inserted
+  T v[DOK_DENSE_ROUNDS];
+  const auto fetch = [&](ll_t base) {
 #pragma unroll
     for (int r = 0; r < DOK_DENSE_ROUNDS; r++) {
       const ll_t i = base + r * DOK_TPB + (int)threadIdx.x;
       v[r] = i < numel ? __ldcs(dense + i) : (T)0;
     }
+  };
+  fetch((ll_t)blockIdx.x * DOK_DENSE_SPAN);
+  for (ll_t base = (ll_t)blockIdx.x * DOK_DENSE_SPAN; base < numel; base += stride) {     // uniform over the block
+    int in_warp = 0;
 #pragma unroll
-    for (int r = 0; r < DOK_DENSE_ROUNDS; r++) {
-      const bool nz = dok_nonzero<T>(v[r], is_float);
-      const unsigned votes = __ballot_sync(0xffffffffu, nz);
-      int at = 0;
-      if ((threadIdx.x & 31) == 0 && votes) at = atomicAdd(&n_found, __popc(votes));
-      at = __shfl_sync(0xffffffffu, at, 0) + __popc(votes & ((1u << (threadIdx.x & 31)) - 1u));
-      if (nz) {
-        found_value[at] = v[r];
-        found_at[at] = base + r * DOK_TPB + (int)threadIdx.x;
+    for (int r = 0; r < DOK_DENSE_ROUNDS; r++) in_warp += __popc(__ballot_sync(0xffffffffu, dok_nonzero<T>(v[r], is_float)));
+    int at = 0;
+    if ((threadIdx.x & 31) == 0 && in_warp) at = atomicAdd(&n_found, in_warp);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (in_warp) {
+#pragma unroll
+      for (int r = 0; r < DOK_DENSE_ROUNDS; r++) {
+        const bool nz = dok_nonzero<T>(v[r], is_float);
+        const unsigned votes = __ballot_sync(0xffffffffu, nz);
+        const int mine = at + __popc(votes & ((1u << (threadIdx.x & 31)) - 1u));
+        if (nz) {
+          found_value[mine] = v[r];
+          found_at[mine] = base + r * DOK_TPB + (int)threadIdx.x;
+        }
+        at += __popc(votes);
       }
     }
+    fetch(base + stride);
     __syncthreads();
     const bool at_end = base + stride >= numel;
     int total = n_found;
@@ -110,17 +134,8 @@ __global__ void __launch_bounds__(DOK_TPB) k_dense_insert(DevTable t, DevHash hp
       if (active) {
         value = found_value[k];
         // unravel the row-major position into the index tuple; each index is one factor of the hash products
-        ull_t rem = (ull_t)found_at[k];
-#pragma unroll
-        for (int d = DOK_MAX_KEY_SIZE - 1; d >= 0; d--) {
-          idx[d] = 0;
-          if (d < shape.ndim) {
-            const ull_t size = (ull_t)shape.sizes[d];
-            const ull_t q = rem / size;
-            idx[d] = (ll_t)(rem - q * size);
-            rem = q;
-          }
-        }
+        if (numel <= 0xffffffffLL) unravel((unsigned)found_at[k], idx);
+        else unravel((ull_t)found_at[k], idx);
         ll_t u = dok_uuid_term(idx[0], hp.a[0], hp.b[0], hp.p[0], hp.m[0]);
         ull_t h = (ull_t)idx[0] * (ull_t)hp.a1[0] + (ull_t)hp.b1[0];
 #pragma unroll
@@ -496,7 +511,8 @@ int dok_dense_insert_nonzero(const dok_table *t, const dok_hash_params *hp, cons
     prod *= shape.sizes[d];
   }
   if (prod != numel) return DOK_BAD_ARG;
-  const unsigned grid = streaming_grid((numel + DOK_DENSE_ROUNDS - 1) / DOK_DENSE_ROUNDS);
+  const ll_t spans = (numel + DOK_DENSE_SPAN - 1) / DOK_DENSE_SPAN;
+  const unsigned grid = (unsigned)(spans < 148 * 4 ? spans : 148 * 4);          // one wave: each block ends with a list that is not full
   cudaStream_t st = (cudaStream_t)stream;
   int rc = DOK_OK;
   switch (dt.vb) {

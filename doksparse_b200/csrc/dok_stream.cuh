@@ -123,8 +123,8 @@ __device__ __forceinline__ void dok_inspect(const LaneRow &lr, const Lines<LW> &
 // The loop.  `step(lane's row, lines, share)` inspects the lines, lets the row go to its next group (dok_next_group) or ends
 // it (done()).
 template <int LW, class Keys, class Step>
-__device__ __forceinline__ void dok_walk_share(WarpQueue &queue, const DevTable &t, const DevHash &hp, const Keys &keys, const Step &step) {
-  WarpShare share = dok_share(keys.total());
+__device__ __forceinline__ void dok_walk_share(WarpQueue &queue, WarpShare share, const DevTable &t, const DevHash &hp, const Keys &keys,
+                                               const Step &step) {
   LaneRow lr = DOK_IDLE_LANE;
   Lines<LW> lines;
   for (;;) {
@@ -133,4 +133,9 @@ __device__ __forceinline__ void dok_walk_share(WarpQueue &queue, const DevTable 
     dok_request<LW>(t, lr, lines);
     step(lr, lines, share);
   }
+}
+// ... of the warp's part of the whole batch
+template <int LW, class Keys, class Step>
+__device__ __forceinline__ void dok_walk_share(WarpQueue &queue, const DevTable &t, const DevHash &hp, const Keys &keys, const Step &step) {
+  dok_walk_share<LW>(queue, dok_share(keys.total()), t, hp, keys, step);
 }

@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(DOK_SMALL_TPB) k_remove_unique_small(DevTable 
 #define DOK_SORT_MAX_ROWS (1LL << 30)      // counts travel in 30 bits beside two flags
 #define DOK_SORT_SPINS (1 << 22)           // bound of every wait for another block; far beyond what one takes
 #define DOK_MAX_RUN 64                     // longest run of equal prefixes with different rows that one thread sorts
-#define DOK_UNIQUE_ROUNDS 4                // rows per thread of the removal; one of them for small batches, likewise
+#define DOK_UNIQUE_ROUNDS 8                // rows per thread of the removal; one of them for small batches, likewise
 
 // zeroed before the first kernel
 struct SortControl {
@@ -457,14 +457,29 @@ __global__ void __launch_bounds__(DOK_TPB) k_sort_ties(SortControl *c, RowKeys k
   }
 }
 
+// The first rows of runs of equal rows, as a key source for the walk.
+struct HeadKeys {
+  const RowKeys &keys;
+  const unsigned *rows;
+  __device__ __forceinline__ ll_t elem(unsigned i) const { return (ll_t)rows[i]; }
+  __device__ __forceinline__ KeyHash hash(const DevHash &hp, ll_t e) const { return keys.hash(hp, e); }
+};
+
 // First row of each run of equal rows: looked up, its slot turned into a tombstone, its flag written at the run's number.
-// Runs are counted across tiles by looking back like in the sort, when the tile's own lookups are done.
+// Runs are counted across tiles by looking back like in the sort, when the tile's own lookups are done.  A tile's runs are
+// gathered first and each warp walks its eighth of them with a lane taking the next when its chain ends (dok_stream.cuh):
+// walked row by row, half the lanes of a batch that holds each key twice were idle, and all but the longest chain's of keys
+// that are no longer there (64 M-operation churn, a table at load 0.9: 5.03 -> 4.64 ms; 4 rows per thread 4.85, 16 spill).
 template <int SB, int ROUNDS>
-__global__ void __launch_bounds__(DOK_TPB) k_remove_unique(DevTable t, DevHash hp, RowKeys keys, SortControl *c, const unsigned *key_a,
-                                                           const unsigned *row_a, const unsigned *key_b, const unsigned *row_b,
-                                                           unsigned *look, unsigned tiles, uint8_t *__restrict__ out_removed,
-                                                           ll_t *__restrict__ out_count, ll_t *counters) {
-  __shared__ unsigned sums[ROUNDS][DOK_TPB / 32], tile_id, base_of_tile;
+__global__ void __launch_bounds__(DOK_TPB, 4) k_remove_unique(DevTable t, DevHash hp, RowKeys keys, SortControl *c, const unsigned *key_a,
+                                                              const unsigned *row_a, const unsigned *key_b, const unsigned *row_b,
+                                                              unsigned *look, unsigned tiles, uint8_t *__restrict__ out_removed,
+                                                              ll_t *__restrict__ out_count, ll_t *counters) {
+  constexpr unsigned TILE = DOK_TPB * ROUNDS;
+  __shared__ unsigned sums[ROUNDS][DOK_WARPS], tile_id, base_of_tile;
+  __shared__ unsigned head_row[TILE];
+  __shared__ uint8_t hit_of[TILE];
+  __shared__ WarpQueue queues[DOK_WARPS];
   __shared__ int removed;
   const unsigned n = (unsigned)keys.n;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -477,32 +492,60 @@ __global__ void __launch_bounds__(DOK_TPB) k_remove_unique(DevTable t, DevHash h
   const unsigned tile = tile_id;
   const unsigned *key = c->final_b ? key_b : key_a, *row = c->final_b ? row_b : row_a;
   const bool whole = dok_prefix_is_row(c, hp.ks);
-  unsigned head_votes[ROUNDS], flags = 0;
-  int hits = 0;
+  unsigned votes[ROUNDS], e[ROUNDS];
 #pragma unroll
   for (int r = 0; r < ROUNDS; r++) {
-    const unsigned i = tile * (DOK_TPB * ROUNDS) + r * DOK_TPB + tid;
+    const unsigned i = tile * TILE + r * DOK_TPB + tid;
     bool head = i < n;
-    const unsigned e = i < n ? row[i] : 0;
+    e[r] = i < n ? row[i] : 0;
     if (head && i > 0 && key[i] == key[i - 1])
-      head = !whole && dok_compare_rows(keys.keys, hp.dtype, hp.ks, e, row[i - 1]) != 0;
-    head_votes[r] = __ballot_sync(0xffffffffu, head);
-    if (lane == 0) sums[r][warp] = __popc(head_votes[r]);
-    KeyHash kh{0, 0};
-    if (head) kh = keys.hash(hp, e);
-    const Located loc = dok_locate<SB, 1, false>(t, kh, 0, head, nullptr, NoEmit());
-    int hit = head && loc.found >= 0;
-    if (hit) hit = dok_cas_tag(t, loc.found, kh.uuid, DOK_REMOVED) == kh.uuid;
-    flags |= (unsigned)hit << r;
-    hits += hit;
+      head = !whole && dok_compare_rows(keys.keys, hp.dtype, hp.ks, e[r], row[i - 1]) != 0;
+    votes[r] = __ballot_sync(0xffffffffu, head);
+    if (lane == 0) sums[r][warp] = __popc(votes[r]);
+  }
+  __syncthreads();
+  unsigned total = 0;
+#pragma unroll
+  for (int r = 0; r < ROUNDS; r++) {
+    unsigned mine = total;
+    for (int w = 0; w < DOK_WARPS; w++) {
+      if (w < warp) mine += sums[r][w];
+      total += sums[r][w];
+    }
+    if ((votes[r] >> lane) & 1u) head_row[mine + __popc(votes[r] & ((1u << lane) - 1u))] = e[r];
+  }
+  if (tid == 0) dok_post(look + tile, (tile == 0 ? DOK_LB_TOTAL : DOK_LB_LOCAL) | total);
+  __syncthreads();
+  int hits = 0;
+  if constexpr (SB == 0) {
+    for (unsigned i = tid; i < total; i += DOK_TPB) {
+      const KeyHash kh = keys.hash(hp, head_row[i]);
+      const Located loc = dok_locate_serial(t, kh, nullptr);
+      const int hit = loc.found >= 0 && dok_cas_tag(t, loc.found, kh.uuid, DOK_REMOVED) == kh.uuid;
+      hit_of[i] = (uint8_t)hit;
+      hits += hit;
+    }
+  } else {
+    const unsigned first = total * warp / DOK_WARPS, last = total * (warp + 1) / DOK_WARPS;
+    dok_walk_share<1>(queues[warp], WarpShare{first, last - first, 0, 0, 0}, t, hp, HeadKeys{keys, head_row},
+                      [&](LaneRow &lr, const Lines<1> &f, const WarpShare &share) {
+      unsigned m, me, match[4], empty[4];
+      dok_inspect<SB, 1>(lr, f, m, me, match, empty);
+      if (!lr.busy()) return;
+      const unsigned pos = me ? (unsigned)__ffs(me) - 1 : 0;
+      const unsigned slot = lr.group * (128 / SB) + pos * 32 / SB;
+      if (me || !dok_next_group<unsigned>(lr.group, lr.word, (unsigned)t.n_groups)) {
+        const int hit = ((m >> pos) & 1u) && dok_cas_tag(t, slot, lr.uuid, DOK_REMOVED) == lr.uuid;
+        hit_of[share.first + lr.row] = (uint8_t)hit;
+        hits += hit;
+        lr.done();
+      }
+    });
   }
   for (int o = 16; o > 0; o >>= 1) hits += __shfl_xor_sync(0xffffffffu, hits, o);
   if (lane == 0 && hits) atomicAdd(&removed, hits);
   __syncthreads();
-  unsigned total = 0;
-  for (int r = 0; r < ROUNDS; r++) for (int w = 0; w < DOK_TPB / 32; w++) total += sums[r][w];
   if (warp == 0) {                                 // 32 predecessors at a time
-    if (lane == 0) dok_post(look + tile, (tile == 0 ? DOK_LB_TOTAL : DOK_LB_LOCAL) | total);
     unsigned before = 0;
     int spins = 0;
     for (ll_t end = tile; end > 0;) {
@@ -529,16 +572,8 @@ __global__ void __launch_bounds__(DOK_TPB) k_remove_unique(DevTable t, DevHash h
     }
   }
   __syncthreads();
-  unsigned at = base_of_tile;
-  for (int r = 0; r < ROUNDS; r++) {
-    unsigned mine = at;
-    for (int w = 0; w < DOK_TPB / 32; w++) {
-      if (w < warp) mine += sums[r][w];
-      at += sums[r][w];
-    }
-    mine += __popc(head_votes[r] & ((1u << lane) - 1u));
-    if (((head_votes[r] >> lane) & 1u) && mine < n) out_removed[mine] = (uint8_t)((flags >> r) & 1u);
-  }
+  for (unsigned i = tid; i < total; i += DOK_TPB)
+    if (base_of_tile + i < n) out_removed[base_of_tile + i] = hit_of[i];
 }
 
 struct SortWork {
