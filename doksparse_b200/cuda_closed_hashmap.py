@@ -68,11 +68,12 @@ _rings = _PinnedRings()
 class _Shared:
     """What shallow clones (views) must see together: the duplicate-resolution stamps with their epoch, and the host-side
     upper bound of n_elements that lets `set` skip a device synchronisation."""
-    __slots__ = ("stamp", "epoch", "bound", "base", "snapshots", "ring", "device")
+    __slots__ = ("stamp", "epoch", "bound", "base", "snapshots", "ring", "device", "known")
 
     def __init__(self, stamp=None, epoch=0, bound=0):
         self.stamp, self.epoch, self.bound, self.base = stamp, epoch, bound, bound
         self.snapshots, self.ring, self.device = [], None, None
+        self.known = False              # the bound is n_elements itself
 
     def __del__(self):
         if self.ring is not None and _rings is not None:         # (None: the interpreter is going down)
@@ -82,6 +83,7 @@ class _Shared:
         """n_elements is known to be n, and nothing enqueued later has been counted in."""
         self.snapshots.clear()
         self.bound = self.base = n
+        self.known = True
 
 
 _Layout = namedtuple("_Layout", "slot_bytes slots_per_group value_offset key_offset stamp_offset n_slots total_bytes")
@@ -257,6 +259,7 @@ class CudaClosedHashmap:
     def _adjust(self, by):
         """n_elements += by (a number or a device scalar) without a change of the slots in use."""
         self._state[_ADJUST] += by
+        self._shared.known = False
         self._shared.bound += by if isinstance(by, int) else 0
 
     def _counter_block(self, block):
@@ -427,6 +430,7 @@ class CudaClosedHashmap:
     # the last one.
     def _after_mutation(self, added):
         sh = self._shared
+        sh.known = False
         sh.bound += added
         for s in sh.snapshots:
             s[1] += added                       # rows that may have been inserted after that snapshot was taken
@@ -697,12 +701,11 @@ class CudaClosedHashmap:
         self._materialise_parameters()
         limit = int(self._rehash_threshold * self.n_buckets)
         row_counted = new_keys.dtype in L.FLOAT_DTYPES
-        # the bound may only be stale (the host runs ahead of the device): fetch the exact count before paying for a pass
-        # that counts the distinct new keys
-        # The distinct new keys (cuda_closed_hashmap.py:350-363) are counted with a scratch set on the device: uuids of
+        # Where the bound may only be stale (the host runs ahead of the device), the exact count is fetched before paying for
+        # a pass that counts the distinct new keys.  The distinct new keys (cuda_closed_hashmap.py:350-363) are counted with a scratch set on the device: uuids of
         # integer keys, ROWS of floating ones like in the reference, because the value cast makes many rows share a uuid.
         plan = self._native_plan()
-        if self._room_for(n, limit) or self.n_elements + n <= limit:
+        if self._room_for(n, limit) or (not self._shared.known and self.n_elements + n <= limit):
             # whatever the number of new keys is, the reference would not rehash: insert and count on the device
             if row_counted:
                 plan.count_new(new_keys, _BY_ROWS, False, self._shared.bound == 0)
@@ -710,7 +713,9 @@ class CudaClosedHashmap:
             self._after_mutation(n)
             return
         state = plan.count_new(new_keys, _COUNTED_NEW, True, self._shared.bound == 0)
-        n_elements, live = self._sizes(state)[:2]
+        n_elements, live, _, failed = self._sizes(state)
+        if failed:
+            self.n_elements             # raises
         n_new = state[_COUNTED_NEW]
         if n_elements + n_new > limit:
             self.rehash(int((n_elements + n_new) * self._rehash_factor), live)
