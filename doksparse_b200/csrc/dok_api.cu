@@ -60,24 +60,24 @@ __global__ void __launch_bounds__(DOK_TPB) k_dense_count(const T *__restrict__ d
 
 struct DenseShape { int ndim; ll_t sizes[DOK_MAX_KEY_SIZE]; };
 
-// A block takes DOK_DENSE_SPAN consecutive elements at a time: every thread looks at DOK_DENSE_ROUNDS of them
-// (coalesced), the non-zero ones are collected in shared memory (position and value), and whenever 256 have come together
-// the block inserts them with every lane busy; what is left over waits for the next span.  An insert costs a block the same
-// few dependent round trips to the table for 20 elements as for 256, and at 1 % density a span holds 20: inserting span by
-// span took 530 us for the 671 k non-zeros of 8192^2 elements.
+// A warp takes DOK_DENSE_SPAN consecutive elements at a time, DOK_DENSE_ROUNDS per lane (coalesced, and requested while the
+// span before is worked on); the non-zero ones are collected in the warp's list in shared memory (position and value), and
+// whenever 32 have come together the warp inserts them with every lane busy; what is left over waits for the next span.
+// Inserting span by span took 530 us for the 671 k non-zeros of 8192^2 elements, with lists of whole blocks, whose warps
+// wait for one another three times a span, 144.
 #define DOK_DENSE_ROUNDS 8
-#define DOK_DENSE_SPAN (DOK_TPB * DOK_DENSE_ROUNDS)
+#define DOK_DENSE_SPAN (32 * DOK_DENSE_ROUNDS)
 
 template <int SB, typename T>
 __global__ void __launch_bounds__(DOK_TPB, 4) k_dense_insert(DevTable t, DevHash hp, const T *__restrict__ dense, ll_t numel,
                                                           int is_float, DenseShape shape, ll_t *counters) {
-  __shared__ ll_t found_at[DOK_DENSE_SPAN + DOK_TPB];
-  __shared__ T found_value[DOK_DENSE_SPAN + DOK_TPB];
-  __shared__ int n_found;
-  const ll_t stride = (ll_t)gridDim.x * DOK_DENSE_SPAN;
-  int claimed = 0, reused = 0, failed = 0, hits = 0;
-  if (threadIdx.x == 0) n_found = 0;
-  __syncthreads();
+  __shared__ ll_t list_at[DOK_WARPS][DOK_DENSE_SPAN + 32];
+  __shared__ T list_value[DOK_WARPS][DOK_DENSE_SPAN + 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  ll_t *const found_at = list_at[warp];
+  T *const found_value = list_value[warp];
+  const ll_t first = ((ll_t)blockIdx.x * DOK_WARPS + warp) * DOK_DENSE_SPAN, stride = (ll_t)gridDim.x * DOK_WARPS * DOK_DENSE_SPAN;
+  int claimed = 0, reused = 0, failed = 0, hits = 0, total = 0;
   const auto unravel = [&](auto rem, ll_t (&idx)[DOK_MAX_KEY_SIZE]) {          // a 64-bit division costs four of 32 bits
     using U = decltype(rem);
 #pragma unroll
@@ -90,42 +90,32 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_dense_insert(DevTable t, DevHash
       }
     }
   };
-  // the next span's elements are on their way while this one's are collected and inserted
   T v[DOK_DENSE_ROUNDS];
   const auto fetch = [&](ll_t base) {
 #pragma unroll
     for (int r = 0; r < DOK_DENSE_ROUNDS; r++) {
-      const ll_t i = base + r * DOK_TPB + (int)threadIdx.x;
+      const ll_t i = base + r * 32 + lane;
       v[r] = i < numel ? __ldcs(dense + i) : (T)0;
     }
   };
-  fetch((ll_t)blockIdx.x * DOK_DENSE_SPAN);
-  for (ll_t base = (ll_t)blockIdx.x * DOK_DENSE_SPAN; base < numel; base += stride) {     // uniform over the block
-    int in_warp = 0;
+  fetch(first);
+  for (ll_t base = first; base < numel; base += stride) {                                 // uniform over the warp
 #pragma unroll
-    for (int r = 0; r < DOK_DENSE_ROUNDS; r++) in_warp += __popc(__ballot_sync(0xffffffffu, dok_nonzero<T>(v[r], is_float)));
-    int at = 0;
-    if ((threadIdx.x & 31) == 0 && in_warp) at = atomicAdd(&n_found, in_warp);
-    at = __shfl_sync(0xffffffffu, at, 0);
-    if (in_warp) {
-#pragma unroll
-      for (int r = 0; r < DOK_DENSE_ROUNDS; r++) {
-        const bool nz = dok_nonzero<T>(v[r], is_float);
-        const unsigned votes = __ballot_sync(0xffffffffu, nz);
-        const int mine = at + __popc(votes & ((1u << (threadIdx.x & 31)) - 1u));
-        if (nz) {
-          found_value[mine] = v[r];
-          found_at[mine] = base + r * DOK_TPB + (int)threadIdx.x;
-        }
-        at += __popc(votes);
+    for (int r = 0; r < DOK_DENSE_ROUNDS; r++) {
+      const bool nz = dok_nonzero<T>(v[r], is_float);
+      const unsigned votes = __ballot_sync(0xffffffffu, nz);
+      if (nz) {
+        const int at = total + __popc(votes & ((1u << lane) - 1u));
+        found_value[at] = v[r];
+        found_at[at] = base + r * 32 + lane;
       }
+      total += __popc(votes);
     }
     fetch(base + stride);
-    __syncthreads();
+    __syncwarp();
     const bool at_end = base + stride >= numel;
-    int total = n_found;
-    while (total >= DOK_TPB || (at_end && total > 0)) {                                   // uniform over the block
-      const int k = total - 1 - (int)threadIdx.x;                                         // from the end of the list
+    while (total >= 32 || (at_end && total > 0)) {                                        // uniform over the warp
+      const int k = total - 1 - lane;                                                     // from the end of the list
       bool active = k >= 0;
       int outcome = -1;
       T value = 0;
@@ -158,11 +148,9 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_dense_insert(DevTable t, DevHash
       reused += outcome == DOK_OUT_REUSED;
       failed += outcome == DOK_OUT_FAILED;
       hits += outcome == DOK_OUT_FOUND;
-      total = total > DOK_TPB ? total - DOK_TPB : 0;
+      total = total > 32 ? total - 32 : 0;
     }
-    __syncthreads();                                     // the lists are added to by the next span
-    if (threadIdx.x == 0) n_found = total;
-    __syncthreads();
+    __syncwarp();                                        // the list is added to by the next span
   }
   if (counters) {
     dok_warp_add(counters + DOK_CNT_CLAIMED_EMPTY, claimed);
@@ -511,8 +499,8 @@ int dok_dense_insert_nonzero(const dok_table *t, const dok_hash_params *hp, cons
     prod *= shape.sizes[d];
   }
   if (prod != numel) return DOK_BAD_ARG;
-  const ll_t spans = (numel + DOK_DENSE_SPAN - 1) / DOK_DENSE_SPAN;
-  const unsigned grid = (unsigned)(spans < 148 * 4 ? spans : 148 * 4);          // one wave: each block ends with a list that is not full
+  const ll_t blocks = (numel + DOK_DENSE_SPAN * DOK_WARPS - 1) / (DOK_DENSE_SPAN * DOK_WARPS);
+  const unsigned grid = (unsigned)(blocks < 148 * 4 ? blocks : 148 * 4);        // one wave: each warp ends with a list that is not full
   cudaStream_t st = (cudaStream_t)stream;
   int rc = DOK_OK;
   switch (dt.vb) {
