@@ -76,6 +76,17 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, De
       }
     } else {
       const EmitValue<SB, LW> emit{t, out_values};
+      // 16-byte values of 32-byte slots: one store by the lane that holds the slot
+      const bool pairs = SB == 32 && t.vb == 16 && ((size_t)out_values & 15) == 0;
+      if (pairs) {
+#pragma unroll
+        for (unsigned r = 0; r < 4; r++) {
+          const unsigned row_r = __shfl_sync(FULL, lr.row, base + r);
+          const unsigned me_r = ((match[r] | empty[r]) >> base) & 0xfu;
+          if ((unsigned)__ffs(me_r) == l + 1 && ((match[r] >> (base + l)) & 1u))
+            *(ulonglong2 *)(out_values + keys.elem(share.first + row_r) * 16) = make_ulonglong2(f.w[r][1], f.w[r][2]);
+        }
+      } else
 #pragma unroll
       for (unsigned r = 0; r < 4; r++) {
         const unsigned row_r = __shfl_sync(FULL, lr.row, base + r);

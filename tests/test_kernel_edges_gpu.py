@@ -187,3 +187,17 @@ def test_sets_with_repeated_keys(n, value_cols):
         keys = rng.integers(0, spread, (n, 1))
         pair.set(keys, rng.standard_normal((n, value_cols)))
         pair.get(keys)
+
+
+@pytest.mark.parametrize("value_cols", [4, 10])
+@pytest.mark.parametrize("offset", [0, 2])
+def test_lookups_into_outputs_that_are_only_8_byte_aligned(value_cols, offset):
+    from doksparse_b200 import CudaClosedHashmap
+    np.random.seed(5)
+    n = 5000
+    table = CudaClosedHashmap(n_buckets=1 << 14)
+    keys, stored = torch.arange(n, device="cuda")[:, None] * 3, torch.randn(n, value_cols, device="cuda")
+    table.set(keys, stored)
+    values = torch.empty(n * value_cols + offset, device="cuda")[offset:].reshape(n, value_cols)
+    out, found = table.get(keys, values=values)
+    assert found.all() and torch.equal(out, stored) and out.data_ptr() == values.data_ptr()
