@@ -541,6 +541,14 @@ struct EmitValue {
       }
     } else {
       const int start = pos * SB + 8 - 32 * l;             // offset of the value relative to this lane's chunk
+      if ((t.vb & 7) == 0) {
+#pragma unroll
+        for (int j = 0; j < LW; j++) {
+          const int rel = 8 * j - start;
+          if ((unsigned)rel < (unsigned)t.vb) *(ull_t *)(dst + rel) = w[j];
+        }
+        return;
+      }
       const int align = (t.vb & -t.vb) < 8 ? (t.vb & -t.vb) : 8;
 #pragma unroll
       for (int j = 0; j < LW; j++) {
