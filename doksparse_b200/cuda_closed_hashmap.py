@@ -18,7 +18,6 @@ What is different (the slot layout is not part of the contract)
 """
 import ctypes
 import math
-import threading
 from collections import namedtuple
 
 import numpy as np
@@ -41,25 +40,30 @@ _COUNTED_NEW = 23        # result of the exact count of a set that may have to g
 class _PinnedRings:
     """Pinned landing places for copies of the counters, 8 per table, cut from chunks that serve 64 tables: pinning memory
     takes milliseconds (33 ms once the process has mapped a few GB), more than anything else a new table does.  A table
-    gives its ring back when it goes; at most 256 are kept."""
+    gives its ring back when it goes; about 256 are kept.
+
+    No lock: `give` runs where the cyclic collector frees a table, which can be in the middle of `take` on the same thread.
+    Taking from and adding to the end of a list are single steps; two threads that both find it empty make a chunk each."""
 
     def __init__(self):
-        self._lock, self._free = threading.Lock(), {}
+        self._free = {}
 
     def take(self, device):
-        with self._lock:
-            free = self._free.setdefault(device, [])
-            if not free:
-                chunk = torch.zeros(64, 8 * _STATE_WORDS, dtype=torch.long, pin_memory=True)
-                free += [L.native().Ring(words, device) for words in chunk]
+        free = self._free.setdefault(device, [])
+        try:
             ring = free.pop()
+        except IndexError:
+            chunk = torch.zeros(64, 8 * _STATE_WORDS, dtype=torch.long, pin_memory=True)
+            rings = [L.native().Ring(words, device) for words in chunk]
+            ring = rings.pop()
+            free.extend(rings)
         ring.wait(-1)                   # the previous owner's copies have landed: nothing writes here any more
         return ring
 
     def give(self, ring, device):
-        with self._lock:
-            if len(self._free[device]) < 256:
-                self._free[device].append(ring)
+        free = self._free[device]
+        if len(free) < 256:
+            free.append(ring)
 
 
 _rings = _PinnedRings()

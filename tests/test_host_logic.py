@@ -68,3 +68,31 @@ def test_sliced_exchange_geometry():
         assert sizes[3] >= world * rows * 8 and sizes[4] >= world * rows
         assert all(o % 256 == 0 for o in offs) and all(offs[i] + sizes[i] == offs[i + 1] for i in range(4))
         assert g["gen_bytes"] == offs[4] + sizes[4]
+
+
+def test_a_table_that_is_collected_while_a_ring_is_taken():
+    """The cyclic collector can free a table, which gives its ring back, while another table's ring is being made."""
+    import threading
+    from types import SimpleNamespace
+    from unittest import mock
+    from doksparse_b200 import cuda_closed_hashmap as M
+
+    rings, made, taken = M._PinnedRings(), [], []
+
+    class Ring:
+        def __init__(self, words, device):
+            made.append(self)
+            if len(made) == 70:                              # in the middle of the second chunk
+                rings.give(taken.pop(), device)
+
+        def wait(self, place):
+            pass
+
+    with mock.patch.object(M.L, "native", lambda: SimpleNamespace(Ring=Ring)), \
+            mock.patch.object(M.torch, "zeros", lambda *shape, **options: range(shape[0])):
+        worker = threading.Thread(target=lambda: [taken.append(rings.take(0)) for _ in range(65)], daemon=True)
+        worker.start()
+        worker.join(timeout=20)
+    assert not worker.is_alive()
+    assert len(made) == 128 and len(taken) == 64 and len(rings._free[0]) == 64
+    assert len(set(map(id, taken + rings._free[0]))) == 128
