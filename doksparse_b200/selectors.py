@@ -54,9 +54,10 @@ def normalise_selectors(selectors, shape, device):
     expanded += [slice(None)] * (ndim - len(expanded))                            # :255
 
     scalar_positions = [i for i, s in enumerate(expanded) if isinstance(s, Tensor) and s.ndim == 0]   # :256
-    tensor_shapes = [s.shape for s in expanded if isinstance(s, Tensor)]
+    tensors = [s for s in expanded if isinstance(s, Tensor)]
     n_slices = sum(isinstance(s, slice) for s in expanded)
-    block_shape = tuple(torch.broadcast_shapes(*tensor_shapes)) if tensor_shapes else ()             # :258-262
+    # (torch.broadcast_shapes imports sympy on its first call, 1.4 s in the first assignment of a process)
+    block_shape = tuple(torch.broadcast_tensors(*tensors)[0].shape) if tensors else ()               # :258-262
     out_ndim = len(block_shape) + n_slices                                        # :264
     first_tensor = next((i for i, s in enumerate(expanded) if isinstance(s, Tensor)), None)
 
