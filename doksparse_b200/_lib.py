@@ -93,6 +93,7 @@ def _declare(lib):
         "dok_map_count_new_rows": ([TP, HP, P, I64, P, I64, P, P], I),
         "dok_map_remove_unique_bytes": ([I64], I64),
         "dok_map_remove_unique": ([TP, HP, P, I64, P, P, P, P, P], I),
+        "dok_map_remove_unique_words": ([TP, HP, P, I64, P, P, I, P, P, P], I),
         "dok_static_scratch_max_rows": ([], I64),
         "dok_map_count_new_static": ([TP, HP, P, I64, P, P], I),
         "dok_map_get_sliced": ([TP, HP, P, I64, I64, P, P, P, P, P, P, P], I),

@@ -424,11 +424,19 @@ PyObject *plan_remove(Plan *self, PyObject *arg) {
     if (bytes) work = at::empty({bytes}, on_device(self, at::kByte));
     volatile int64_t *count = pinned_words();
     *count = -2;
-    const int status = dok_map_remove_unique(&self->table, &self->hash, keys->data_ptr(), n, (uint8_t *)removed.data_ptr(),
-                                             bytes ? work.data_ptr() : nullptr, (int64_t *)count, self->state + STATE_REMOVE, stream.stream());
+    int status = dok_map_remove_unique(&self->table, &self->hash, keys->data_ptr(), n, (uint8_t *)removed.data_ptr(),
+                                       bytes ? work.data_ptr() : nullptr, (int64_t *)count, self->state + STATE_REMOVE, stream.stream());
     if (status == DOK_TOO_LARGE) Py_RETURN_NONE;
     if (!check(status, "dok_map_remove_unique")) return nullptr;
     wait_for(stream);
+    if (*count < -DOK_SORT_ALL_WORDS) {
+      const int words = (int)(-*count - DOK_SORT_ALL_WORDS);
+      *count = -2;
+      status = dok_map_remove_unique_words(&self->table, &self->hash, keys->data_ptr(), n, (uint8_t *)removed.data_ptr(), work.data_ptr(), words,
+                                           (int64_t *)count, self->state + STATE_REMOVE, stream.stream());
+      if (!check(status, "dok_map_remove_unique_words")) return nullptr;
+      wait_for(stream);
+    }
     if (*count == -1) Py_RETURN_NONE;
     if (*count < 0) { PyErr_SetString(dok_error, "dok_map_remove_unique: a wait between blocks ran out"); return nullptr; }
     return THPVariable_Wrap(removed.narrow(0, 0, *count));

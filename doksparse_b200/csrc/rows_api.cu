@@ -1,5 +1,7 @@
 // Row-wise passes that the reference leaves to `unique(dim=0)`: the count of the distinct new rows of a float-key set
 // (cuda_closed_hashmap.py:350-363) and the removal of a batch's sorted unique rows (:438-454).
+#include <cstddef>
+#include <type_traits>
 #include "dok_kernels.cuh"
 
 // ---------------------------------------------------------------------------------------------------------
@@ -7,8 +9,8 @@
 // ---------------------------------------------------------------------------------------------------------
 
 // Element as an unsigned number of the type's width that sorts like the element: the sign bit flipped for signed
-// integers, all bits for negative floats.  The two float zeros compare equal, so they get one image; *nan is set for a
-// NaN, which compares with nothing.
+// integers; for floats, the magnitude's bits above or below the middle, which gives the two zeros, equal, one image and
+// keeps the mantissa's low zeros of whole numbers of either sign.  *nan is set for a NaN, which compares with nothing.
 __device__ __forceinline__ ull_t dok_ordered(const void *keys, int dtype, ll_t idx, bool *nan) {
   switch (dtype) {
     case DOK_I64: return ((const ull_t *)keys)[idx] ^ 0x8000000000000000ULL;
@@ -17,22 +19,19 @@ __device__ __forceinline__ ull_t dok_ordered(const void *keys, int dtype, ll_t i
     case DOK_I8: return (unsigned)(((const unsigned char *)keys)[idx] ^ 0x80u);
     case DOK_U8: return ((const unsigned char *)keys)[idx];
     case DOK_F64: {
-      ull_t b = ((const ull_t *)keys)[idx];
-      if ((b << 1) == 0) b = 0;
-      *nan |= (b << 1) > 0xffe0000000000000ULL;
-      return (b >> 63) ? ~b : b | 0x8000000000000000ULL;
+      const ull_t b = ((const ull_t *)keys)[idx], size = b & 0x7fffffffffffffffULL;
+      *nan |= size > 0x7ff0000000000000ULL;
+      return (b >> 63) ? 0x8000000000000000ULL - size : 0x8000000000000000ULL + size;
     }
     case DOK_F32: {
-      unsigned b = ((const unsigned *)keys)[idx];
-      if ((b << 1) == 0) b = 0;
-      *nan |= (b << 1) > 0xff000000u;
-      return (b >> 31) ? (unsigned)~b : b | 0x80000000u;
+      const unsigned b = ((const unsigned *)keys)[idx], size = b & 0x7fffffffu;
+      *nan |= size > 0x7f800000u;
+      return (b >> 31) ? 0x80000000u - size : 0x80000000u + size;
     }
     default: {
-      unsigned b = ((const unsigned short *)keys)[idx];
-      if ((b & 0x7fffu) == 0) b = 0;
-      *nan |= (b & 0x7fffu) > (dtype == DOK_F16 ? 0x7c00u : 0x7f80u);
-      return (b >> 15) ? (~b & 0xffffu) : b | 0x8000u;
+      const unsigned b = ((const unsigned short *)keys)[idx], size = b & 0x7fffu;
+      *nan |= size > (dtype == DOK_F16 ? 0x7c00u : 0x7f80u);
+      return (b >> 15) ? 0x8000u - size : 0x8000u + size;
     }
   }
 }
@@ -202,107 +201,247 @@ __global__ void __launch_bounds__(DOK_SMALL_TPB) k_remove_unique_small(DevTable 
 // the same for larger batches: radix sort of 32-bit prefixes, ties by row
 // ---------------------------------------------------------------------------------------------------------
 
-// A row's columns are packed, first column on top, each in as many bits as the batch's smallest and largest value differ
-// by; the leading 32 bits of that are the prefix, and four passes of a single-pass-per-digit radix sort (D. Merrill and
-// M. Garland, "Single-pass parallel prefix scan with decoupled look-back", 2016; A. Adinets and D. Merrill, "Onesweep",
-// 2022) bring the row numbers into prefix order.  Where the packed columns have more than 32 bits, runs of equal prefixes
-// that hold different rows -- a handful for scattered keys -- are put in order by one thread each.  Half the passes of a
-// 64-bit sort, and rows of any number of columns at the price of one; a comparison sort of rows took 0.37 ms for 250 k
-// rows of three floats.  Digits that all rows share are skipped.
+// A row's columns are packed, first column on top, each in as many bits as its values differ in: those of the largest less
+// the smallest, without the low bits that all rows share (the empty end of the mantissa of whole numbers).  The leading 32
+// bits of that are the prefix, and four passes of a single-pass-per-digit radix sort (D. Merrill and M. Garland,
+// "Single-pass parallel prefix scan with decoupled look-back", 2016; A. Adinets and D. Merrill, "Onesweep", 2022) bring the
+// row numbers into prefix order.  Digits that all rows share are skipped.  Where the packed row has more than 32 bits, runs
+// of equal prefixes that hold different rows -- a handful for scattered keys -- are put in order afterwards.  Half the
+// passes of a 64-bit sort, and rows of any number of columns at the price of one; a comparison sort of rows took 0.37 ms
+// for 250 k rows of three floats.
+//
+// Where such runs are the rule (ids of a few bits more than 32 of which the small ones are in every batch, few values in the
+// first columns), the rows are sorted by every word of the packed row instead, the last word first: the host is told how
+// many there are and calls again.  Whether they are the rule is estimated before the first pass, on samples of the batch
+// (a call of remove(), 1 M / 6.4 M rows, us.  Ids that are Zipf-distributed over 2^34: 647 / 2023 where a batch with a run of
+// more than 64 rows was given back to the library after the passes, 272 / 796 by all words.  Three floats below 1000: 838 /
+// 4288, 317 / 1279.  The prefix alone tells three floats below 2^20 well enough apart: 263 at 1 M, 465 by all words).
 #define DOK_SORT_TPB 256
 #define DOK_SORT_ITEMS 16                  // per thread; a quarter where that leaves SMs without a tile
 #define DOK_SORT_SMALL_ITEMS 4
 #define DOK_SORT_SMALL (148LL * DOK_SORT_TPB * DOK_SORT_ITEMS)
 #define DOK_SORT_MAX_ROWS (1LL << 30)      // counts travel in 30 bits beside two flags
 #define DOK_SORT_SPINS (1 << 22)           // bound of every wait for another block; far beyond what one takes
-#define DOK_MAX_RUN 64                     // longest run of equal prefixes with different rows that one thread sorts
+#define DOK_MAX_RUN 16                     // longest run of equal prefixes with different rows that one thread sorts
+#define DOK_LONG_RUNS 4096                 // places for longer ones, which a block sorts:
+#define DOK_TIES_TPB 1024
+#define DOK_BLOCK_RUN 4096                 // by a network up to here, ...
+#define DOK_MAX_DISTINCT 32                // ... beyond if they hold no more different rows than this
+#define DOK_CLUMP_SLOTS 1024               // rows per block that are looked at for the estimate
+#define DOK_CLUMPED_MIN 8
 #define DOK_UNIQUE_ROUNDS 8                // rows per thread of the removal; one of them for small batches, likewise
+
+// why nothing was removed
+enum { DOK_REFUSED_ROWS = 1, DOK_REFUSED_WAIT = 2, DOK_REFUSED_PREFIX = 3 };
 
 // zeroed before the first kernel
 struct SortControl {
   ull_t not_min[DOK_MAX_KEY_SIZE], max[DOK_MAX_KEY_SIZE];     // of the ordered images, ~min so that 0 is neutral
+  ull_t varying[DOK_MAX_KEY_SIZE];                            // bits in which a row's image differs from the first row's
+  // and again before the first word of a sort by all words
+  unsigned final_b;       // the rows in order are in buffer b
+  unsigned refused;       // DOK_REFUSED_ROWS: a NaN, or a wait of the sort that ran out; _WAIT: a wait of the removal; _PREFIX:
+                          // the sort by prefixes is not worth it, or has left a run that nobody sorts
+  // and again before each word
   unsigned hist[4][256];
   unsigned ticket[5];                                         // next tile of each pass, and of the removal
-  unsigned refused;       // 1: a NaN, a long mixed run, or a wait that ran out in the sort; 2: a wait in the removal
-  unsigned n_mixed;
-  unsigned skip[4], from_b[4], final_b;                       // plan of the passes
+  unsigned n_mixed, n_long, differ;                           // short and long mixed runs; rows of the samples in mixed runs
+  unsigned skip[4], from_b[4];                                // plan of the passes
+  unsigned long_set[DOK_LONG_RUNS], long_run[DOK_LONG_RUNS];  // the long ones' starts, + 1: as a set, and in a row
 };
 
+__device__ __forceinline__ int dok_column_shift(const SortControl *c, int i) {      // (0 in a column of one value)
+  const int shift = __ffsll((ll_t)c->varying[i]) - 1;
+  return shift < 0 ? 0 : shift;
+}
 __device__ __forceinline__ int dok_column_bits(const SortControl *c, int i) {
-  const ull_t span = c->max[i] - ~c->not_min[i];
+  const ull_t span = (c->max[i] - ~c->not_min[i]) >> dok_column_shift(c, i);
   return span ? 64 - __clzll(span) : 0;
 }
-// the leading 32 bits of the packed row (all of it when there are no more)
-__device__ __forceinline__ unsigned dok_row_prefix(const SortControl *c, const void *keys, int dtype, int ks, ll_t e) {
-  bool nan = false;
-  ull_t acc = 0;
-  int left = 32;
-  for (int i = 0; i < ks && left > 0; i++) {
-    const int w = dok_column_bits(c, i);
-    const ull_t v = dok_ordered(keys, dtype, e * ks + i, &nan) - ~c->not_min[i];
-    if (w <= left) { acc = (acc << w) | v; left -= w; }
-    else { acc = (acc << left) | (v >> (w - left)); left = 0; }
-  }
-  return (unsigned)acc;
-}
-__device__ __forceinline__ bool dok_prefix_is_row(const SortControl *c, int ks) {
+__device__ __forceinline__ int dok_row_words(const SortControl *c, int ks) {
   int bits = 0;
   for (int i = 0; i < ks; i++) bits += dok_column_bits(c, i);
-  return bits <= 32;
+  return bits <= 32 ? 1 : (bits + 31) / 32;
+}
+__device__ __forceinline__ bool dok_prefix_is_row(const SortControl *c, int ks) { return dok_row_words(c, ks) == 1; }
+
+// How a row is packed, in shared memory.
+struct RowPack {
+  ull_t min[DOK_MAX_KEY_SIZE];
+  int shift[DOK_MAX_KEY_SIZE], bits[DOK_MAX_KEY_SIZE];
+};
+__device__ __forceinline__ void dok_load_pack(RowPack &pack, const SortControl *c, int ks) {
+  const int i = threadIdx.x;
+  if (i < ks) {
+    pack.min[i] = ~c->not_min[i];
+    pack.shift[i] = dok_column_shift(c, i);
+    pack.bits[i] = dok_column_bits(c, i);
+  }
+}
+// Bits 32 * word .. 32 * word + 31 of the packed row, counted from its leading bit; the last word has what is left.
+// HASH: with a hash of the whole row.
+template <bool HASH>
+__device__ __forceinline__ unsigned dok_row_word(const RowPack &pack, const void *keys, int dtype, int ks, ll_t e, int word, unsigned *rest) {
+  bool nan = false;
+  ull_t acc = 0, hash = 0;
+  const int from = 32 * word, to = from + 32;
+  int at = 0;
+  for (int i = 0; i < ks && (HASH || at < to); i++) {
+    const int end = at + pack.bits[i], lo = at > from ? at : from, hi = end < to ? end : to;
+    if (HASH || lo < hi) {
+      const ull_t v = (dok_ordered(keys, dtype, e * ks + i, &nan) - pack.min[i]) >> pack.shift[i];
+      if (lo < hi) acc = (acc << (hi - lo)) | ((v >> (end - hi)) & ((1ULL << (hi - lo)) - 1ULL));
+      if (HASH) hash = (hash ^ v) * 0x9e3779b97f4a7c15ULL;
+    }
+    at = end;
+  }
+  if (HASH) *rest = (unsigned)(hash >> 32);
+  return (unsigned)acc;
 }
 
-__global__ void __launch_bounds__(DOK_TPB) k_row_range(RowKeys keys, int dtype, int ks, SortControl *c) {
-  __shared__ ull_t lo_hi[2 * DOK_MAX_KEY_SIZE];
-  if (threadIdx.x < 2 * DOK_MAX_KEY_SIZE) lo_hi[threadIdx.x] = 0;
+// The loop below knows the type, so that four loads are on their way at a time.
+template <class F>
+__device__ __forceinline__ void dok_with_dtype(int dtype, const F &f) {
+  switch (dtype) {
+    case DOK_I64: f(std::integral_constant<int, DOK_I64>()); break;
+    case DOK_I32: f(std::integral_constant<int, DOK_I32>()); break;
+    case DOK_I16: f(std::integral_constant<int, DOK_I16>()); break;
+    case DOK_I8: f(std::integral_constant<int, DOK_I8>()); break;
+    case DOK_U8: f(std::integral_constant<int, DOK_U8>()); break;
+    case DOK_F64: f(std::integral_constant<int, DOK_F64>()); break;
+    case DOK_F32: f(std::integral_constant<int, DOK_F32>()); break;
+    case DOK_F16: f(std::integral_constant<int, DOK_F16>()); break;
+    default: f(std::integral_constant<int, DOK_BF16>()); break;
+  }
+}
+
+struct ColumnRange { ull_t not_min, max, varying; };
+
+#define DOK_RANGE_BLOCKS 5                 // per SM, resident
+__global__ void __launch_bounds__(DOK_TPB, DOK_RANGE_BLOCKS) k_row_range(RowKeys keys, int dtype, int ks, SortControl *c) {
+  __shared__ ull_t lo_hi[3 * DOK_MAX_KEY_SIZE];
+  if (threadIdx.x < 3 * DOK_MAX_KEY_SIZE) lo_hi[threadIdx.x] = 0;
   __syncthreads();
   bool nan = false;
-  const ll_t stride = (ll_t)gridDim.x * DOK_TPB;
+  const ll_t stride = (ll_t)gridDim.x * DOK_TPB, n = keys.n;
   for (int i = 0; i < ks; i++) {
-    ull_t not_min = 0, max = 0;
-    for (ll_t e = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x; e < keys.n; e += stride) {
-      const ull_t v = dok_ordered(keys.keys, dtype, e * ks + i, &nan);
-      not_min = ~v > not_min ? ~v : not_min;
-      max = v > max ? v : max;
-    }
+    ColumnRange r{0, 0, 0};
+    dok_with_dtype(dtype, [&](auto type) {
+      constexpr int TYPE = decltype(type)::value;
+      const ull_t first = dok_ordered(keys.keys, TYPE, i, &nan);
+      const auto add = [&](ull_t v) {
+        r.not_min = ~v > r.not_min ? ~v : r.not_min;
+        r.max = v > r.max ? v : r.max;
+        r.varying |= v ^ first;
+      };
+      ll_t e = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x;
+      for (; e + 3 * stride < n; e += 4 * stride) {
+        ull_t v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = dok_ordered(keys.keys, TYPE, (e + k * stride) * ks + i, &nan);
+#pragma unroll
+        for (int k = 0; k < 4; k++) add(v[k]);
+      }
+      for (; e < n; e += stride) add(dok_ordered(keys.keys, TYPE, e * ks + i, &nan));
+    });
     for (int o = 16; o > 0; o >>= 1) {
-      const ull_t a = __shfl_xor_sync(0xffffffffu, not_min, o), b = __shfl_xor_sync(0xffffffffu, max, o);
-      not_min = a > not_min ? a : not_min;
-      max = b > max ? b : max;
+      const ull_t a = __shfl_xor_sync(0xffffffffu, r.not_min, o), b = __shfl_xor_sync(0xffffffffu, r.max, o);
+      r.not_min = a > r.not_min ? a : r.not_min;
+      r.max = b > r.max ? b : r.max;
+      r.varying |= __shfl_xor_sync(0xffffffffu, r.varying, o);
     }
     if ((threadIdx.x & 31) == 0) {
-      atomicMax(&lo_hi[2 * i], not_min);
-      atomicMax(&lo_hi[2 * i + 1], max);
+      atomicMax(&lo_hi[3 * i], r.not_min);
+      atomicMax(&lo_hi[3 * i + 1], r.max);
+      atomicOr(&lo_hi[3 * i + 2], r.varying);
     }
   }
   nan = __syncthreads_or(nan);
   if (threadIdx.x < ks) {
-    atomicMax(&c->not_min[threadIdx.x], lo_hi[2 * threadIdx.x]);
-    atomicMax(&c->max[threadIdx.x], lo_hi[2 * threadIdx.x + 1]);
+    atomicMax(&c->not_min[threadIdx.x], lo_hi[3 * threadIdx.x]);
+    atomicMax(&c->max[threadIdx.x], lo_hi[3 * threadIdx.x + 1]);
+    atomicOr(&c->varying[threadIdx.x], lo_hi[3 * threadIdx.x + 2]);
   }
-  if (threadIdx.x == 0 && nan) c->refused = 1;
+  if (threadIdx.x == 0 && nan) c->refused = DOK_REFUSED_ROWS;
 }
 
-__global__ void __launch_bounds__(DOK_TPB) k_row_prefix(RowKeys keys, int dtype, int ks, SortControl *c, unsigned *prefix, unsigned *row) {
+__device__ __forceinline__ void dok_count_digits(unsigned (&hist)[4][256], unsigned word) {
+#pragma unroll
+  for (int d = 0; d < 4; d++) atomicAdd(&hist[d][(word >> (8 * d)) & 255u], 1u);
+}
+__device__ __forceinline__ void dok_add_digits(SortControl *c, const unsigned (&hist)[4][256]) {
+  for (int i = threadIdx.x; i < 1024; i += DOK_TPB)
+    if (((const unsigned *)hist)[i]) atomicAdd((unsigned *)c->hist + i, ((const unsigned *)hist)[i]);
+}
+
+__device__ __forceinline__ void dok_warp_count(unsigned *counter, int v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0 && v) atomicAdd(counter, (unsigned)v);
+}
+
+// The prefixes of the rows, and how many rows of the block's first DOK_CLUMP_SLOTS meet their prefix there with another
+// row: by a table that keeps the last row of each prefix (of each place, which two prefixes may share).
+__global__ void __launch_bounds__(DOK_TPB, 8) k_row_prefix(RowKeys keys, int dtype, int ks, SortControl *c, unsigned *prefix, unsigned *row) {
   __shared__ unsigned hist[4][256];
+  __shared__ ull_t seen[DOK_CLUMP_SLOTS];
+  __shared__ RowPack pack;
+  dok_load_pack(pack, c, ks);
   for (int i = threadIdx.x; i < 1024; i += DOK_TPB) ((unsigned *)hist)[i] = 0;
+  for (int i = threadIdx.x; i < DOK_CLUMP_SLOTS; i += DOK_TPB) seen[i] = ~0ULL;
   __syncthreads();
+  int bits = 0;
+  for (int i = 0; i < ks; i++) bits += pack.bits[i];
   const ll_t stride = (ll_t)gridDim.x * DOK_TPB;
-  for (ll_t e = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x; e < keys.n; e += stride) {
-    const unsigned p = dok_row_prefix(c, keys.keys, dtype, ks, e);
+  ll_t e = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x;
+  const auto put = [&](unsigned p) {
     prefix[e] = p;
     row[e] = (unsigned)e;
-#pragma unroll
-    for (int d = 0; d < 4; d++) atomicAdd(&hist[d][(p >> (8 * d)) & 255u], 1u);
+    dok_count_digits(hist, p);
+  };
+  if (bits > 32) {
+    int differ = 0;
+    for (int looked = 0; e < keys.n && looked < DOK_CLUMP_SLOTS; e += stride, looked += DOK_TPB) {
+      unsigned rest;
+      const unsigned p = dok_row_word<true>(pack, keys.keys, dtype, ks, e, 0, &rest);
+      const ull_t mine = (ull_t)p << 32 | rest, other = atomicExch(&seen[(p * 0x9e3779b1u) >> 22], mine);
+      differ += (unsigned)(other >> 32) == p && other != mine && other != ~0ULL;
+      put(p);
+    }
+    dok_warp_count(&c->differ, differ);
   }
+  for (; e < keys.n; e += stride) put(dok_row_word<false>(pack, keys.keys, dtype, ks, e, 0, nullptr));
   __syncthreads();
-  for (int i = threadIdx.x; i < 1024; i += DOK_TPB)
-    if (((unsigned *)hist)[i]) atomicAdd((unsigned *)c->hist + i, ((unsigned *)hist)[i]);
+  dok_add_digits(c, hist);
 }
 
-// digit counts -> exclusive offsets; which passes move anything, and from which buffer each one reads
-__global__ void __launch_bounds__(256) k_sort_plan(SortControl *c, unsigned n) {
+// One word of the packed rows, in the order that the rows have so far (first: their own).
+__global__ void __launch_bounds__(DOK_TPB, 8) k_row_word(RowKeys keys, int dtype, int ks, SortControl *c, int word, bool first, unsigned *key_a,
+                                                      unsigned *row_a, unsigned *key_b, unsigned *row_b) {
+  __shared__ unsigned hist[4][256];
+  __shared__ RowPack pack;
+  dok_load_pack(pack, c, ks);
+  for (int i = threadIdx.x; i < 1024; i += DOK_TPB) ((unsigned *)hist)[i] = 0;
+  __syncthreads();
+  unsigned *key = c->final_b ? key_b : key_a, *row = c->final_b ? row_b : row_a;
+  const ll_t stride = (ll_t)gridDim.x * DOK_TPB;
+  for (ll_t i = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x; i < keys.n; i += stride) {
+    if (first) row[i] = (unsigned)i;
+    const unsigned e = first ? (unsigned)i : row[i];
+    if (e >= keys.n) continue;                                // (a wait of an earlier pass ran out: nothing is removed)
+    const unsigned w = dok_row_word<false>(pack, keys.keys, dtype, ks, e, word, nullptr);
+    key[i] = w;
+    dok_count_digits(hist, w);
+  }
+  __syncthreads();
+  dok_add_digits(c, hist);
+}
+
+// digit counts -> exclusive offsets; which passes move anything, and from which buffer each one reads.  None does where the
+// sort by prefixes gives up: `clumped` rows of the samples or more are in mixed runs (0: no limit).
+__global__ void __launch_bounds__(256) k_sort_plan(SortControl *c, unsigned n, unsigned clumped) {
   __shared__ unsigned sums[8];
-  unsigned in_b = 0;
+  const bool give_up = c->refused != 0 || (clumped && c->differ >= clumped);
+  unsigned in_b = c->final_b;
   for (int d = 0; d < 4; d++) {
     const unsigned own = c->hist[d][threadIdx.x];
     unsigned v = own;
@@ -311,14 +450,17 @@ __global__ void __launch_bounds__(256) k_sort_plan(SortControl *c, unsigned n) {
       if ((threadIdx.x & 31) >= o) v += u;
     }
     if ((threadIdx.x & 31) == 31) sums[threadIdx.x >> 5] = v;
-    const bool same = __syncthreads_or(own == n);
+    const bool same = __syncthreads_or(own == n) || give_up;
     for (int w = 0; w < (int)(threadIdx.x >> 5); w++) v += sums[w];
     c->hist[d][threadIdx.x] = v - own;
     if (threadIdx.x == 0) { c->skip[d] = same; c->from_b[d] = in_b; }
     if (!same) in_b ^= 1;
     __syncthreads();
   }
-  if (threadIdx.x == 0) c->final_b = in_b;
+  if (threadIdx.x == 0) {
+    c->final_b = in_b;
+    if (give_up && c->refused == 0) c->refused = DOK_REFUSED_PREFIX;
+  }
 }
 
 #define DOK_LB_LOCAL 0x40000000u           // a tile's own count
@@ -390,7 +532,7 @@ __global__ void __launch_bounds__(DOK_SORT_TPB) k_sort_pass(SortControl *c, int 
     const unsigned s = dok_peek(look + (size_t)(p - 1) * 256 + tid);
     if (s == 0) {
       if (++spins < DOK_SORT_SPINS) continue;
-      c->refused = 1;
+      c->refused = DOK_REFUSED_ROWS;
       break;
     }
     before += s & DOK_LB_VALUE;
@@ -416,43 +558,134 @@ __global__ void __launch_bounds__(DOK_SORT_TPB) k_sort_pass(SortControl *c, int 
   }
 }
 
-// Runs of equal prefixes that hold different rows.  LIST: the first place where two neighbours of such a run differ lists
-// the run's start (nothing is written to the rows meanwhile); otherwise: one thread per listed run sorts it by insertion.
-template <bool LIST>
-__global__ void __launch_bounds__(DOK_TPB) k_sort_ties(SortControl *c, RowKeys keys, int dtype, int ks, unsigned *key_a, unsigned *row_a,
-                                                       unsigned *key_b, unsigned *row_b) {
+// first place of [lo, hi) whose key is >= k, of a sorted array
+__device__ __forceinline__ unsigned dok_lower_bound(const unsigned *key, unsigned lo, unsigned hi, unsigned k) {
+  while (lo < hi) {
+    const unsigned mid = lo + (hi - lo) / 2;
+    if (key[mid] < k) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+// Runs of equal prefixes that hold different rows are listed by their start: at the first place where two neighbours differ,
+// in a run of more than DOK_MAX_RUN rows by each such place that has none in the DOK_MAX_RUN rows before it.
+__global__ void __launch_bounds__(DOK_TPB) k_list_ties(SortControl *c, RowKeys keys, int dtype, int ks, unsigned *key_a, const unsigned *row_a,
+                                                       unsigned *key_b, const unsigned *row_b) {
   const unsigned n = (unsigned)keys.n;
   if (c->refused || dok_prefix_is_row(c, ks)) return;
-  const unsigned *key = c->final_b ? key_b : key_a;
-  unsigned *row = c->final_b ? row_b : row_a, *list = c->final_b ? key_a : key_b;
+  const unsigned *key = c->final_b ? key_b : key_a, *row = c->final_b ? row_b : row_a;
+  unsigned *list = c->final_b ? key_a : key_b;
   const unsigned stride = gridDim.x * DOK_TPB;
-  if (LIST) {
-    for (unsigned i = blockIdx.x * DOK_TPB + threadIdx.x; i + 1 < n; i += stride) {
-      if (key[i] != key[i + 1] || dok_compare_rows(keys.keys, dtype, ks, row[i], row[i + 1]) == 0) continue;
-      unsigned lo = i;
-      int steps = 0;
-      bool first = true;
-      while (lo > 0 && key[lo - 1] == key[i] && first && steps < DOK_MAX_RUN) {
-        first = dok_compare_rows(keys.keys, dtype, ks, row[lo - 1], row[lo]) == 0;
-        lo--;
-        steps++;
-      }
-      if (!first) continue;                          // an earlier place lists the run
-      if (steps == DOK_MAX_RUN) { c->refused = 1; return; }
-      list[atomicAdd(&c->n_mixed, 1u)] = lo;
+  for (unsigned i = blockIdx.x * DOK_TPB + threadIdx.x; i + 1 < n; i += stride) {
+    if (key[i] != key[i + 1] || dok_compare_rows(keys.keys, dtype, ks, row[i], row[i + 1]) == 0) continue;
+    unsigned lo = i;
+    bool first = true;
+    while (first && lo > 0 && key[lo - 1] == key[i] && i - lo < DOK_MAX_RUN) {
+      first = dok_compare_rows(keys.keys, dtype, ks, row[lo - 1], row[lo]) == 0;
+      lo--;
     }
-  } else {
-    for (unsigned m = blockIdx.x * DOK_TPB + threadIdx.x; m < c->n_mixed; m += stride) {
-      const unsigned lo = list[m];
-      unsigned hi = lo + 1;
-      while (hi < n && hi - lo <= DOK_MAX_RUN && key[hi] == key[lo]) hi++;
-      if (hi - lo > DOK_MAX_RUN) { c->refused = 1; return; }
-      for (unsigned i = lo + 1; i < hi; i++) {
-        const unsigned r = row[i];
-        unsigned j = i;
-        for (; j > lo && dok_compare_rows(keys.keys, dtype, ks, r, row[j - 1]) < 0; j--) row[j] = row[j - 1];
-        row[j] = r;
+    if (!first) continue;                          // an earlier place lists the run
+    if (n - lo <= DOK_MAX_RUN || key[lo + DOK_MAX_RUN] != key[i]) {
+      list[atomicAdd(&c->n_mixed, 1u)] = lo;
+      continue;
+    }
+    lo = dok_lower_bound(key, 0, i, key[i]);
+    unsigned at = lo * 0x9e3779b1u % DOK_LONG_RUNS, tries = 0;
+    for (; tries < DOK_LONG_RUNS; tries++) {
+      const unsigned old = atomicCAS(&c->long_set[at], 0u, lo + 1);
+      if (old == 0) c->long_run[atomicAdd(&c->n_long, 1u)] = lo + 1;
+      if (old == 0 || old == lo + 1) break;
+      at = (at + 1) % DOK_LONG_RUNS;
+    }
+    if (tries == DOK_LONG_RUNS) { c->refused = DOK_REFUSED_PREFIX; return; }
+  }
+}
+
+// The smallest row of a block's threads, and how many hold one that equals it.
+struct SmallestRow { unsigned row, count; };
+#define DOK_NO_ROW 0xffffffffu
+__device__ __forceinline__ SmallestRow dok_smaller(const RowKeys &keys, int dtype, int ks, SmallestRow a, SmallestRow b) {
+  if (a.row == DOK_NO_ROW) return b;
+  if (b.row == DOK_NO_ROW) return a;
+  const int order = dok_compare_rows(keys.keys, dtype, ks, a.row, b.row);
+  if (order) return order < 0 ? a : b;
+  return SmallestRow{min(a.row, b.row), a.count + b.count};
+}
+
+// A listed run of up to DOK_MAX_RUN rows is sorted by insertion, by one thread (each step waits for the one before: 64 rows
+// took 0.3 ms).  A longer one is sorted by a block: by a bitonic network where its rows fit; beyond that it is most often a
+// key that the batch repeats and another that shares its prefix, and the block looks for the smallest row, the next larger
+// one and so on, and writes each as often as it occurs (which of several equal rows it is makes no difference).  A batch of
+// 6.4 M rows with 2.5 M different keys, Zipf-distributed, has about ten long runs.
+__global__ void __launch_bounds__(DOK_TIES_TPB) k_sort_ties(SortControl *c, RowKeys keys, int dtype, int ks, const unsigned *key_a, unsigned *row_a,
+                                                       const unsigned *key_b, unsigned *row_b) {
+  __shared__ SmallestRow best_of[DOK_TIES_TPB / 32];
+  __shared__ unsigned run[DOK_BLOCK_RUN];
+  const unsigned n = (unsigned)keys.n;
+  if (c->refused == DOK_REFUSED_ROWS || dok_prefix_is_row(c, ks)) return;      // (_PREFIX: set before, or by a block of this kernel)
+  const unsigned *key = c->final_b ? key_b : key_a;
+  const unsigned *list = c->final_b ? key_a : key_b;
+  unsigned *row = c->final_b ? row_b : row_a, *sorted = c->final_b ? row_a : row_b;
+  const unsigned n_long = c->n_long;
+  for (unsigned r = blockIdx.x; r < n_long; r += gridDim.x) {
+    const unsigned lo = c->long_run[r] - 1, k = key[lo], hi = k == 0xffffffffu ? n : dok_lower_bound(key, lo, n, k + 1);
+    if (hi - lo <= DOK_BLOCK_RUN) {                                             // uniform over the block
+      unsigned padded = 2;
+      while (padded < hi - lo) padded *= 2;
+      for (unsigned i = threadIdx.x; i < padded; i += DOK_TIES_TPB) run[i] = lo + i < hi ? row[lo + i] : DOK_NO_ROW;
+      __syncthreads();
+      const auto before = [&](unsigned a, unsigned b) {                         // the padding is behind every row
+        if (a == DOK_NO_ROW || b == DOK_NO_ROW) return a < b;
+        return dok_compare_rows(keys.keys, dtype, ks, a, b) < 0;
+      };
+      for (unsigned size = 2; size <= padded; size *= 2)
+        for (unsigned step = size / 2; step > 0; step /= 2) {
+          for (unsigned i = threadIdx.x; i < padded / 2; i += DOK_TIES_TPB) {
+            const unsigned p = 2 * i - (i & (step - 1)), q = p + step, a = run[p], b = run[q];
+            if ((p & size) == 0 ? before(b, a) : before(a, b)) { run[p] = b; run[q] = a; }
+          }
+          __syncthreads();
+        }
+      for (unsigned i = threadIdx.x; i < hi - lo; i += DOK_TIES_TPB) row[lo + i] = run[i];
+      __syncthreads();
+      continue;
+    }
+    unsigned out = lo, last = 0;
+    for (int d = 0; out < hi; d++) {
+      SmallestRow best{DOK_NO_ROW, 0};
+      if (d < DOK_MAX_DISTINCT)
+        for (unsigned i = lo + threadIdx.x; i < hi; i += DOK_TIES_TPB)
+          if (d == 0 || dok_compare_rows(keys.keys, dtype, ks, row[i], last) > 0)
+            best = dok_smaller(keys, dtype, ks, best, SmallestRow{row[i], 1});
+      for (int o = 16; o > 0; o >>= 1)
+        best = dok_smaller(keys, dtype, ks, best, SmallestRow{__shfl_xor_sync(0xffffffffu, best.row, o), __shfl_xor_sync(0xffffffffu, best.count, o)});
+      __syncthreads();
+      if ((threadIdx.x & 31) == 0) best_of[threadIdx.x >> 5] = best;
+      __syncthreads();
+      best = best_of[0];
+      for (int w = 1; w < DOK_TIES_TPB / 32; w++) best = dok_smaller(keys, dtype, ks, best, best_of[w]);
+      if (best.row == DOK_NO_ROW) {                                             // too many different rows
+        if (threadIdx.x == 0) c->refused = DOK_REFUSED_PREFIX;
+        break;
       }
+      last = best.row;
+      for (unsigned i = out + threadIdx.x; i < out + best.count; i += DOK_TIES_TPB) sorted[i] = last;
+      out += best.count;
+    }
+    __syncthreads();
+    if (out == hi)
+      for (unsigned i = lo + threadIdx.x; i < hi; i += DOK_TIES_TPB) row[i] = sorted[i];
+  }
+  const unsigned stride = gridDim.x * DOK_TIES_TPB, mixed = c->n_mixed;
+  for (unsigned m = blockIdx.x * DOK_TIES_TPB + threadIdx.x; m < mixed; m += stride) {
+    const unsigned lo = list[m];
+    unsigned hi = lo + 1;
+    while (hi < n && hi - lo <= DOK_MAX_RUN && key[hi] == key[lo]) hi++;
+    for (unsigned i = lo + 1; i < hi; i++) {
+      const unsigned r = row[i];
+      unsigned j = i;
+      for (; j > lo && dok_compare_rows(keys.keys, dtype, ks, r, row[j - 1]) < 0; j--) row[j] = row[j - 1];
+      row[j] = r;
     }
   }
 }
@@ -483,8 +716,9 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_remove_unique(DevTable t, DevHas
   __shared__ int removed;
   const unsigned n = (unsigned)keys.n;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (c->refused == 1) {                           // set before this kernel: nothing has been removed
-    if (blockIdx.x == 0 && tid == 0) *out_count = -1;
+  const unsigned refused = *(volatile unsigned *)&c->refused;
+  if (refused == DOK_REFUSED_ROWS || refused == DOK_REFUSED_PREFIX) {      // set before this kernel: nothing has been removed
+    if (blockIdx.x == 0 && tid == 0) *out_count = refused == DOK_REFUSED_ROWS ? -1 : -DOK_SORT_ALL_WORDS - dok_row_words(c, hp.ks);
     return;
   }
   if (tid == 0) { tile_id = atomicAdd(&c->ticket[4], 1u); removed = 0; }
@@ -553,7 +787,7 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_remove_unique(DevTable t, DevHas
       const unsigned s = p >= 0 ? dok_peek(look + p) : DOK_LB_TOTAL;
       if (__any_sync(0xffffffffu, s == 0)) {
         if (++spins < DOK_SORT_SPINS) continue;
-        if (lane == 0) c->refused = 2;
+        if (lane == 0) c->refused = DOK_REFUSED_WAIT;
         break;
       }
       const unsigned totals = __ballot_sync(0xffffffffu, (s & DOK_LB_TOTAL) != 0);
@@ -567,7 +801,7 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_remove_unique(DevTable t, DevHas
     if (lane == 0) {
       if (tile > 0) dok_post(look + tile, DOK_LB_TOTAL | (before + total));
       base_of_tile = before;
-      if (tile == tiles - 1) *out_count = *(volatile unsigned *)&c->refused == 2 ? -2 : (ll_t)before + total;
+      if (tile == tiles - 1) *out_count = *(volatile unsigned *)&c->refused == DOK_REFUSED_WAIT ? -2 : (ll_t)before + total;
       if (removed && counters) atomicAdd((ull_t *)counters + DOK_CNT_HITS, (ull_t)removed);
     }
   }
@@ -602,6 +836,36 @@ static SortWork sort_work(void *base, ll_t n) {
   w.row_b = (unsigned *)take((size_t)n * sizeof(unsigned));
   w.bytes = at;
   return w;
+}
+
+static unsigned rows_grid(ll_t n, ll_t per_sm = 8) {
+  const ll_t blocks = (n + DOK_TPB - 1) / DOK_TPB, quarter = (n + 4 * DOK_TPB - 1) / (4 * DOK_TPB);
+  // one per SM first, then four rows per thread: each block adds a thousand digit counts to the batch's
+  return (unsigned)(blocks < 148 ? blocks : quarter < 148 ? 148 : quarter < 148 * per_sm ? quarter : 148 * per_sm);
+}
+
+// the four passes over one word
+static int sort_rows(const SortWork &w, ll_t n, unsigned clumped, cudaStream_t st) {
+  int rc;
+  k_sort_plan<<<1, 256, 0, st>>>(w.control, (unsigned)n, clumped);
+  if ((rc = dok_check_launch()) != DOK_OK) return rc;
+  for (int d = 0; d < 4; d++) {
+    const auto pass = w.small ? k_sort_pass<DOK_SORT_SMALL_ITEMS> : k_sort_pass<DOK_SORT_ITEMS>;
+    pass<<<w.tiles, DOK_SORT_TPB, 0, st>>>(w.control, d, (unsigned)n, w.key_a, w.row_a, w.key_b, w.row_b,
+                                           w.look + (size_t)d * w.tiles * 256);
+    if ((rc = dok_check_launch()) != DOK_OK) return rc;
+  }
+  return DOK_OK;
+}
+
+static int remove_sorted(const DevTable &dt, const DevHash &dh, const RowKeys &rk, const SortWork &w, uint8_t *out_removed, int64_t *out_count,
+                         int64_t *counters, cudaStream_t st) {
+  const auto remove = [&](auto kernel) {
+    kernel<<<w.unique_tiles, DOK_TPB, 0, st>>>(dt, dh, rk, w.control, w.key_a, w.row_a, w.key_b, w.row_b, w.unique_look, w.unique_tiles,
+                                               out_removed, (ll_t *)out_count, (ll_t *)counters);
+  };
+  DOK_DISPATCH_SB(dt, (w.small ? remove(k_remove_unique<SB, 1>) : remove(k_remove_unique<SB, DOK_UNIQUE_ROUNDS>)));
+  return dok_check_launch();
 }
 
 extern "C" {
@@ -646,31 +910,47 @@ int dok_map_remove_unique(const dok_table *t, const dok_hash_params *hp, const v
   if (!work) return DOK_BAD_ARG;
   const SortWork w = sort_work(work, n);
   if (cudaMemsetAsync(work, 0, w.zeroed, st) != cudaSuccess) return dok_check_launch();
-  const ll_t blocks = (n + DOK_TPB - 1) / DOK_TPB;
-  const unsigned grid = (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8);
   int rc;
-  k_row_range<<<grid, DOK_TPB, 0, st>>>(rk, dh.dtype, dh.ks, w.control);
+  const unsigned grid = rows_grid(n);
+  k_row_range<<<rows_grid(n, DOK_RANGE_BLOCKS), DOK_TPB, 0, st>>>(rk, dh.dtype, dh.ks, w.control);
   if ((rc = dok_check_launch()) != DOK_OK) return rc;
   k_row_prefix<<<grid, DOK_TPB, 0, st>>>(rk, dh.dtype, dh.ks, w.control, w.key_a, w.row_a);
   if ((rc = dok_check_launch()) != DOK_OK) return rc;
-  k_sort_plan<<<1, 256, 0, st>>>(w.control, (unsigned)n);
+  // A row with m mates (other rows of its prefix) finds one among the rows before it of a block's sample of s rows in s / 2n * m
+  // of the cases.  The sort by all words is taken from four mates per row on, on average: below, the runs cost less than the
+  // further passes; and from as many as one run of more than DOK_BLOCK_RUN rows gives, which might be refused in the end (at
+  // DOK_CLUMPED_MIN such rows chance is out of the question).
+  const double block_rows = n < (ll_t)grid * DOK_CLUMP_SLOTS ? (double)n / grid : DOK_CLUMP_SLOTS, samples = block_rows * grid;
+  const double one_run = (double)DOK_BLOCK_RUN * DOK_BLOCK_RUN / n, clumped = (one_run < 4 ? one_run : 4) * samples * block_rows / (2.0 * n);
+  if ((rc = sort_rows(w, n, clumped < DOK_CLUMPED_MIN ? DOK_CLUMPED_MIN : (unsigned)clumped, st)) != DOK_OK) return rc;
+  k_list_ties<<<grid, DOK_TPB, 0, st>>>(w.control, rk, dh.dtype, dh.ks, w.key_a, w.row_a, w.key_b, w.row_b);
   if ((rc = dok_check_launch()) != DOK_OK) return rc;
-  for (int d = 0; d < 4; d++) {
-    const auto pass = w.small ? k_sort_pass<DOK_SORT_SMALL_ITEMS> : k_sort_pass<DOK_SORT_ITEMS>;
-    pass<<<w.tiles, DOK_SORT_TPB, 0, st>>>(w.control, d, (unsigned)n, w.key_a, w.row_a, w.key_b, w.row_b,
-                                           w.look + (size_t)d * w.tiles * 256);
+  k_sort_ties<<<grid < 148 ? grid : 148, DOK_TIES_TPB, 0, st>>>(w.control, rk, dh.dtype, dh.ks, w.key_a, w.row_a, w.key_b, w.row_b);
+  if ((rc = dok_check_launch()) != DOK_OK) return rc;
+  return remove_sorted(dt, dh, rk, w, out_removed, out_count, counters, st);
+}
+
+int dok_map_remove_unique_words(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n, uint8_t *out_removed,
+                                void *work, int words, int64_t *out_count, int64_t *counters, void *stream) {
+  DevHash dh;
+  DevTable dt;
+  if (!dok_make_hash(hp, &dh) || !dok_make_table(t, &dt) || dt.kb != dh.ks * dh.elem_bytes || n <= DOK_SMALL_ROWS || n > DOK_SORT_MAX_ROWS ||
+      !keys || !out_removed || !out_count || !work || words < 2 || words > 2 * DOK_MAX_KEY_SIZE || dok_window_passes(dt) > 1)
+    return DOK_BAD_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
+  RowKeys rk{keys, n};
+  const SortWork w = sort_work(work, n);
+  const unsigned grid = rows_grid(n);
+  int rc;
+  for (int word = words - 1; word >= 0; word--) {
+    const bool first = word == words - 1;
+    const size_t from = first ? offsetof(SortControl, final_b) : offsetof(SortControl, hist);
+    if (cudaMemsetAsync((char *)work + from, 0, w.zeroed - from, st) != cudaSuccess) return dok_check_launch();
+    k_row_word<<<grid, DOK_TPB, 0, st>>>(rk, dh.dtype, dh.ks, w.control, word, first, w.key_a, w.row_a, w.key_b, w.row_b);
     if ((rc = dok_check_launch()) != DOK_OK) return rc;
+    if ((rc = sort_rows(w, n, 0, st)) != DOK_OK) return rc;
   }
-  k_sort_ties<true><<<grid, DOK_TPB, 0, st>>>(w.control, rk, dh.dtype, dh.ks, w.key_a, w.row_a, w.key_b, w.row_b);
-  if ((rc = dok_check_launch()) != DOK_OK) return rc;
-  k_sort_ties<false><<<grid < 148 ? grid : 148, DOK_TPB, 0, st>>>(w.control, rk, dh.dtype, dh.ks, w.key_a, w.row_a, w.key_b, w.row_b);
-  if ((rc = dok_check_launch()) != DOK_OK) return rc;
-  const auto remove = [&](auto kernel) {
-    kernel<<<w.unique_tiles, DOK_TPB, 0, st>>>(dt, dh, rk, w.control, w.key_a, w.row_a, w.key_b, w.row_b, w.unique_look, w.unique_tiles,
-                                               out_removed, (ll_t *)out_count, (ll_t *)counters);
-  };
-  DOK_DISPATCH_SB(dt, (w.small ? remove(k_remove_unique<SB, 1>) : remove(k_remove_unique<SB, DOK_UNIQUE_ROUNDS>)));
-  return dok_check_launch();
+  return remove_sorted(dt, dh, rk, w, out_removed, out_count, counters, st);
 }
 
 }  // extern "C"

@@ -219,12 +219,17 @@ int dok_map_count_new_rows(const dok_table *t, const dok_hash_params *hp, const 
 
 /* CudaClosedHashmap.remove (cuda_closed_hashmap.py:438-454): removes the batch's unique rows and writes their flags in
  * sorted order to out_removed (room for n), their number to *out_count, which may be pinned host memory and has to hold
- * -2 before the call.  -1: a row holds a NaN, or many rows differ only in their last bits; nothing was removed, and the
- * rows have to be made unique another way.  -2 afterwards: a wait inside the kernels ran out.
+ * -2 before the call.  -1: a row holds a NaN; nothing was removed, and the rows have to be made unique another way.
+ * -DOK_SORT_ALL_WORDS - w: the rows' leading 32 bits do not tell them apart; nothing was removed, and
+ * dok_map_remove_unique_words(..., w, ...) with the same arguments and the untouched work does.  -2 afterwards: a wait inside
+ * the kernels ran out.
  * work: dok_map_remove_unique_bytes(n) bytes of device memory (0: none needed, -1: n is too large). */
+#define DOK_SORT_ALL_WORDS 16
 int64_t dok_map_remove_unique_bytes(int64_t n);
 int dok_map_remove_unique(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n, uint8_t *out_removed,
                           void *work, int64_t *out_count, int64_t *counters, void *stream);
+int dok_map_remove_unique_words(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n, uint8_t *out_removed,
+                                void *work, int words, int64_t *out_count, int64_t *counters, void *stream);
 
 /* ---- sliced batches -------------------------------------------------------------------------------------
  * The same three operations on a batch that arrives as n_slices slices of slice_rows rows each (keys / values /

@@ -87,6 +87,54 @@ def test_removal_of_sorted_unique_rows(kind, n):
     pair.get(stored)
 
 
+def _rows_alike(rng, kind, n):
+    """Rows whose leading 32 bits do not tell them apart."""
+    wide = lambda *shape: rng.integers(-2 ** 62, 2 ** 62, shape)
+    if kind == "zipf 2^34":                        # a few bits more than 32, the small ids in most rows
+        return np.minimum(rng.zipf(1.1, (n, 1)), 2 ** 34 - 1 - rng.integers(0, 9, (n, 1)))
+    if kind == "whole f32x3":
+        return rng.integers(-500, 500, (n, 3)).astype(np.float32)
+    if kind == "whole f64 and halves":
+        return (rng.integers(-10 ** 6, 10 ** 6, (n, 2)) / 2).astype(np.float64)
+    if kind == "f16x5":
+        return rng.integers(-300, 300, (n, 5)).astype(np.float16)
+    if kind == "few leading values":               # 62 + 62 bits: four words
+        return np.concatenate([wide(7, 1)[rng.integers(0, 7, n)], wide(n // 2 + 1, 1)[rng.integers(0, n // 2 + 1, n)]], axis=1)
+    if kind == "all words":                        # 8 columns of 64 bits, the last ones different
+        return np.concatenate([wide(1, 6)[np.zeros(n, int)] + rng.integers(0, 2, (n, 6)) * 2 ** 61, wide(n, 2)], axis=1)
+    if kind == "last word":
+        return np.concatenate([wide(2, 2)[rng.integers(0, 2, n)], rng.integers(0, 3 * n, (n, 1))], axis=1)
+    rows = wide(n, 1)                              # scattered, and ...
+    if kind == "popular":                          # ... runs of one key's repetitions and a few others
+        for k in range(40):
+            rows[k * (n // 60):(k + 1) * (n // 60)] = rows[-1 - k]
+            rows[k * (n // 60):k * (n // 60) + k % 31] += np.arange(1, k % 31 + 1)[:, None]
+    if kind == "clumps":                           # ... runs of many different rows
+        for k, m in enumerate((16, 17, 200, 900, 1100)):
+            rows[k * (n // 6):k * (n // 6) + min(m, n // 6)] = (rows[-1 - k] >> 13 << 13) + rng.integers(0, 4 * m, (min(m, n // 6), 1))
+    if kind == "short runs":
+        rows[:3000] = (rows[:3000] // 64) * 64 + rng.integers(0, 64, (3000, 1))
+        rows[:3000] = np.repeat(rows[:60], 50, axis=0) + rng.integers(0, 40, (3000, 1))
+    return rows[rng.permutation(n)]
+
+
+@pytest.mark.parametrize("kind", ["zipf 2^34", "whole f32x3", "whole f64 and halves", "f16x5", "few leading values", "all words", "last word",
+                                  "popular", "clumps", "short runs"])
+@pytest.mark.parametrize("n", [4097, 8193, 70001, 700001])
+def test_removal_of_rows_with_equal_leading_bits(kind, n, monkeypatch):
+    """Sorted by every word of the packed rows, or by the first and its runs put in order; not by the library."""
+    rng = np.random.default_rng(n)
+    rows = _rows_alike(rng, kind, n)
+    half = rows[:n // 2]
+    pair = Pair(seed=n, n_buckets=1 << 21)
+    pair.set(half, rng.standard_normal((len(half), 1)))
+    for library in (torch, torch.Tensor):
+        monkeypatch.setattr(library, "unique", None)
+    flags = pair.remove(rows)
+    assert flags.shape[0] == np.unique(rows, axis=0).shape[0]
+    pair.get(rows[:5000])
+
+
 @pytest.mark.parametrize("n", [100, 6000])
 def test_removal_of_rows_with_nans(n):
     from doksparse_b200 import CudaClosedHashmap
