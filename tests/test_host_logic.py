@@ -96,3 +96,43 @@ def test_a_table_that_is_collected_while_a_ring_is_taken():
     assert not worker.is_alive()
     assert len(made) == 128 and len(taken) == 64 and len(rings._free[0]) == 64
     assert len(set(map(id, taken + rings._free[0]))) == 128
+
+
+def test_pieces_of_a_host_batch_hide_their_host_time():
+    """A piece costs about 75 us on the host.  Two of them have to move what the link takes that long for, 55 bytes in a
+    nanosecond (a lone operation has nothing else to overlap with: less will do)."""
+    from types import SimpleNamespace
+    import torch
+    from doksparse_b200.host_batch import HostBatch
+
+    class Offline(HostBatch):
+        def __init__(self):
+            self.chunk_rows, self._takes_outputs, self._staged_set_rows = 1 << 22, True, 0
+            self.table = SimpleNamespace(_slots=0, remove_rows=None, remove=None, _element_bound=lambda: 0, _rehash_threshold=0.75, n_buckets=1 << 30)
+
+        def _ring(self, *shape):
+            pass
+
+        def _execute(self, chunks):
+            self.pieces = [[t.shape[0] for _, t in inputs] for inputs, _ in chunks]
+
+    batch = Offline()
+    for log2 in range(10, 24):
+        for n in (1 << log2, 3 << (log2 - 1)):
+            for cols in (1, 2, 4):
+                keys, values, flags = torch.empty(n, 1, dtype=torch.long), torch.empty(n, cols), torch.empty(n, dtype=torch.bool)
+                ops = {"get": ((keys, values, flags), 9 + 4 * cols), "set": ((keys, values), 8 + 4 * cols), "remove_rows": ((keys, flags), 9)}
+                for name, (args, row_bytes) in ops.items():
+                    getattr(batch, name)(*args)
+                    alone = [p[0] for p in batch.pieces]
+                    batch.run([(name, *args)])
+                    assert [p[0] for p in batch.pieces] == alone and sum(alone) == n
+                    batch.run([(name, *args)] * 2)
+                    together = [p[0] for p in batch.pieces]
+                    assert sum(together) == 2 * n
+                    for pieces, least in ((alone, 3.2e6), (together[:len(together) // 2], 75e-6 * 55e9)):
+                        assert len(pieces) <= 4
+                        if len(pieces) > 1 and n <= batch.chunk_rows:
+                            assert sum(pieces) / len(pieces) * row_bytes >= least
+                    if n == 1 << 22:
+                        assert len(alone) == 4
