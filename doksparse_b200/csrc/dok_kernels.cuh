@@ -16,10 +16,10 @@
 // get
 // ---------------------------------------------------------------------------------------------------------
 // One row per thread: for 32-byte slots with values of at most 8 bytes, whose walk fits 32 registers, so that 64 warps are
-// resident (8.4 M lookups at load 0.6: 251 us; the form below, with half the instructions but 32 warps: 291), and for slots
-// wider than a line, which a lane walks by itself.
+// resident (8.4 M lookups at load 0.6: 251 us; the form below, with half the instructions but 32 warps: 291), for slots
+// wider than a line, which a lane walks by itself, and for batches of a few rows per lane (DOK_FEW_ROWS).
 template <int SB, int LW, class Keys>
-__global__ void __launch_bounds__(DOK_TPB, SB == 32 ? 8 : 1) k_get_row(DevTable t, DevHash hp, Keys keys, char *__restrict__ out_values,
+__global__ void __launch_bounds__(DOK_TPB, LW == 2 ? (SB == 32 ? 8 : 6) : 1) k_get_row(DevTable t, DevHash hp, Keys keys, char *__restrict__ out_values,
                                                     uint8_t *__restrict__ out_found, Fallback fb, ll_t *counters,
                                                     int count_probes) {
   __shared__ BlockTally tally;
@@ -155,6 +155,14 @@ inline dim3 dok_stream_grid(const Keys &keys) {
 #define DOK_STREAM(t, rc, st, keys, KERNEL, ...) \
   DOK_FOR_WINDOWS(t, rc, (KERNEL<<<dok_stream_grid<KERNEL>(keys), DOK_TPB, 0, st>>>(wt, __VA_ARGS__)))
 
+// Batches of fewer key rows go to k_get_row: with less than two rows for each lane of k_get, there are too few chains for a
+// lane to take up when its own ends.  k_get_row's time over k_get's, means over hits, Zipf-distributed hits and misses at
+// loads of 0.3 to 0.85: 40-byte values, 10 k rows 0.71, 100 k 0.72, 200 k 0.84, 300 k 0.94, 500 k 1.10, 1 M 1.32; 16-byte
+// values 0.87, 0.84, 0.94, 1.02, 1.15, 1.36; 4-byte values in 64-byte slots 1.03, 0.91, 0.81, 0.94, 1.00, 1.13, the misses at
+// 0.85 alone 0.83 at 200 k and 1.13 at 300 k.  Selections of a tensor, whose index arithmetic a share does for 32 rows at a
+// time, differ by a tenth either way and stay with k_get.
+#define DOK_FEW_ROWS(LW) (148LL * DOK_TPB * ((LW) == 4 ? 3 : 4) * 2)
+
 template <class Keys>
 inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, void *out_values, uint8_t *out_found,
                       const void *fallback, int64_t *counters, int count_probes, cudaStream_t st) {
@@ -168,24 +176,24 @@ inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, vo
   ll_t *cnt = (ll_t *)counters;
   // tag and value fit the first 16 bytes of the slot: half the load width
   const bool narrow = t.vb <= 8;
-  constexpr bool ROWS = std::is_same<Keys, RowKeys>::value;
+  const auto launch = [&](auto slot_bytes, auto words) {
+    constexpr int SB = decltype(slot_bytes)::value, LW = decltype(words)::value;
+    constexpr bool ROWS = std::is_same<Keys, RowKeys>::value, ONLY_ROWS = SB == 0 || (ROWS && SB == 32 && LW == 2);
+    if constexpr (ROWS || SB == 0)
+      if (ONLY_ROWS || n < DOK_FEW_ROWS(LW)) {
+        DOK_FOR_WINDOWS(t, rc, (k_get_row<SB, LW, Keys><<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, values, out_found, fb, cnt, count_probes)));
+        return;
+      }
+    if constexpr (!ONLY_ROWS) DOK_STREAM(t, rc, st, keys, (k_get<SB, LW, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
+  };
+  const auto by_width = [&](auto slot_bytes) {
+    if (narrow) launch(slot_bytes, std::integral_constant<int, 2>()); else launch(slot_bytes, std::integral_constant<int, 4>());
+  };
   switch (t.sb) {
-    case 32:
-      if (!narrow) DOK_STREAM(t, rc, st, keys, (k_get<32, 4, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
-      else if constexpr (ROWS)
-        DOK_FOR_WINDOWS(t, rc, (k_get_row<32, 2, Keys><<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, values, out_found, fb, cnt, count_probes)));
-      else DOK_STREAM(t, rc, st, keys, (k_get<32, 2, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
-      break;
-    case 64:
-      if (narrow) DOK_STREAM(t, rc, st, keys, (k_get<64, 2, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
-      else DOK_STREAM(t, rc, st, keys, (k_get<64, 4, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
-      break;
-    case 128:
-      if (narrow) DOK_STREAM(t, rc, st, keys, (k_get<128, 2, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
-      else DOK_STREAM(t, rc, st, keys, (k_get<128, 4, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
-      break;
-    default:
-      DOK_FOR_WINDOWS(t, rc, (k_get_row<0, 4, Keys><<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, values, out_found, fb, cnt, count_probes)));
+    case 32: by_width(std::integral_constant<int, 32>()); break;
+    case 64: by_width(std::integral_constant<int, 64>()); break;
+    case 128: by_width(std::integral_constant<int, 128>()); break;
+    default: launch(std::integral_constant<int, 0>(), std::integral_constant<int, 4>());
   }
   return rc;
 }

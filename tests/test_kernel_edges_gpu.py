@@ -225,6 +225,13 @@ def test_lookups_over_warp_shares(n, key_cols, value_dtype, value_cols):
     assert (values[~found] == 7).all() and torch.equal(values[found], all_values[query[found]])
 
 
+@pytest.mark.parametrize("n", [148 * 256 * 6 - 1, 148 * 256 * 6, 148 * 256 * 8 - 1, 148 * 256 * 8])
+@pytest.mark.parametrize("key_cols,value_dtype,value_cols", [(1, torch.float32, 4), (4, torch.float32, 1), (1, torch.int64, 5), (2, torch.float64, 12)])
+def test_lookups_where_the_form_changes(n, key_cols, value_dtype, value_cols):
+    """One row per thread below two rows for each lane of the resident warps, shares of the batch from there."""
+    test_lookups_over_warp_shares(n, key_cols, value_dtype, value_cols)
+
+
 @pytest.mark.parametrize("n", [1, 2, 1024, 1025, 2049, 8192, 8193, 65535, 65537, 200_001])
 @pytest.mark.parametrize("value_cols", [2, 4, 31])              # stamps in the slot, in an array of their own, slots wider than a line
 def test_sets_with_repeated_keys(n, value_cols):
