@@ -135,6 +135,16 @@ def test_removal_of_rows_with_equal_leading_bits(kind, n, monkeypatch):
     pair.get(rows[:5000])
 
 
+def test_removal_flags_hold_no_memory_of_repeated_rows():
+    from doksparse_b200 import CudaClosedHashmap
+    np.random.seed(1)
+    t = CudaClosedHashmap(n_buckets=1 << 12)
+    keys = torch.arange(1000, device="cuda")[:, None]
+    t.set(keys, torch.ones(1000, 1, device="cuda"))
+    flags = t.remove(keys.repeat(1000, 1))
+    assert flags.shape == (1000,) and flags.all() and flags.untyped_storage().nbytes() == 1000
+
+
 @pytest.mark.parametrize("n", [100, 6000])
 def test_removal_of_rows_with_nans(n):
     from doksparse_b200 import CudaClosedHashmap
