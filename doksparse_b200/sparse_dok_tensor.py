@@ -415,6 +415,8 @@ class SparseDOKTensor(object):
         src_strides = (ctypes.c_int64 * L.MAX_SELECTOR_NDIM)(*src.stride())
         epoch = hashmap._next_epoch()
         words = L.lib().dok_set_scratch_words(hashmap._c_table(), n_sel)
+        if words < 0:
+            raise L.DokError(f"an assignment may select up to 2^32 - 1 positions, got {n_sel}")
         scratch = torch.empty(words, device=self.device, dtype=torch.long)
         with L.on(self.device):
             # n_elements grows by the selected positions that were not stored; duplicates over-count, like the reference (:474)

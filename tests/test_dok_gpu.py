@@ -312,3 +312,16 @@ def test_flatten_and_reshape_rekey_in_one_pass():
     consume_fresh_map_draws(1024, 2, 700)
     expected = np.random.get_state()[1][:8].copy(), np.random.get_state()[2]
     assert (after_reshape[0] == expected[0]).all() and after_reshape[1] == expected[1]
+
+
+@pytest.mark.parametrize("value", [2.0, torch.tensor(2)])             # the native call, and the general one
+def test_assignment_beyond_the_batch_limit(value):
+    """2^33 positions, on a table that is told not to grow: an error of the library's, nothing stored."""
+    from doksparse_b200 import CudaClosedHashmap, SparseDOKTensor
+    from doksparse_b200._lib import DokError
+    np.random.seed(0)
+    table = CudaClosedHashmap(n_buckets=1024, device="cuda:0", rehash_threshold=1e9)
+    t = SparseDOKTensor((1 << 17, 1 << 16), torch.tensor([[3, 5], [4, 9]]), torch.ones(2), device="cuda:0", storage=table)
+    with pytest.raises(DokError):
+        t[:, :] = value.cuda() if isinstance(value, torch.Tensor) else value
+    assert t._nnz() == 2 and float(t[3, 4]) == 1
