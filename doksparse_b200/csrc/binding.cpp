@@ -198,6 +198,10 @@ int ring_init(Ring *self, PyObject *args, PyObject *) {
   return 0;
 }
 void ring_dealloc(Ring *self) {
+  // a copy on its way would land in memory that the allocator has given to somebody else
+  Py_BEGIN_ALLOW_THREADS
+  for (int i = 0; i < 8; i++) if ((self->used >> i) & 1u) (void)cudaEventSynchronize(self->events[i]);
+  Py_END_ALLOW_THREADS
   for (int i = 0; i < 8; i++) if (self->events[i]) cudaEventDestroy(self->events[i]);
   Py_XDECREF(self->memory);
   Py_TYPE(self)->tp_free((PyObject *)self);

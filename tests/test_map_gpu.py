@@ -492,3 +492,17 @@ def test_state_dict_round_trip(tmp_path):
         np.testing.assert_array_equal(x, y)
     empty = CudaClosedHashmap.from_state_dict(CudaClosedHashmap(n_buckets=64, device="cuda:0").state_dict())
     assert empty.n_elements == 0 and empty.n_buckets == 64
+
+
+def test_a_ring_that_goes_waits_for_its_copies():
+    """The pinned words go back to the allocator with the ring: nothing may be on its way to them."""
+    from doksparse_b200 import CudaClosedHashmap, _lib
+    np.random.seed(0)
+    table = CudaClosedHashmap(n_buckets=1 << 10)
+    table.set(torch.arange(100, device="cuda")[:, None], torch.ones(100, 1, device="cuda"))
+    words = torch.full((256,), -7, dtype=torch.long, pin_memory=True)
+    ring = _lib.native().Ring(words, table._slots.device.index)
+    torch.cuda._sleep(100_000_000)
+    ring.copy(table._native_plan(), 0)
+    del ring
+    assert words[0] == 100
