@@ -391,17 +391,6 @@ PyObject *plan_count_new(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
   });
 }
 
-// init(): empty tags, zero counters
-PyObject *plan_init_table(Plan *self, PyObject *) {
-  return guarded([&]() -> PyObject * {
-    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
-    if (!check(dok_map_init_state(&self->table, self->state, STATE_WORDS, c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()),
-               "dok_map_init_state"))
-      return nullptr;
-    Py_RETURN_NONE;
-  });
-}
-
 // reinsert(plan): the live rows of another table of the same row shape
 PyObject *plan_reinsert(Plan *self, PyObject *arg) {
   return guarded([&]() -> PyObject * {
@@ -670,7 +659,6 @@ PyMethodDef plan_methods[] = {
     {"remove", (PyCFunction)plan_remove, METH_O, nullptr},
     {"read", (PyCFunction)plan_read, METH_NOARGS, nullptr},
     {"count_new", (PyCFunction)(void *)plan_count_new, METH_FASTCALL, nullptr},
-    {"init", (PyCFunction)plan_init_table, METH_NOARGS, nullptr},
     {"reinsert", (PyCFunction)plan_reinsert, METH_O, nullptr},
     {"index", (PyCFunction)(void *)plan_index, METH_FASTCALL, nullptr},
     {"assign", (PyCFunction)(void *)plan_assign, METH_FASTCALL, nullptr},
