@@ -163,6 +163,7 @@ class HostBatch:
     def _execute(self, chunks):
         """Copy-in of chunk i + 1 is enqueued before the kernels of chunk i."""
         chunks = iter(chunks)
+        self._staged_set_rows = 0                   # (an operation before this one may have raised)
 
         def stage(chunk):
             if chunk is None:

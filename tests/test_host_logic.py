@@ -136,3 +136,26 @@ def test_pieces_of_a_host_batch_hide_their_host_time():
                             assert sum(pieces) / len(pieces) * row_bytes >= least
                     if n == 1 << 22:
                         assert len(alone) == 4
+
+
+def test_a_set_that_raises_leaves_no_staged_rows():
+    """Rows staged for a set that never ran would keep later sets from going in pieces."""
+    import pytest
+    import torch
+    from doksparse_b200.host_batch import HostBatch
+
+    class Offline(HostBatch):
+        def __init__(self):
+            self._staged_set_rows = 0
+
+    batch = Offline()
+
+    def chunks():
+        batch._staged_set_rows += 100
+        raise ValueError
+        yield
+
+    with pytest.raises(ValueError):
+        batch._execute(chunks())
+    batch._execute([])
+    assert batch._staged_set_rows == 0
