@@ -203,7 +203,7 @@ def test_native_selectors_agree_with_the_general_ones(name):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.uint8, torch.float64])
 @pytest.mark.parametrize("shape,density", [((1,), 1.0), ((2047,), 0.5), ((2048, 3), 1.0), ((129, 17, 5), 0.02), ((700, 1500), 0.001), ((1300, 1000), 0.4)])
 def test_dense_round_trip(dtype, shape, density):
-    """Spans of 2048 elements whose non-zeros are inserted 256 at a time: few, exactly full and many per span."""
+    """Few, all and many non-zeros, on fewer elements than a wave takes and on more."""
     from doksparse_b200 import SparseDOKTensor
     np.random.seed(2)
     rng = np.random.default_rng(1)
@@ -213,6 +213,20 @@ def test_dense_round_trip(dtype, shape, density):
     assert torch.equal(t.to_dense(), dense) and torch.equal(t.to_sparse_coo().to_dense(), dense)
     if len(shape) > 1:
         assert torch.equal(t.transpose(0, 1).to_dense(), dense.transpose(0, 1))
+
+
+@pytest.mark.parametrize("numel", [255, 256, 257, 2049, 148 * 4 * 2048 + 1, 4 * 148 * 4 * 2048 + 300])
+@pytest.mark.parametrize("counts", [(31,), (32,), (33,), (31, 1, 0, 33), (256, 0, 1)])
+def test_dense_lists_of_a_warp(numel, counts):
+    """A warp takes spans of 256 elements and inserts whenever it has found 32 non-zeros; `counts` in its spans, in turn."""
+    from doksparse_b200 import SparseDOKTensor
+    np.random.seed(2)
+    at = torch.arange(numel, device="cuda")
+    order = (at * 37) % 256                                  # where the non-zeros of a span lie
+    share = torch.tensor(counts, device="cuda")[(at // 256) // (148 * 4 * 8) % len(counts)]
+    dense = torch.where(order < share, at + 1, 0)
+    t = SparseDOKTensor.from_dense(dense)
+    assert t._nnz() == int((dense != 0).sum()) and torch.equal(t.to_dense(), dense)
 
 
 @pytest.mark.parametrize("n", [1, 31, 33, 257, 148 * 3 * 256 - 1, 148 * 4 * 256 + 33, 400_003])
