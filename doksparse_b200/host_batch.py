@@ -100,18 +100,17 @@ class HostBatch:
     # 350, 2^21 rows 27 MB 611 / 509 / 476, 2^22 rows 1154 / 947 / 859; a set of 16-byte values, 2^18 rows 6.3 MB 299 / 301 /
     # 337, 2^20 rows 25 MB 624 / 591 / 585; set, get and remove in one run with 8-byte values, 2^19 rows 8 MB each 418 / 504 /
     # 913, 3 * 2^18 rows 13 MB 576 / 574 / 916, 2^20 rows 17 MB 745 / 718 / 943, 2^22 rows 2716 / 2479 / 2454.
-    def _chunks(self, n, row_bytes, alone, divisible=True):
+    def _chunks(self, n, moved, alone, divisible=True):
         rows = self.chunk_rows
         if divisible and self._takes_outputs:
-            moved = n * row_bytes
             pieces = 4 if moved >= (24e6 if alone else 32e6) else 2 if moved >= (6.5e6 if alone else 12e6) else 1
             rows = min(rows, max(1, -(-n // pieces)))
         for lo in range(0, n, rows):
             yield lo, min(n, lo + rows)
 
     @staticmethod
-    def _row_bytes(*tensors):
-        return sum(t[:1].numel() * t.element_size() for t in tensors if t is not None)
+    def _bytes(*tensors):
+        return sum(t.numel() * t.element_size() for t in tensors if t is not None)
 
     def _set_is_divisible(self, keys_host):
         """Whether the pieces of a set leave the table as the whole would: where it might have to grow, the size it grows
@@ -124,7 +123,7 @@ class HostBatch:
     def _get_chunks(self, keys_host, out_values_host, out_found_host, fallback_value=None, *, alone=True):
         vr = self._ring("ov", out_values_host.shape[1:], out_values_host.dtype)
         fr = self._ring("of", (), torch.bool)
-        for lo, hi in self._chunks(keys_host.shape[0], self._row_bytes(keys_host, out_values_host, out_found_host), alone):
+        for lo, hi in self._chunks(keys_host.shape[0], self._bytes(keys_host, out_values_host, out_found_host), alone):
             def body(keys, lo=lo, hi=hi):
                 vi, vbuf = vr.take(self.s_run)
                 fi, fbuf = fr.take(self.s_run)
@@ -139,7 +138,7 @@ class HostBatch:
             yield [("k", keys_host[lo:hi])], body
 
     def _set_chunks(self, keys_host, values_host, assume_unique=False, *, alone=True):
-        for lo, hi in self._chunks(keys_host.shape[0], self._row_bytes(keys_host, values_host), alone, self._set_is_divisible(keys_host)):
+        for lo, hi in self._chunks(keys_host.shape[0], self._bytes(keys_host, values_host), alone, self._set_is_divisible(keys_host)):
             def body(keys, values):
                 self.table.set(keys, values, assume_unique=assume_unique)
                 self._staged_set_rows -= keys.shape[0]
@@ -150,7 +149,7 @@ class HostBatch:
     def _remove_chunks(self, keys_host, out_flags_host=None, *, alone=True):
         remove = getattr(self.table, "remove_rows", None) or self.table.remove
         fr = self._ring("rf", (), torch.bool)
-        for lo, hi in self._chunks(keys_host.shape[0], self._row_bytes(keys_host, out_flags_host), alone):
+        for lo, hi in self._chunks(keys_host.shape[0], self._bytes(keys_host, out_flags_host), alone):
             def body(keys, lo=lo, hi=hi):
                 flags = remove(keys)
                 if out_flags_host is None:
