@@ -158,10 +158,12 @@ inline dim3 dok_stream_grid(const Keys &keys) {
 // Batches of fewer key rows go to k_get_row: with less than two rows for each lane of k_get, there are too few chains for a
 // lane to take up when its own ends.  k_get_row's time over k_get's, means over hits, Zipf-distributed hits and misses at
 // loads of 0.3 to 0.85: 40-byte values, 10 k rows 0.71, 100 k 0.72, 200 k 0.84, 300 k 0.94, 500 k 1.10, 1 M 1.32; 16-byte
-// values 0.87, 0.84, 0.94, 1.02, 1.15, 1.36; 4-byte values in 64-byte slots 1.03, 0.91, 0.81, 0.94, 1.00, 1.13, the misses at
-// 0.85 alone 0.83 at 200 k and 1.13 at 300 k.  Selections of a tensor, whose index arithmetic a share does for 32 rows at a
-// time, differ by a tenth either way and stay with k_get.
+// values 0.87, 0.84, 0.94, 1.02, 1.15, 1.36; 4-byte values in 64-byte slots 1.03, 0.91, 0.81, 0.94, 1.00, 1.13 (at 30 k rows
+// 0.99, at 60 k 0.94, so these stay with k_get below a block per SM), the misses at 0.85 alone 0.83 at 200 k and 1.13 at
+// 300 k.  Selections of a tensor, whose index arithmetic a share does for 32 rows at a time, differ by a tenth either way and
+// stay with k_get.
 #define DOK_FEW_ROWS(LW) (148LL * DOK_TPB * ((LW) == 4 ? 3 : 4) * 2)
+#define DOK_LEAST_ROWS(LW) ((LW) == 4 ? 0LL : 148LL * DOK_TPB)
 
 template <class Keys>
 inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, void *out_values, uint8_t *out_found,
@@ -180,7 +182,7 @@ inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, vo
     constexpr int SB = decltype(slot_bytes)::value, LW = decltype(words)::value;
     constexpr bool ROWS = std::is_same<Keys, RowKeys>::value, ONLY_ROWS = SB == 0 || (ROWS && SB == 32 && LW == 2);
     if constexpr (ROWS || SB == 0)
-      if (ONLY_ROWS || n < DOK_FEW_ROWS(LW)) {
+      if (ONLY_ROWS || (n < DOK_FEW_ROWS(LW) && n >= DOK_LEAST_ROWS(LW))) {
         DOK_FOR_WINDOWS(t, rc, (k_get_row<SB, LW, Keys><<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, values, out_found, fb, cnt, count_probes)));
         return;
       }

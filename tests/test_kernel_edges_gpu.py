@@ -249,10 +249,11 @@ def test_lookups_over_warp_shares(n, key_cols, value_dtype, value_cols):
     assert (values[~found] == 7).all() and torch.equal(values[found], all_values[query[found]])
 
 
-@pytest.mark.parametrize("n", [148 * 256 * 6 - 1, 148 * 256 * 6, 148 * 256 * 8 - 1, 148 * 256 * 8])
+@pytest.mark.parametrize("n", [148 * 256 - 1, 148 * 256, 148 * 256 * 6 - 1, 148 * 256 * 6, 148 * 256 * 8 - 1, 148 * 256 * 8])
 @pytest.mark.parametrize("key_cols,value_dtype,value_cols", [(1, torch.float32, 4), (4, torch.float32, 1), (1, torch.int64, 5), (2, torch.float64, 12)])
 def test_lookups_where_the_form_changes(n, key_cols, value_dtype, value_cols):
-    """One row per thread below two rows for each lane of the resident warps, shares of the batch from there."""
+    """One row per thread below two rows for each lane of the resident warps, shares of the batch from there (and, for narrow
+    values, below a block per SM)."""
     test_lookups_over_warp_shares(n, key_cols, value_dtype, value_cols)
 
 
