@@ -364,8 +364,8 @@ PyObject *plan_read(Plan *self, PyObject *) {
   });
 }
 
-// count_new(keys, word, exact, empty table): adds the number of distinct new keys to the counter `word`; exact: sets it, and answers
-// the counters
+// count_new(keys, word, exact, empty table): adds the number of distinct new keys to the counter `word`; exact: sets it, and
+// answers the counters
 PyObject *plan_count_new(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
   return guarded([&]() -> PyObject * {
     if (nargs != 4) { PyErr_SetString(PyExc_TypeError, "count_new takes 4 arguments"); return nullptr; }

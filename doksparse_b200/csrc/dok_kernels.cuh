@@ -47,9 +47,9 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 2 ? (SB == 32 ? 8 : 6) : 1) k_g
   }
 }
 
-// A warp's share of the batch (dok_stream.cuh): for everything else.  Wider values need the registers of whole lines (3
+// A warp's share of the batch (dok_stream.cuh): for larger batches of everything else.  Wider values need the registers of whole lines (3
 // blocks of 256 per SM in either form), and where a line holds fewer slots the chains are longer, so that a warp that waits
-// for its longest chain leaves most of its lanes idle: 8.4 M lookups of 16-byte values 544 -> 354 us, 8.4 M misses in
+// for its longest chain leaves most of its lanes idle: 8.4 M lookups of 16-byte values 544 -> 303 us, 8.4 M misses in
 // 64-byte slots at load 0.69 750 -> 595, selections of 32-byte slots 153 -> 141.
 // Values of at most 8 bytes lie behind the tag in the word pair that a lane has loaded: the key's own lane fetches it from
 // the lane of the slot that matched, and stores value (or fallback) and flag of its row -- one store for 32 rows of which
@@ -160,8 +160,8 @@ inline dim3 dok_stream_grid(const Keys &keys) {
 // loads of 0.3 to 0.85: 40-byte values, 10 k rows 0.71, 100 k 0.72, 200 k 0.84, 300 k 0.94, 500 k 1.10, 1 M 1.32; 16-byte
 // values 0.87, 0.84, 0.94, 1.02, 1.15, 1.36; 4-byte values in 64-byte slots 1.03, 0.91, 0.81, 0.94, 1.00, 1.13 (at 30 k rows
 // 0.99, at 60 k 0.94, so these stay with k_get below a block per SM), the misses at 0.85 alone 0.83 at 200 k and 1.13 at
-// 300 k.  Selections of a tensor, whose index arithmetic a share does for 32 rows at a time, differ by a tenth either way and
-// stay with k_get.
+// 300 k.  Selections of a tensor, whose index arithmetic a share does for 32 rows at a time, differ by a tenth either way
+// and stay with k_get.
 #define DOK_FEW_ROWS(LW) (148LL * DOK_TPB * ((LW) == 4 ? 3 : 4) * 2)
 #define DOK_LEAST_ROWS(LW) ((LW) == 4 ? 0LL : 148LL * DOK_TPB)
 
@@ -358,8 +358,9 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
       // A key that the block holds several times is probably all over the batch.  If a later row has already stamped its
       // slot -- blocks start from the batch's end, so one has unless it is still running -- this row has nothing to write,
       // and a line that most of the blocks want is read, not written: writes to one line come 140 ns apart.  In a batch with
-      // many repetitions (one row in 16 so far, by a sample) the same goes for the keys that a block holds once: one in a thousand rows of a Zipf batch of 12.8 M
-      // is 12,800 writes to one line.  Elsewhere the look would cost every row a round trip for nothing.
+      // many repetitions (one row in 16 so far, by a sample) the same goes for the keys that a block holds once: one in a
+      // thousand rows of a Zipf batch of 12.8 M is 12,800 writes to one line.  Elsewhere the look would cost every row a round
+      // trip for nothing.
       const bool contended = filter && (ull_t)twins.signal.x * DOK_SIGNAL_SAMPLE * 16 > ((ull_t)blockIdx.y * gridDim.x + blockIdx.x) * DOK_TPB;
       ull_t old = (same.more || contended) && !fresh ? __ldcg(stamp) : 0;
       const bool over = old > (dok_stamp(epoch, e) | 3);

@@ -155,9 +155,9 @@ static __global__ void k_part_shard_counts(const ll_t *tile_offsets, int n_shard
 }
 
 // Where the rows of each owner go.  Local exchange buffer: every owner the same base, row0 < 0 = "at the start of
-// the owner's segment in this rank's grouped order".  Peer exchange: base = the owner GPU's receive buffer (mapped into this process), row0 = where THIS rank's segment
-// starts inside it; the rows then cross NVLink as plain stores while the tile is being partitioned, and no separate
-// exchange pass follows.
+// the owner's segment in this rank's grouped order".  Peer exchange: base = the owner GPU's receive buffer (mapped into
+// this process), row0 = where THIS rank's segment starts inside it; the rows then cross NVLink as plain stores while the
+// tile is being partitioned, and no separate exchange pass follows.
 struct PartDest {
   char *keys[DOK_MAX_SHARDS];
   char *values[DOK_MAX_SHARDS];

@@ -706,8 +706,9 @@ class CudaClosedHashmap:
         limit = int(self._rehash_threshold * self.n_buckets)
         row_counted = new_keys.dtype in L.FLOAT_DTYPES
         # Where the bound may only be stale (the host runs ahead of the device), the exact count is fetched before paying for
-        # a pass that counts the distinct new keys.  The distinct new keys (cuda_closed_hashmap.py:350-363) are counted with a scratch set on the device: uuids of
-        # integer keys, ROWS of floating ones like in the reference, because the value cast makes many rows share a uuid.
+        # a pass that counts the distinct new keys.  These (cuda_closed_hashmap.py:350-363) are counted with a scratch set on
+        # the device: uuids of integer keys, ROWS of floating ones like in the reference, because the value cast makes many
+        # rows share a uuid.
         plan = self._native_plan()
         if self._room_for(n, limit) or (not self._shared.known and self.n_elements + n <= limit):
             # whatever the number of new keys is, the reference would not rehash: insert and count on the device
