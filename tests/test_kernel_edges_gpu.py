@@ -98,6 +98,8 @@ def _rows_alike(rng, kind, n):
         return (rng.integers(-10 ** 6, 10 ** 6, (n, 2)) / 2).astype(np.float64)
     if kind == "f16x5":
         return rng.integers(-300, 300, (n, 5)).astype(np.float16)
+    if kind == "zeros of both signs":
+        return (rng.integers(-12, 12, (n, 4)) * rng.choice([-2.0 ** 20, 2.0 ** 20], (n, 4))).astype(np.float32)
     if kind == "few leading values":               # 62 + 62 bits: four words
         return np.concatenate([wide(7, 1)[rng.integers(0, 7, n)], wide(n // 2 + 1, 1)[rng.integers(0, n // 2 + 1, n)]], axis=1)
     if kind == "all words":                        # 8 columns of 64 bits, the last ones different
@@ -118,7 +120,7 @@ def _rows_alike(rng, kind, n):
     return rows[rng.permutation(n)]
 
 
-@pytest.mark.parametrize("kind", ["zipf 2^34", "whole f32x3", "whole f64 and halves", "f16x5", "few leading values", "all words", "last word",
+@pytest.mark.parametrize("kind", ["zipf 2^34", "whole f32x3", "whole f64 and halves", "f16x5", "zeros of both signs", "few leading values", "all words", "last word",
                                   "popular", "clumps", "short runs"])
 @pytest.mark.parametrize("n", [4097, 8193, 70001, 700001])
 def test_removal_of_rows_with_equal_leading_bits(kind, n, monkeypatch):
