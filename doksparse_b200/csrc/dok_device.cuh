@@ -384,21 +384,25 @@ __device__ __forceinline__ Located dok_locate_serial(const DevTable &t, const Ke
 
 // No-op hit handler for walks that only need the slot.
 struct NoEmit {
+  static constexpr bool L1 = false;
   template <int LW>
   __device__ __forceinline__ void operator()(ll_t, int, const ull_t (&)[LW]) const {}
 };
 
-// LW 8-byte words of a line chunk with one load that allocates in L2 only (L2 is the point of coherence for the
-// CAS claims; the table is touched at random, so L1 lines would be dead on arrival)
-template <int LW>
+// LW 8-byte words of a line chunk with one load.  Walks that claim or remove read through L2, the point of coherence for
+// their CAS.  Lookups change nothing and go through L1: batches of real ids are skewed, and the lines of the popular ones,
+// which otherwise come from a single L2 slice each, stay there (39.5 M Zipf(0.99) hits of 16-byte values: 1255 -> 1050 us;
+// 33.5 M uniform ones: 987 us either way).
+template <int LW, bool L1>
 __device__ __forceinline__ void dok_load_words(const char *p, ull_t (&w)[LW]) {
   if constexpr (LW == 4) {
-    asm volatile("ld.global.cg.v4.u64 {%0,%1,%2,%3}, [%4];" : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3]) : "l"(p));
+    if constexpr (L1) asm volatile("ld.global.ca.v4.u64 {%0,%1,%2,%3}, [%4];" : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3]) : "l"(p));
+    else asm volatile("ld.global.cg.v4.u64 {%0,%1,%2,%3}, [%4];" : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3]) : "l"(p));
   } else if constexpr (LW == 2) {
-    const ulonglong2 v = __ldcg((const ulonglong2 *)p);
+    const ulonglong2 v = L1 ? __ldca((const ulonglong2 *)p) : __ldcg((const ulonglong2 *)p);
     w[0] = v.x; w[1] = v.y;
   } else {
-    w[0] = __ldcg((const ull_t *)p);
+    w[0] = L1 ? __ldca((const ull_t *)p) : __ldcg((const ull_t *)p);
   }
 }
 
@@ -462,7 +466,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const KeyH
 #pragma unroll
     for (unsigned r = 0; r < 4; r++) {
       g[r] = __shfl_sync(FULL, group, base + r);
-      if (g[r] != NONE) dok_load_words<LW>(my_base + (ull_t)g[r] * 128u, w[r]);
+      if (g[r] != NONE) dok_load_words<LW, Emit::L1>(my_base + (ull_t)g[r] * 128u, w[r]);
     }
     unsigned bits = 0, tbits = 0;
 #pragma unroll
@@ -504,7 +508,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const KeyH
     if (!quad) g_r = NONE;
     const ll_t uuid_r = __shfl_sync(FULL, kh.uuid, base + r);
     ull_t wl[LW];
-    if (g_r != NONE) dok_load_words<LW>(my_base + (ull_t)g_r * 128u, wl);
+    if (g_r != NONE) dok_load_words<LW, Emit::L1>(my_base + (ull_t)g_r * 128u, wl);
     const ll_t tag = (has_tag && g_r != NONE) ? (ll_t)wl[0] : DOK_BLOCKED;
     unsigned bits = ((unsigned)(tag == uuid_r) | ((unsigned)(tag == DOK_EMPTY) << 4) |
                      (TOMB ? (unsigned)(tag == DOK_REMOVED) << 8 : 0u)) << my_slot;
@@ -529,6 +533,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const KeyH
 // a hit needs no second access to the table.  LW = 2 serves 32-byte slots whose value is one word behind the tag.
 template <int SB, int LW>
 struct EmitValue {
+  static constexpr bool L1 = true;
   const DevTable &t;
   char *out_values;
   __device__ __forceinline__ void operator()(ll_t e_r, int pos, const ull_t (&w)[LW]) const {

@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, De
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ WarpQueue queues[DOK_WARPS];
   int hits = 0, probes = 0;
-  dok_walk_share<LW>(queues[threadIdx.x >> 5], t, hp, keys, [&](LaneRow &lr, const Lines<LW> &f, const WarpShare &share) {
+  dok_walk_share<LW, true>(queues[threadIdx.x >> 5], t, hp, keys, [&](LaneRow &lr, const Lines<LW> &f, const WarpShare &share) {
     unsigned m, me, match[4], empty[4];
     dok_inspect<SB, LW>(lr, f, m, me, match, empty);
     const unsigned l = threadIdx.x & 3u, base = threadIdx.x & 28u;

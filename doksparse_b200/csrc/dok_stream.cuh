@@ -92,12 +92,12 @@ __device__ __forceinline__ bool dok_refill(const WarpQueue &q, WarpShare &s, Lan
 // One group for each lane: four requests, each for the lines of a quad's key in its turn.
 template <int LW>
 struct Lines { ull_t w[4][LW]; };
-template <int LW>
+template <int LW, bool L1>
 __device__ __forceinline__ void dok_request(const DevTable &t, const LaneRow &lr, Lines<LW> &f) {
   const char *my_base = t.slots + 32 * (threadIdx.x & 3u);
 #pragma unroll
   for (unsigned r = 0; r < 4; r++)
-    dok_load_words<LW>(my_base + (ull_t)__shfl_sync(0xffffffffu, lr.group, (threadIdx.x & 28u) + r) * 128u, f.w[r]);
+    dok_load_words<LW, L1>(my_base + (ull_t)__shfl_sync(0xffffffffu, lr.group, (threadIdx.x & 28u) + r) * 128u, f.w[r]);
 }
 
 // m / me: match and match-or-empty bits of the lane's own group by LANE of the quad (the slot at lane position p of a group
@@ -122,7 +122,7 @@ __device__ __forceinline__ void dok_inspect(const LaneRow &lr, const Lines<LW> &
 
 // The loop.  `step(lane's row, lines, share)` inspects the lines, lets the row go to its next group (dok_next_group) or ends
 // it (done()).
-template <int LW, class Keys, class Step>
+template <int LW, bool L1, class Keys, class Step>
 __device__ __forceinline__ void dok_walk_share(WarpQueue &queue, WarpShare share, const DevTable &t, const DevHash &hp, const Keys &keys,
                                                const Step &step) {
   LaneRow lr = DOK_IDLE_LANE;
@@ -130,12 +130,12 @@ __device__ __forceinline__ void dok_walk_share(WarpQueue &queue, WarpShare share
   for (;;) {
     dok_fill_queue(queue, share, t, hp, keys);
     if (!dok_refill(queue, share, lr, t)) break;
-    dok_request<LW>(t, lr, lines);
+    dok_request<LW, L1>(t, lr, lines);
     step(lr, lines, share);
   }
 }
 // ... of the warp's part of the whole batch
-template <int LW, class Keys, class Step>
+template <int LW, bool L1, class Keys, class Step>
 __device__ __forceinline__ void dok_walk_share(WarpQueue &queue, const DevTable &t, const DevHash &hp, const Keys &keys, const Step &step) {
-  dok_walk_share<LW>(queue, dok_share(keys.total()), t, hp, keys, step);
+  dok_walk_share<LW, L1>(queue, dok_share(keys.total()), t, hp, keys, step);
 }

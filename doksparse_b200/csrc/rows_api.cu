@@ -763,7 +763,7 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_remove_unique(DevTable t, DevHas
     }
   } else {
     const unsigned first = total * warp / DOK_WARPS, last = total * (warp + 1) / DOK_WARPS;
-    dok_walk_share<1>(queues[warp], WarpShare{first, last - first, 0, 0, 0}, t, hp, HeadKeys{keys, head_row},
+    dok_walk_share<1, false>(queues[warp], WarpShare{first, last - first, 0, 0, 0}, t, hp, HeadKeys{keys, head_row},
                       [&](LaneRow &lr, const Lines<1> &f, const WarpShare &share) {
       unsigned m, me, match[4], empty[4];
       dok_inspect<SB, 1>(lr, f, m, me, match, empty);
