@@ -139,6 +139,14 @@ __device__ __forceinline__ ll_t dok_start_group(const KeyHash &h, const DevTable
 __device__ __forceinline__ unsigned dok_chain_word(const KeyHash &h, const DevTable &t) {
   return t.n_groups > 64 ? (unsigned)dok_chain_hash(h) & 63u : DOK_CHAIN_LINEAR;
 }
+// The chain of a key, its hash mixed: for walks that come back to where the chain starts.
+struct ChainKey { ll_t uuid; unsigned hash, word; };
+__device__ __forceinline__ ChainKey dok_chain(const KeyHash &h, const DevTable &t) {
+  const ull_t mixed = dok_chain_hash(h);
+  return ChainKey{h.uuid, (unsigned)(mixed >> 32), t.n_groups > 64 ? (unsigned)mixed & 63u : DOK_CHAIN_LINEAR};
+}
+__device__ __forceinline__ ll_t dok_start_group(const ChainKey &k, const DevTable &t) { return (ll_t)__umulhi(k.hash, (unsigned)t.n_groups); }
+__device__ __forceinline__ unsigned dok_chain_word(const ChainKey &k, const DevTable &) { return k.word; }
 // steps to the next group of the chain; false when every group has been inspected
 template <class Index>
 __device__ __forceinline__ bool dok_next_group(Index &group, unsigned &word, Index n_groups) {
@@ -153,6 +161,26 @@ __device__ __forceinline__ bool dok_next_group(Index &group, unsigned &word, Ind
   group += step;
   if (group >= n_groups) group -= n_groups;
   return true;
+}
+// Groups that a key went past.  Lookups of absent keys would inspect every group up to one with an empty slot: at load 0.745
+// with 2 slots per group 2.6 of them.  Most full groups hold just the keys that start there, so each group remembers whether a
+// key was ever placed behind it: in the highest bit of its first slot's value word, where values of at most 7 bytes leave
+// padding and where a lookup has it in a register already.  Insertion sets it, and nothing clears it but a new table; a walk
+// that looks for a place ignores it.  8.4 M lookups of a 4-D selection, nearly all misses: 587 -> 402 us; 4 M lookups at load
+// 0.8, 30 % hits: 335 -> 210; filling that table with 50 M rows: 8.3 -> 8.9 ms.  With 4 slots per group fewer keys go past
+// one (load 0.36: 1.06 groups per miss); there a table that grows to 300 k rows lost more (880 -> 910 us) than lookups won.
+#define DOK_PASSED 0x8000000000000000ULL
+__host__ __device__ __forceinline__ bool dok_has_passed_bits(const DevTable &t) { return t.vb < 8 && t.spg <= 2; }
+// a key was placed in `slot`: marks the groups before it on its chain
+__device__ __forceinline__ void dok_mark_passed(const DevTable &t, const ChainKey &kh, ll_t slot) {
+  if (!dok_has_passed_bits(t)) return;
+  const unsigned placed = (unsigned)slot / (unsigned)t.spg, n_groups = (unsigned)t.n_groups;
+  unsigned group = (unsigned)dok_start_group(kh, t), word = dok_chain_word(kh, t);
+  while (group != placed) {
+    ull_t *first = (ull_t *)(t.slots + (ull_t)group * 128u + 8u);       // (no slot with such a value is wider than a line)
+    if (!(__ldcg(first) & DOK_PASSED)) atomicOr(first, DOK_PASSED);
+    if (!dok_next_group<unsigned>(group, word, n_groups)) break;
+  }
 }
 // does this launch serve the row?  (rows outside the window belong to another pass over the same batch)
 __device__ __forceinline__ bool dok_in_window(const DevTable &t, const KeyHash &h, bool active) {
@@ -365,7 +393,8 @@ struct Located { ll_t found, empty, tomb; };
 
 // Walk by ONE lane, the reference's loop (closed_hashmap_impl_class.cu:280-312, 368-407) over this library's chain.
 // Used for slots wider than a line (one slot per group).
-__device__ __forceinline__ Located dok_locate_serial(const DevTable &t, const KeyHash &kh, int *probes) {
+template <class Key>
+__device__ __forceinline__ Located dok_locate_serial(const DevTable &t, const Key &kh, int *probes) {
   Located r{-1, -1, -1};
   ll_t group = dok_start_group(kh, t);
   unsigned word = dok_chain_word(kh, t);
@@ -384,7 +413,7 @@ __device__ __forceinline__ Located dok_locate_serial(const DevTable &t, const Ke
 
 // No-op hit handler for walks that only need the slot.
 struct NoEmit {
-  static constexpr bool L1 = false;
+  static constexpr bool L1 = false, ENDS = false;
   template <int LW>
   __device__ __forceinline__ void operator()(ll_t, int, const ull_t (&)[LW]) const {}
 };
@@ -421,8 +450,8 @@ __device__ __forceinline__ void dok_load_words(const char *p, ull_t (&w)[LW]) {
 // Every lane of the warp must call this (inactive lanes pass active = false), with CONSECUTIVE batch elements e in
 // consecutive lanes.  SB = slot bytes (32, 64, 128).  Slot indices are 32-bit here: the host refuses cooperative
 // tables of 2^32 - 1 slots or more.
-template <int SB, int LW, bool TOMB, class Emit>
-__device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const KeyHash &kh, ll_t e, bool active,
+template <int SB, int LW, bool TOMB, class Key, class Emit>
+__device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key &kh, ll_t e, bool active,
                                                    int *probes, const Emit &emit) {
   constexpr int SPG = 128 / SB;
   constexpr unsigned FULL = 0xffffffffu;
@@ -440,6 +469,9 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const KeyH
     group = (unsigned)dok_start_group(kh, t);
     word = dok_chain_word(kh, t);
   }
+
+  // a group that no key went past ends a chain like an empty last slot (in the bits of its first slot's lane)
+  auto ends = [&](const ull_t (&w)[LW]) -> unsigned { return l == 0 && !(w[LW > 1 ? 1 : 0] & DOK_PASSED) ? 1u << (3 + SPG) : 0u; };
 
   // what the owner lane does with the outcome of one inspected group: m / me / tb = match, match-or-empty and
   // tombstone bits by slot
@@ -475,6 +507,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const KeyH
       if (has_tag && g[r] != NONE) {
         const ll_t tag = (ll_t)w[r][0];
         bits |= ((unsigned)(tag == uuid_r) | ((unsigned)(tag == DOK_EMPTY) << 4)) << (8u * r + my_slot);
+        if constexpr (Emit::ENDS) bits |= ends(w[r]) << (8u * r);
         if (TOMB) tbits |= (unsigned)(tag == DOK_REMOVED) << (4u * r + my_slot);
       }
     }
@@ -512,6 +545,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const KeyH
     const ll_t tag = (has_tag && g_r != NONE) ? (ll_t)wl[0] : DOK_BLOCKED;
     unsigned bits = ((unsigned)(tag == uuid_r) | ((unsigned)(tag == DOK_EMPTY) << 4) |
                      (TOMB ? (unsigned)(tag == DOK_REMOVED) << 8 : 0u)) << my_slot;
+    if constexpr (Emit::ENDS) if (g_r != NONE) bits |= ends(wl);
     bits |= __shfl_xor_sync(FULL, bits, 1);
     bits |= __shfl_xor_sync(FULL, bits, 2);
     const unsigned m = bits & 0xfu, me = (bits | (bits >> 4)) & 0xfu;
@@ -529,11 +563,11 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const KeyH
   return res;
 }
 
-// Hit handler of `get`: the lanes of the quad write the value straight from the registers that hold the line, so
+// Hit handler of `get` (PASSED: of a table whose groups remember that a key went past them): the lanes of the quad write the value straight from the registers that hold the line, so
 // a hit needs no second access to the table.  LW = 2 serves 32-byte slots whose value is one word behind the tag.
-template <int SB, int LW>
+template <int SB, int LW, bool PASSED>
 struct EmitValue {
-  static constexpr bool L1 = true;
+  static constexpr bool L1 = true, ENDS = PASSED;
   const DevTable &t;
   char *out_values;
   __device__ __forceinline__ void operator()(ll_t e_r, int pos, const ull_t (&w)[LW]) const {
@@ -565,8 +599,8 @@ struct EmitValue {
 };
 
 // SB == 0 selects the serial walk (slots wider than one line); emit is not called there.
-template <int SB, int LW, bool TOMB, class Emit>
-__device__ __forceinline__ Located dok_locate(const DevTable &t, const KeyHash &kh, ll_t e, bool active, int *probes,
+template <int SB, int LW, bool TOMB, class Key, class Emit>
+__device__ __forceinline__ Located dok_locate(const DevTable &t, const Key &kh, ll_t e, bool active, int *probes,
                                               const Emit &emit) {
   if constexpr (SB == 0) {
     if (probes) *probes = 0;
@@ -588,7 +622,7 @@ enum { DOK_OUT_FOUND = 0, DOK_OUT_CLAIMED_EMPTY = 1, DOK_OUT_REUSED = 2, DOK_OUT
 // unless a tombstone was seen.  Phase 2 walks it again and takes the first slot that is free, tombstone or empty.  No slot
 // becomes free while a set runs, so rows with equal uuids meet: the one that comes later finds the slot the first one
 // took, in the walk or because its CAS loses to the SAME uuid.
-static __device__ __forceinline__ ll_t dok_find_or_claim_serial(const DevTable &t, const KeyHash &kh, int *outcome) {
+static __device__ __forceinline__ ll_t dok_find_or_claim_serial(const DevTable &t, const ChainKey &kh, int *outcome) {
   const ll_t uuid = kh.uuid;
   bool reuse = false;                                    // a tombstone was seen
   for (int phase = 0; phase < 2; phase++) {
@@ -603,7 +637,11 @@ static __device__ __forceinline__ ll_t dok_find_or_claim_serial(const DevTable &
         if (tag == DOK_EMPTY && phase == 0 && reuse) { more = false; break; }
         if (tag == DOK_EMPTY || (tag == DOK_REMOVED && phase == 1)) {
           const ll_t old = dok_cas_tag(t, slot, tag, uuid);
-          if (old == tag) { *outcome = tag == DOK_EMPTY ? DOK_OUT_CLAIMED_EMPTY : DOK_OUT_REUSED; return slot; }
+          if (old == tag) {
+            *outcome = tag == DOK_EMPTY ? DOK_OUT_CLAIMED_EMPTY : DOK_OUT_REUSED;
+            dok_mark_passed(t, kh, slot);
+            return slot;
+          }
           tag = old;
         }
         if (tag == uuid) { *outcome = DOK_OUT_FOUND; return slot; }
@@ -621,17 +659,18 @@ static __device__ __forceinline__ ll_t dok_find_or_claim_serial(const DevTable &
 // CAS.  Losing the CAS to the same uuid means a twin row of the batch claimed it: join.  Losing it to another
 // uuid is rare; that lane redoes the whole operation with the serial walk.  Every lane of the warp must call.
 template <int SB>
-__device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHash &kh, bool active, int *outcome) {
+__device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHash &key, bool active, int *outcome) {
+  const ChainKey kh = dok_chain(key, t);
   const Located loc = dok_locate<SB, 1, true>(t, kh, 0, active, nullptr, NoEmit());   // the tags are all a claim needs
   if (!active) return -1;
   if (loc.found >= 0) { *outcome = DOK_OUT_FOUND; return loc.found; }
   if (loc.tomb >= 0) {
     const ll_t old = dok_cas_tag(t, loc.tomb, DOK_REMOVED, kh.uuid);
-    if (old == DOK_REMOVED) { *outcome = DOK_OUT_REUSED; return loc.tomb; }
+    if (old == DOK_REMOVED) { *outcome = DOK_OUT_REUSED; if (SB >= 64) dok_mark_passed(t, kh, loc.tomb); return loc.tomb; }
     if (old == kh.uuid) { *outcome = DOK_OUT_FOUND; return loc.tomb; }
   } else if (loc.empty >= 0) {
     const ll_t old = dok_cas_tag(t, loc.empty, DOK_EMPTY, kh.uuid);
-    if (old == DOK_EMPTY) { *outcome = DOK_OUT_CLAIMED_EMPTY; return loc.empty; }
+    if (old == DOK_EMPTY) { *outcome = DOK_OUT_CLAIMED_EMPTY; if (SB >= 64) dok_mark_passed(t, kh, loc.empty); return loc.empty; }
     if (old == kh.uuid) { *outcome = DOK_OUT_FOUND; return loc.empty; }
   } else {
     *outcome = DOK_OUT_FAILED;       // no match, no tombstone, no empty slot: the table is full

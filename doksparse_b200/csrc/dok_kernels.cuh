@@ -18,7 +18,7 @@
 // One row per thread: for 32-byte slots with values of at most 8 bytes, whose walk fits 32 registers, so that 64 warps are
 // resident (8.4 M lookups at load 0.6: 251 us; the form below, with half the instructions but 32 warps: 291), for slots
 // wider than a line, which a lane walks by itself, and for batches of a few rows per lane (DOK_FEW_ROWS).
-template <int SB, int LW, class Keys>
+template <int SB, int LW, bool PASSED, class Keys>
 __global__ void __launch_bounds__(DOK_TPB, LW == 2 ? (SB == 32 ? 8 : 6) : 1) k_get_row(DevTable t, DevHash hp, Keys keys, char *__restrict__ out_values,
                                                     uint8_t *__restrict__ out_found, Fallback fb, ll_t *counters,
                                                     int count_probes) {
@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 2 ? (SB == 32 ? 8 : 6) : 1) k_g
   active = dok_in_window(t, kh, active);
   int probes = 0;
   // on a hit the quad writes the value from the registers that hold the line
-  const Located loc = dok_locate<SB, LW, false>(t, kh, e, active, &probes, EmitValue<(SB == 0 ? 32 : SB), LW>{t, out_values});
+  const Located loc = dok_locate<SB, LW, false>(t, kh, e, active, &probes, EmitValue<(SB == 0 ? 32 : SB), LW, PASSED>{t, out_values});
   const int hit = active && loc.found >= 0;
   if (active) {
     char *dst = out_values + e * (ll_t)t.vb;
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 2 ? (SB == 32 ? 8 : 6) : 1) k_g
 // the lane of the slot that matched, and stores value (or fallback) and flag of its row -- one store for 32 rows of which
 // most are neighbours.  Wider values are written by the quad from the registers that hold the line.  Either way a hit needs
 // no second access to the table.
-template <int SB, int LW, class Keys>
+template <int SB, int LW, bool PASSED, class Keys>
 __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, DevHash hp, Keys keys, char *__restrict__ out_values,
                                                                   uint8_t *__restrict__ out_found, Fallback fb, ll_t *counters,
                                                                   int count_probes) {
@@ -63,19 +63,21 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, De
   __shared__ WarpQueue queues[DOK_WARPS];
   int hits = 0, probes = 0;
   dok_walk_share<LW, true>(queues[threadIdx.x >> 5], t, hp, keys, [&](LaneRow &lr, const Lines<LW> &f, const WarpShare &share) {
-    unsigned m, me, match[4], empty[4];
-    dok_inspect<SB, LW>(lr, f, m, me, match, empty);
     const unsigned l = threadIdx.x & 3u, base = threadIdx.x & 28u;
+    unsigned m, me, match[4], empty[4];
     ull_t value = 0;
     if constexpr (LW == 2) {
-      const unsigned from = base + (me ? (unsigned)(__ffs(me) - 1) : 0u);
+      const unsigned bits = dok_inspect<SB, LW, PASSED>(lr, f);
+      m = dok_matches(bits, l); me = dok_ends(bits, l);
+      const unsigned from = base + (me ? (unsigned)(__ffs(me) - 1) * (SB / 32) : 0u);
 #pragma unroll
       for (unsigned r = 0; r < 4; r++) {
         const ull_t v = __shfl_sync(FULL, f.w[r][1], from);
         if (l == r) value = v;
       }
     } else {
-      const EmitValue<SB, LW> emit{t, out_values};
+      dok_inspect_votes<SB, LW>(lr, f, m, me, match, empty);
+      const EmitValue<SB, LW, false> emit{t, out_values};
       // 16-byte values of 32-byte slots: one store by the lane that holds the slot
       const bool pairs = SB == 32 && t.vb == 16 && ((size_t)out_values & 15) == 0;
       if (pairs) {
@@ -178,24 +180,27 @@ inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, vo
   ll_t *cnt = (ll_t *)counters;
   // tag and value fit the first 16 bytes of the slot: half the load width
   const bool narrow = t.vb <= 8;
-  const auto launch = [&](auto slot_bytes, auto words) {
+  const auto launch = [&](auto slot_bytes, auto words, auto passed) {
     constexpr int SB = decltype(slot_bytes)::value, LW = decltype(words)::value;
+    constexpr bool PASSED = decltype(passed)::value;
     constexpr bool ROWS = std::is_same<Keys, RowKeys>::value, ONLY_ROWS = SB == 0 || (ROWS && SB == 32 && LW == 2);
     if constexpr (ROWS || SB == 0)
       if (ONLY_ROWS || (n < DOK_FEW_ROWS(LW) && n >= DOK_LEAST_ROWS(LW))) {
-        DOK_FOR_WINDOWS(t, rc, (k_get_row<SB, LW, Keys><<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, values, out_found, fb, cnt, count_probes)));
+        DOK_FOR_WINDOWS(t, rc, (k_get_row<SB, LW, PASSED, Keys><<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, values, out_found, fb, cnt, count_probes)));
         return;
       }
-    if constexpr (!ONLY_ROWS) DOK_STREAM(t, rc, st, keys, (k_get<SB, LW, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
+    if constexpr (!ONLY_ROWS) DOK_STREAM(t, rc, st, keys, (k_get<SB, LW, PASSED, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
   };
   const auto by_width = [&](auto slot_bytes) {
-    if (narrow) launch(slot_bytes, std::integral_constant<int, 2>()); else launch(slot_bytes, std::integral_constant<int, 4>());
+    if (dok_has_passed_bits(t)) launch(slot_bytes, std::integral_constant<int, 2>(), std::true_type());
+    else if (narrow) launch(slot_bytes, std::integral_constant<int, 2>(), std::false_type());
+    else launch(slot_bytes, std::integral_constant<int, 4>(), std::false_type());
   };
   switch (t.sb) {
     case 32: by_width(std::integral_constant<int, 32>()); break;
     case 64: by_width(std::integral_constant<int, 64>()); break;
     case 128: by_width(std::integral_constant<int, 128>()); break;
-    default: launch(std::integral_constant<int, 0>(), std::integral_constant<int, 4>());
+    default: launch(std::integral_constant<int, 0>(), std::integral_constant<int, 4>(), std::false_type());
   }
   return rc;
 }

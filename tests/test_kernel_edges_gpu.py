@@ -35,6 +35,34 @@ def test_chains_of_a_full_table(n_buckets, key_size, value_cols):
     pair.get(rows(0, n_buckets + gone + 50)[0])
 
 
+@pytest.mark.parametrize("n_buckets", [1, 7, 255, 257, 260, 1021, 40000])
+@pytest.mark.parametrize("key_size", [1, 3, 7])                                # 4, 2 and 1 slots per group
+@pytest.mark.parametrize("dtype,cols", [(np.float32, 1), (np.float16, 3), (np.uint8, 7)])
+def test_lookups_end_at_groups_that_no_key_went_past(n_buckets, key_size, dtype, cols):
+    """Values of at most 7 bytes: every way of placing a key marks the full groups before it, tombstones included."""
+    rng = np.random.default_rng(n_buckets + key_size)
+    rows = lambda lo, hi: np.stack([np.arange(lo, hi) * (j + 3) + j for j in range(key_size)], axis=1).astype(np.int64)
+    values = lambda k: rng.integers(0, 100, (k, cols)).astype(dtype)
+    long = lambda v: [v[j % 3] + 2 * (j // 3) for j in range(key_size)]
+    pair = Pair(seed=3, n_buckets=n_buckets, key_size=key_size, rehash_threshold=1.0, **{k: long(v) for k, v in params(3).items()})
+    most = max(1, 19 * n_buckets // 20)                       # chains of many groups, and empty slots
+    half = most // 2
+    pair.set(rows(0, half), values(half), assume_unique=True)
+    pair.set(rows(half, most), values(most - half))
+    everything = rows(0, 2 * n_buckets + 50)
+    pair.get(everything)
+    gone = most // 3
+    if gone:
+        pair.remove(rows(0, gone))
+        pair.get(everything)
+        pair.set(rows(most, most + gone), values(gone))       # into the tombstones
+        pair.get(everything)
+        pair.c.rebuild()
+        pair.get(everything)
+    pair.set(rows(most + gone, n_buckets + gone), values(n_buckets - most))
+    pair.get(everything)
+
+
 @pytest.mark.parametrize("n", [1, 31, 300, 5000, 70000])
 def test_assignment_counts_repeated_new_positions(n):
     """n_elements grows by every selected position that was not stored, repetitions included; the last one's value stays."""
