@@ -168,7 +168,8 @@ __device__ __forceinline__ bool dok_next_group(Index &group, unsigned &word, Ind
 // padding and where a lookup has it in a register already.  Insertion sets it, and nothing clears it but a new table; a walk
 // that looks for a place ignores it.  8.4 M lookups of a 4-D selection, nearly all misses: 587 -> 402 us; 4 M lookups at load
 // 0.8, 30 % hits: 335 -> 210; filling that table with 50 M rows: 8.3 -> 8.9 ms.  With 4 slots per group fewer keys go past
-// one (load 0.36: 1.06 groups per miss); there a table that grows to 300 k rows lost more (880 -> 910 us) than lookups won.
+// one: at load 0.36 4 M lookups went from 140 to 127 us, but a table that grows to 300 k rows from 880 to 910 and a dense
+// tensor's conversion from 348 to 359 (398 where the bit is written without a look), so those stay without.
 #define DOK_PASSED 0x8000000000000000ULL
 __host__ __device__ __forceinline__ bool dok_has_passed_bits(const DevTable &t) { return t.vb < 8 && t.spg <= 2; }
 // a key was placed in `slot`: marks the groups before it on its chain
@@ -563,7 +564,8 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
   return res;
 }
 
-// Hit handler of `get` (PASSED: of a table whose groups remember that a key went past them): the lanes of the quad write the value straight from the registers that hold the line, so
+// Hit handler of `get` (PASSED: of a table whose groups remember that a key went past them): the lanes of the quad write
+// the value straight from the registers that hold the line, so
 // a hit needs no second access to the table.  LW = 2 serves 32-byte slots whose value is one word behind the tag.
 template <int SB, int LW, bool PASSED>
 struct EmitValue {
