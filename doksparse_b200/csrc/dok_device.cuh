@@ -306,11 +306,18 @@ struct SelKeys {
   __device__ __forceinline__ bool idle(unsigned = 0) const { return false; }
   __device__ __forceinline__ bool row(ll_t &e, unsigned block) const { return at((ll_t)block * DOK_TPB + threadIdx.x, e); }
   __device__ __forceinline__ ll_t index(int d, ll_t off) const { return s.ptr[d] ? s.ptr[d][off] : s.base[d] + off; }
-  // element offsets of batch element e into each of the ndim index tensors (fully unrolled over the
-  // maximum ndim with predication, so `off` stays in registers)
-  __device__ __forceinline__ void offsets(ll_t e, ll_t (&off)[DOK_MAX_KEY_SIZE]) const {
+  // Element offsets of batch element e into each of the N index tensors.  N is the number of dims, or the most there can be:
+  // the loops are unrolled so that `off` stays in registers, and every dim that is not there would cost its instructions all
+  // the same (8 instead of 2: a third of those of a 2-D lookup).
+  template <int N>
+  __device__ __forceinline__ void offsets(ll_t e, ll_t (&off)[N]) const {
+    if (s.selector_ndim == 1) {        // one index tensor per dim, most often: nothing to unravel
 #pragma unroll
-    for (int d = 0; d < DOK_MAX_KEY_SIZE; d++) off[d] = 0;
+      for (int d = 0; d < N; d++) off[d] = d < s.ndim ? e * s.strides[d][0] : 0;
+      return;
+    }
+#pragma unroll
+    for (int d = 0; d < N; d++) off[d] = 0;
     unsigned rem = (unsigned)e;        // batches have fewer than 2^32 elements; the outermost index is what is left
     for (int j = s.selector_ndim - 1; j >= 0; j--) {
       const unsigned size = (unsigned)s.sizes[j];
@@ -318,39 +325,48 @@ struct SelKeys {
       const ll_t idx = (ll_t)(rem - q * size);
       rem = q;
 #pragma unroll
-      for (int d = 0; d < DOK_MAX_KEY_SIZE; d++) if (d < s.ndim) off[d] += idx * s.strides[d][j];
+      for (int d = 0; d < N; d++) if (d < s.ndim) off[d] += idx * s.strides[d][j];
     }
   }
-  __device__ __forceinline__ KeyHash hash(const DevHash &hp, ll_t e) const {
-    ll_t off[DOK_MAX_KEY_SIZE];
-    offsets(e, off);
-    ll_t k = index(0, off[0]);
-    ll_t u = dok_uuid_term(k, hp.a[0], hp.b[0], hp.p[0], hp.m[0]);
-    ull_t h = (ull_t)k * (ull_t)hp.a1[0] + (ull_t)hp.b1[0];
+  template <int N>
+  __device__ __forceinline__ KeyHash hash_dims(const DevHash &hp, ll_t e) const {
+    ll_t off[N], k[N];
+    offsets<N>(e, off);
 #pragma unroll
-    for (int d = 1; d < DOK_MAX_KEY_SIZE; d++)
+    for (int d = 0; d < N; d++) k[d] = d < s.ndim ? index(d, off[d]) : 0;          // on their way together
+    ll_t u = dok_uuid_term(k[0], hp.a[0], hp.b[0], hp.p[0], hp.m[0]);
+    ull_t h = (ull_t)k[0] * (ull_t)hp.a1[0] + (ull_t)hp.b1[0];
+#pragma unroll
+    for (int d = 1; d < N; d++)
       if (d < s.ndim) {
-        k = index(d, off[d]);
-        u = (ll_t)((ull_t)u * (ull_t)dok_uuid_term(k, hp.a[d], hp.b[d], hp.p[d], hp.m[d]));
-        h *= (ull_t)k * (ull_t)hp.a1[d] + (ull_t)hp.b1[d];
+        u = (ll_t)((ull_t)u * (ull_t)dok_uuid_term(k[d], hp.a[d], hp.b[d], hp.p[d], hp.m[d]));
+        h *= (ull_t)k[d] * (ull_t)hp.a1[d] + (ull_t)hp.b1[d];
       }
     return KeyHash{dok_llabs(u), (ll_t)h};
   }
-  __device__ __forceinline__ void store_key(const DevTable &t, const DevHash &hp, ll_t e, char *slot) const {
-    ll_t off[DOK_MAX_KEY_SIZE];
-    offsets(e, off);
+  __device__ __forceinline__ KeyHash hash(const DevHash &hp, ll_t e) const {
+    return s.ndim <= 2 ? hash_dims<2>(hp, e) : s.ndim <= 4 ? hash_dims<4>(hp, e) : hash_dims<DOK_MAX_KEY_SIZE>(hp, e);
+  }
+  template <int N>
+  __device__ __forceinline__ void store_key_dims(const DevTable &t, const DevHash &hp, ll_t e, char *slot) const {
+    ll_t off[N];
+    offsets<N>(e, off);
     char *dst_row = slot + t.key_off;
     if (hp.in_order && (t.key_off & 8) == 0) {
 #pragma unroll
-      for (int d = 0; d < DOK_MAX_KEY_SIZE; d += 2) {
+      for (int d = 0; d < N; d += 2) {
         if (d + 1 < s.ndim) *(longlong2 *)(dst_row + 8 * d) = make_longlong2(index(d, off[d]), index(d + 1, off[d + 1]));
         else if (d < s.ndim) *(ll_t *)(dst_row + 8 * d) = index(d, off[d]);
       }
       return;
     }
 #pragma unroll
-    for (int d = 0; d < DOK_MAX_KEY_SIZE; d++)
+    for (int d = 0; d < N; d++)
       if (d < s.ndim) ((ll_t *)dst_row)[hp.perm[d]] = index(d, off[d]);
+  }
+  __device__ __forceinline__ void store_key(const DevTable &t, const DevHash &hp, ll_t e, char *slot) const {
+    if (s.ndim <= 2) store_key_dims<2>(t, hp, e, slot);
+    else store_key_dims<DOK_MAX_KEY_SIZE>(t, hp, e, slot);
   }
 };
 
