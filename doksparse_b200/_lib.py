@@ -112,6 +112,9 @@ def _declare(lib):
         "dok_dok_assign": ([TP, HP, SP, P, P, P, I64, I64, P, P, P], I),
         "dok_set_scratch_words": ([TP, I64], I64),
         "dok_map_set_with": ([TP, HP, P, P, I64, P, I64, I64, P, P], I),
+        "dok_set_takes_sequence": ([TP, HP, I64], I),
+        "dok_map_set_sequenced": ([TP, HP, P, P, I64, P, P, P], I),
+        "dok_dok_assign_sequenced": ([TP, HP, SP, P, P, P, P, P, P], I),
         "dok_dok_to_dense": ([TP, HP, P, P, P], I),
         "dok_dense_count_nonzero": ([P, I64, I, I, P, P], I),
         "dok_dense_insert_nonzero": ([TP, HP, P, P, I64, I, P, P], I),

@@ -31,7 +31,7 @@ struct Plan {
   at::ScalarType key_type, value_type;
 };
 
-enum { STATE_SET = 0, STATE_REMOVE = 8, STATE_BULK = 24, STATE_ADJUST = 7, STATE_WORDS = 32 };   // int64 offsets of the counter blocks
+enum { STATE_SET = 0, STATE_REMOVE = 8, STATE_SEQUENCE = 18, STATE_BULK = 24, STATE_ADJUST = 7, STATE_WORDS = 32 };   // int64 offsets of the counter blocks
 
 PyObject *dok_error = nullptr;
 extern PyTypeObject plan_type;
@@ -281,6 +281,19 @@ PyObject *plan_get(Plan *self, PyObject *arg) {
   });
 }
 
+// in the slots, or in an array that the table has already
+bool has_stamps(const dok_table &table) {
+  dok_layout_info lay;
+  return table.stamp || (dok_table_layout(table.value_bytes, table.key_bytes, table.n_buckets, &lay) == DOK_OK && lay.stamp_offset >= 0);
+}
+
+// in_word(n) -> whether a general set of n rows does without stamps
+PyObject *plan_in_word(Plan *self, PyObject *arg) {
+  const long long n = PyLong_AsLongLong(arg);
+  if (n == -1 && PyErr_Occurred()) return nullptr;
+  return PyBool_FromLong(dok_set_takes_sequence(&self->table, &self->hash, n));
+}
+
 // set(keys, values, assume_unique, epoch, stamp address) -> the number of rows, or None
 PyObject *plan_set(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
   return guarded([&]() -> PyObject * {
@@ -302,7 +315,13 @@ PyObject *plan_set(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
       if (!check(dok_map_set_unique(&table, &self->hash, keys->data_ptr(), values->data_ptr(), n, nullptr, self->state + STATE_SET, stream),
                  "dok_map_set_unique"))
         return nullptr;
+    } else if (dok_set_takes_sequence(&table, &self->hash, n)) {
+      if (!check(dok_map_set_sequenced(&table, &self->hash, keys->data_ptr(), values->data_ptr(), n, self->state + STATE_SEQUENCE,
+                                       self->state + STATE_SET, stream),
+                 "dok_map_set_sequenced"))
+        return nullptr;
     } else {
+      if (!has_stamps(table)) Py_RETURN_NONE;
       const int64_t words = dok_set_scratch_words(&table, n);
       at::Tensor scratch;
       if (words > 0) scratch = at::empty({words}, on_device(self, at::kLong));
@@ -626,7 +645,14 @@ PyObject *plan_assign(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
       }
       values = at::full({}, value, on_device(self, self->value_type)).expand(s.shape);
     }
-    if (s.n > 0) {
+    if (dok_set_takes_sequence(&table, &self->hash, s.n)) {
+      if (!check(dok_dok_assign_sequenced(&table, &self->hash, &s.sel, values.data_ptr(), values.strides().data(), self->state + STATE_SEQUENCE,
+                                          self->state + STATE_SET, self->state + STATE_ADJUST,
+                                          c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()),
+                 "dok_dok_assign_sequenced"))
+        return nullptr;
+    } else if (s.n > 0) {
+      if (!has_stamps(table)) Py_RETURN_NONE;
       const int64_t words = dok_set_scratch_words(&table, s.n);
       at::Tensor scratch;
       if (words > 0) scratch = at::empty({words}, on_device(self, at::kLong));
@@ -655,6 +681,7 @@ PyMethodDef plan_methods[] = {
     {"set_hash", (PyCFunction)(void *)plan_set_hash, METH_FASTCALL, nullptr},
     {"get", (PyCFunction)plan_get, METH_O, nullptr},
     {"set", (PyCFunction)(void *)plan_set, METH_FASTCALL, nullptr},
+    {"in_word", (PyCFunction)plan_in_word, METH_O, nullptr},
     {"remove_rows", (PyCFunction)plan_remove_rows, METH_O, nullptr},
     {"remove", (PyCFunction)plan_remove, METH_O, nullptr},
     {"read", (PyCFunction)plan_read, METH_NOARGS, nullptr},

@@ -11,6 +11,7 @@ struct StridedValues {
   ll_t sizes[DOK_MAX_SELECTOR_NDIM];
   ll_t strides[DOK_MAX_SELECTOR_NDIM];
   __device__ __forceinline__ const char *row(const DevTable &t, ll_t e) const {
+    if (selector_ndim == 1) return src + e * strides[0] * (ll_t)t.vb;
     unsigned rem = (unsigned)e;        // batches have fewer than 2^32 elements
     ll_t off = 0;
     for (int j = selector_ndim - 1; j >= 0; j--) {
@@ -363,6 +364,17 @@ int dok_dok_set_dense(const dok_table *t, const dok_hash_params *hp, const dok_s
   return dok_dok_assign(t, hp, sel, src, src_strides, slot_scratch, n + 1, epoch, counters, nullptr, stream);
 }
 
+static StridedValues strided(const dok_selectors *sel, const void *src, const int64_t *src_strides) {
+  StridedValues sv;
+  sv.src = (const char *)src;
+  sv.selector_ndim = sel->selector_ndim;
+  for (int j = 0; j < DOK_MAX_SELECTOR_NDIM; j++) {
+    sv.sizes[j] = j < sel->selector_ndim ? sel->sizes[j] : 1;
+    sv.strides[j] = j < sel->selector_ndim ? src_strides[j] : 0;
+  }
+  return sv;
+}
+
 int dok_dok_assign(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel, const void *src,
                    const int64_t *src_strides, int64_t *scratch, int64_t scratch_words, int64_t epoch, int64_t *counters,
                    int64_t *more, void *stream) {
@@ -373,14 +385,17 @@ int dok_dok_assign(const dok_table *t, const dok_hash_params *hp, const dok_sele
   if (sk.n == 0) return DOK_OK;
   if (!dok_set_is_small(dt, sk.n) && (!scratch || scratch_words < sk.n + 1)) return DOK_BAD_ARG;
   if (!src || !src_strides || !dok_has_stamps(dt) || epoch < 1 || epoch > DOK_MAX_EPOCH) return DOK_BAD_ARG;
-  StridedValues sv;
-  sv.src = (const char *)src;
-  sv.selector_ndim = sel->selector_ndim;
-  for (int j = 0; j < DOK_MAX_SELECTOR_NDIM; j++) {
-    sv.sizes[j] = j < sel->selector_ndim ? sel->sizes[j] : 1;
-    sv.strides[j] = j < sel->selector_ndim ? src_strides[j] : 0;
-  }
-  return launch_set_general(dt, dh, sk, sv, scratch, epoch, nullptr, counters, (cudaStream_t)stream, more, scratch_words);
+  return launch_set_general(dt, dh, sk, strided(sel, src, src_strides), scratch, epoch, nullptr, counters, (cudaStream_t)stream, more, scratch_words);
+}
+
+int dok_dok_assign_sequenced(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel, const void *src,
+                             const int64_t *src_strides, int64_t *sequence, int64_t *counters, int64_t *more, void *stream) {
+  DevHash dh;
+  DevTable dt;
+  SelKeys sk;
+  if (!prepare(t, hp, &dt, &dh) || !make_sel(sel, dh, &sk) || sk.n < 1 || !dok_set_in_word(dt, dh, sk.n) || !src || !src_strides || !sequence)
+    return DOK_BAD_ARG;
+  return launch_set_word(dt, dh, sk, strided(sel, src, src_strides), sequence, counters, more, (cudaStream_t)stream);
 }
 
 int dok_dok_gather_insert(const dok_table *src, const dok_hash_params *src_hp, const dok_selectors *sel,

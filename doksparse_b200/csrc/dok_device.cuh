@@ -406,7 +406,8 @@ __device__ __forceinline__ void dok_store_word(char *dst, ull_t w, int nbytes, i
 // What a walk of one key's chain found.  found >= 0: the slot holding the uuid.  Otherwise `empty` is the first
 // empty slot of the chain (-1: the whole table was walked without meeting one) and `tomb` the first tombstone
 // met before it (-1: none) -- the two places ClosedHashmap::set may claim (closed_hashmap_impl_class.cu:368-427).
-struct Located { ll_t found, empty, tomb; };
+// word: the value word of the slot that ended the walk, for handlers that ask for it.
+struct Located { ll_t found, empty, tomb; ull_t word = 0; };
 
 // Walk by ONE lane, the reference's loop (closed_hashmap_impl_class.cu:280-312, 368-407) over this library's chain.
 // Used for slots wider than a line (one slot per group).
@@ -430,7 +431,21 @@ __device__ __forceinline__ Located dok_locate_serial(const DevTable &t, const Ke
 
 // No-op hit handler for walks that only need the slot.
 struct NoEmit {
-  static constexpr bool L1 = false, ENDS = false;
+  static constexpr bool L1 = false, ENDS = false, WORD = false;
+  template <int LW>
+  __device__ __forceinline__ void operator()(ll_t, int, const ull_t (&)[LW]) const {}
+};
+
+// {tag, value word} of a slot, in one piece: what a 128-bit CAS has written is seen as a whole
+__device__ __forceinline__ ulonglong2 dok_load_pair(const char *slot) {
+  ulonglong2 v;
+  asm volatile("{\n\t.reg .b128 v;\n\tld.relaxed.gpu.global.b128 v, [%2];\n\tmov.b128 {%0, %1}, v;\n\t}" : "=l"(v.x), "=l"(v.y) : "l"(slot));
+  return v;
+}
+
+// A walk whose owner lanes get the value word of the slot that was found, or of the empty one (of 32-byte slots).
+struct NeedsWord {
+  static constexpr bool L1 = false, ENDS = false, WORD = true;
   template <int LW>
   __device__ __forceinline__ void operator()(ll_t, int, const ull_t (&)[LW]) const {}
 };
@@ -467,6 +482,15 @@ __device__ __forceinline__ void dok_load_words(const char *p, ull_t (&w)[LW]) {
 // Every lane of the warp must call this (inactive lanes pass active = false), with CONSECUTIVE batch elements e in
 // consecutive lanes.  SB = slot bytes (32, 64, 128).  Slot indices are 32-bit here: the host refuses cooperative
 // tables of 2^32 - 1 slots or more.
+template <class Emit, int LW>
+__device__ __forceinline__ void dok_load_line(const char *p, ull_t (&w)[LW]) {
+  if constexpr (Emit::WORD) {
+    const ulonglong2 v = dok_load_pair(p);
+    w[0] = v.x; w[1] = v.y;
+  } else {
+    dok_load_words<LW, Emit::L1>(p, w);
+  }
+}
 template <int SB, int LW, bool TOMB, class Key, class Emit>
 __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key &kh, ll_t e, bool active,
                                                    int *probes, const Emit &emit) {
@@ -479,6 +503,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
   const ll_t e_quad = e - l;                          // batch element of the quad's first lane (elements are consecutive)
   const unsigned n_groups = (unsigned)t.n_groups;     // < 2^32 (checked on the host)
   const char *my_base = t.slots + 32 * l;
+  ull_t word_of = 0;
   // results as 32-bit group-relative codes until the end: slot = group * SPG + position
   unsigned found = NONE, empty = NONE, tomb = NONE;
   unsigned group = NONE, word = 0, walked = 0;
@@ -515,7 +540,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
 #pragma unroll
     for (unsigned r = 0; r < 4; r++) {
       g[r] = __shfl_sync(FULL, group, base + r);
-      if (g[r] != NONE) dok_load_words<LW, Emit::L1>(my_base + (ull_t)g[r] * 128u, w[r]);
+      if (g[r] != NONE) dok_load_line<Emit>(my_base + (ull_t)g[r] * 128u, w[r]);
     }
     unsigned bits = 0, tbits = 0;
 #pragma unroll
@@ -542,6 +567,14 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
         if ((m >> pos) & 1u) emit(e_quad + r, pos, w[r]);
       }
     }
+    if constexpr (Emit::WORD) {
+#pragma unroll
+      for (unsigned r = 0; r < 4; r++) {
+        const unsigned me = ((bits >> (8u * r)) | (bits >> (8u * r + 4u))) & 0xfu;
+        const ull_t v = __shfl_sync(FULL, w[r][LW - 1], base + (me ? __ffs(me) - 1 : 0));
+        if (l == r) word_of = v;
+      }
+    }
     if (group != NONE) {
       const unsigned mine = bits >> (8u * l);
       advance(mine & 0xfu, (mine | (mine >> 4)) & 0xfu, TOMB ? (tbits >> (4u * l)) & 0xfu : 0u);
@@ -558,7 +591,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
     if (!quad) g_r = NONE;
     const ll_t uuid_r = __shfl_sync(FULL, kh.uuid, base + r);
     ull_t wl[LW];
-    if (g_r != NONE) dok_load_words<LW, Emit::L1>(my_base + (ull_t)g_r * 128u, wl);
+    if (g_r != NONE) dok_load_line<Emit>(my_base + (ull_t)g_r * 128u, wl);
     const ll_t tag = (has_tag && g_r != NONE) ? (ll_t)wl[0] : DOK_BLOCKED;
     unsigned bits = ((unsigned)(tag == uuid_r) | ((unsigned)(tag == DOK_EMPTY) << 4) |
                      (TOMB ? (unsigned)(tag == DOK_REMOVED) << 8 : 0u)) << my_slot;
@@ -570,6 +603,10 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
       const int pos = __ffs(me) - 1;
       if ((m >> pos) & 1u) emit(e_quad + r, pos, wl);
     }
+    if constexpr (Emit::WORD) {
+      const ull_t v = __shfl_sync(FULL, wl[LW - 1], base + (me ? __ffs(me) - 1 : 0));
+      if (l == r && group != NONE) word_of = v;
+    }
     if (l == r && group != NONE) advance(m, me, (bits >> 8) & 0xfu);
   }
   if (probes) *probes = (int)walked;
@@ -577,6 +614,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
   res.found = found == NONE ? -1 : (ll_t)found;
   res.empty = empty == NONE ? -1 : (ll_t)empty;
   res.tomb = tomb == NONE ? -1 : (ll_t)tomb;
+  res.word = word_of;
   return res;
 }
 
@@ -585,7 +623,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
 // a hit needs no second access to the table.  LW = 2 serves 32-byte slots whose value is one word behind the tag.
 template <int SB, int LW, bool PASSED>
 struct EmitValue {
-  static constexpr bool L1 = true, ENDS = PASSED;
+  static constexpr bool L1 = true, ENDS = PASSED, WORD = false;
   const DevTable &t;
   char *out_values;
   __device__ __forceinline__ void operator()(ll_t e_r, int pos, const ull_t (&w)[LW]) const {

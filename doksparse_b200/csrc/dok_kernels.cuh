@@ -295,13 +295,14 @@ struct BlockTwins {
 };
 struct Twins { int last; bool more; };     // thread of the key's last row; whether there are others
 
-// every thread of the block must call
-__device__ __forceinline__ Twins dok_find_twins(BlockTwins &b, const KeyHash &kh, bool active) {
+// every thread of the block must call; any: the block has such rows
+__device__ __forceinline__ Twins dok_find_twins(BlockTwins &b, const KeyHash &kh, bool active, bool &any) {
 #pragma unroll
   for (int i = threadIdx.x; i < DOK_TWIN_SLOTS; i += DOK_TPB) { b.chain[i] = DOK_EMPTY; b.more[i] = 0; }
   b.uuid[threadIdx.x] = active ? kh.uuid : DOK_EMPTY;
   __syncthreads();
   int at = 0;
+  bool met = false;
   if (active) {
     const ll_t mine = ((ll_t)dok_chain_hash(kh) & 0x7fffffffffffff00LL) | threadIdx.x;
     at = (int)(mine >> 8) & (DOK_TWIN_SLOTS - 1);
@@ -311,13 +312,14 @@ __device__ __forceinline__ Twins dok_find_twins(BlockTwins &b, const KeyHash &kh
       if (((old ^ mine) >> 8) == 0) {
         atomicMax(&b.chain[at], mine);
         b.more[at] = 1;
+        met = true;
         break;
       }
       at = (at + 1) & (DOK_TWIN_SLOTS - 1);
     }
   }
   asm volatile("cp.async.wait_all;" ::: "memory");              // (k_set_claim: the signal)
-  __syncthreads();
+  any = __syncthreads_or(met);
   Twins w{(int)threadIdx.x, false};
   if (active) {
     const int last = (int)(b.chain[at] & 255);
@@ -349,7 +351,8 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
   KeyHash kh{0, 0};
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
-  const Twins same = dok_find_twins(twins, kh, active);
+  bool any_twins;
+  const Twins same = dok_find_twins(twins, kh, active, any_twins);
   const bool last = active && same.last == (int)threadIdx.x;
   int outcome = -1, conflict = 0, dup = 0;
   ll_t slot = dok_find_or_claim<SB>(t, kh, last, &outcome);
@@ -549,6 +552,8 @@ inline int launch_set_small(const DevTable &t, const DevHash &hp, const Keys &ke
 inline bool dok_is_sliced(const RowKeys &k) { return k.slice_rows != 0; }
 inline bool dok_is_sliced(const SelKeys &) { return false; }
 inline bool dok_set_is_small(const DevTable &t, ll_t n) { return n <= DOK_SMALL_SET_ROWS && dok_window_passes(t) == 1; }
+
+#include "dok_word.cuh"
 
 // contiguous value rows [n, value_bytes]
 template <class Keys, class Values>

@@ -113,6 +113,21 @@ int dok_map_set_with(const dok_table *t, const dok_hash_params *hp, const void *
   return launch_set(dt, dh, rk, (const char *)values, scratch, epoch, nullptr, counters, (cudaStream_t)stream, scratch_words);
 }
 
+int dok_set_takes_sequence(const dok_table *t, const dok_hash_params *hp, int64_t n) {
+  DevHash dh;
+  DevTable dt;
+  return prepare(t, hp, &dt, &dh) && n > 0 && dok_set_in_word(dt, dh, n);
+}
+
+int dok_map_set_sequenced(const dok_table *t, const dok_hash_params *hp, const void *keys, const void *values, int64_t n,
+                          int64_t *sequence, int64_t *counters, void *stream) {
+  DevHash dh;
+  DevTable dt;
+  if (!prepare(t, hp, &dt, &dh) || n < 1 || !dok_set_in_word(dt, dh, n) || !keys || !values || !sequence) return DOK_BAD_ARG;
+  RowKeys rk{keys, n};
+  return launch_set_word(dt, dh, rk, RowValues{(const char *)values}, sequence, counters, nullptr, (cudaStream_t)stream);
+}
+
 int dok_map_remove(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n, uint8_t *out_removed,
                    int64_t *counters, void *stream) {
   DevHash dh;

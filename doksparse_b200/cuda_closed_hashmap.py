@@ -34,6 +34,7 @@ _PARAM_NAMES = ("prime1", "prime2", "alpha1", "alpha2", "beta1", "beta2")
 _STATE_WORDS = 32
 _BY_SET, _BY_REMOVE, _BY_ROWS, _BY_BULK = 0, 8, 16, 24      # set | remove | distinct new rows of float keys | bulk inserts
 _ADJUST = 7              # what n_elements differs by from the slots in use (the reference's DOK assignments over-count)
+_SEQUENCE = 18           # three words: numbers of the rows of sets that need no stamps
 _COUNTED_NEW = 23        # result of the exact count of a set that may have to grow the table
 
 
@@ -671,7 +672,8 @@ class CudaClosedHashmap:
     # ------------------------------------------------------------------ set
     def _launch_set(self, keys, values, assume_unique):
         """The set kernels on contiguous rows of this table."""
-        epoch = self._shared.epoch if assume_unique else self._next_epoch()
+        unstamped = assume_unique or self._native_plan().in_word(keys.shape[0])
+        epoch = self._shared.epoch if unstamped else self._next_epoch()
         self._native_plan().set(keys, values, assume_unique, epoch, self._stamp_address() or 0)
 
     def set(self, new_keys, new_values, assume_unique=False):
@@ -680,8 +682,7 @@ class CudaClosedHashmap:
         plan, sh = self._plan, self._shared
         if plan is not None and self._key_dtype not in L.FLOAT_DTYPES and sh.epoch < L.MAX_EPOCH - 1 \
                 and self._room_for(new_keys.shape[0], int(self._rehash_threshold * self._n_buckets)):
-            stamp = self._stamp_address()
-            rows = None if stamp is None else plan.set(new_keys, new_values, assume_unique, sh.epoch + 1, stamp)
+            rows = plan.set(new_keys, new_values, assume_unique, sh.epoch + 1, self._stamp_address() or 0)
             if rows is not None:
                 sh.epoch += 1
                 self._after_mutation(rows)

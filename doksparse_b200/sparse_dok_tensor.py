@@ -358,17 +358,16 @@ class SparseDOKTensor(object):
         hashmap = self._hashmap
         plan, sh = hashmap._plan or hashmap._native_plan(), hashmap._shared
         if plan is not None and hashmap._value_dtype == self._dtype and sh.epoch < L.MAX_EPOCH - 1:
-            stamp = hashmap._stamp_address()
-            if stamp is not None:
-                limit = hashmap._n_buckets * hashmap._rehash_threshold
-                n = plan.assign(selectors, self._size, values, limit - hashmap._element_bound(), sh.epoch + 1, stamp)
-                if n is not None and n < 0 and hashmap._room_for(-n, limit):
-                    n = plan.assign(selectors, self._size, values, -n, sh.epoch + 1, stamp)
-                if n is not None and n >= 0:
-                    if n:
-                        sh.epoch += 1
-                        hashmap._after_mutation(n)
-                    return
+            stamp = hashmap._stamp_address() or 0
+            limit = hashmap._n_buckets * hashmap._rehash_threshold
+            n = plan.assign(selectors, self._size, values, limit - hashmap._element_bound(), sh.epoch + 1, stamp)
+            if n is not None and n < 0 and hashmap._room_for(-n, limit):
+                n = plan.assign(selectors, self._size, values, -n, sh.epoch + 1, stamp)
+            if n is not None and n >= 0:
+                if n:
+                    sh.epoch += 1
+                    hashmap._after_mutation(n)
+                return
         selectors, _ = self._handle_selectors(selectors)
         shape = selectors[0].shape
         if isinstance(values, SparseDOKTensor) or (isinstance(values, Tensor) and values.is_sparse):
@@ -413,6 +412,14 @@ class SparseDOKTensor(object):
                 hashmap.rehash(math.ceil((n_elements + n_sel) * hashmap._rehash_factor))
         sel = _selectors_struct(selectors)
         src_strides = (ctypes.c_int64 * L.MAX_SELECTOR_NDIM)(*src.stride())
+        if hashmap._native_plan().in_word(n_sel):
+            with L.on(self.device):
+                L.check(L.lib().dok_dok_assign_sequenced(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(src), src_strides,
+                                                         hashmap._counter_block(M._SEQUENCE), hashmap._counter_block(M._BY_SET),
+                                                         hashmap._counter_block(M._ADJUST), L.stream_ptr(self.device)),
+                        "dok_dok_assign_sequenced")
+            hashmap._after_mutation(n_sel)
+            return
         epoch = hashmap._next_epoch()
         words = L.lib().dok_set_scratch_words(hashmap._c_table(), n_sel)
         if words < 0:

@@ -212,7 +212,14 @@ int64_t dok_set_scratch_words(const dok_table *t, int64_t n);
 int dok_map_set_with(const dok_table *t, const dok_hash_params *hp, const void *keys, const void *values, int64_t n,
                      int64_t *scratch, int64_t scratch_words, int64_t epoch, int64_t *counters, void *stream);
 
-/* The same for keys whose identity is the row, as the reference counts every key type (:363): distinct absent ROWS, by
+/* dok_map_set for batches whose values share a word of the slot with their row's number (integer keys, values of at most 4
+ * bytes in 32-byte slots, more rows than the smallest batches have: dok_set_takes_sequence answers 1).  Neither stamps nor
+ * scratch are needed.  sequence: device int64[3] that belong to the table, zero when its slots are initialised. */
+int dok_set_takes_sequence(const dok_table *t, const dok_hash_params *hp, int64_t n);
+int dok_map_set_sequenced(const dok_table *t, const dok_hash_params *hp, const void *keys, const void *values, int64_t n,
+                          int64_t *sequence, int64_t *counters, void *stream);
+
+/* dok_map_count_new for keys whose identity is the row, as the reference counts every key type (:363): distinct absent ROWS, by
  * value (float keys, where the value cast gives different rows one uuid; a row with a NaN counts each time). */
 int dok_map_count_new_rows(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n,
                            int64_t *scratch, int64_t scratch_slots, int64_t *counters, void *stream);
@@ -297,6 +304,10 @@ int dok_dok_set_dense(const dok_table *t, const dok_hash_params *hp, const dok_s
 int dok_dok_assign(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel,
                    const void *src, const int64_t *src_strides, int64_t *scratch, int64_t scratch_words, int64_t epoch,
                    int64_t *counters, int64_t *more, void *stream);
+
+/* dok_dok_assign for batches that dok_set_takes_sequence accepts, sequence as for dok_map_set_sequenced. */
+int dok_dok_assign_sequenced(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel, const void *src,
+                             const int64_t *src_strides, int64_t *sequence, int64_t *counters, int64_t *more, void *stream);
 
 /* Value of every stored element to its position of a dense row-major tensor of the given sizes (HOST int64[key_size]; one
  * value element of 1, 2, 4 or 8 bytes), which the caller has zeroed.  Positions outside the sizes are left out.  Replaces

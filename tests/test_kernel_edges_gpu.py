@@ -83,6 +83,68 @@ def test_assignment_counts_repeated_new_positions(n):
         np.testing.assert_array_equal(host(t.to_dense()), dense)
 
 
+@pytest.mark.parametrize("n", [8192, 8193, 70000])
+@pytest.mark.parametrize("dtype", [np.float32, np.float16, np.int8])
+def test_sets_whose_values_carry_the_row(n, dtype):
+    """Up to 4 bytes in 32-byte slots: the last row of a key stays, within a batch and across the point where the rows'
+    numbers start over; tombstones are reused, and rows of a full table counted."""
+    from doksparse_b200.cuda_closed_hashmap import _SEQUENCE
+    rng = np.random.default_rng(n)
+    pair = Pair(seed=5, n_buckets=100000, rehash_threshold=1.0, **params(1))
+    values = lambda k: rng.integers(-100, 100, (k, 1)).astype(dtype)
+    for spread in (30, 40000, 90000):
+        keys = (rng.zipf(1.3, (n, 1)) % spread) * 7919
+        pair.set(keys, values(n))
+        pair.get(np.arange(100000)[:, None] * 7919)
+        if spread == 40000:
+            pair.remove(keys[: n // 3])
+            pair.c._state[_SEQUENCE] = 0x7ffffff0 - n // 2        # the next set's numbers do not fit any more
+    full = np.arange(160000)[:, None] * 13 + 10 ** 12
+    pair.c.set_rows(dev(np.concatenate([full, full[:5]])), dev(np.concatenate([values(160000)] + [values(5)])))
+    stored = pair.c.get(dev(full))[1].cpu().numpy()
+    assert pair.c.last_set_failed == (~stored).sum() + (~stored[:5]).sum() > 0
+    assert pair.c.nonempty_mask.all()
+
+
+@pytest.mark.parametrize("n", [8192, 8193, 70000])
+def test_assignment_of_narrow_values_counts_repeated_new_positions(n):
+    from doksparse_b200 import SparseDOKTensor
+    rng = np.random.default_rng(n)
+    np.random.seed(1)
+    t = SparseDOKTensor((900, 700), dev(rng.integers(0, 700, (2, 20000))), dev(rng.standard_normal(20000).astype(np.float32)))
+    for distinct in (3, n // 3, n):
+        i, j = rng.integers(0, 900, distinct), rng.integers(0, 700, distinct)
+        pick = rng.integers(0, distinct, n)
+        i, j, v = i[pick], j[pick], rng.standard_normal(n).astype(np.float32)
+        dense = host(t.to_dense())
+        stored, before, live, buckets = t.count_items((dev(i), dev(j))), t._nnz(), t.values().numel(), t.storage().n_buckets
+        t[dev(i), dev(j)] = dev(v)
+        dense[i, j] = v
+        before = before if t.storage().n_buckets == buckets else live        # a rehash counts again
+        assert t._nnz() == before + n - stored
+        np.testing.assert_array_equal(host(t.to_dense()), dense)
+
+
+def test_a_captured_set_counts_on_when_it_is_replayed():
+    from doksparse_b200 import CudaClosedHashmap
+    n = 20000
+    table = CudaClosedHashmap(n_buckets=1 << 18, device="cuda:0")
+    keys, values = torch.arange(n, device="cuda")[:, None] % 9000, torch.rand(n, 1, device="cuda")
+    table.set(keys, values)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        table.set(keys, values)
+    for _ in range(3):
+        order = torch.randperm(n, device="cuda")
+        keys.copy_(keys[order].clone())
+        values.copy_(torch.rand(n, 1, device="cuda"))
+        graph.replay()
+        last = torch.full((9000,), -1, device="cuda").scatter_reduce(0, keys[:, 0], torch.arange(n, device="cuda"), "amax")
+        got, found = table.get(torch.arange(9000, device="cuda")[:, None])
+        assert bool(found.all()) and torch.equal(got, values[last])
+
+
 def _rows(rng, kind, n):
     if kind == "i64":
         return rng.integers(-2 ** 62, 2 ** 62, (n, 1))
