@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_gather_insert(DevTable src, DevHash
   const bool active = sel.row(e);
   KeyHash kh{0, 0};
   if (active) kh = sel.hash(shp, e);
-  const Located loc = dok_locate<SBS, 1, false>(src, kh, e, active, nullptr, NoEmit());
+  const Located loc = dok_locate<SBS, 1, false>(src, kh, e, active, nullptr, NoEmit<false>());
   const bool hit = active && loc.found >= 0;
   ll_t idx[DOK_MAX_KEY_SIZE];
   KeyHash kd{0, 0};

@@ -430,8 +430,9 @@ __device__ __forceinline__ Located dok_locate_serial(const DevTable &t, const Ke
 }
 
 // No-op hit handler for walks that only need the slot.
+template <bool FEW>
 struct NoEmit {
-  static constexpr bool L1 = false, ENDS = false, WORD = false;
+  static constexpr bool L1 = false, ENDS = false, WORD = false, BOTH = FEW;
   template <int LW>
   __device__ __forceinline__ void operator()(ll_t, int, const ull_t (&)[LW]) const {}
 };
@@ -444,8 +445,9 @@ __device__ __forceinline__ ulonglong2 dok_load_pair(const char *slot) {
 }
 
 // A walk whose owner lanes get the value word of the slot that was found, or of the empty one (of 32-byte slots).
+template <bool FEW>
 struct NeedsWord {
-  static constexpr bool L1 = false, ENDS = false, WORD = true;
+  static constexpr bool L1 = false, ENDS = false, WORD = true, BOTH = FEW;
   template <int LW>
   __device__ __forceinline__ void operator()(ll_t, int, const ull_t (&)[LW]) const {}
 };
@@ -533,8 +535,8 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
     }
   };
 
-  // ---- first groups of the quad's four keys: four requests in flight, one packed exchange
-  {
+  // ---- a group of each of the quad's four keys: four requests in flight, one packed exchange
+  auto inspect_all = [&]() {
     ull_t w[4][LW];
     unsigned g[4];
 #pragma unroll
@@ -572,19 +574,17 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
       for (unsigned r = 0; r < 4; r++) {
         const unsigned me = ((bits >> (8u * r)) | (bits >> (8u * r + 4u))) & 0xfu;
         const ull_t v = __shfl_sync(FULL, w[r][LW - 1], base + (me ? __ffs(me) - 1 : 0));
-        if (l == r) word_of = v;
+        if (l == r && group != NONE) word_of = v;
       }
     }
     if (group != NONE) {
       const unsigned mine = bits >> (8u * l);
       advance(mine & 0xfu, (mine | (mine >> 4)) & 0xfu, TOMB ? (tbits >> (4u * l)) & 0xfu : 0u);
     }
-  }
+  };
 
-  // ---- keys whose chain runs into further groups (few below 90 % load): one key per quad and iteration
-  for (;;) {
-    const unsigned pend = __ballot_sync(FULL, group != NONE);
-    if (pend == 0) break;
+  // ---- of one of them
+  auto inspect_one = [&](unsigned pend) {
     const unsigned quad = (pend >> base) & 0xfu;
     const unsigned r = quad ? (unsigned)(__ffs(quad) - 1) : 0u;     // the quad's lowest unfinished key
     unsigned g_r = __shfl_sync(FULL, group, base + r);
@@ -608,6 +608,24 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
       if (l == r && group != NONE) word_of = v;
     }
     if (l == r && group != NONE) advance(m, me, (bits >> 8) & 0xfu);
+  };
+
+  // Keys whose chain runs into further groups.  A large batch, which keeps the memory busy, has the fewest instructions with
+  // one key per quad and iteration.  A small one waits for the iterations: all of the quad's keys at once while a quad has
+  // more than one (sets of 30 k rows of 64-byte slots at load 0.65 55 -> 49 us, lookups 31 -> 27, a table that grows to 300 k
+  // rows 803 -> 767; no difference at 300 k rows; sets of 33.5 M rows 2694 -> 2713).
+  if constexpr (Emit::BOTH) {
+    unsigned pend = FULL;
+    for (bool all = true;;) {
+      if (all) inspect_all(); else inspect_one(pend);
+      pend = __ballot_sync(FULL, group != NONE);
+      if (pend == 0) break;
+      const unsigned per_quad = (pend & 0x11111111u) + ((pend >> 1) & 0x11111111u) + ((pend >> 2) & 0x11111111u) + ((pend >> 3) & 0x11111111u);
+      all = (per_quad & 0x66666666u) != 0;
+    }
+  } else {
+    inspect_all();
+    while (const unsigned pend = __ballot_sync(FULL, group != NONE)) inspect_one(pend);
   }
   if (probes) *probes = (int)walked;
   Located res;
@@ -623,7 +641,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
 // a hit needs no second access to the table.  LW = 2 serves 32-byte slots whose value is one word behind the tag.
 template <int SB, int LW, bool PASSED>
 struct EmitValue {
-  static constexpr bool L1 = true, ENDS = PASSED, WORD = false;
+  static constexpr bool L1 = true, ENDS = PASSED, WORD = false, BOTH = LW != 2;
   const DevTable &t;
   char *out_values;
   __device__ __forceinline__ void operator()(ll_t e_r, int pos, const ull_t (&w)[LW]) const {
@@ -714,10 +732,10 @@ static __device__ __forceinline__ ll_t dok_find_or_claim_serial(const DevTable &
 // where the chain offers a place (first tombstone, else first empty slot); the owner claims that place with one
 // CAS.  Losing the CAS to the same uuid means a twin row of the batch claimed it: join.  Losing it to another
 // uuid is rare; that lane redoes the whole operation with the serial walk.  Every lane of the warp must call.
-template <int SB>
+template <int SB, bool FEW = false>
 __device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHash &key, bool active, int *outcome) {
   const ChainKey kh = dok_chain(key, t);
-  const Located loc = dok_locate<SB, 1, true>(t, kh, 0, active, nullptr, NoEmit());   // the tags are all a claim needs
+  const Located loc = dok_locate<SB, 1, true>(t, kh, 0, active, nullptr, NoEmit<FEW>());   // the tags are all a claim needs
   if (!active) return -1;
   if (loc.found >= 0) { *outcome = DOK_OUT_FOUND; return loc.found; }
   if (loc.tomb >= 0) {

@@ -124,6 +124,12 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, De
   }
 }
 
+// Kernels whose walk has a form for few rows (dok_locate_quad): up to four blocks per SM.
+#define DOK_FEW_BLOCKS (148 * 4)
+#define DOK_BY_SIZE(blocks, CALL)                                    \
+  if ((blocks) <= DOK_FEW_BLOCKS) { constexpr bool FEW = true; CALL; } \
+  else { constexpr bool FEW = false; CALL; }
+
 #define DOK_DISPATCH_SB(t, CALL)                        \
   switch ((t).sb) {                                     \
     case 32: { constexpr int SB = 32; CALL; break; }    \
@@ -333,7 +339,7 @@ __device__ __forceinline__ Twins dok_find_twins(BlockTwins &b, const KeyHash &kh
 // for a batch without equal uuids that is all there is to do.  A row that finds the slot already stamped in
 // this epoch sets the conflict bit and counts a duplicate (in slot_out[n], zeroed by the host before the
 // launch); the second kernel then lets the slot's last row rewrite it.
-template <int SB, class Keys, class Values>
+template <int SB, bool FEW, class Keys, class Values>
 __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp, Keys keys, Values values,
                                                        ll_t *__restrict__ slot_out, unsigned *filter, ll_t epoch, int mark_fresh,
                                                        uint8_t *__restrict__ out_stored, ll_t *counters) {
@@ -355,7 +361,7 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
   const Twins same = dok_find_twins(twins, kh, active, any_twins);
   const bool last = active && same.last == (int)threadIdx.x;
   int outcome = -1, conflict = 0, dup = 0;
-  ll_t slot = dok_find_or_claim<SB>(t, kh, last, &outcome);
+  ll_t slot = dok_find_or_claim<SB, FEW>(t, kh, last, &outcome);
   if (last) {
     const bool fresh = outcome == DOK_OUT_CLAIMED_EMPTY || outcome == DOK_OUT_REUSED;
     slot_out[e] = mark_fresh && fresh ? slot | DOK_ROW_FRESH : slot;
@@ -492,7 +498,7 @@ __global__ void __launch_bounds__(DOK_SMALL_SET_TPB) k_set_small(DevTable t, Dev
   KeyHash kh{0, 0};
   if (active) kh = keys.hash(hp, e);
   int outcome = -1, dup = 0, again = 0;
-  const ll_t slot = dok_find_or_claim<SB>(t, kh, active, &outcome);
+  const ll_t slot = dok_find_or_claim<SB, true>(t, kh, active, &outcome);
   const bool placed = active && slot >= 0, fresh = outcome == DOK_OUT_CLAIMED_EMPTY || outcome == DOK_OUT_REUSED;
   ull_t *stamp = placed ? (ull_t *)dok_stamp_ptr(t, slot) : nullptr;
   if (placed) {
@@ -530,22 +536,21 @@ __global__ void __launch_bounds__(DOK_SMALL_SET_TPB) k_set_small(DevTable t, Dev
   dok_tally_flush(tally, counters, more);
 }
 
-template <int SB, class Keys, class Values>
-inline int launch_set_small(const DevTable &t, const DevHash &hp, const Keys &keys, const Values &values, ll_t epoch, ll_t *counters,
-                            ll_t *more, cudaStream_t st) {
+template <class Kernel, class... Args>
+inline int dok_launch_cluster(ll_t rows, cudaStream_t st, Kernel kernel, Args... args) {
   unsigned blocks = 1;
-  while ((ll_t)blocks * DOK_SMALL_SET_TPB < keys.n) blocks *= 2;
+  while ((ll_t)blocks * DOK_SMALL_SET_TPB < rows) blocks *= 2;
   cudaLaunchAttribute cluster;
   cluster.id = cudaLaunchAttributeClusterDimension;
   cluster.val.clusterDim.x = blocks;
   cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(blocks);
-  config.blockDim = dim3(blocks > 1 ? DOK_SMALL_SET_TPB : (unsigned)((keys.n + 63) / 64 * 64));
+  config.blockDim = dim3(blocks > 1 ? DOK_SMALL_SET_TPB : (unsigned)((rows + 63) / 64 * 64));
   config.stream = st;
   config.attrs = &cluster;
   config.numAttrs = 1;
-  cudaLaunchKernelEx(&config, k_set_small<SB, Keys, Values>, t, hp, keys, values, epoch, counters, more);
+  cudaLaunchKernelEx(&config, kernel, args...);
   return dok_check_launch();
 }
 
@@ -562,7 +567,7 @@ inline int launch_set_general(const DevTable &t, const DevHash &hp, const Keys &
                               int64_t *more = nullptr, int64_t scratch_words = 0) {
   if (!out_stored && !dok_is_sliced(keys) && dok_set_is_small(t, keys.n)) {
     int rc = DOK_OK;
-    DOK_DISPATCH_SB(t, (rc = launch_set_small<SB>(t, hp, keys, values, (ll_t)epoch, (ll_t *)counters, (ll_t *)more, st)));
+    DOK_DISPATCH_SB(t, (rc = dok_launch_cluster(keys.n, st, k_set_small<SB, Keys, Values>, t, hp, keys, values, (ll_t)epoch, (ll_t *)counters, (ll_t *)more)));
     return rc;
   }
   const bool filtered = keys.n >= DOK_FILTER_FROM && scratch_words >= keys.n + 1 + DOK_FILTER_ALL;
@@ -571,8 +576,8 @@ inline int launch_set_general(const DevTable &t, const DevHash &hp, const Keys &
   if (cudaMemsetAsync(slot_scratch + keys.n, 0, zeroed, st) != cudaSuccess) return dok_check_launch();
   const dim3 grid = dok_grid(keys);
   int rc = DOK_OK;
-  DOK_DISPATCH_SB(t, DOK_FOR_WINDOWS(t, rc, (k_set_claim<SB><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, (ll_t *)slot_scratch, filter,
-                                                                                       (ll_t)epoch, more != nullptr, out_stored, (ll_t *)counters))));
+  DOK_DISPATCH_SB(t, DOK_BY_SIZE(grid.x * grid.y, DOK_FOR_WINDOWS(t, rc, (k_set_claim<SB, FEW><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, (ll_t *)slot_scratch, filter,
+                                                                                       (ll_t)epoch, more != nullptr, out_stored, (ll_t *)counters)))));
   if (rc != DOK_OK) return rc;
   dim3 few = grid;
   if (few.x > 148 * 8) few.x = 148 * 8;
@@ -603,7 +608,7 @@ inline int launch_set_unique(const DevTable &t, const DevHash &hp, const RowKeys
 
 // REMOVE = 1: the tag is swapped to the tombstone by CAS so that equal uuids in one batch report exactly once
 // (ClosedHashmap::remove, closed_hashmap_impl_class.cu:459-484, stores it non-atomically).
-template <int SB, int REMOVE, class Keys>
+template <int SB, int REMOVE, bool FEW, class Keys>
 __global__ void __launch_bounds__(DOK_TPB) k_find(DevTable t, DevHash hp, Keys keys, uint8_t *__restrict__ out_flags,
                                                   ll_t *counters) {
   __shared__ BlockTally tally;
@@ -614,7 +619,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_find(DevTable t, DevHash hp, Keys k
   KeyHash kh{0, 0};
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
-  const Located loc = dok_locate<SB, 1, false>(t, kh, e, active, nullptr, NoEmit());
+  const Located loc = dok_locate<SB, 1, false>(t, kh, e, active, nullptr, NoEmit<FEW>());
   int hit = active && loc.found >= 0;
   if (REMOVE && hit) hit = dok_cas_tag(t, loc.found, kh.uuid, DOK_REMOVED) == kh.uuid;
   if (active && out_flags) out_flags[e] = (uint8_t)hit;
@@ -629,7 +634,7 @@ inline int launch_find(const DevTable &t, const DevHash &hp, const Keys &keys, u
                        cudaStream_t st) {
   const dim3 grid = dok_grid(keys);
   int rc = DOK_OK;
-  DOK_DISPATCH_SB(t, DOK_FOR_WINDOWS(t, rc, (k_find<SB, REMOVE><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, out_flags, (ll_t *)counters))));
+  DOK_DISPATCH_SB(t, DOK_BY_SIZE(grid.x * grid.y, DOK_FOR_WINDOWS(t, rc, (k_find<SB, REMOVE, FEW><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, out_flags, (ll_t *)counters)))));
   return rc;
 }
 
@@ -639,7 +644,7 @@ static __global__ void k_fill_i64(ll_t *p, ll_t n, ll_t v) {
 
 // Rows absent from the table insert their uuid into a scratch tag set; the number of successful claims is the
 // number of distinct absent uuids.
-template <int SB, class Keys>
+template <int SB, bool FEW, class Keys>
 __global__ void __launch_bounds__(DOK_TPB) k_count_new(DevTable t, DevHash hp, Keys keys, ll_t *__restrict__ scratch,
                                                        ll_t scratch_slots, ll_t *counters) {
   __shared__ BlockTally tally;
@@ -651,7 +656,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_count_new(DevTable t, DevHash hp, K
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
   Located loc{-1, -1, -1};
-  if (t.n_groups > 0) loc = dok_locate<SB, 1, false>(t, kh, e, active, nullptr, NoEmit());      // (0: no table, every row is absent)
+  if (t.n_groups > 0) loc = dok_locate<SB, 1, false>(t, kh, e, active, nullptr, NoEmit<FEW>());      // (0: no table, every row is absent)
   int claimed = 0;
   if (active && loc.found < 0) {
     const ll_t uuid = kh.uuid;
@@ -679,7 +684,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_count_new(DevTable t, DevHash hp, K
 // the reference's rehash = two boolean-mask gathers plus a full `set` with its pre-get and unique
 // (cuda_closed_hashmap.py:456-468) and this library's own compaction + insert.  Live keys are pairwise different,
 // so every row claims a fresh slot; tombstones stay behind.
-template <int SB>
+template <int SB, bool FEW>
 __global__ void __launch_bounds__(DOK_TPB) k_reinsert(DevTable src, DevTable dst, DevHash hp, ll_t *counters) {
   const ll_t stride = (ll_t)gridDim.x * DOK_TPB;
   int claimed = 0, failed = 0, found = 0;
@@ -702,7 +707,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_reinsert(DevTable src, DevTable dst
     }
     active = dok_in_window(dst, kh, active);
     int outcome = -1;
-    const ll_t slot = dok_find_or_claim<SB>(dst, kh, active, &outcome);
+    const ll_t slot = dok_find_or_claim<SB, FEW>(dst, kh, active, &outcome);
     if (active && slot >= 0) {
       char *drow = dok_key_row(dst, slot);
       if ((dst.kb & 7) == 0) for (int i = 0; i < (dst.kb >> 3); i++) ((ull_t *)drow)[i] = ((const ull_t *)krow)[i];

@@ -22,18 +22,20 @@
 enum { DOK_SEQ_NEXT = 0, DOK_SEQ_BASE = 1, DOK_SEQ_TICKET = 2 };
 
 inline bool dok_set_in_word(const DevTable &t, const DevHash &hp, ll_t n) {
-  return t.sb == 32 && t.vb <= 4 && hp.dtype < DOK_F16 && !dok_set_is_small(t, n) && n <= DOK_WORD_ROWS;
+  return t.sb == 32 && t.vb <= 4 && hp.dtype < DOK_F16 && n <= DOK_WORD_ROWS;
 }
 
+__device__ __forceinline__ void dok_clear_numbers(const DevTable &t) {
+  for (ll_t i = (ll_t)blockIdx.x * blockDim.x + threadIdx.x; i < t.n_slots; i += (ll_t)gridDim.x * blockDim.x)
+    *(unsigned *)(dok_value_ptr(t, i) + 4) = 0;
+}
 // The numbers of this set's rows: base + 1 ... base + n.
 static __global__ void __launch_bounds__(DOK_TPB) k_word_begin(DevTable t, ll_t *sequence, ll_t n) {
   __shared__ ll_t next;
   if (threadIdx.x == 0) next = *(volatile ll_t *)&sequence[DOK_SEQ_NEXT];
   __syncthreads();
   const bool over = next + n > DOK_WORD_ROWS;
-  if (over)
-    for (ll_t i = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x; i < t.n_slots; i += (ll_t)gridDim.x * DOK_TPB)
-      *(unsigned *)(dok_value_ptr(t, i) + 4) = 0;
+  if (over) dok_clear_numbers(t);
   __syncthreads();
   if (threadIdx.x != 0) return;
   __threadfence();
@@ -81,9 +83,10 @@ static __device__ __forceinline__ WordSlot dok_claim_word_serial(const DevTable 
 }
 
 // dok_find_or_claim with words.  Every lane of the warp must call.
+template <bool FEW>
 __device__ __forceinline__ WordSlot dok_find_or_claim_word(const DevTable &t, const KeyHash &kh, bool active, ull_t word) {
   const ChainKey key = dok_chain(kh, t);
-  const Located loc = dok_locate_quad<32, 2, true>(t, key, 0, active, nullptr, NeedsWord());
+  const Located loc = dok_locate_quad<32, 2, true>(t, key, 0, active, nullptr, NeedsWord<FEW>());
   if (!active) return WordSlot{-1, -1, 0};
   if (loc.found >= 0) return WordSlot{loc.found, DOK_OUT_FOUND, loc.word};
   const bool reuse = loc.tomb >= 0;
@@ -101,7 +104,33 @@ __device__ __forceinline__ WordSlot dok_find_or_claim_word(const DevTable &t, co
   return dok_claim_word_serial(t, key, word);
 }
 
-template <class Keys, class Values>
+__device__ __forceinline__ ull_t dok_narrow_value(const char *src, int vb) {
+  if (vb == 4) return *(const unsigned *)src;
+  if (vb == 2) return *(const unsigned short *)src;
+  ull_t v = 0;
+  for (int b = 0; b < vb; b++) v |= (ull_t)(unsigned char)src[b] << (8 * b);
+  return v;
+}
+
+// What became of a row that goes to the table.
+struct WordOutcome {
+  bool claimed, met;       // met: another row of this batch was there before,
+  ull_t fresh;             // ... and this batch claimed the slot
+};
+template <class Keys>
+__device__ __forceinline__ WordOutcome dok_write_word(const DevTable &t, const DevHash &hp, const Keys &keys, ll_t e, const WordSlot &found,
+                                                      ll_t base, ull_t word) {
+  WordOutcome o;
+  const ull_t before = found.word >> DOK_WORD_SHIFT;
+  o.claimed = found.outcome == DOK_OUT_CLAIMED_EMPTY || found.outcome == DOK_OUT_REUSED;
+  o.met = found.outcome == DOK_OUT_FOUND && before > (ull_t)base;
+  o.fresh = o.met ? found.word & DOK_WORD_FRESH : 0;
+  if (o.claimed) keys.store_key(t, hp, e, dok_slot_ptr(t, found.slot));
+  if (found.outcome == DOK_OUT_FOUND && before < word >> DOK_WORD_SHIFT) atomicMax((ull_t *)dok_value_ptr(t, found.slot), word | o.fresh);
+  return o;
+}
+
+template <bool FEW, class Keys, class Values>
 __global__ void __launch_bounds__(DOK_TPB, 6) k_set_word(DevTable t, DevHash hp, Keys keys, Values values, const ll_t *sequence,
                                                          ll_t *counters, ll_t *more) {
   __shared__ BlockTally tally;
@@ -115,25 +144,18 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_word(DevTable t, DevHash hp,
   ull_t value = 0;
   if (active) {
     kh = keys.hash(hp, e);
-    const char *src = values.row(t, e);
-    value = t.vb == 4 ? *(const unsigned *)src : t.vb == 2 ? *(const unsigned short *)src : 0;
-    if (t.vb == 1 || t.vb == 3) for (int b = 0; b < t.vb; b++) value |= (ull_t)(unsigned char)src[b] << (8 * b);
+    value = dok_narrow_value(values.row(t, e), t.vb);
   }
   active = dok_in_window(t, kh, active);
   bool any_twins;
   const Twins same = dok_find_twins(twins, kh, active, any_twins);
   const bool last = active && same.last == (int)threadIdx.x;
-  const ull_t number = (ull_t)(base + e + 1), word = number << DOK_WORD_SHIFT | value;
-  const WordSlot found = dok_find_or_claim_word(t, kh, last, word | DOK_WORD_FRESH);
-  const bool claimed = found.outcome == DOK_OUT_CLAIMED_EMPTY || found.outcome == DOK_OUT_REUSED;
-  const ull_t before = found.word >> DOK_WORD_SHIFT;
-  const bool met = found.outcome == DOK_OUT_FOUND && before > (ull_t)base;              // by another row of this batch,
-  const ull_t fresh = met ? found.word & DOK_WORD_FRESH : 0;                            // ... which claimed the slot
-  int failed = found.outcome == DOK_OUT_FAILED, again = failed || fresh != 0, twin = active && !last;
-  if (claimed) keys.store_key(t, hp, e, dok_slot_ptr(t, found.slot));
-  if (found.outcome == DOK_OUT_FOUND && before < number) atomicMax((ull_t *)dok_value_ptr(t, found.slot), word | fresh);
+  const ull_t word = (ull_t)(base + e + 1) << DOK_WORD_SHIFT | value;
+  const WordSlot found = dok_find_or_claim_word<FEW>(t, kh, last, word | DOK_WORD_FRESH);
+  const WordOutcome o = dok_write_word(t, hp, keys, e, found, base, word);
+  int failed = found.outcome == DOK_OUT_FAILED, again = failed || o.fresh != 0, twin = active && !last;
   if (any_twins) {                                           // uniform over the block
-    if (last) twins.slot[threadIdx.x] = failed ? 2 : claimed || fresh;
+    if (last) twins.slot[threadIdx.x] = failed ? 2 : o.claimed || o.fresh;
     __syncthreads();
     if (twin) {
       const ll_t how = twins.slot[same.last];
@@ -147,17 +169,61 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_word(DevTable t, DevHash hp,
     dok_tally_add(tally, DOK_CNT_REUSED_REMOVED, found.outcome == DOK_OUT_REUSED);
     dok_tally_add(tally, DOK_CNT_FAILED, failed);
     dok_tally_add(tally, DOK_CNT_HITS, (twin && !failed) || found.outcome == DOK_OUT_FOUND);
-    dok_tally_add(tally, DOK_CNT_DUPLICATES, twin || met);
+    dok_tally_add(tally, DOK_CNT_DUPLICATES, twin || o.met);
   }
   dok_tally_flush(tally, counters, more);
+}
+
+// The same for a batch that one cluster holds (k_set_small), in one launch: the blocks read the next number together, and the
+// first one moves it on when all have.
+template <class Keys, class Values>
+__global__ void __launch_bounds__(DOK_SMALL_SET_TPB) k_set_word_small(DevTable t, DevHash hp, Keys keys, Values values, ll_t *sequence,
+                                                                      ll_t *counters, ll_t *more) {
+  __shared__ BlockTally tally;
+  dok_tally_begin(tally);
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  ll_t base = *(volatile ll_t *)&sequence[DOK_SEQ_NEXT];
+  const bool over = base + keys.count() > DOK_WORD_ROWS;     // uniform over the launch
+  if (over) {
+    base = 0;
+    dok_clear_numbers(t);
+    cluster.sync();
+  }
+  const ll_t e = (ll_t)blockIdx.x * DOK_SMALL_SET_TPB + threadIdx.x;
+  const bool active = e < keys.count();
+  KeyHash kh{0, 0};
+  ull_t value = 0;
+  if (active) {
+    kh = keys.hash(hp, e);
+    value = dok_narrow_value(values.row(t, e), t.vb);
+  }
+  const ull_t word = (ull_t)(base + e + 1) << DOK_WORD_SHIFT | value;
+  const WordSlot found = dok_find_or_claim_word<true>(t, kh, active, word | DOK_WORD_FRESH);
+  const WordOutcome o = dok_write_word(t, hp, keys, e, found, base, word);
+  const int failed = found.outcome == DOK_OUT_FAILED;
+  dok_tally_add(tally, DOK_TALLY_EXTRA, failed || o.fresh != 0);
+  if (counters) {
+    dok_tally_add(tally, DOK_CNT_CLAIMED_EMPTY, found.outcome == DOK_OUT_CLAIMED_EMPTY);
+    dok_tally_add(tally, DOK_CNT_REUSED_REMOVED, found.outcome == DOK_OUT_REUSED);
+    dok_tally_add(tally, DOK_CNT_FAILED, failed);
+    dok_tally_add(tally, DOK_CNT_HITS, found.outcome == DOK_OUT_FOUND);
+    dok_tally_add(tally, DOK_CNT_DUPLICATES, o.met);
+  }
+  dok_tally_flush(tally, counters, more);
+  cluster.sync();
+  if (blockIdx.x == 0 && threadIdx.x == 0) sequence[DOK_SEQ_NEXT] = base + keys.count();
 }
 
 template <class Keys, class Values>
 inline int launch_set_word(const DevTable &t, const DevHash &hp, const Keys &keys, const Values &values, int64_t *sequence, int64_t *counters,
                            int64_t *more, cudaStream_t st) {
+  if (dok_set_is_small(t, keys.n))
+    return dok_launch_cluster(keys.n, st, k_set_word_small<Keys, Values>, t, hp, keys, values, (ll_t *)sequence, (ll_t *)counters, (ll_t *)more);
   k_word_begin<<<148, DOK_TPB, 0, st>>>(t, (ll_t *)sequence, keys.n);
   int rc = dok_check_launch();
   if (rc != DOK_OK) return rc;
-  DOK_FOR_WINDOWS(t, rc, (k_set_word<<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, values, (const ll_t *)sequence, (ll_t *)counters, (ll_t *)more)));
+  const dim3 grid = dok_grid(keys);
+  DOK_BY_SIZE(grid.x, DOK_FOR_WINDOWS(t, rc, (k_set_word<FEW><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, (const ll_t *)sequence,
+                                                                                     (ll_t *)counters, (ll_t *)more))));
   return rc;
 }

@@ -165,8 +165,8 @@ int dok_map_count_new(const dok_table *t, const dok_hash_params *hp, const void 
   if (rc != DOK_OK) return rc;
   RowKeys rk{keys, n};
   rc = DOK_OK;
-  DOK_DISPATCH_SB(dt, DOK_FOR_WINDOWS(dt, rc, (k_count_new<SB><<<grid_for(n), DOK_TPB, 0, (cudaStream_t)stream>>>(
-                                                  wt, dh, rk, (ll_t *)scratch_tags, scratch_slots, (ll_t *)counters))));
+  DOK_DISPATCH_SB(dt, DOK_BY_SIZE(grid_for(n), DOK_FOR_WINDOWS(dt, rc, (k_count_new<SB, FEW><<<grid_for(n), DOK_TPB, 0, (cudaStream_t)stream>>>(
+                                                  wt, dh, rk, (ll_t *)scratch_tags, scratch_slots, (ll_t *)counters)))));
   return rc;
 }
 
@@ -267,8 +267,8 @@ int dok_map_reinsert(const dok_table *src, const dok_table *dst, const dok_hash_
   if (blocks > 148 * 8) blocks = 148 * 8;            // 8 resident blocks of 256 threads per SM, grid-stride over the slots
   if (blocks < 1) blocks = 1;
   int rc = DOK_OK;
-  DOK_DISPATCH_SB(dt, DOK_FOR_WINDOWS(dt, rc, (k_reinsert<SB><<<(unsigned)blocks, DOK_TPB, 0, (cudaStream_t)stream>>>(
-                                                  st_, wt, dh, (ll_t *)counters))));
+  DOK_DISPATCH_SB(dt, DOK_BY_SIZE(blocks, DOK_FOR_WINDOWS(dt, rc, (k_reinsert<SB, FEW><<<(unsigned)blocks, DOK_TPB, 0, (cudaStream_t)stream>>>(
+                                                  st_, wt, dh, (ll_t *)counters)))));
   return rc;
 }
 

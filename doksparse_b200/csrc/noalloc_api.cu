@@ -77,7 +77,7 @@ int dok_map_count_new_static(const dok_table *t, const dok_hash_params *hp, cons
   RowKeys rk{keys, n};
   const unsigned grid = (unsigned)((n + DOK_TPB - 1) / DOK_TPB);
   rc = DOK_OK;
-  DOK_DISPATCH_SB(dt, DOK_FOR_WINDOWS(dt, rc, (k_count_new<SB><<<grid, DOK_TPB, 0, st>>>(wt, dh, rk, scratch, slots, (ll_t *)counters))));
+  DOK_DISPATCH_SB(dt, DOK_FOR_WINDOWS(dt, rc, (k_count_new<SB, false><<<grid, DOK_TPB, 0, st>>>(wt, dh, rk, scratch, slots, (ll_t *)counters))));
   return rc;
 }
 

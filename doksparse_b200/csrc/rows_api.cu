@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_count_new_rows(DevTable t, DevHash 
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
   Located loc{-1, -1, -1};
-  if (t.n_groups > 0) loc = dok_locate<SB, 1, false>(t, kh, e, active, nullptr, NoEmit());      // (0: no table, every row is absent)
+  if (t.n_groups > 0) loc = dok_locate<SB, 1, false>(t, kh, e, active, nullptr, NoEmit<false>());      // (0: no table, every row is absent)
   int claimed = 0;
   if (active && loc.found < 0) {
     bool nan = false;
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(DOK_SMALL_TPB) k_remove_unique_small(DevTable 
     const ll_t e = active ? s.row[i] : 0;
     KeyHash kh{0, 0};
     if (active) kh = keys.hash(hp, e);
-    const Located loc = dok_locate<SB, 1, false>(t, kh, 0, active, nullptr, NoEmit());
+    const Located loc = dok_locate<SB, 1, false>(t, kh, 0, active, nullptr, NoEmit<true>());
     int hit = active && loc.found >= 0;
     if (hit) hit = dok_cas_tag(t, loc.found, kh.uuid, DOK_REMOVED) == kh.uuid;
     if (active) out_removed[i] = (uint8_t)hit;

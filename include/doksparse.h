@@ -213,8 +213,8 @@ int dok_map_set_with(const dok_table *t, const dok_hash_params *hp, const void *
                      int64_t *scratch, int64_t scratch_words, int64_t epoch, int64_t *counters, void *stream);
 
 /* dok_map_set for batches whose values share a word of the slot with their row's number (integer keys, values of at most 4
- * bytes in 32-byte slots, more rows than the smallest batches have: dok_set_takes_sequence answers 1).  Neither stamps nor
- * scratch are needed.  sequence: device int64[3] that belong to the table, zero when its slots are initialised. */
+ * bytes in 32-byte slots: dok_set_takes_sequence answers 1).  Neither stamps nor scratch are needed.  sequence: device
+ * int64[3] that belong to the table, zero when its slots are initialised. */
 int dok_set_takes_sequence(const dok_table *t, const dok_hash_params *hp, int64_t n);
 int dok_map_set_sequenced(const dok_table *t, const dok_hash_params *hp, const void *keys, const void *values, int64_t n,
                           int64_t *sequence, int64_t *counters, void *stream);

@@ -83,7 +83,7 @@ def test_assignment_counts_repeated_new_positions(n):
         np.testing.assert_array_equal(host(t.to_dense()), dense)
 
 
-@pytest.mark.parametrize("n", [8192, 8193, 70000])
+@pytest.mark.parametrize("n", [3, 1024, 1025, 8192, 8193, 70000])
 @pytest.mark.parametrize("dtype", [np.float32, np.float16, np.int8])
 def test_sets_whose_values_carry_the_row(n, dtype):
     """Up to 4 bytes in 32-byte slots: the last row of a key stays, within a batch and across the point where the rows'
@@ -106,13 +106,13 @@ def test_sets_whose_values_carry_the_row(n, dtype):
     assert pair.c.nonempty_mask.all()
 
 
-@pytest.mark.parametrize("n", [8192, 8193, 70000])
+@pytest.mark.parametrize("n", [3, 1025, 8192, 8193, 70000])
 def test_assignment_of_narrow_values_counts_repeated_new_positions(n):
     from doksparse_b200 import SparseDOKTensor
     rng = np.random.default_rng(n)
     np.random.seed(1)
     t = SparseDOKTensor((900, 700), dev(rng.integers(0, 700, (2, 20000))), dev(rng.standard_normal(20000).astype(np.float32)))
-    for distinct in (3, n // 3, n):
+    for distinct in (1, n // 3, n):
         i, j = rng.integers(0, 900, distinct), rng.integers(0, 700, distinct)
         pick = rng.integers(0, distinct, n)
         i, j, v = i[pick], j[pick], rng.standard_normal(n).astype(np.float32)
