@@ -444,6 +444,14 @@ __device__ __forceinline__ ulonglong2 dok_load_pair(const char *slot) {
   return v;
 }
 
+// A lookup that only needs the slot.
+template <bool FEW>
+struct Probe {
+  static constexpr bool L1 = true, ENDS = false, WORD = false, BOTH = FEW;
+  template <int LW>
+  __device__ __forceinline__ void operator()(ll_t, int, const ull_t (&)[LW]) const {}
+};
+
 // A walk whose owner lanes get the value word of the slot that was found, or of the empty one (of 32-byte slots).
 template <bool FEW>
 struct NeedsWord {
@@ -636,38 +644,34 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
   return res;
 }
 
-// Hit handler of `get` (PASSED: of a table whose groups remember that a key went past them): the lanes of the quad write
-// the value straight from the registers that hold the line, so
-// a hit needs no second access to the table.  LW = 2 serves 32-byte slots whose value is one word behind the tag.
+// Hit handler of `get` (PASSED: of a table whose groups remember that a key went past them): the lane that holds the slot
+// writes the value straight from its registers, so a hit needs no second access to the table.  LW = 2 serves values of at
+// most 8 bytes, one word behind the tag, LW = 4 the whole of a 32-byte slot.
 template <int SB, int LW, bool PASSED>
 struct EmitValue {
-  static constexpr bool L1 = true, ENDS = PASSED, WORD = false, BOTH = LW != 2;
+  static constexpr bool L1 = true, ENDS = PASSED, WORD = false, BOTH = false;
   const DevTable &t;
   char *out_values;
   __device__ __forceinline__ void operator()(ll_t e_r, int pos, const ull_t (&w)[LW]) const {
-    const int l = (int)(threadIdx.x & 3u);
+    if ((int)(threadIdx.x & 3u) != pos * (SB / 32)) return;
     char *dst = out_values + e_r * (ll_t)t.vb;
-    if constexpr (SB == 32 && LW == 2) {
-      if (l == pos) {
-        if (t.vb == 8) *(ull_t *)dst = w[1];
-        else dok_store_word(dst, w[1], t.vb, (t.vb & -t.vb));
+    if constexpr (LW == 2) {
+      if (t.vb == 8) *(ull_t *)dst = w[1];
+      else dok_store_word(dst, w[1], t.vb, (t.vb & -t.vb));
+    } else if ((t.vb & 7) == 0) {
+#pragma unroll
+      for (int j = 1; j < LW; j++) if (8 * j <= t.vb) *(ull_t *)(dst + 8 * j - 8) = w[j];
+    } else if ((t.vb & 3) == 0) {
+#pragma unroll
+      for (int j = 1; j < LW; j++) {
+        if (8 * j - 4 <= t.vb) *(unsigned *)(dst + 8 * j - 8) = (unsigned)w[j];
+        if (8 * j <= t.vb) *(unsigned *)(dst + 8 * j - 4) = (unsigned)(w[j] >> 32);
       }
     } else {
-      const int start = pos * SB + 8 - 32 * l;             // offset of the value relative to this lane's chunk
-      if ((t.vb & 7) == 0) {
+      const int align = t.vb & -t.vb;
 #pragma unroll
-        for (int j = 0; j < LW; j++) {
-          const int rel = 8 * j - start;
-          if ((unsigned)rel < (unsigned)t.vb) *(ull_t *)(dst + rel) = w[j];
-        }
-        return;
-      }
-      const int align = (t.vb & -t.vb) < 8 ? (t.vb & -t.vb) : 8;
-#pragma unroll
-      for (int j = 0; j < LW; j++) {
-        const int rel = 8 * j - start;
-        if (rel >= 0 && rel < t.vb) dok_store_word(dst + rel, w[j], t.vb - rel < 8 ? t.vb - rel : 8, align);
-      }
+      for (int j = 1; j < LW; j++)
+        if (8 * j - 8 < t.vb) dok_store_word(dst + 8 * j - 8, w[j], t.vb - 8 * j + 8 < 8 ? t.vb - 8 * j + 8 : 8, align);
     }
   }
 };
@@ -773,18 +777,23 @@ __device__ __forceinline__ void dok_store_value(const DevTable &t, ll_t slot, co
 }
 
 // slot -> value row
+template <bool L1, class T>
+__device__ __forceinline__ T dok_load_as(const T *p) {
+  return L1 ? __ldca(p) : __ldcg(p);
+}
+template <bool L1 = false>
 __device__ __forceinline__ void dok_load_value(const DevTable &t, ll_t slot, char *dst) {
   const ull_t *src = (const ull_t *)dok_value_ptr(t, slot);
-  if (t.vb == 8) { *(ull_t *)dst = __ldcg(src); return; }
-  if (t.vb == 4) { *(unsigned *)dst = __ldcg((const unsigned *)src); return; }
+  if (t.vb == 8) { *(ull_t *)dst = dok_load_as<L1>(src); return; }
+  if (t.vb == 4) { *(unsigned *)dst = dok_load_as<L1>((const unsigned *)src); return; }
   if ((t.vb & 7) == 0) {
-    for (int w = 0; w < t.vwords; w++) ((ull_t *)dst)[w] = __ldcg(src + w);
+    for (int w = 0; w < t.vwords; w++) ((ull_t *)dst)[w] = dok_load_as<L1>(src + w);
   } else if ((t.vb & 3) == 0) {
-    for (int w = 0; w < (t.vb >> 2); w++) ((unsigned *)dst)[w] = __ldcg((const unsigned *)src + w);
+    for (int w = 0; w < (t.vb >> 2); w++) ((unsigned *)dst)[w] = dok_load_as<L1>((const unsigned *)src + w);
   } else if ((t.vb & 1) == 0) {
-    for (int w = 0; w < (t.vb >> 1); w++) ((unsigned short *)dst)[w] = __ldcg((const unsigned short *)src + w);
+    for (int w = 0; w < (t.vb >> 1); w++) ((unsigned short *)dst)[w] = dok_load_as<L1>((const unsigned short *)src + w);
   } else {
-    for (int w = 0; w < t.vb; w++) dst[w] = __ldcg((const char *)src + w);
+    for (int w = 0; w < t.vb; w++) dst[w] = dok_load_as<L1>((const char *)src + w);
   }
 }
 

@@ -16,12 +16,19 @@
 // get
 // ---------------------------------------------------------------------------------------------------------
 // One row per thread: for 32-byte slots with values of at most 8 bytes, whose walk fits 32 registers, so that 64 warps are
-// resident (8.4 M lookups at load 0.6: 251 us; the form below, with half the instructions but 32 warps: 291), for slots
-// wider than a line, which a lane walks by itself, and for batches of a few rows per lane (DOK_FEW_ROWS).
-template <int SB, int LW, bool PASSED, class Keys>
-__global__ void __launch_bounds__(DOK_TPB, LW == 2 ? (SB == 32 ? 8 : 6) : 1) k_get_row(DevTable t, DevHash hp, Keys keys, char *__restrict__ out_values,
-                                                    uint8_t *__restrict__ out_found, Fallback fb, ll_t *counters,
-                                                    int count_probes) {
+// resident (8.4 M lookups at load 0.6: 251 us; the form below, with half the instructions but 32 warps: 291), for wider
+// values of all other slots, and for batches that dok_get_by_rows names.
+// For values of more than 8 bytes the walk reads the tags alone, so that 64 warps are resident here too, and the row's own
+// lane reads the value where it was found -- from L1, as its sector has just come in, and further sectors of the line from
+// L2.  Against whole lines in the registers of 24 warps: 40-byte values, 8 M lookups at load 0.6 499 -> 443 us, 1 M 69 -> 52,
+// 300 k 52 -> 36; 16-byte values, 200 k 24 -> 18, 3000 15 -> 11.  (8 M of those in 32-byte slots: 290 -> 326, so they stay below.)
+// Lines through cp.async and shared memory, 40 warps: 445, 62 and 50 for 40-byte values, 292 for 16-byte ones, and 2053
+// instead of 1800 for the churn's, whose popular lines are then not in L1.
+template <int SB, int LW, bool PASSED, bool FEW, class Keys>
+__global__ void __launch_bounds__(DOK_TPB, SB == 0 ? 1 : SB != 32 && LW == 2 ? 6 : 8)
+    k_get_row(DevTable t, DevHash hp, Keys keys, char *__restrict__ out_values, uint8_t *__restrict__ out_found, Fallback fb, ll_t *counters,
+              int count_probes) {
+  constexpr bool AGAIN = LW == 4;                          // the value is read when its slot is known
   __shared__ BlockTally tally;
   if (keys.idle()) return;
   if (counters) dok_tally_begin(tally);
@@ -31,12 +38,14 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 2 ? (SB == 32 ? 8 : 6) : 1) k_g
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
   int probes = 0;
-  // on a hit the quad writes the value from the registers that hold the line
-  const Located loc = dok_locate<SB, LW, false>(t, kh, e, active, &probes, EmitValue<(SB == 0 ? 32 : SB), LW, PASSED>{t, out_values});
+  Located loc;
+  if constexpr (AGAIN) loc = dok_locate<SB, 1, false>(t, kh, e, active, &probes, Probe<FEW>());
+  // ... or on a hit the quad writes it from the registers that hold the line
+  else loc = dok_locate<SB, LW, false>(t, kh, e, active, &probes, EmitValue<SB, LW, PASSED>{t, out_values});
   const int hit = active && loc.found >= 0;
   if (active) {
     char *dst = out_values + e * (ll_t)t.vb;
-    if (SB == 0 && hit) dok_load_value(t, loc.found, dst);
+    if (AGAIN && hit) dok_load_value<SB != 0>(t, loc.found, dst);
     if (!hit) dok_store_fallback(t, fb, dst);
   }
   if (active && out_found) out_found[e] = (uint8_t)hit;
@@ -78,8 +87,8 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, De
     } else {
       dok_inspect_votes<SB, LW>(lr, f, m, me, match, empty);
       const EmitValue<SB, LW, false> emit{t, out_values};
-      // 16-byte values of 32-byte slots: one store by the lane that holds the slot
-      const bool pairs = SB == 32 && t.vb == 16 && ((size_t)out_values & 15) == 0;
+      // 16-byte values: one store
+      const bool pairs = t.vb == 16 && ((size_t)out_values & 15) == 0;
       if (pairs) {
 #pragma unroll
         for (unsigned r = 0; r < 4; r++) {
@@ -94,8 +103,8 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, De
         const unsigned row_r = __shfl_sync(FULL, lr.row, base + r);
         const unsigned m_r = (match[r] >> base) & 0xfu, me_r = m_r | ((empty[r] >> base) & 0xfu);
         if (me_r) {
-          const int lane = __ffs(me_r) - 1, pos = lane * 32 / SB;
-          if ((m_r >> lane) & 1u) emit(keys.elem(share.first + row_r), pos, f.w[r]);
+          const int pos = __ffs(me_r) - 1;
+          if ((m_r >> pos) & 1u) emit(keys.elem(share.first + row_r), pos, f.w[r]);
         }
       }
     }
@@ -163,15 +172,20 @@ inline dim3 dok_stream_grid(const Keys &keys) {
 #define DOK_STREAM(t, rc, st, keys, KERNEL, ...) \
   DOK_FOR_WINDOWS(t, rc, (KERNEL<<<dok_stream_grid<KERNEL>(keys), DOK_TPB, 0, st>>>(wt, __VA_ARGS__)))
 
-// Batches of fewer key rows go to k_get_row: with less than two rows for each lane of k_get, there are too few chains for a
-// lane to take up when its own ends.  k_get_row's time over k_get's, means over hits, Zipf-distributed hits and misses at
-// loads of 0.3 to 0.85: 40-byte values, 10 k rows 0.71, 100 k 0.72, 200 k 0.84, 300 k 0.94, 500 k 1.10, 1 M 1.32; 16-byte
-// values 0.87, 0.84, 0.94, 1.02, 1.15, 1.36; 4-byte values in 64-byte slots 1.03, 0.91, 0.81, 0.94, 1.00, 1.13 (at 30 k rows
-// 0.99, at 60 k 0.94, so these stay with k_get below a block per SM), the misses at 0.85 alone 0.83 at 200 k and 1.13 at
-// 300 k.  Selections of a tensor, whose index arithmetic a share does for 32 rows at a time, differ by a tenth either way
-// and stay with k_get.
-#define DOK_FEW_ROWS(LW) (148LL * DOK_TPB * ((LW) == 4 ? 3 : 4) * 2)
-#define DOK_LEAST_ROWS(LW) ((LW) == 4 ? 0LL : 148LL * DOK_TPB)
+// Which batches of key rows go to k_get_row.  Values of at most 8 bytes in 64- and 128-byte slots: with less than two rows for
+// each lane of k_get there are too few chains for a lane to take up when its own ends (k_get_row's time over k_get's, means
+// over hits, Zipf-distributed hits and misses at loads of 0.3 to 0.85: 30 k rows 0.99, 60 k 0.94, 100 k 0.91, 200 k 0.81,
+// 300 k 0.94, 500 k 1.00, 1 M 1.13), and below a block per SM they stay with k_get.  Wider values of 32-byte slots, where
+// k_get_row looks at the slot a second time: that costs nothing while address translation covers the table (a second access
+// to a sector just read is free in 256 MB, and in 4 GB it costs as much as a line), or the batch is all latency.  16-byte
+// values, k_get / k_get_row, us: 1 M rows, load 0.6, table of 32 MB 42 / 32, 256 MB 50 / 42, 512 MB 52 / 48, 2 GB 54 / 56; 8 M
+// rows 216 / 153, 259 / 200, 271 / 280, 290 / 357; 300 k rows 24..28 / 17..24.  Of 9 to 15 bytes, which no single store
+// takes, 8 M rows 273 / 159 ... 325 / 339, and misses at 0.8 527 / 484.  Selections of a tensor, whose index arithmetic a
+// share does for 32 rows at a time, differ by a tenth either way and stay with k_get.
+inline bool dok_get_by_rows(const DevTable &t, ll_t n) {
+  if (t.vb <= 8) return n >= 148LL * DOK_TPB && n < 148LL * DOK_TPB * 4 * 2;
+  return t.vb < 16 || n < 900000 || t.n_slots * t.sb <= 512LL << 20;
+}
 
 template <class Keys>
 inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, void *out_values, uint8_t *out_found,
@@ -186,13 +200,15 @@ inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, vo
   ll_t *cnt = (ll_t *)counters;
   // tag and value fit the first 16 bytes of the slot: half the load width
   const bool narrow = t.vb <= 8;
+  const dim3 grid = dok_grid(keys);
   const auto launch = [&](auto slot_bytes, auto words, auto passed) {
     constexpr int SB = decltype(slot_bytes)::value, LW = decltype(words)::value;
-    constexpr bool PASSED = decltype(passed)::value;
-    constexpr bool ROWS = std::is_same<Keys, RowKeys>::value, ONLY_ROWS = SB == 0 || (ROWS && SB == 32 && LW == 2);
-    if constexpr (ROWS || SB == 0)
-      if (ONLY_ROWS || (n < DOK_FEW_ROWS(LW) && n >= DOK_LEAST_ROWS(LW))) {
-        DOK_FOR_WINDOWS(t, rc, (k_get_row<SB, LW, PASSED, Keys><<<dok_grid(keys), DOK_TPB, 0, st>>>(wt, hp, keys, values, out_found, fb, cnt, count_probes)));
+    constexpr bool PASSED = decltype(passed)::value, ROWS = std::is_same<Keys, RowKeys>::value;
+    constexpr bool ONLY_ROWS = SB == 0 || (LW == 4 && SB != 32) || (ROWS && SB == 32 && LW == 2);
+    if constexpr (ROWS || ONLY_ROWS)
+      if (ONLY_ROWS || dok_get_by_rows(t, n)) {
+        DOK_BY_SIZE(grid.x * grid.y, DOK_FOR_WINDOWS(t, rc, (k_get_row<SB, LW, PASSED, FEW && LW == 4 && SB != 0, Keys>
+                                                             <<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, out_found, fb, cnt, count_probes))));
         return;
       }
     if constexpr (!ONLY_ROWS) DOK_STREAM(t, rc, st, keys, (k_get<SB, LW, PASSED, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
