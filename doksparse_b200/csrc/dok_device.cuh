@@ -738,23 +738,25 @@ static __device__ __forceinline__ ll_t dok_find_or_claim_serial(const DevTable &
 // uuid is rare; that lane redoes the whole operation with the serial walk.  Every lane of the warp must call.
 template <int SB, bool FEW = false>
 __device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHash &key, bool active, int *outcome) {
-  const ChainKey kh = dok_chain(key, t);
+  // (mixed once where the walk is followed by dok_mark_passed; kept in registers elsewhere it cost an insert of 32-byte slots
+  // a fifth: 160 k non-zeros 35 -> 42 us)
+  const auto kh = [&] { if constexpr (SB >= 64) return dok_chain(key, t); else return key; }();
   const Located loc = dok_locate<SB, 1, true>(t, kh, 0, active, nullptr, NoEmit<FEW>());   // the tags are all a claim needs
   if (!active) return -1;
   if (loc.found >= 0) { *outcome = DOK_OUT_FOUND; return loc.found; }
   if (loc.tomb >= 0) {
     const ll_t old = dok_cas_tag(t, loc.tomb, DOK_REMOVED, kh.uuid);
-    if (old == DOK_REMOVED) { *outcome = DOK_OUT_REUSED; if (SB >= 64) dok_mark_passed(t, kh, loc.tomb); return loc.tomb; }
+    if (old == DOK_REMOVED) { *outcome = DOK_OUT_REUSED; if constexpr (SB >= 64) dok_mark_passed(t, kh, loc.tomb); return loc.tomb; }
     if (old == kh.uuid) { *outcome = DOK_OUT_FOUND; return loc.tomb; }
   } else if (loc.empty >= 0) {
     const ll_t old = dok_cas_tag(t, loc.empty, DOK_EMPTY, kh.uuid);
-    if (old == DOK_EMPTY) { *outcome = DOK_OUT_CLAIMED_EMPTY; if (SB >= 64) dok_mark_passed(t, kh, loc.empty); return loc.empty; }
+    if (old == DOK_EMPTY) { *outcome = DOK_OUT_CLAIMED_EMPTY; if constexpr (SB >= 64) dok_mark_passed(t, kh, loc.empty); return loc.empty; }
     if (old == kh.uuid) { *outcome = DOK_OUT_FOUND; return loc.empty; }
   } else {
     *outcome = DOK_OUT_FAILED;       // no match, no tombstone, no empty slot: the table is full
     return -1;
   }
-  return dok_find_or_claim_serial(t, kh, outcome);
+  return dok_find_or_claim_serial(t, dok_chain(key, t), outcome);
 }
 
 // value row (vb bytes at `src`, alignment of the widest power of two dividing vb, capped at 8) -> slot
