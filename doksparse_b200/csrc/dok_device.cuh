@@ -695,68 +695,43 @@ __device__ __forceinline__ Located dok_locate(const DevTable &t, const Key &kh, 
 
 enum { DOK_OUT_FOUND = 0, DOK_OUT_CLAIMED_EMPTY = 1, DOK_OUT_REUSED = 2, DOK_OUT_FAILED = 3 };
 
-// Insert-or-find by one lane, slot by slot (ClosedHashmap::set, closed_hashmap_impl_class.cu:368-427, without
-// the row stores).  Phase 1 walks the chain: a matching tag is a hit; at the first empty tag the slot is claimed by CAS
-// unless a tombstone was seen.  Phase 2 walks it again and takes the first slot that is free, tombstone or empty.  No slot
-// becomes free while a set runs, so rows with equal uuids meet: the one that comes later finds the slot the first one
-// took, in the walk or because its CAS loses to the SAME uuid.
-static __device__ __forceinline__ ll_t dok_find_or_claim_serial(const DevTable &t, const ChainKey &kh, int *outcome) {
-  const ll_t uuid = kh.uuid;
-  bool reuse = false;                                    // a tombstone was seen
-  for (int phase = 0; phase < 2; phase++) {
-    ll_t group = dok_start_group(kh, t);
-    unsigned word = dok_chain_word(kh, t);
-    bool more = true;
-    while (more) {
-      for (int i = 0; i < t.spg && more; i++) {
-        const ll_t slot = group * t.spg + i;
-        ll_t tag = dok_load_tag(t, slot);
-        if (tag == DOK_REMOVED && phase == 0) reuse = true;
-        if (tag == DOK_EMPTY && phase == 0 && reuse) { more = false; break; }
-        if (tag == DOK_EMPTY || (tag == DOK_REMOVED && phase == 1)) {
-          const ll_t old = dok_cas_tag(t, slot, tag, uuid);
-          if (old == tag) {
-            *outcome = tag == DOK_EMPTY ? DOK_OUT_CLAIMED_EMPTY : DOK_OUT_REUSED;
-            dok_mark_passed(t, kh, slot);
-            return slot;
-          }
-          tag = old;
-        }
-        if (tag == uuid) { *outcome = DOK_OUT_FOUND; return slot; }
-      }
-      more = more && dok_next_group<ll_t>(group, word, t.n_groups);
-    }
-    if (!reuse) break;
-  }
-  *outcome = DOK_OUT_FAILED;
-  return -1;
-}
-
-// Insert-or-find for the 32 keys of a warp: one cooperative walk tells every owner lane where its uuid is or
-// where the chain offers a place (first tombstone, else first empty slot); the owner claims that place with one
-// CAS.  Losing the CAS to the same uuid means a twin row of the batch claimed it: join.  Losing it to another
-// uuid is rare; that lane redoes the whole operation with the serial walk.  Every lane of the warp must call.
+// Insert-or-find for the 32 keys of a warp (ClosedHashmap::set, closed_hashmap_impl_class.cu:368-427, without the row
+// stores): one cooperative walk tells every owner lane where its uuid is or where the chain offers a place (first tombstone,
+// else first empty slot); the owner claims that place with one CAS.  Losing the CAS to the same uuid means a twin row of the
+// batch claimed it: join.  Losing it to another uuid means another walk for that lane: no slot becomes free while a set runs,
+// so each lost CAS is a slot taken.  In a table that fills up that is no exception -- the rows that are on their way at a time
+// see the same first places -- and a lane that went on by itself, slot by slot, held its warp up: sets of a fifth new rows,
+// 300 k rows of 32-byte slots 60 -> 54 us, 1 M 113 -> 107, 30 k rows of 64-byte slots 59 -> 48.  Every lane of the warp must call.
 template <int SB, bool FEW = false>
 __device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHash &key, bool active, int *outcome) {
   // (mixed once where the walk is followed by dok_mark_passed; kept in registers elsewhere it cost an insert of 32-byte slots
-  // a fifth: 160 k non-zeros 35 -> 42 us)
+  // a fifth)
   const auto kh = [&] { if constexpr (SB >= 64) return dok_chain(key, t); else return key; }();
-  const Located loc = dok_locate<SB, 1, true>(t, kh, 0, active, nullptr, NoEmit<FEW>());   // the tags are all a claim needs
-  if (!active) return -1;
-  if (loc.found >= 0) { *outcome = DOK_OUT_FOUND; return loc.found; }
-  if (loc.tomb >= 0) {
-    const ll_t old = dok_cas_tag(t, loc.tomb, DOK_REMOVED, kh.uuid);
-    if (old == DOK_REMOVED) { *outcome = DOK_OUT_REUSED; if constexpr (SB >= 64) dok_mark_passed(t, kh, loc.tomb); return loc.tomb; }
-    if (old == kh.uuid) { *outcome = DOK_OUT_FOUND; return loc.tomb; }
-  } else if (loc.empty >= 0) {
-    const ll_t old = dok_cas_tag(t, loc.empty, DOK_EMPTY, kh.uuid);
-    if (old == DOK_EMPTY) { *outcome = DOK_OUT_CLAIMED_EMPTY; if constexpr (SB >= 64) dok_mark_passed(t, kh, loc.empty); return loc.empty; }
-    if (old == kh.uuid) { *outcome = DOK_OUT_FOUND; return loc.empty; }
-  } else {
-    *outcome = DOK_OUT_FAILED;       // no match, no tombstone, no empty slot: the table is full
-    return -1;
-  }
-  return dok_find_or_claim_serial(t, dok_chain(key, t), outcome);
+  ll_t slot = -1;
+  do {
+    const Located loc = dok_locate<SB, 1, true>(t, kh, 0, active, nullptr, NoEmit<FEW>());   // the tags are all a claim needs
+    if (active) {
+      active = false;
+      slot = loc.found;
+      *outcome = DOK_OUT_FOUND;
+      if (slot < 0) {
+        slot = loc.tomb >= 0 ? loc.tomb : loc.empty;
+        const ll_t expect = loc.tomb >= 0 ? DOK_REMOVED : DOK_EMPTY;
+        if (slot < 0) {
+          *outcome = DOK_OUT_FAILED;                     // no match, no tombstone, no empty slot: the table is full
+        } else {
+          const ll_t old = dok_cas_tag(t, slot, expect, key.uuid);
+          if (old == expect) {
+            *outcome = expect == DOK_EMPTY ? DOK_OUT_CLAIMED_EMPTY : DOK_OUT_REUSED;
+            if constexpr (SB >= 64) dok_mark_passed(t, kh, slot);
+          } else {
+            active = old != key.uuid;
+          }
+        }
+      }
+    }
+  } while (__any_sync(0xffffffffu, active));
+  return slot;
 }
 
 // value row (vb bytes at `src`, alignment of the widest power of two dividing vb, capped at 8) -> slot
