@@ -117,6 +117,8 @@ def _declare(lib):
         "dok_dok_assign_sequenced": ([TP, HP, SP, P, P, P, P, P, P], I),
         "dok_dok_to_dense": ([TP, HP, P, P, P], I),
         "dok_dense_count_nonzero": ([P, I64, I, I, P, P], I),
+        "dok_dense_collect_nonzero": ([P, I64, I, I, P, I64, P, P], I),
+        "dok_dense_insert_list": ([TP, HP, P, I64, I64, P, P, P], I),
         "dok_dense_insert_nonzero": ([TP, HP, P, P, I64, I, P, P], I),
         "dok_partition_tiles": ([I64], I64),
         "dok_partition_offset_words": ([I64, I], I64),

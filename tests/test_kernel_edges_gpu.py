@@ -307,6 +307,24 @@ def test_dense_round_trip(dtype, shape, density):
         assert torch.equal(t.transpose(0, 1).to_dense(), dense.transpose(0, 1))
 
 
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.bfloat16, torch.float32, torch.int64])
+@pytest.mark.parametrize("numel", [1, 15, 513, 4097, 700001, 1 << 21])
+@pytest.mark.parametrize("density", [0.003, 0.1, 0.14])                 # the list holds an eighth, or 65,536
+@pytest.mark.parametrize("offset", [0, 1])                              # not on a 16-byte boundary: the other way
+def test_dense_tensor_by_the_list_of_its_non_zeros(dtype, numel, density, offset):
+    from doksparse_b200 import SparseDOKTensor
+    np.random.seed(2)
+    g = torch.Generator(device="cuda").manual_seed(numel)
+    dense = torch.randint(1, 100, (numel + offset,), generator=g, device="cuda").to(dtype)
+    dense *= (torch.rand(numel + offset, generator=g, device="cuda") < density).to(dtype)
+    dense = dense[offset:]
+    dense[-1] = 7
+    if dtype.is_floating_point:
+        dense[0] = -0.0 if numel > 1 else 7
+    t = SparseDOKTensor.from_dense(dense)
+    assert t._nnz() == int((dense != 0).sum()) and torch.equal(t.to_dense(), dense)
+
+
 @pytest.mark.parametrize("numel", [255, 256, 257, 2049, 148 * 4 * 2048 + 1, 4 * 148 * 4 * 2048 + 300])
 @pytest.mark.parametrize("counts", [(31,), (32,), (33,), (31, 1, 0, 33), (256, 0, 1)])
 def test_dense_lists_of_a_warp(numel, counts):
