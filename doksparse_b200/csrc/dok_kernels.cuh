@@ -56,14 +56,14 @@ __global__ void __launch_bounds__(DOK_TPB, SB == 0 ? 1 : SB != 32 && LW == 2 ? 6
   }
 }
 
-// A warp's share of the batch (dok_stream.cuh): for larger batches of everything else.  Wider values need the registers of whole lines (3
-// blocks of 256 per SM in either form), and where a line holds fewer slots the chains are longer, so that a warp that waits
-// for its longest chain leaves most of its lanes idle: 8.4 M lookups of 16-byte values 544 -> 303 us, 8.4 M misses in
-// 64-byte slots at load 0.69 750 -> 595, selections of 32-byte slots 153 -> 141.
+// A warp's share of the batch (dok_stream.cuh): for larger batches of everything else.  16-byte values need the registers of
+// whole lines (3 blocks of 256 per SM in either form), and where a line holds fewer slots the chains are longer, so that a
+// warp that waits for its longest chain leaves most of its lanes idle: 8.4 M lookups of 16-byte values 544 -> 303 us, 8.4 M
+// misses in 64-byte slots at load 0.69 750 -> 595, selections of 32-byte slots 153 -> 141.
 // Values of at most 8 bytes lie behind the tag in the word pair that a lane has loaded: the key's own lane fetches it from
 // the lane of the slot that matched, and stores value (or fallback) and flag of its row -- one store for 32 rows of which
-// most are neighbours.  Wider values are written by the quad from the registers that hold the line.  Either way a hit needs
-// no second access to the table.
+// most are neighbours.  16-byte values of 32-byte slots (dok_get_by_rows) are written by the lane that holds the slot.  Either
+// way a hit needs no second access to the table.
 template <int SB, int LW, bool PASSED, class Keys>
 __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, DevHash hp, Keys keys, char *__restrict__ out_values,
                                                                   uint8_t *__restrict__ out_found, Fallback fb, ll_t *counters,
