@@ -70,13 +70,23 @@ class _PinnedRings:
 _rings = _PinnedRings()
 
 
-class _Shared:
-    """What shallow clones (views) must see together: the duplicate-resolution stamps with their epoch, and the host-side
-    upper bound of n_elements that lets `set` skip a device synchronisation."""
-    __slots__ = ("stamp", "epoch", "bound", "base", "snapshots", "ring", "device", "known")
+class _Marks:
+    """What general sets have left in one slot array, for as long as there is that array: every map that writes its slots
+    has these marks, and a new slot array gets new ones.  `epoch`: the largest one in a stamp.  `stamp`: the stamps, where
+    the slots have no room for them."""
+    __slots__ = ("stamp", "epoch")
 
-    def __init__(self, stamp=None, epoch=0, bound=0):
-        self.stamp, self.epoch, self.bound, self.base = stamp, epoch, bound, bound
+    def __init__(self, stamp=None, epoch=0):
+        self.stamp, self.epoch = stamp, epoch
+
+
+class _Shared:
+    """What the maps of one slot array (shallow clones, views) must see together besides its counters and marks: the
+    host-side upper bound of n_elements that lets `set` skip a device synchronisation."""
+    __slots__ = ("bound", "base", "snapshots", "ring", "device", "known")
+
+    def __init__(self, bound=0):
+        self.bound, self.base = bound, bound
         self.snapshots, self.ring, self.device = [], None, None
         self.known = False              # the bound is n_elements itself
 
@@ -125,6 +135,7 @@ class CudaClosedHashmap:
         self._key_shape = None
         self._key_dtype = None
         self._shared = _Shared()
+        self._marks = _Marks()
         self._value_shape = None
         self._value_dtype = None
 
@@ -297,7 +308,7 @@ class CudaClosedHashmap:
         self._value_bytes, self._key_bytes = value_bytes, key_size * key_dtype.itemsize
         self._value_shape, self._value_dtype = torch.Size(value_shape), value_dtype
         self._key_shape, self._key_dtype = torch.Size(key_shape), key_dtype
-        self._shared.stamp = None
+        self._marks = _Marks()
         self._hp = self._plan = None
         device = torch.cuda.current_device() if self.device.index is None else self.device.index
         self._bare_plan, self._slots, self._counters_of_table, layout = L.native().allocate(
@@ -357,18 +368,18 @@ class CudaClosedHashmap:
     def _next_epoch(self):
         """Epoch of the next general set: larger than every epoch stamped on this table before.  The stamps live in
         the slots when the layout has room for them, else in a separate array allocated on first use."""
-        sh = self._shared
-        if self._layout.stamp_offset < 0 and sh.stamp is None:
-            sh.stamp = torch.zeros(self._layout.n_slots, device=self.device, dtype=torch.long)
-        if sh.epoch >= L.MAX_EPOCH - 1:
+        marks = self._marks
+        if self._layout.stamp_offset < 0 and marks.stamp is None:
+            marks.stamp = torch.zeros(self._layout.n_slots, device=self.device, dtype=torch.long)
+        if marks.epoch >= L.MAX_EPOCH - 1:
             raise L.DokError("stamp epochs exhausted: rehash() the map to start over")
-        sh.epoch += 1
-        return sh.epoch
+        marks.epoch += 1
+        return marks.epoch
 
     def _c_table(self):
         t = L.Table()
         t.slots = self._slots.data_ptr()
-        stamp = self._shared.stamp
+        stamp = self._marks.stamp
         t.stamp = stamp.data_ptr() if stamp is not None else None
         t.n_buckets = self._n_buckets
         t.slot_bytes = self._layout.slot_bytes
@@ -421,7 +432,7 @@ class CudaClosedHashmap:
         """Address of the separate stamp array (0: the stamps are in the slots), None while it has yet to be made."""
         if self._layout.stamp_offset >= 0:
             return 0
-        stamp = self._shared.stamp
+        stamp = self._marks.stamp
         return None if stamp is None else stamp.data_ptr()
 
     def _counters(self):
@@ -550,20 +561,22 @@ class CudaClosedHashmap:
             rehash_factor=self._rehash_factor, rehash_threshold=self._rehash_threshold,
             tombstone_threshold=self._tombstone_threshold,
         )
+        if self._slots is None:
+            return new           # each will have slots of its own, and whatever goes with them
         new._tombstone_host_bound = self._tombstone_host_bound
-        if self._slots is not None:
-            new._slots = cp(self._slots)
-            new._layout = self._layout
-            new._value_bytes, new._key_bytes = self._value_bytes, self._key_bytes
-            new._value_shape, new._value_dtype = self._value_shape, self._value_dtype
-            new._key_shape, new._key_dtype = self._key_shape, self._key_dtype
+        new._slots = cp(self._slots)
+        new._layout = self._layout
+        new._value_bytes, new._key_bytes = self._value_bytes, self._key_bytes
+        new._value_shape, new._value_dtype = self._value_shape, self._value_dtype
+        new._key_shape, new._key_dtype = self._key_shape, self._key_dtype
         new._counters_of_table = cp(self._state)
         if deepclone:
             # in-slot stamps were copied with the slots: continue their epochs; a separate array is copied too
-            sh = self._shared
-            new._shared = _Shared(None if sh.stamp is None else sh.stamp.clone(), sh.epoch, sh.bound)
+            marks = self._marks
+            new._marks = _Marks(None if marks.stamp is None else marks.stamp.clone(), marks.epoch)
+            new._shared = _Shared(self._shared.bound)
         else:
-            new._shared = self._shared   # a view writes the same slots: same stamps, epoch and bound
+            new._marks, new._shared = self._marks, self._shared   # a view writes the same slots
         return new
 
     # ------------------------------------------------------------------ sizes
@@ -673,18 +686,18 @@ class CudaClosedHashmap:
     def _launch_set(self, keys, values, assume_unique):
         """The set kernels on contiguous rows of this table."""
         unstamped = assume_unique or self._native_plan().in_word(keys.shape[0])
-        epoch = self._shared.epoch if unstamped else self._next_epoch()
+        epoch = self._marks.epoch if unstamped else self._next_epoch()
         self._native_plan().set(keys, values, assume_unique, epoch, self._stamp_address() or 0)
 
     def set(self, new_keys, new_values, assume_unique=False):
         """Insert-or-assign a batch.  `assume_unique=True` promises pairwise different keys and runs one kernel
         instead of two.  Returns None like the reference."""
-        plan, sh = self._plan, self._shared
-        if plan is not None and self._key_dtype not in L.FLOAT_DTYPES and sh.epoch < L.MAX_EPOCH - 1 \
+        plan, marks = self._plan, self._marks
+        if plan is not None and self._key_dtype not in L.FLOAT_DTYPES and marks.epoch < L.MAX_EPOCH - 1 \
                 and self._room_for(new_keys.shape[0], int(self._rehash_threshold * self._n_buckets)):
-            rows = plan.set(new_keys, new_values, assume_unique, sh.epoch + 1, self._stamp_address() or 0)
+            rows = plan.set(new_keys, new_values, assume_unique, marks.epoch + 1, self._stamp_address() or 0)
             if rows is not None:
-                sh.epoch += 1
+                marks.epoch += 1
                 self._after_mutation(rows)
                 return
         assert new_keys.shape[0] == new_values.shape[0]
@@ -917,10 +930,11 @@ class CudaClosedHashmap:
     def rebuild(self):
         """The same table without its tombstones: a fresh slot array of the same geometry, every live slot re-inserted
         with the SAME hash parameters (one kernel, dok_map_reinsert).  Lookups, sizes and parameters are unchanged;
-        shallow clones made before keep the old slot array (as after a rehash in the reference)."""
+        shallow clones made before keep the old slot array (as after a rehash in the reference) with its counters and
+        marks."""
         if self._slots is None:
             return
-        old_slots, old_stamp = self._slots, self._shared.stamp
+        old_slots, old_state, old_stamp = self._slots, self._state, self._marks.stamp
         source = L.Table()
         source.slots = old_slots.data_ptr()
         source.stamp = old_stamp.data_ptr() if old_stamp is not None else None
@@ -928,21 +942,22 @@ class CudaClosedHashmap:
         source.slot_bytes = self._layout.slot_bytes
         source.value_bytes, source.key_bytes = self._value_bytes, self._key_bytes
         fresh = torch.empty(self._layout.total_bytes, device=self.device, dtype=torch.uint8)     # may raise: nothing changed yet
-        self._slots = fresh
+        state = old_state.clone()
+        # the sizes are those of before; only the tombstones are gone: reused = removed
+        gone = state[_BY_REMOVE + L.CNT_HITS] - state[L.CNT_REUSED_REMOVED]
+        state[L.CNT_CLAIMED_EMPTY] -= gone
+        state[L.CNT_REUSED_REMOVED] += gone
+        known = self._shared.known
+        self._slots, self._counters_of_table, self._marks, self._shared = fresh, state, _Marks(), _Shared(self._shared.bound)
+        self._shared.known = known
         self._plan = self._bare_plan = None
-        self._shared.stamp = None
-        self._shared.epoch = 0
-        state = self._state.clone()
         with L.on(self.device):
             st = L.stream_ptr(self.device)
             L.check(L.lib().dok_map_init(self._c_table(), st), "dok_map_init")
             L.check(L.lib().dok_map_reinsert(ctypes.byref(source), self._c_table(), self._c_hash(), None, st),
                     "dok_map_reinsert")
-        old_slots.record_stream(torch.cuda.current_stream(self.device))
-        # the sizes are those of before; only the tombstones are gone: reused = removed
-        gone = state[_BY_REMOVE + L.CNT_HITS] - state[L.CNT_REUSED_REMOVED]
-        self._state[L.CNT_CLAIMED_EMPTY] -= gone
-        self._state[L.CNT_REUSED_REMOVED] += gone
+        for old in (old_slots, old_state):
+            old.record_stream(torch.cuda.current_stream(self.device))
         self._tombstone_host_bound = 0
 
     @property

@@ -371,16 +371,16 @@ class SparseDOKTensor(object):
         """Dense assignment (sparse_dok_tensor.py:317-327 -> sparse_dok_tensor_impl.py:412-474).  A Python scalar is
         treated like a 0-dim tensor, as the reference's README documents."""
         hashmap = self._hashmap
-        plan, sh = hashmap._plan or hashmap._native_plan(), hashmap._shared
-        if plan is not None and hashmap._value_dtype == self._dtype and sh.epoch < L.MAX_EPOCH - 1:
+        plan, marks = hashmap._plan or hashmap._native_plan(), hashmap._marks
+        if plan is not None and hashmap._value_dtype == self._dtype and marks.epoch < L.MAX_EPOCH - 1:
             stamp = hashmap._stamp_address() or 0
             limit = hashmap._n_buckets * hashmap._rehash_threshold
-            n = plan.assign(selectors, self._size, values, limit - hashmap._element_bound(), sh.epoch + 1, stamp)
+            n = plan.assign(selectors, self._size, values, limit - hashmap._element_bound(), marks.epoch + 1, stamp)
             if n is not None and n < 0 and hashmap._room_for(-n, limit):
-                n = plan.assign(selectors, self._size, values, -n, sh.epoch + 1, stamp)
+                n = plan.assign(selectors, self._size, values, -n, marks.epoch + 1, stamp)
             if n is not None and n >= 0:
                 if n:
-                    sh.epoch += 1
+                    marks.epoch += 1
                     hashmap._after_mutation(n)
                 return
         selectors, _ = self._handle_selectors(selectors)
