@@ -18,6 +18,7 @@ MAX_SELECTOR_NDIM = 8
 MAX_SHARDS = 64
 N_COUNTERS = 8
 MAX_EPOCH = (1 << 30) - 1
+MAX_BATCH = (1 << 32) - 1
 CNT_CLAIMED_EMPTY, CNT_REUSED_REMOVED, CNT_FAILED, CNT_HITS, CNT_DUPLICATES, CNT_PROBES = range(6)
 
 DTYPE_CODES = {
@@ -112,9 +113,10 @@ def _declare(lib):
         "dok_dok_assign": ([TP, HP, SP, P, P, P, I64, I64, P, P, P], I),
         "dok_set_scratch_words": ([TP, I64], I64),
         "dok_map_set_with": ([TP, HP, P, P, I64, P, I64, I64, P, P], I),
-        "dok_set_takes_sequence": ([TP, HP, I64], I),
-        "dok_map_set_sequenced": ([TP, HP, P, P, I64, P, P, P], I),
-        "dok_dok_assign_sequenced": ([TP, HP, SP, P, P, P, P, P, P], I),
+        "dok_set_takes_numbers": ([TP, HP, I64], I),
+        "dok_map_set_numbered": ([TP, HP, P, P, I64, I64, P, P], I),
+        "dok_map_clear_numbers": ([TP, P], I),
+        "dok_dok_assign_numbered": ([TP, HP, SP, P, P, I64, P, P, P], I),
         "dok_dok_to_dense": ([TP, HP, P, P, P], I),
         "dok_dense_count_nonzero": ([P, I64, I, I, P, P], I),
         "dok_dense_collect_nonzero": ([P, I64, I, I, P, I64, P, P], I),

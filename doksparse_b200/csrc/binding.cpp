@@ -12,6 +12,7 @@
 #include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
+#include <structmember.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -31,7 +32,7 @@ struct Plan {
   at::ScalarType key_type, value_type;
 };
 
-enum { STATE_SET = 0, STATE_REMOVE = 8, STATE_SEQUENCE = 18, STATE_BULK = 24, STATE_ADJUST = 7, STATE_WORDS = 32 };   // int64 offsets of the counter blocks
+enum { STATE_SET = 0, STATE_REMOVE = 8, STATE_BULK = 24, STATE_ADJUST = 7, STATE_WORDS = 32 };   // int64 offsets of the counter blocks
 
 PyObject *dok_error = nullptr;
 extern PyTypeObject plan_type;
@@ -67,8 +68,8 @@ PyObject *guarded(F f) {
   END_HANDLE_TH_ERRORS
 }
 
-int shape_from(PyObject *tuple, int64_t *out) {
-  if (!PyTuple_Check(tuple) || PyTuple_GET_SIZE(tuple) > 7) return -1;
+int shape_from(PyObject *tuple, int64_t *out, int most = 7) {
+  if (!PyTuple_Check(tuple) || PyTuple_GET_SIZE(tuple) > most) return -1;
   const int n = (int)PyTuple_GET_SIZE(tuple);
   for (int i = 0; i < n; i++) {
     out[i] = PyLong_AsLongLong(PyTuple_GET_ITEM(tuple, i));
@@ -170,6 +171,102 @@ PyObject *plan_set_hash(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
   self->hash.key_size = (int32_t)n;
   Py_RETURN_NONE;
 }
+
+// ---- what sets leave behind in one slot array ---------------------------------------------------------------
+
+// For as long as there is the slot array: every map that writes it has these marks, a new one gets new ones.  They are changed
+// with the interpreter's lock held, so that sets from several threads and on several streams never share an epoch or numbers.
+struct Marks {
+  PyObject_HEAD
+  PyObject *stamp;             // the stamps (a tensor), where the slots have no room for them and a set has needed them
+  long long epoch;             // largest one in a stamp
+  long long numbered;          // largest number of a row that shares its value's word with it
+  long long renumbered;        // ... that sets in graphs use again and again
+  cudaStream_t stream;         // of the numbered sets so far
+  bool any, several;           // there were some; on more than one stream, or in a graph
+};
+
+void marks_dealloc(Marks *self) {
+  Py_XDECREF(self->stamp);
+  Py_TYPE(self)->tp_free((PyObject *)self);
+}
+
+// Marks(), or Marks(other, stamp): for a copy of other's slots, `stamp` the copy of its stamps or None
+int marks_init(Marks *self, PyObject *args, PyObject *) {
+  PyObject *other = nullptr, *stamp = Py_None;
+  if (!PyArg_ParseTuple(args, "|OO", &other, &stamp)) return -1;
+  if (other && Py_TYPE(other) != Py_TYPE(self)) { PyErr_SetString(PyExc_TypeError, "Marks: other marks expected"); return -1; }
+  if (other) {
+    const Marks *m = (const Marks *)other;
+    self->epoch = m->epoch;
+    self->numbered = m->numbered;
+  }
+  Py_INCREF(stamp);
+  Py_XSETREF(self->stamp, stamp);
+  return 0;
+}
+
+// in the slots, or in an array that the marks have
+bool add_stamps(const Marks *m, dok_table *table) {
+  const at::Tensor *stamp = m->stamp ? tensor_of(m->stamp) : nullptr;
+  table->stamp = stamp ? (int64_t *)stamp->data_ptr() : nullptr;
+  dok_layout_info lay;
+  return stamp || (dok_table_layout(table->value_bytes, table->key_bytes, table->n_buckets, &lay) == DOK_OK && lay.stamp_offset >= 0);
+}
+
+// A new start for the numbers: nothing that numbers rows of these slots is on its way, and nothing starts before they are
+// cleared.  false where there is no quiet moment for it (or, with several streams, where one of them captures); the caller
+// stamps its rows then.
+bool start_over(const Plan *p, Marks *m, cudaStream_t stream) {
+  for (int i = 0; i < 4; i++) {
+    const int64_t launched = dok_launch_count();
+    cudaError_t e;
+    Py_BEGIN_ALLOW_THREADS
+    e = m->several || m->stream != stream ? cudaDeviceSynchronize() : cudaStreamSynchronize(stream);
+    Py_END_ALLOW_THREADS
+    if (e == cudaErrorStreamCaptureUnsupported) { (void)cudaGetLastError(); return false; }
+    C10_CUDA_CHECK(e);
+    if (dok_launch_count() != launched) continue;            // another thread had the interpreter meanwhile
+    if (dok_map_clear_numbers(&p->table, stream) != DOK_OK) return false;
+    C10_CUDA_CHECK(cudaStreamSynchronize(stream));
+    m->numbered = m->renumbered;
+    m->any = false;
+    m->several = m->renumbered > 0;
+    return true;
+  }
+  return false;
+}
+
+// Numbers for n rows, to `base`; false where their set has to be stamped.
+bool take_numbers(const Plan *p, Marks *m, int64_t n, cudaStream_t stream, int64_t *base) {
+  if (!dok_set_takes_numbers(&p->table, &p->hash, n)) return false;
+  cudaStreamCaptureStatus capturing;
+  C10_CUDA_CHECK(cudaStreamIsCapturing(stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) {
+    m->renumbered = std::max<long long>(m->renumbered, n);
+    m->numbered = std::max(m->numbered, m->renumbered);
+    m->several = true;
+    *base = DOK_RENUMBER;
+    return true;
+  }
+  if (m->numbered > DOK_MAX_NUMBER - n && (m->renumbered > DOK_MAX_NUMBER - n || !start_over(p, m, stream) || m->numbered > DOK_MAX_NUMBER - n))
+    return false;
+  m->several = m->several || (m->any && m->stream != stream);
+  m->any = true;
+  m->stream = stream;
+  *base = m->numbered;
+  m->numbered += n;
+  return true;
+}
+
+// An epoch for a stamped set, and its table with the stamps; false where the stamps have yet to be made or epochs are used up
+bool take_epoch(Marks *m, dok_table *table, int64_t *epoch) {
+  if (!add_stamps(m, table) || m->epoch >= DOK_MAX_EPOCH - 1) return false;
+  *epoch = ++m->epoch;
+  return true;
+}
+
+Marks *marks_of(PyObject *o);
 
 // ---- counts that travel to the host by themselves -----------------------------------------------------------
 
@@ -281,23 +378,11 @@ PyObject *plan_get(Plan *self, PyObject *arg) {
   });
 }
 
-// in the slots, or in an array that the table has already
-bool has_stamps(const dok_table &table) {
-  dok_layout_info lay;
-  return table.stamp || (dok_table_layout(table.value_bytes, table.key_bytes, table.n_buckets, &lay) == DOK_OK && lay.stamp_offset >= 0);
-}
-
-// in_word(n) -> whether a general set of n rows does without stamps
-PyObject *plan_in_word(Plan *self, PyObject *arg) {
-  const long long n = PyLong_AsLongLong(arg);
-  if (n == -1 && PyErr_Occurred()) return nullptr;
-  return PyBool_FromLong(dok_set_takes_sequence(&self->table, &self->hash, n));
-}
-
-// set(keys, values, assume_unique, epoch, stamp address) -> the number of rows, or None
+// set(keys, values, assume_unique, marks) -> the number of rows, or None
 PyObject *plan_set(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
   return guarded([&]() -> PyObject * {
-    if (nargs != 5) { PyErr_SetString(PyExc_TypeError, "set takes 5 arguments"); return nullptr; }
+    Marks *marks = nargs == 4 ? marks_of(args[3]) : nullptr;
+    if (!marks) { PyErr_SetString(PyExc_TypeError, "set takes keys, values, assume_unique and Marks"); return nullptr; }
     const at::Tensor *keys = tensor_of(args[0]), *values = tensor_of(args[1]);
     if (!keys || !values || !rows_match(*keys, self->device, self->key_type, self->key_ndim, self->key_shape) ||
         !rows_match(*values, self->device, self->value_type, self->value_ndim, self->value_shape) || keys->size(0) != values->size(0) ||
@@ -305,23 +390,22 @@ PyObject *plan_set(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
       Py_RETURN_NONE;
     const int64_t n = keys->size(0);
     const int unique = PyObject_IsTrue(args[2]);
-    const int64_t epoch = PyLong_AsLongLong(args[3]);
-    dok_table table = self->table;
-    table.stamp = (int64_t *)PyLong_AsVoidPtr(args[4]);
-    if (unique < 0 || PyErr_Occurred()) return nullptr;
+    if (unique < 0) return nullptr;
     const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
-    void *stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream();
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream();
+    dok_table table = self->table;
+    int64_t base, epoch;
     if (unique) {
+      add_stamps(marks, &table);         // (windows are cut by the bytes of slots and stamps)
       if (!check(dok_map_set_unique(&table, &self->hash, keys->data_ptr(), values->data_ptr(), n, nullptr, self->state + STATE_SET, stream),
                  "dok_map_set_unique"))
         return nullptr;
-    } else if (dok_set_takes_sequence(&table, &self->hash, n)) {
-      if (!check(dok_map_set_sequenced(&table, &self->hash, keys->data_ptr(), values->data_ptr(), n, self->state + STATE_SEQUENCE,
-                                       self->state + STATE_SET, stream),
-                 "dok_map_set_sequenced"))
+    } else if (take_numbers(self, marks, n, stream, &base)) {
+      if (!check(dok_map_set_numbered(&table, &self->hash, keys->data_ptr(), values->data_ptr(), n, base, self->state + STATE_SET, stream),
+                 "dok_map_set_numbered"))
         return nullptr;
     } else {
-      if (!has_stamps(table)) Py_RETURN_NONE;
+      if (!take_epoch(marks, &table, &epoch)) Py_RETURN_NONE;
       const int64_t words = dok_set_scratch_words(&table, n);
       at::Tensor scratch;
       if (words > 0) scratch = at::empty({words}, on_device(self, at::kLong));
@@ -583,8 +667,8 @@ bool parse_selection(PyObject *selectors, const int64_t *size, int ndim, int dev
 PyObject *plan_index(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
   return guarded([&]() -> PyObject * {
     if (nargs != 2) { PyErr_SetString(PyExc_TypeError, "index takes 2 arguments"); return nullptr; }
-    int64_t size[8];
-    const int ndim = shape_from(args[1], size);
+    int64_t size[DOK_MAX_KEY_SIZE];
+    const int ndim = shape_from(args[1], size, DOK_MAX_KEY_SIZE);
     if (ndim < 1 || ndim > DOK_MAX_KEY_SIZE || ndim != self->hash.key_size || self->value_ndim != 1 || self->value_shape[0] != 1) {
       PyErr_Clear();
       Py_RETURN_NONE;
@@ -606,13 +690,14 @@ PyObject *plan_index(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
   });
 }
 
-// assign(selectors, size, values, room, epoch, stamp address) -> the number of positions, or None; its negative, and
-// nothing done, when it is more than `room`, so that the table might have to grow
+// assign(selectors, size, values, room, marks) -> the number of positions, or None; its negative, and nothing done, when it
+// is more than `room`, so that the table might have to grow
 PyObject *plan_assign(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
   return guarded([&]() -> PyObject * {
-    if (nargs != 6) { PyErr_SetString(PyExc_TypeError, "assign takes 6 arguments"); return nullptr; }
-    int64_t size[8];
-    const int ndim = shape_from(args[1], size);
+    Marks *marks = nargs == 5 ? marks_of(args[4]) : nullptr;
+    if (!marks) { PyErr_SetString(PyExc_TypeError, "assign takes selectors, size, values, room and Marks"); return nullptr; }
+    int64_t size[DOK_MAX_KEY_SIZE];
+    const int ndim = shape_from(args[1], size, DOK_MAX_KEY_SIZE);
     const at::Tensor *given = tensor_of(args[2]);
     const bool number = PyFloat_CheckExact(args[2]) ? at::isFloatingType(self->value_type)
                                                     : PyLong_CheckExact(args[2]) && (at::isFloatingType(self->value_type) || self->value_type == at::kLong);
@@ -624,11 +709,11 @@ PyObject *plan_assign(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
       Py_RETURN_NONE;
     }
     const double room = PyFloat_AsDouble(args[3]);
-    const int64_t epoch = PyLong_AsLongLong(args[4]);
-    dok_table table = self->table;
-    table.stamp = (int64_t *)PyLong_AsVoidPtr(args[5]);
     if (PyErr_Occurred()) return nullptr;
     const c10::cuda::CUDAGuard guard((c10::DeviceIndex)self->device);
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream();
+    dok_table table = self->table;
+    int64_t base, epoch;
     Selection s;
     if (!parse_selection(args[0], size, ndim, self->device, &s)) Py_RETURN_NONE;
     if ((double)s.n > room) return PyLong_FromLongLong(-s.n);
@@ -645,20 +730,18 @@ PyObject *plan_assign(Plan *self, PyObject *const *args, Py_ssize_t nargs) {
       }
       values = at::full({}, value, on_device(self, self->value_type)).expand(s.shape);
     }
-    if (dok_set_takes_sequence(&table, &self->hash, s.n)) {
-      if (!check(dok_dok_assign_sequenced(&table, &self->hash, &s.sel, values.data_ptr(), values.strides().data(), self->state + STATE_SEQUENCE,
-                                          self->state + STATE_SET, self->state + STATE_ADJUST,
-                                          c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()),
-                 "dok_dok_assign_sequenced"))
+    if (take_numbers(self, marks, s.n, stream, &base)) {
+      if (!check(dok_dok_assign_numbered(&table, &self->hash, &s.sel, values.data_ptr(), values.strides().data(), base, self->state + STATE_SET,
+                                         self->state + STATE_ADJUST, stream),
+                 "dok_dok_assign_numbered"))
         return nullptr;
     } else if (s.n > 0) {
-      if (!has_stamps(table)) Py_RETURN_NONE;
+      if (!take_epoch(marks, &table, &epoch)) Py_RETURN_NONE;
       const int64_t words = dok_set_scratch_words(&table, s.n);
       at::Tensor scratch;
       if (words > 0) scratch = at::empty({words}, on_device(self, at::kLong));
       if (!check(dok_dok_assign(&table, &self->hash, &s.sel, values.data_ptr(), values.strides().data(),
-                                words > 0 ? (int64_t *)scratch.data_ptr() : nullptr, words, epoch, self->state + STATE_SET, self->state + STATE_ADJUST,
-                                c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)self->device).stream()),
+                                words > 0 ? (int64_t *)scratch.data_ptr() : nullptr, words, epoch, self->state + STATE_SET, self->state + STATE_ADJUST, stream),
                  "dok_dok_assign"))
         return nullptr;
     }
@@ -675,13 +758,22 @@ PyMethodDef ring_methods[] = {
 
 PyTypeObject ring_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
+PyMemberDef marks_members[] = {{"stamp", T_OBJECT, offsetof(Marks, stamp), 0, nullptr},
+                               {"epoch", T_LONGLONG, offsetof(Marks, epoch), 0, nullptr},
+                               {"numbered", T_LONGLONG, offsetof(Marks, numbered), 0, nullptr},
+                               {"renumbered", T_LONGLONG, offsetof(Marks, renumbered), READONLY, nullptr},
+                               {nullptr, 0, 0, 0, nullptr}};
+
+PyTypeObject marks_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+Marks *marks_of(PyObject *o) { return Py_TYPE(o) == &marks_type ? (Marks *)o : nullptr; }
+
 PyMethodDef module_methods[] = {{"allocate", (PyCFunction)plan_allocate, METH_VARARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
 
 PyMethodDef plan_methods[] = {
     {"set_hash", (PyCFunction)(void *)plan_set_hash, METH_FASTCALL, nullptr},
     {"get", (PyCFunction)plan_get, METH_O, nullptr},
     {"set", (PyCFunction)(void *)plan_set, METH_FASTCALL, nullptr},
-    {"in_word", (PyCFunction)plan_in_word, METH_O, nullptr},
     {"remove_rows", (PyCFunction)plan_remove_rows, METH_O, nullptr},
     {"remove", (PyCFunction)plan_remove, METH_O, nullptr},
     {"read", (PyCFunction)plan_read, METH_NOARGS, nullptr},
@@ -712,12 +804,23 @@ PyMODINIT_FUNC PyInit__native(void) {
   ring_type.tp_init = (initproc)ring_init;
   ring_type.tp_dealloc = (destructor)ring_dealloc;
   ring_type.tp_methods = ring_methods;
-  if (PyType_Ready(&plan_type) < 0 || PyType_Ready(&ring_type) < 0) return nullptr;
+  marks_type.tp_name = "doksparse_b200._native.Marks";
+  marks_type.tp_basicsize = sizeof(Marks);
+  marks_type.tp_flags = Py_TPFLAGS_DEFAULT;
+  marks_type.tp_new = PyType_GenericNew;
+  marks_type.tp_init = (initproc)marks_init;
+  marks_type.tp_dealloc = (destructor)marks_dealloc;
+  marks_type.tp_members = marks_members;
+  if (PyType_Ready(&plan_type) < 0 || PyType_Ready(&ring_type) < 0 || PyType_Ready(&marks_type) < 0) return nullptr;
   PyObject *lib = PyImport_ImportModule("doksparse_b200._lib");
   if (!lib) return nullptr;
   dok_error = PyObject_GetAttrString(lib, "DokError");
   Py_DECREF(lib);
   PyObject *m = dok_error ? PyModule_Create(&module) : nullptr;
-  if (m && (PyModule_AddObjectRef(m, "Plan", (PyObject *)&plan_type) < 0 || PyModule_AddObjectRef(m, "Ring", (PyObject *)&ring_type) < 0)) { Py_DECREF(m); return nullptr; }
+  if (m && (PyModule_AddObjectRef(m, "Plan", (PyObject *)&plan_type) < 0 || PyModule_AddObjectRef(m, "Ring", (PyObject *)&ring_type) < 0 ||
+            PyModule_AddObjectRef(m, "Marks", (PyObject *)&marks_type) < 0)) {
+    Py_DECREF(m);
+    return nullptr;
+  }
   return m;
 }

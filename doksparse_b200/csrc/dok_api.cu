@@ -508,14 +508,15 @@ int dok_dok_assign(const dok_table *t, const dok_hash_params *hp, const dok_sele
   return launch_set_general(dt, dh, sk, strided(sel, src, src_strides), scratch, epoch, nullptr, counters, (cudaStream_t)stream, more, scratch_words);
 }
 
-int dok_dok_assign_sequenced(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel, const void *src,
-                             const int64_t *src_strides, int64_t *sequence, int64_t *counters, int64_t *more, void *stream) {
+int dok_dok_assign_numbered(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel, const void *src,
+                            const int64_t *src_strides, int64_t base, int64_t *counters, int64_t *more, void *stream) {
   DevHash dh;
   DevTable dt;
   SelKeys sk;
-  if (!prepare(t, hp, &dt, &dh) || !make_sel(sel, dh, &sk) || sk.n < 1 || !dok_set_in_word(dt, dh, sk.n) || !src || !src_strides || !sequence)
+  if (!prepare(t, hp, &dt, &dh) || !make_sel(sel, dh, &sk) || !dok_set_in_word(dt, dh, sk.n) || !dok_numbers_fit(base, sk.n) || !src ||
+      !src_strides)
     return DOK_BAD_ARG;
-  return launch_set_word(dt, dh, sk, strided(sel, src, src_strides), sequence, counters, more, (cudaStream_t)stream);
+  return launch_set_word(dt, dh, sk, strided(sel, src, src_strides), base, counters, more, (cudaStream_t)stream);
 }
 
 int dok_dok_gather_insert(const dok_table *src, const dok_hash_params *src_hp, const dok_selectors *sel,

@@ -6,7 +6,6 @@
 #include "dok_device.cuh"
 
 #define DOK_MAX_BATCH 0xffffffffLL   // row indices are packed into 32 bits of the set stamp
-#define DOK_MAX_EPOCH 0x3fffffffLL   // 30 bits of the stamp above the row index and two flags
 
 // contiguous value rows [n, value_bytes]
 struct RowValues {

@@ -8,41 +8,41 @@
 // what the reference's count of an assignment asks for, and there is nothing left for further kernels.  (Slots of 64 and 128
 // bytes have other use for that padding: dok_mark_passed.)
 //
-// Numbers go on from set to set: a table's `sequence` on the device holds the next one, so that a captured set counts on
-// when it is replayed.  Before they run out at 2^31 rows k_word_begin clears them.
+// Numbers go on from set to set.  The host hands them out (`base` of a launch), so that sets on several streams have ranges of
+// their own and whatever is ordered after a set has larger ones; k_word_clear makes a new start when they have run out at
+// 2^31 rows.  A set in a graph, whose base would be old when it is replayed, first takes the numbers of the slots that it will
+// write away (k_word_release: another walk) and has base 0.
 //
-// 4 M-pair assignment to a 2-D tensor: 393 + 56 + 25 us of k_set_claim, k_set_resolve, k_set_count; here 219 + 4.  8.4 M rows of
+// 4 M-pair assignment to a 2-D tensor: 393 + 56 + 25 us of k_set_claim, k_set_resolve, k_set_count; here 219.  8.4 M rows of
 // 4-byte values in a table of 2^26 keys, a fifth of them new: 688 -> 564; 800 k Zipf ids 97 -> 52.
 #pragma once
 
 // row's number (31 bits) | this batch claimed the slot | value (32 bits)
 #define DOK_WORD_FRESH (1ULL << 32)
 #define DOK_WORD_SHIFT 33
-#define DOK_WORD_ROWS 0x7ffffff0LL
-enum { DOK_SEQ_NEXT = 0, DOK_SEQ_BASE = 1, DOK_SEQ_TICKET = 2 };
 
+inline bool dok_values_in_word(const DevTable &t) { return t.sb == 32 && t.vb <= 4; }
 inline bool dok_set_in_word(const DevTable &t, const DevHash &hp, ll_t n) {
-  return t.sb == 32 && t.vb <= 4 && hp.dtype < DOK_F16 && n <= DOK_WORD_ROWS;
+  return dok_values_in_word(t) && hp.dtype < DOK_F16 && n > 0 && n <= DOK_MAX_NUMBER;
+}
+inline bool dok_numbers_fit(ll_t base, ll_t n) { return base == DOK_RENUMBER || (base >= 0 && base <= DOK_MAX_NUMBER - n); }
+
+__device__ __forceinline__ unsigned *dok_number_ptr(const DevTable &t, ll_t slot) { return (unsigned *)(dok_value_ptr(t, slot) + 4); }
+
+static __global__ void __launch_bounds__(DOK_TPB) k_word_clear(DevTable t) {
+  for (ll_t i = (ll_t)blockIdx.x * DOK_TPB + threadIdx.x; i < t.n_slots; i += (ll_t)gridDim.x * DOK_TPB) *dok_number_ptr(t, i) = 0;
 }
 
-__device__ __forceinline__ void dok_clear_numbers(const DevTable &t) {
-  for (ll_t i = (ll_t)blockIdx.x * blockDim.x + threadIdx.x; i < t.n_slots; i += (ll_t)gridDim.x * blockDim.x)
-    *(unsigned *)(dok_value_ptr(t, i) + 4) = 0;
-}
-// The numbers of this set's rows: base + 1 ... base + n.
-static __global__ void __launch_bounds__(DOK_TPB) k_word_begin(DevTable t, ll_t *sequence, ll_t n) {
-  __shared__ ll_t next;
-  if (threadIdx.x == 0) next = *(volatile ll_t *)&sequence[DOK_SEQ_NEXT];
-  __syncthreads();
-  const bool over = next + n > DOK_WORD_ROWS;
-  if (over) dok_clear_numbers(t);
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  __threadfence();
-  if (atomicAdd((ull_t *)&sequence[DOK_SEQ_TICKET], 1ULL) != gridDim.x - 1) return;
-  sequence[DOK_SEQ_BASE] = over ? 0 : next;                  // the last block: all have read
-  sequence[DOK_SEQ_NEXT] = (over ? 0 : next) + n;
-  sequence[DOK_SEQ_TICKET] = 0;
+// The numbers of the slots that hold the batch's keys.
+template <bool FEW, class Keys>
+__global__ void __launch_bounds__(DOK_TPB) k_word_release(DevTable t, DevHash hp, Keys keys) {
+  ll_t e;
+  bool active = keys.row(e);
+  KeyHash kh{0, 0};
+  if (active) kh = keys.hash(hp, e);
+  active = dok_in_window(t, kh, active);
+  const Located loc = dok_locate<32, 1, false>(t, kh, e, active, nullptr, NoEmit<FEW>());
+  if (active && loc.found >= 0) *dok_number_ptr(t, loc.found) = 0;
 }
 
 __device__ __forceinline__ ulonglong2 dok_cas_pair(char *slot, ulonglong2 expect, ulonglong2 desired) {
@@ -73,8 +73,8 @@ static __device__ __forceinline__ WordSlot dok_claim_word_serial(const DevTable 
         if ((ll_t)now.x == DOK_EMPTY && phase == 0 && reuse) { more = false; break; }
         if ((ll_t)now.x == DOK_EMPTY || ((ll_t)now.x == DOK_REMOVED && phase == 1)) {
           const ulonglong2 old = dok_cas_pair(dok_slot_ptr(t, slot), now, make_ulonglong2((ull_t)key.uuid, word));
-          if (old.x == now.x) return WordSlot{slot, (ll_t)now.x == DOK_EMPTY ? DOK_OUT_CLAIMED_EMPTY : DOK_OUT_REUSED, 0};
-          now = old;                                         // (the word of a free slot does not change while a set runs)
+          if (old.x == now.x && old.y == now.y) return WordSlot{slot, (ll_t)now.x == DOK_EMPTY ? DOK_OUT_CLAIMED_EMPTY : DOK_OUT_REUSED, 0};
+          now = old;               // (the word of a free slot stays as it is while sets and removals of one key are in order)
         }
         if ((ll_t)now.x == key.uuid) return WordSlot{slot, DOK_OUT_FOUND, now.y};
       }
@@ -100,7 +100,7 @@ __device__ __forceinline__ WordSlot dok_find_or_claim_word(const DevTable &t, co
   if (reuse) free = dok_load_pair(at);
   if ((ll_t)free.x == DOK_EMPTY || (ll_t)free.x == DOK_REMOVED) {
     const ulonglong2 old = dok_cas_pair(at, free, make_ulonglong2((ull_t)key.uuid, word));
-    if (old.x == free.x) return WordSlot{slot, reuse ? DOK_OUT_REUSED : DOK_OUT_CLAIMED_EMPTY, 0};
+    if (old.x == free.x && old.y == free.y) return WordSlot{slot, reuse ? DOK_OUT_REUSED : DOK_OUT_CLAIMED_EMPTY, 0};
     free = old;
   }
   if ((ll_t)free.x == key.uuid) return WordSlot{slot, DOK_OUT_FOUND, free.y};
@@ -134,13 +134,12 @@ __device__ __forceinline__ WordOutcome dok_write_word(const DevTable &t, const D
 }
 
 template <bool FEW, class Keys, class Values>
-__global__ void __launch_bounds__(DOK_TPB, 6) k_set_word(DevTable t, DevHash hp, Keys keys, Values values, const ll_t *sequence,
-                                                         ll_t *counters, ll_t *more) {
+__global__ void __launch_bounds__(DOK_TPB, 6) k_set_word(DevTable t, DevHash hp, Keys keys, Values values, ll_t base, ll_t *counters,
+                                                         ll_t *more) {
   __shared__ BlockTally tally;
   __shared__ BlockTwins twins;
   const unsigned block = gridDim.x - 1 - blockIdx.x;         // from the end of the batch: a popular key's last rows first
   dok_tally_begin(tally);
-  const ll_t base = sequence[DOK_SEQ_BASE];
   ll_t e;
   bool active = keys.row(e, block);
   KeyHash kh{0, 0};
@@ -177,23 +176,14 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_word(DevTable t, DevHash hp,
   dok_tally_flush(tally, counters, more);
 }
 
-// The same for a batch that one cluster holds (k_set_small), in one launch: the blocks read the next number together, and the
-// first one moves it on when all have.
+// The same for a batch of few rows (k_set_small), which has no popular keys to look for.
 template <class Keys, class Values>
-__global__ void __launch_bounds__(DOK_SMALL_SET_TPB) k_set_word_small(DevTable t, DevHash hp, Keys keys, Values values, ll_t *sequence,
-                                                                      ll_t *counters, ll_t *more) {
+__global__ void __launch_bounds__(DOK_TPB, 4) k_set_word_small(DevTable t, DevHash hp, Keys keys, Values values, ll_t base, ll_t *counters,
+                                                            ll_t *more) {
   __shared__ BlockTally tally;
   dok_tally_begin(tally);
-  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
-  ll_t base = *(volatile ll_t *)&sequence[DOK_SEQ_NEXT];
-  const bool over = base + keys.count() > DOK_WORD_ROWS;     // uniform over the launch
-  if (over) {
-    base = 0;
-    dok_clear_numbers(t);
-    cluster.sync();
-  }
-  const ll_t e = (ll_t)blockIdx.x * DOK_SMALL_SET_TPB + threadIdx.x;
-  const bool active = e < keys.count();
+  ll_t e;
+  const bool active = keys.row(e);
   KeyHash kh{0, 0};
   ull_t value = 0;
   if (active) {
@@ -213,20 +203,23 @@ __global__ void __launch_bounds__(DOK_SMALL_SET_TPB) k_set_word_small(DevTable t
     dok_tally_add(tally, DOK_CNT_DUPLICATES, o.met);
   }
   dok_tally_flush(tally, counters, more);
-  cluster.sync();
-  if (blockIdx.x == 0 && threadIdx.x == 0) sequence[DOK_SEQ_NEXT] = base + keys.count();
 }
 
 template <class Keys, class Values>
-inline int launch_set_word(const DevTable &t, const DevHash &hp, const Keys &keys, const Values &values, int64_t *sequence, int64_t *counters,
+inline int launch_set_word(const DevTable &t, const DevHash &hp, const Keys &keys, const Values &values, int64_t base, int64_t *counters,
                            int64_t *more, cudaStream_t st) {
-  if (dok_set_is_small(t, keys.n))
-    return dok_launch_cluster(keys.n, st, k_set_word_small<Keys, Values>, t, hp, keys, values, (ll_t *)sequence, (ll_t *)counters, (ll_t *)more);
-  k_word_begin<<<148, DOK_TPB, 0, st>>>(t, (ll_t *)sequence, keys.n);
-  int rc = dok_check_launch();
-  if (rc != DOK_OK) return rc;
   const dim3 grid = dok_grid(keys);
-  DOK_BY_SIZE(grid.x, DOK_FOR_WINDOWS(t, rc, (k_set_word<FEW><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, (const ll_t *)sequence,
-                                                                                     (ll_t *)counters, (ll_t *)more))));
+  int rc = DOK_OK;
+  if (base == DOK_RENUMBER) {
+    base = 0;
+    DOK_BY_SIZE(grid.x, DOK_FOR_WINDOWS(t, rc, (k_word_release<FEW><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys))));
+    if (rc != DOK_OK) return rc;
+  }
+  if (dok_set_is_small(t, keys.n)) {
+    k_set_word_small<<<grid, DOK_TPB, 0, st>>>(t, hp, keys, values, (ll_t)base, (ll_t *)counters, (ll_t *)more);
+    return dok_check_launch();
+  }
+  DOK_BY_SIZE(grid.x, DOK_FOR_WINDOWS(t, rc, (k_set_word<FEW><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, (ll_t)base, (ll_t *)counters,
+                                                                                     (ll_t *)more))));
   return rc;
 }

@@ -10,7 +10,7 @@ static unsigned grid_for(ll_t n) { return (unsigned)((n + DOK_TPB - 1) / DOK_TPB
 
 extern "C" {
 
-int dok_version(void) { return 2; }
+int dok_version(void) { return 3; }
 int dok_last_cuda_error(void) { return dok_last_error_slot(); }
 int64_t dok_launch_count(void) { return dok_launch_counter(); }
 
@@ -113,19 +113,27 @@ int dok_map_set_with(const dok_table *t, const dok_hash_params *hp, const void *
   return launch_set(dt, dh, rk, (const char *)values, scratch, epoch, nullptr, counters, (cudaStream_t)stream, scratch_words);
 }
 
-int dok_set_takes_sequence(const dok_table *t, const dok_hash_params *hp, int64_t n) {
+int dok_set_takes_numbers(const dok_table *t, const dok_hash_params *hp, int64_t n) {
   DevHash dh;
   DevTable dt;
-  return prepare(t, hp, &dt, &dh) && n > 0 && dok_set_in_word(dt, dh, n);
+  return prepare(t, hp, &dt, &dh) && dok_set_in_word(dt, dh, n);
 }
 
-int dok_map_set_sequenced(const dok_table *t, const dok_hash_params *hp, const void *keys, const void *values, int64_t n,
-                          int64_t *sequence, int64_t *counters, void *stream) {
+int dok_map_set_numbered(const dok_table *t, const dok_hash_params *hp, const void *keys, const void *values, int64_t n,
+                         int64_t base, int64_t *counters, void *stream) {
   DevHash dh;
   DevTable dt;
-  if (!prepare(t, hp, &dt, &dh) || n < 1 || !dok_set_in_word(dt, dh, n) || !keys || !values || !sequence) return DOK_BAD_ARG;
+  if (!prepare(t, hp, &dt, &dh) || !dok_set_in_word(dt, dh, n) || !dok_numbers_fit(base, n) || !keys || !values) return DOK_BAD_ARG;
   RowKeys rk{keys, n};
-  return launch_set_word(dt, dh, rk, RowValues{(const char *)values}, sequence, counters, nullptr, (cudaStream_t)stream);
+  return launch_set_word(dt, dh, rk, RowValues{(const char *)values}, base, counters, nullptr, (cudaStream_t)stream);
+}
+
+int dok_map_clear_numbers(const dok_table *t, void *stream) {
+  DevTable dt;
+  if (!dok_make_table(t, &dt) || !dok_values_in_word(dt)) return DOK_BAD_ARG;
+  const ll_t blocks = (dt.n_slots + DOK_TPB - 1) / DOK_TPB;
+  k_word_clear<<<(unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), DOK_TPB, 0, (cudaStream_t)stream>>>(dt);
+  return dok_check_launch();
 }
 
 int dok_map_remove(const dok_table *t, const dok_hash_params *hp, const void *keys, int64_t n, uint8_t *out_removed,

@@ -34,7 +34,7 @@ _PARAM_NAMES = ("prime1", "prime2", "alpha1", "alpha2", "beta1", "beta2")
 _STATE_WORDS = 32
 _BY_SET, _BY_REMOVE, _BY_ROWS, _BY_BULK = 0, 8, 16, 24      # set | remove | distinct new rows of float keys | bulk inserts
 _ADJUST = 7              # what n_elements differs by from the slots in use (the reference's DOK assignments over-count)
-_SEQUENCE = 18           # three words: numbers of the rows of sets that need no stamps
+_SEQUENCE = 18           # (three words that are free: row numbers are handed out by the host, see _native.Marks)
 _COUNTED_NEW = 23        # result of the exact count of a set that may have to grow the table
 
 
@@ -68,16 +68,6 @@ class _PinnedRings:
 
 
 _rings = _PinnedRings()
-
-
-class _Marks:
-    """What general sets have left in one slot array, for as long as there is that array: every map that writes its slots
-    has these marks, and a new slot array gets new ones.  `epoch`: the largest one in a stamp.  `stamp`: the stamps, where
-    the slots have no room for them."""
-    __slots__ = ("stamp", "epoch")
-
-    def __init__(self, stamp=None, epoch=0):
-        self.stamp, self.epoch = stamp, epoch
 
 
 class _Shared:
@@ -135,7 +125,7 @@ class CudaClosedHashmap:
         self._key_shape = None
         self._key_dtype = None
         self._shared = _Shared()
-        self._marks = _Marks()
+        self._marks = None           # what sets have left in the slot array (_native.Marks)
         self._value_shape = None
         self._value_dtype = None
 
@@ -308,7 +298,7 @@ class CudaClosedHashmap:
         self._value_bytes, self._key_bytes = value_bytes, key_size * key_dtype.itemsize
         self._value_shape, self._value_dtype = torch.Size(value_shape), value_dtype
         self._key_shape, self._key_dtype = torch.Size(key_shape), key_dtype
-        self._marks = _Marks()
+        self._marks = L.native().Marks()
         self._hp = self._plan = None
         device = torch.cuda.current_device() if self.device.index is None else self.device.index
         self._bare_plan, self._slots, self._counters_of_table, layout = L.native().allocate(
@@ -366,15 +356,18 @@ class CudaClosedHashmap:
         return self._slot_view(self._key_dtype, self._key_shape, self._layout.key_offset)
 
     def _next_epoch(self):
-        """Epoch of the next general set: larger than every epoch stamped on this table before.  The stamps live in
-        the slots when the layout has room for them, else in a separate array allocated on first use."""
+        """Epoch of the next stamped set: larger than every epoch stamped on this table before."""
+        self._ready_stamps()
+        epoch = self._marks.epoch = self._marks.epoch + 1
+        return epoch
+
+    def _ready_stamps(self):
+        """The stamps live in the slots when the layout has room for them, else in a separate array allocated on first use."""
         marks = self._marks
         if self._layout.stamp_offset < 0 and marks.stamp is None:
             marks.stamp = torch.zeros(self._layout.n_slots, device=self.device, dtype=torch.long)
         if marks.epoch >= L.MAX_EPOCH - 1:
             raise L.DokError("stamp epochs exhausted: rehash() the map to start over")
-        marks.epoch += 1
-        return marks.epoch
 
     def _c_table(self):
         t = L.Table()
@@ -427,13 +420,6 @@ class CudaClosedHashmap:
             self._plan = L.native().Plan(bytes(self._table), bytes(self._hp), self._state.data_ptr(), self._slots.device.index,
                                        tuple(self._key_shape), self._key_dtype, tuple(self._value_shape), self._value_dtype)
         return self._plan
-
-    def _stamp_address(self):
-        """Address of the separate stamp array (0: the stamps are in the slots), None while it has yet to be made."""
-        if self._layout.stamp_offset >= 0:
-            return 0
-        stamp = self._marks.stamp
-        return None if stamp is None else stamp.data_ptr()
 
     def _counters(self):
         return torch.zeros(L.N_COUNTERS, device=self.device, dtype=torch.long)
@@ -571,9 +557,9 @@ class CudaClosedHashmap:
         new._key_shape, new._key_dtype = self._key_shape, self._key_dtype
         new._counters_of_table = cp(self._state)
         if deepclone:
-            # in-slot stamps were copied with the slots: continue their epochs; a separate array is copied too
-            marks = self._marks
-            new._marks = _Marks(None if marks.stamp is None else marks.stamp.clone(), marks.epoch)
+            # stamps and numbers in the slots were copied with them: continue; a separate array is copied too
+            stamp = self._marks.stamp
+            new._marks = L.native().Marks(self._marks, None if stamp is None else stamp.clone())
             new._shared = _Shared(self._shared.bound)
         else:
             new._marks, new._shared = self._marks, self._shared   # a view writes the same slots
@@ -685,19 +671,19 @@ class CudaClosedHashmap:
     # ------------------------------------------------------------------ set
     def _launch_set(self, keys, values, assume_unique):
         """The set kernels on contiguous rows of this table."""
-        unstamped = assume_unique or self._native_plan().in_word(keys.shape[0])
-        epoch = self._marks.epoch if unstamped else self._next_epoch()
-        self._native_plan().set(keys, values, assume_unique, epoch, self._stamp_address() or 0)
+        plan = self._native_plan()
+        if plan.set(keys, values, assume_unique, self._marks) is None:
+            self._ready_stamps()
+            plan.set(keys, values, assume_unique, self._marks)
 
     def set(self, new_keys, new_values, assume_unique=False):
         """Insert-or-assign a batch.  `assume_unique=True` promises pairwise different keys and runs one kernel
         instead of two.  Returns None like the reference."""
-        plan, marks = self._plan, self._marks
-        if plan is not None and self._key_dtype not in L.FLOAT_DTYPES and marks.epoch < L.MAX_EPOCH - 1 \
+        plan = self._plan
+        if plan is not None and self._key_dtype not in L.FLOAT_DTYPES \
                 and self._room_for(new_keys.shape[0], int(self._rehash_threshold * self._n_buckets)):
-            rows = plan.set(new_keys, new_values, assume_unique, marks.epoch + 1, self._stamp_address() or 0)
+            rows = plan.set(new_keys, new_values, assume_unique, self._marks)
             if rows is not None:
-                marks.epoch += 1
                 self._after_mutation(rows)
                 return
         assert new_keys.shape[0] == new_values.shape[0]
@@ -948,7 +934,7 @@ class CudaClosedHashmap:
         state[L.CNT_CLAIMED_EMPTY] -= gone
         state[L.CNT_REUSED_REMOVED] += gone
         known = self._shared.known
-        self._slots, self._counters_of_table, self._marks, self._shared = fresh, state, _Marks(), _Shared(self._shared.bound)
+        self._slots, self._counters_of_table, self._marks, self._shared = fresh, state, L.native().Marks(), _Shared(self._shared.bound)
         self._shared.known = known
         self._plan = self._bare_plan = None
         with L.on(self.device):

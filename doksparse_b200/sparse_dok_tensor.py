@@ -372,15 +372,13 @@ class SparseDOKTensor(object):
         treated like a 0-dim tensor, as the reference's README documents."""
         hashmap = self._hashmap
         plan, marks = hashmap._plan or hashmap._native_plan(), hashmap._marks
-        if plan is not None and hashmap._value_dtype == self._dtype and marks.epoch < L.MAX_EPOCH - 1:
-            stamp = hashmap._stamp_address() or 0
+        if plan is not None and hashmap._value_dtype == self._dtype:
             limit = hashmap._n_buckets * hashmap._rehash_threshold
-            n = plan.assign(selectors, self._size, values, limit - hashmap._element_bound(), marks.epoch + 1, stamp)
+            n = plan.assign(selectors, self._size, values, limit - hashmap._element_bound(), marks)
             if n is not None and n < 0 and hashmap._room_for(-n, limit):
-                n = plan.assign(selectors, self._size, values, -n, marks.epoch + 1, stamp)
+                n = plan.assign(selectors, self._size, values, -n, marks)
             if n is not None and n >= 0:
                 if n:
-                    marks.epoch += 1
                     hashmap._after_mutation(n)
                 return
         selectors, _ = self._handle_selectors(selectors)
@@ -425,26 +423,14 @@ class SparseDOKTensor(object):
             n_elements = hashmap.n_elements
             if n_elements + n_sel > hashmap.n_buckets * hashmap._rehash_threshold:
                 hashmap.rehash(math.ceil((n_elements + n_sel) * hashmap._rehash_factor))
-        sel = _selectors_struct(selectors)
-        src_strides = (ctypes.c_int64 * L.MAX_SELECTOR_NDIM)(*src.stride())
-        if hashmap._native_plan().in_word(n_sel):
-            with L.on(self.device):
-                L.check(L.lib().dok_dok_assign_sequenced(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(src), src_strides,
-                                                         hashmap._counter_block(M._SEQUENCE), hashmap._counter_block(M._BY_SET),
-                                                         hashmap._counter_block(M._ADJUST), L.stream_ptr(self.device)),
-                        "dok_dok_assign_sequenced")
-            hashmap._after_mutation(n_sel)
-            return
-        epoch = hashmap._next_epoch()
-        words = L.lib().dok_set_scratch_words(hashmap._c_table(), n_sel)
-        if words < 0:
+        if n_sel > L.MAX_BATCH:
             raise L.DokError(f"an assignment may select up to 2^32 - 1 positions, got {n_sel}")
-        scratch = torch.empty(words, device=self.device, dtype=torch.long)
-        with L.on(self.device):
-            # n_elements grows by the selected positions that were not stored; duplicates over-count, like the reference (:474)
-            L.check(L.lib().dok_dok_assign(hashmap._c_table(), hashmap._c_hash(), ctypes.byref(sel), L.ptr(src),
-                                           src_strides, L.ptr(scratch), words, epoch, hashmap._counter_block(M._BY_SET),
-                                           hashmap._counter_block(M._ADJUST), L.stream_ptr(self.device)), "dok_dok_assign")
+        # n_elements grows by the selected positions that were not stored; duplicates over-count, like the reference (:474)
+        plan, selectors = hashmap._native_plan(), tuple(selectors)
+        if plan.assign(selectors, self._size, src, n_sel, hashmap._marks) is None:
+            hashmap._ready_stamps()
+            if plan.assign(selectors, self._size, src, n_sel, hashmap._marks) is None:
+                raise L.DokError(f"an assignment to selectors of shape {tuple(selectors[0].shape)} (at most {L.MAX_SELECTOR_NDIM} dims) failed")
         hashmap._after_mutation(n_sel)
 
     def zero_items(self, selectors):

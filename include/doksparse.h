@@ -13,6 +13,9 @@
  * the start slot is free (the slot layout is not part of the contract) and is derived from the uuid
  * and the first-hash parameters with a 64-bit mixer.
  *
+ * Calls on one table may run at the same time on several streams as long as no key of a set is in another call that sets or
+ * removes it; calls that share such keys, and those that replace or clear slots, are ordered by the caller.
+ *
  * Storage of a table (owned by the caller, 128-byte aligned, sized by dok_table_layout): n_slots slots of
  * slot_bytes (32, 64, 128, or a larger multiple of 128 for very wide rows):
  *     { int64 tag | value (padded to 8) | key row (padded to 8) | int64 stamp (if it fits without growing the slot) }
@@ -39,6 +42,9 @@ extern "C" {
 #define DOK_MAX_VALUE_BYTES 248 /* value bytes per row  */
 #define DOK_MAX_SELECTOR_NDIM 8 /* dims of a broadcast selector shape */
 #define DOK_MAX_SHARDS 64
+#define DOK_MAX_EPOCH 0x3fffffffLL  /* 30 bits of a stamp */
+#define DOK_MAX_NUMBER 0x7ffffff0LL /* number of a row in the word of its value */
+#define DOK_RENUMBER (-1LL)
 
 #define DOK_TAG_EMPTY (-1LL)   /* cuda_closed_hashmap.py:36 */
 #define DOK_TAG_REMOVED (-3LL) /* cuda_closed_hashmap.py:37 */
@@ -212,12 +218,17 @@ int64_t dok_set_scratch_words(const dok_table *t, int64_t n);
 int dok_map_set_with(const dok_table *t, const dok_hash_params *hp, const void *keys, const void *values, int64_t n,
                      int64_t *scratch, int64_t scratch_words, int64_t epoch, int64_t *counters, void *stream);
 
-/* dok_map_set for batches whose values share a word of the slot with their row's number (integer keys, values of at most 4
- * bytes in 32-byte slots: dok_set_takes_sequence answers 1).  Neither stamps nor scratch are needed.  sequence: device
- * int64[3] that belong to the table, zero when its slots are initialised. */
-int dok_set_takes_sequence(const dok_table *t, const dok_hash_params *hp, int64_t n);
-int dok_map_set_sequenced(const dok_table *t, const dok_hash_params *hp, const void *keys, const void *values, int64_t n,
-                          int64_t *sequence, int64_t *counters, void *stream);
+/* dok_map_set for batches whose values share a word of the slot with the number of the row that wrote them (integer keys,
+ * values of at most 4 bytes in 32-byte slots: dok_set_takes_numbers answers 1).  Neither stamps nor scratch are needed.  The
+ * rows have the numbers base + 1 ... base + n, up to DOK_MAX_NUMBER; base is at least every number that was used on these
+ * slots before, 0 for new ones, and the ranges of sets that may run at the same time do not overlap.  When the numbers have
+ * run out, dok_map_clear_numbers gives the slots a new start; no set of the table may run meanwhile.
+ * base = DOK_RENUMBER: the numbers of the slots that hold the batch's keys are cleared first, then the rows have 1 ... n.
+ * For a set in a graph, right whenever it is replayed; sets outside of the graph go on from n or more. */
+int dok_set_takes_numbers(const dok_table *t, const dok_hash_params *hp, int64_t n);
+int dok_map_set_numbered(const dok_table *t, const dok_hash_params *hp, const void *keys, const void *values, int64_t n,
+                         int64_t base, int64_t *counters, void *stream);
+int dok_map_clear_numbers(const dok_table *t, void *stream);
 
 /* dok_map_count_new for keys whose identity is the row, as the reference counts every key type (:363): distinct absent ROWS, by
  * value (float keys, where the value cast gives different rows one uuid; a row with a NaN counts each time). */
@@ -305,9 +316,9 @@ int dok_dok_assign(const dok_table *t, const dok_hash_params *hp, const dok_sele
                    const void *src, const int64_t *src_strides, int64_t *scratch, int64_t scratch_words, int64_t epoch,
                    int64_t *counters, int64_t *more, void *stream);
 
-/* dok_dok_assign for batches that dok_set_takes_sequence accepts, sequence as for dok_map_set_sequenced. */
-int dok_dok_assign_sequenced(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel, const void *src,
-                             const int64_t *src_strides, int64_t *sequence, int64_t *counters, int64_t *more, void *stream);
+/* dok_dok_assign for batches that dok_set_takes_numbers accepts, base as for dok_map_set_numbered. */
+int dok_dok_assign_numbered(const dok_table *t, const dok_hash_params *hp, const dok_selectors *sel, const void *src,
+                            const int64_t *src_strides, int64_t base, int64_t *counters, int64_t *more, void *stream);
 
 /* Value of every stored element to its position of a dense row-major tensor of the given sizes (HOST int64[key_size]; one
  * value element of 1, 2, 4 or 8 bytes), which the caller has zeroed.  Positions outside the sizes are left out.  Replaces

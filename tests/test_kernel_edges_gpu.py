@@ -88,7 +88,6 @@ def test_assignment_counts_repeated_new_positions(n):
 def test_sets_whose_values_carry_the_row(n, dtype):
     """Up to 4 bytes in 32-byte slots: the last row of a key stays, within a batch and across the point where the rows'
     numbers start over; tombstones are reused, and rows of a full table counted."""
-    from doksparse_b200.cuda_closed_hashmap import _SEQUENCE
     rng = np.random.default_rng(n)
     pair = Pair(seed=5, n_buckets=100000, rehash_threshold=1.0, **params(1))
     values = lambda k: rng.integers(-100, 100, (k, 1)).astype(dtype)
@@ -98,7 +97,7 @@ def test_sets_whose_values_carry_the_row(n, dtype):
         pair.get(np.arange(100000)[:, None] * 7919)
         if spread == 40000:
             pair.remove(keys[: n // 3])
-            pair.c._state[_SEQUENCE] = 0x7ffffff0 - n // 2        # the next set's numbers do not fit any more
+            pair.c._marks.numbered = 0x7ffffff0 - n // 2          # the next set's numbers do not fit any more
     full = np.arange(160000)[:, None] * 13 + 10 ** 12
     pair.c.set_rows(dev(np.concatenate([full, full[:5]])), dev(np.concatenate([values(160000)] + [values(5)])))
     stored = pair.c.get(dev(full))[1].cpu().numpy()

@@ -72,3 +72,107 @@ def test_a_rebuilt_map_and_a_clone_that_keeps_the_old_slots(kind, n):
         for c, o in ((a, oa), (b, ob)):
             _both_set(c, o, batch(), values(n))
             _same(c, o, everything)
+
+
+@pytest.mark.parametrize("kind", sorted(VALUES))
+@pytest.mark.parametrize("n", [700, 20000])
+def test_sets_of_different_keys_on_two_streams(kind, n):
+    """Each stream sets keys of its own, with repetitions, while the other does; after both, one set of all of them."""
+    cols = VALUES[kind][1]
+    table, oracle = _maps(n_buckets=1 << 18, key_size=1, **params(1))
+    rng = np.random.default_rng(n)
+    everything = np.arange(2 * n)[:, None]
+    _both_set(table, oracle, everything, np.zeros((2 * n, cols), np.float32))
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for _ in range(15):
+        rows = (n, n // 9)
+        batches = [[(rng.integers(0, n, (rows[s], 1)) + s * n, rng.standard_normal((rows[s], cols)).astype(np.float32)) for _ in range(3)] for s in range(2)]
+        on_device = [[(dev(k), dev(v)) for k, v in parts] for parts in batches]
+        torch.cuda.synchronize()
+        for stream in streams:
+            with torch.cuda.stream(stream):
+                torch.cuda._sleep(1 << 20)               # until all of the sets are queued
+        for k in range(3):
+            for s in range(2):
+                with torch.cuda.stream(streams[s]):
+                    table.set(*on_device[s][k])
+        torch.cuda.synchronize()
+        for parts in batches:
+            for k, v in parts:
+                oracle.set(k, v)
+        _same(table, oracle, everything)
+        _both_set(table, oracle, everything[::-1].copy(), rng.standard_normal((2 * n, cols)).astype(np.float32))
+        _same(table, oracle, everything)
+
+
+@pytest.mark.parametrize("n", [700, 20000])
+def test_row_numbers_start_over_while_another_stream_sets(n):
+    table, oracle = _maps(n_buckets=1 << 18, key_size=1, **params(1))
+    rng = np.random.default_rng(n)
+    everything = np.arange(2 * n)[:, None]
+    _both_set(table, oracle, everything, np.zeros((2 * n, 1), np.float32))
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for _ in range(4):
+        batches = [(rng.integers(0, n, (n, 1)) + s * n, rng.standard_normal((n, 1)).astype(np.float32)) for s in (0, 1, 0, 1)]
+        on_device = [(dev(k), dev(v)) for k, v in batches]
+        torch.cuda.synchronize()
+        table._marks.numbered = 0x7ffffff0 - 2 * n + 1           # room for one of the four
+        for i in range(4):
+            with torch.cuda.stream(streams[i % 2]):
+                table.set(*on_device[i])
+        assert table._marks.numbered == 3 * n
+        torch.cuda.synchronize()
+        for k, v in batches:
+            oracle.set(k, v)
+        _same(table, oracle, everything)
+
+
+@pytest.mark.parametrize("n", [700, 20000])
+@pytest.mark.parametrize("dtype", [np.float32, np.uint8])
+def test_replayed_sets_among_others(n, dtype):
+    """A set in a graph wins over what came before its replay and loses against what comes after it, whatever numbers the
+    slots hold, and reuses tombstones."""
+    table, oracle = _maps(n_buckets=1 << 19, key_size=1, **params(1))
+    rng = np.random.default_rng(n)
+    everything = np.arange(2 * n)[:, None]
+    batch = lambda m: (rng.integers(0, 2 * n, (m, 1)), rng.integers(0, 100, (m, 1)).astype(dtype))
+    _both_set(table, oracle, *batch(n))
+    keys, values = (dev(x) for x in batch(n))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        table.set(keys, values)
+    for i in range(6):
+        k, v = batch(n)
+        keys.copy_(dev(k))
+        values.copy_(dev(v))
+        graph.replay()
+        oracle.set(k, v)
+        _same(table, oracle, everything)
+        if i % 2:
+            _both_set(table, oracle, *batch(n // 3))
+        if i == 2:
+            table._marks.numbered = 0x7ffffff0                 # the next one starts the numbers over
+        gone = np.unique(rng.integers(0, 2 * n, n // 5))[:, None]
+        np.testing.assert_array_equal(host(table.remove(dev(gone))), oracle.remove(gone))
+        _same(table, oracle, everything)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_assignment_by_selectors_of_the_general_way(dtype):
+    """Lists, arrays, other integer types and values of another type or device, up to eight dims."""
+    from doksparse_b200 import SparseDOKTensor
+    shape = (3, 2, 4, 2, 3, 2, 2, 5)
+    np.random.seed(1)
+    t, dense = SparseDOKTensor(shape, dtype=dtype), torch.zeros(shape, device="cuda", dtype=dtype)
+    rng = np.random.default_rng(0)
+    for _ in range(3):
+        i, j = rng.integers(0, 3, 6), torch.from_numpy(rng.integers(0, 5, 6)).to(torch.int32)
+        picked = (i.tolist(), 1, slice(1, 3), 0, rng.integers(0, 3, 6), slice(None), 1, j)
+        at = tuple(torch.as_tensor(p).cuda().long() if isinstance(p, (list, np.ndarray, torch.Tensor)) else p for p in picked)
+        values = torch.randint(0, 100, tuple(t[at].shape))
+        t[picked] = values
+        for e in range(6):                                       # the last one of equal positions stays
+            one = tuple(p[e] if isinstance(p, torch.Tensor) else p for p in at)
+            dense[one] = values[e].to("cuda", dtype)
+        assert torch.equal(t.to_dense(), dense)
