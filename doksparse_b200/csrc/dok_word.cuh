@@ -129,7 +129,8 @@ __device__ __forceinline__ WordOutcome dok_write_word(const DevTable &t, const D
   o.met = found.outcome == DOK_OUT_FOUND && before > (ull_t)base;
   o.fresh = o.met ? found.word & DOK_WORD_FRESH : 0;
   if (o.claimed) keys.store_key(t, hp, e, dok_slot_ptr(t, found.slot));
-  if (found.outcome == DOK_OUT_FOUND && before < word >> DOK_WORD_SHIFT) atomicMax((ull_t *)dok_value_ptr(t, found.slot), word | o.fresh);
+  if (found.outcome == DOK_OUT_FOUND && before < word >> DOK_WORD_SHIFT)
+    o.met |= atomicMax((ull_t *)dok_value_ptr(t, found.slot), word | o.fresh) >> DOK_WORD_SHIFT > (ull_t)base;
   return o;
 }
 

@@ -176,3 +176,18 @@ def test_assignment_by_selectors_of_the_general_way(dtype):
             one = tuple(p[e] if isinstance(p, torch.Tensor) else p for p in at)
             dense[one] = values[e].to("cuda", dtype)
         assert torch.equal(t.to_dense(), dense)
+
+
+@pytest.mark.parametrize("kind", sorted(VALUES))
+@pytest.mark.parametrize("n", [700, 8193, 70000])
+@pytest.mark.parametrize("distinct", [1, 3, 300])
+def test_rows_that_lost_to_a_later_one_are_counted(kind, n, distinct):
+    from doksparse_b200._lib import CNT_DUPLICATES
+    table, _ = _maps(n_buckets=1 << 18, key_size=1, **params(1))
+    rng = np.random.default_rng(n)
+    cols = VALUES[kind][1]
+    for _ in range(3):                                           # new keys, then stored ones
+        keys = rng.integers(0, distinct, (n, 1)) * 7919
+        before = int(table._state[CNT_DUPLICATES])
+        table.set(dev(keys), torch.zeros(n, cols, device="cuda"))
+        assert int(table._state[CNT_DUPLICATES]) - before == n - len(np.unique(keys))
