@@ -19,6 +19,7 @@ MAX_SHARDS = 64
 N_COUNTERS = 8
 MAX_EPOCH = (1 << 30) - 1
 MAX_BATCH = (1 << 32) - 1
+UNLISTED = 1 << 62
 CNT_CLAIMED_EMPTY, CNT_REUSED_REMOVED, CNT_FAILED, CNT_HITS, CNT_DUPLICATES, CNT_PROBES = range(6)
 
 DTYPE_CODES = {

@@ -305,11 +305,11 @@ class CudaClosedHashmap:
             device, self._n_buckets, self._key_shape, key_dtype, self._value_shape, value_dtype, self._counters_of_table)
         self._layout = _Layout(*layout)
 
-    def _begin_bulk_insert(self, key_shape, key_dtype, value_shape, value_dtype, n_new):
+    def _begin_bulk_insert(self, key_shape, key_dtype, value_shape, value_dtype, n_new, spare=()):
         """What `set` does to a never-used map before its kernel runs, for a batch known to hold `n_new` pairwise
         different new keys: allocate, draw the parameters, grow if the reference's trigger fires (which re-draws them,
         cuda_closed_hashmap.py:365-366, 456-468).  The caller then inserts the rows with a kernel that counts into
-        `_counter_block(_BY_BULK)`."""
+        `_counter_block(_BY_BULK)`.  `spare`: a list of memory that is dropped where there is no room beside it."""
         assert self._slots is None
         if n_new == 0:
             self._allocate(key_shape, key_dtype, value_shape, value_dtype)
@@ -320,7 +320,14 @@ class CudaClosedHashmap:
             self.__init__(n_buckets=int(n_new * self._rehash_factor), device=self.device, key_perm=self._key_perm,
                           rehash_factor=self._rehash_factor, rehash_threshold=self._rehash_threshold,
                           tombstone_threshold=self._tombstone_threshold)
-        self._allocate(key_shape, key_dtype, value_shape, value_dtype)
+        try:
+            self._allocate(key_shape, key_dtype, value_shape, value_dtype)
+        except torch.OutOfMemoryError:
+            if not spare:
+                raise
+            spare.clear()
+        if self._slots is None:
+            self._allocate(key_shape, key_dtype, value_shape, value_dtype)
         self._materialise_parameters()
         self._shared.exact(n_new)
 

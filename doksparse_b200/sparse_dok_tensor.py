@@ -84,7 +84,8 @@ class SparseDOKTensor(object):
     def from_dense(cls, tensor):
         """Same result as the reference's `from_sparse_coo(tensor.to_sparse())` (sparse_dok_tensor.py:86-90): a map of
         next_power_of_2(nnz) buckets (grown like `set` would grow it) holding every non-zero element.  The pass that
-        counts them keeps their positions and values, up to an eighth of the tensor; a tensor with more is scanned again.
+        counts them keeps their positions and values, up to an eighth of the tensor; a tensor with more is scanned again, and
+        so is one whose table has no room beside the list.
         No COO index tensor is built."""
         assert isinstance(tensor, Tensor)
         assert tensor.layout == torch.strided
@@ -96,30 +97,33 @@ class SparseDOKTensor(object):
         device = dense.device
         es = dense.element_size()
         is_float = int(dense.dtype.is_floating_point)
-        numel, kept, room = dense.numel(), None, 0
+        numel, room, kept = dense.numel(), 0, []
         if 0 < numel < 1 << 32 and dense.data_ptr() % 16 == 0 and es in (1, 2, 4, 8):
             room = (max(numel // 8, min(numel, 1 << 16)) + 1) // 2 * 2
             try:
-                kept = torch.empty(room * (4 + es), device=device, dtype=torch.uint8)
+                kept.append(torch.empty(room * (4 + es), device=device, dtype=torch.uint8))
             except torch.OutOfMemoryError:
-                kept, room = None, 0
+                pass
         with L.on(device):
             st = L.stream_ptr(device)
-            count = torch.zeros(1, device=device, dtype=torch.long)
-            if kept is not None:
-                L.check(lib.dok_dense_collect_nonzero(L.ptr(dense), numel, es, is_float, L.ptr(kept), room, L.ptr(count), st),
+            count = (torch.empty if kept else torch.zeros)(1, device=device, dtype=torch.long)
+            if kept:
+                L.check(lib.dok_dense_collect_nonzero(L.ptr(dense), numel, es, is_float, L.ptr(kept[0]), room, L.ptr(count), st),
                         "dok_dense_collect_nonzero")
             else:
                 L.check(lib.dok_dense_count_nonzero(L.ptr(dense), numel, es, is_float, L.ptr(count), st), "dok_dense_count_nonzero")
             nnz = int(count.item())
+        if nnz > room:                                   # more than the list holds, or (L.UNLISTED) not listed at all
+            kept.clear()
+            nnz %= L.UNLISTED
         hashmap = CudaClosedHashmap(n_buckets=next_power_of_2(nnz), device=device)
         new = cls(size=tuple(dense.shape), dtype=dense.dtype, storage=hashmap)
-        hashmap._begin_bulk_insert((dense.ndim,), torch.long, (1,), dense.dtype, nnz)
+        hashmap._begin_bulk_insert((dense.ndim,), torch.long, (1,), dense.dtype, nnz, spare=kept)
         if nnz:
             sizes = (ctypes.c_int64 * dense.ndim)(*dense.shape)
             with L.on(device):
-                if nnz <= room:
-                    L.check(lib.dok_dense_insert_list(hashmap._c_table(), hashmap._c_hash(), L.ptr(kept), room, nnz, sizes,
+                if kept:
+                    L.check(lib.dok_dense_insert_list(hashmap._c_table(), hashmap._c_hash(), L.ptr(kept[0]), room, nnz, sizes,
                                                       hashmap._counter_block(M._BY_BULK), L.stream_ptr(device)),
                             "dok_dense_insert_list")
                 else:

@@ -345,9 +345,11 @@ int dok_dok_gather_insert(const dok_table *src, const dok_hash_params *src_hp, c
  * sizes[ndim] is the dense shape, ndim = hp->key_size, keys are int64. */
 int dok_dense_count_nonzero(const void *dense, int64_t numel, int elem_bytes, int is_float, int64_t *count_out,
                             void *stream);
-/* The count that also lists what it finds (numel < 2^32, dense 16-byte aligned): *count_out grows by the number of
+/* The count that also lists what it finds (numel < 2^32, dense 16-byte aligned): *count_out becomes the number of
  * non-zeros, and the first `capacity` (even) of them, in no particular order, go to list: uint32 positions[capacity], then
- * elements[capacity].  If all of them fit, dok_dense_insert_list inserts n of them in place of step 2. */
+ * elements[capacity].  Where a sample shows more than the list would hold nothing is listed, and *count_out is that number +
+ * DOK_UNLISTED.  If all are listed, dok_dense_insert_list inserts them in place of step 2. */
+#define DOK_UNLISTED (1LL << 62)
 int dok_dense_collect_nonzero(const void *dense, int64_t numel, int elem_bytes, int is_float, void *list, int64_t capacity,
                               int64_t *count_out, void *stream);
 int dok_dense_insert_list(const dok_table *t, const dok_hash_params *hp, const void *list, int64_t capacity, int64_t n,

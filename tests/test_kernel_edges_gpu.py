@@ -390,3 +390,56 @@ def test_lookups_into_outputs_that_are_only_8_byte_aligned(value_cols, offset):
     values = torch.empty(n * value_cols + offset, device="cuda")[offset:].reshape(n, value_cols)
     out, found = table.get(keys, values=values)
     assert found.all() and torch.equal(out, stored) and out.data_ptr() == values.data_ptr()
+
+
+def _looked_at(numel, elem_bytes):
+    """Positions of the sample that decides whether the non-zeros of a dense tensor are listed."""
+    each, piece = 16 // elem_bytes, np.arange(1024, dtype=np.uint64)
+    spacing = np.uint64(numel // each // 1024)
+    first = piece * spacing + (spacing * (piece * np.uint64(0x9e3779b1) % np.uint64(1 << 32)) >> np.uint64(32))
+    return (first[:, None].astype(np.int64) * each + np.arange(each)).ravel()
+
+
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.float16, torch.float32, torch.float64])
+@pytest.mark.parametrize("numel", [70001, (1 << 20) + 3, 1 << 22])
+@pytest.mark.parametrize("kind", ["only there", "all but there", "full", "none", "second half"])
+def test_dense_tensors_whose_sample_misleads(dtype, numel, kind):
+    from doksparse_b200 import SparseDOKTensor
+    np.random.seed(2)
+    there = torch.zeros(numel, dtype=torch.bool, device="cuda")
+    there[dev(_looked_at(numel, dtype.itemsize))] = True
+    at = torch.arange(numel, device="cuda")
+    nonzero = {"only there": there, "all but there": ~there & (at % 7 == 0), "full": at >= 0, "none": at < 0, "second half": at >= numel // 2}[kind]
+    dense = torch.where(nonzero, at % 100 + 1, 0).to(dtype)
+    t = SparseDOKTensor.from_dense(dense)
+    assert t._nnz() == int(nonzero.sum()) and torch.equal(t.to_dense(), dense)
+
+
+@pytest.mark.parametrize("density", [0.01, 0.3, 1.0])
+def test_memory_of_a_dense_tensors_conversion(density, monkeypatch):
+    """No list beside a table that needs the room: above an eighth of non-zeros there is none, and below it is dropped."""
+    from doksparse_b200 import CudaClosedHashmap, SparseDOKTensor
+    numel = 1 << 24
+    dense = (torch.rand(numel + 1, device="cuda") < density).float()
+    peaks = []
+    for start in (1, 0):                                         # off a 16-byte boundary: without a list
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        SparseDOKTensor.from_dense(dense[start:start + numel])
+        peaks.append(torch.cuda.max_memory_allocated() - before)
+    assert peaks[1] <= peaks[0] + (numel + 4096 if density < 0.125 else 4096)
+    allocate, calls = CudaClosedHashmap._allocate, []
+
+    def short_of_memory(self, *args):
+        calls.append(torch.cuda.memory_allocated())
+        if len(calls) == 1:
+            raise torch.OutOfMemoryError("no room beside the list")
+        return allocate(self, *args)
+
+    monkeypatch.setattr(CudaClosedHashmap, "_allocate", short_of_memory)
+    if density < 0.125:
+        t = SparseDOKTensor.from_dense(dense[:numel])
+        assert torch.equal(t.to_dense(), dense[:numel]) and calls[0] - calls[1] >= numel
+    else:
+        with pytest.raises(torch.OutOfMemoryError):
+            SparseDOKTensor.from_dense(dense[:numel])
