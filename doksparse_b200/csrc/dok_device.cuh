@@ -166,13 +166,14 @@ __device__ __forceinline__ bool dok_next_group(Index &group, unsigned &word, Ind
 // with 2 slots per group 2.6 of them.  Most full groups hold just the keys that start there, so each group remembers whether a
 // key was ever placed behind it: in the highest bit of its first slot's value word, where values of at most 7 bytes leave
 // padding and where a lookup has it in a register already.  Insertion sets it, and nothing clears it but a new table; a walk
-// that looks for a place ignores it.  8.4 M lookups of a 4-D selection, nearly all misses: 587 -> 402 us; 4 M lookups at load
+// that looks for a place ignores it.  A key that was found is marked too: a key of the same uuid whose hash differs has been
+// placed from another start (alpha2 = 0 in a column), and a lookup has to get past the groups that this walk went past.  8.4 M lookups of a 4-D selection, nearly all misses: 587 -> 402 us; 4 M lookups at load
 // 0.8, 30 % hits: 335 -> 210; filling that table with 50 M rows: 8.3 -> 8.9 ms.  With 4 slots per group fewer keys go past
 // one: at load 0.36 4 M lookups went from 140 to 127 us, but a table that grows to 300 k rows from 880 to 910 and a dense
 // tensor's conversion from 348 to 359 (398 where the bit is written without a look), so those stay without.
 #define DOK_PASSED 0x8000000000000000ULL
 __host__ __device__ __forceinline__ bool dok_has_passed_bits(const DevTable &t) { return t.vb < 8 && t.spg <= 2; }
-// a key was placed in `slot`: marks the groups before it on its chain
+// a key was placed or found in `slot`: marks the groups before it on its chain
 __device__ __forceinline__ void dok_mark_passed(const DevTable &t, const ChainKey &kh, ll_t slot) {
   if (!dok_has_passed_bits(t)) return;
   const unsigned placed = (unsigned)slot / (unsigned)t.spg, n_groups = (unsigned)t.n_groups;
@@ -723,12 +724,12 @@ __device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHa
           const ll_t old = dok_cas_tag(t, slot, expect, key.uuid);
           if (old == expect) {
             *outcome = expect == DOK_EMPTY ? DOK_OUT_CLAIMED_EMPTY : DOK_OUT_REUSED;
-            if constexpr (SB >= 64) dok_mark_passed(t, kh, slot);
           } else {
             active = old != key.uuid;
           }
         }
       }
+      if constexpr (SB >= 64) if (!active && slot >= 0) dok_mark_passed(t, kh, slot);
     }
   } while (__any_sync(0xffffffffu, active));
   return slot;

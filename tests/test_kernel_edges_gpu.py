@@ -63,6 +63,31 @@ def test_lookups_end_at_groups_that_no_key_went_past(n_buckets, key_size, dtype,
     pair.get(everything)
 
 
+@pytest.mark.parametrize("n_buckets", [40, 120, 250, 1000])
+@pytest.mark.parametrize("key_size", [3, 7])                                   # 2 and 1 slots per group
+@pytest.mark.parametrize("unique", [False, True])
+def test_keys_of_one_uuid_that_start_in_different_groups(n_buckets, key_size, unique):
+    """A column that the uuid does not depend on: a set finds the slot that another key made, and lookups have to as well."""
+    from doksparse_b200 import CudaClosedHashmap
+    long = lambda v: [v[j % 3] + 2 * (j // 3) for j in range(key_size)]
+    drawn = {k: long(v) for k, v in params(3).items()}
+    drawn["alpha2"][-1] = 0
+    most, joined = 17 * n_buckets // 20, 0
+    for first in range(0, 10 * n_buckets, n_buckets):
+        table = CudaClosedHashmap(n_buckets=n_buckets, key_size=key_size, rehash_threshold=2.0, tombstone_threshold=None, **drawn)
+        keys = (first + torch.arange(most, device="cuda"))[:, None] * torch.arange(3, 3 + key_size, device="cuda")
+        table.set(keys, torch.zeros(most, 1, device="cuda"), assume_unique=unique)
+        others = keys.clone()
+        others[:, -1] += 1
+        others = others[:n_buckets // 10]
+        values = 1 + torch.arange(len(others), device="cuda", dtype=torch.float32)[:, None]
+        table.set(others, values, assume_unique=unique)
+        joined += most + len(others) - table.n_elements
+        stored, found = table.get(others)
+        assert found.all() and torch.equal(stored, values) and table.remove_rows(others).all()
+    assert joined > 0
+
+
 @pytest.mark.parametrize("n", [1, 31, 300, 5000, 70000])
 def test_assignment_counts_repeated_new_positions(n):
     """n_elements grows by every selected position that was not stored, repetitions included; the last one's value stays."""
