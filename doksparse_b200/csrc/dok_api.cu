@@ -703,7 +703,7 @@ int dok_dense_insert_list(const dok_table *t, const dok_hash_params *hp, const v
   const RowValues values{(const char *)list + 4 * capacity};
   const unsigned grid = (unsigned)((n + DOK_TPB - 1) / DOK_TPB);
   int rc = DOK_OK;
-  DOK_DISPATCH_SB(dt, DOK_FOR_WINDOWS(dt, rc, (k_set_unique<SB><<<grid, DOK_TPB, 0, (cudaStream_t)stream>>>(wt, dh, keys, values, (uint8_t *)nullptr, (ll_t *)counters))));
+  DOK_DISPATCH_MARKS(dt, DOK_FOR_WINDOWS(dt, rc, (k_set_unique<SB, MARKS><<<grid, DOK_TPB, 0, (cudaStream_t)stream>>>(wt, dh, keys, values, (uint8_t *)nullptr, (ll_t *)counters))));
   return rc;
 }
 

@@ -167,20 +167,24 @@ __device__ __forceinline__ bool dok_next_group(Index &group, unsigned &word, Ind
 // key was ever placed behind it: in the highest bit of its first slot's value word, where values of at most 7 bytes leave
 // padding and where a lookup has it in a register already.  Insertion sets it, and nothing clears it but a new table; a walk
 // that looks for a place ignores it.  A key that was found is marked too: a key of the same uuid whose hash differs has been
-// placed from another start (alpha2 = 0 in a column), and a lookup has to get past the groups that this walk went past.  8.4 M lookups of a 4-D selection, nearly all misses: 587 -> 402 us; 4 M lookups at load
-// 0.8, 30 % hits: 335 -> 210; filling that table with 50 M rows: 8.3 -> 8.9 ms.  With 4 slots per group fewer keys go past
-// one: at load 0.36 4 M lookups went from 140 to 127 us, but a table that grows to 300 k rows from 880 to 910 and a dense
-// tensor's conversion from 348 to 359 (398 where the bit is written without a look), so those stay without.
+// placed from another start (alpha2 = 0 in a column), and a lookup has to get past the groups that this walk went past.
+// 8.4 M lookups of a 4-D selection, nearly all misses: 587 -> 402 us; 4 M lookups at load 0.8, 30 % hits: 335 -> 210.  What it
+// costs: filling a 4-D tensor with 50 M rows 8.02 -> 8.29 ms (8.63 where the groups are read again for their marks), a table of
+// 2 slots per group up to load 0.8 1.60 -> 1.69, of one 2.53 -> 2.71; general sets of stored keys 2 to 3 %.  With 4 slots per
+// group fewer keys go past one: at load 0.36 4 M lookups went from 140 to 127 us, but a table that grows to 300 k rows from 880
+// to 910 and a dense tensor's conversion from 348 to 359 (398 where the bit is written without a look), so those stay without.
 #define DOK_PASSED 0x8000000000000000ULL
 __host__ __device__ __forceinline__ bool dok_has_passed_bits(const DevTable &t) { return t.vb < 8 && t.spg <= 2; }
-// a key was placed or found in `slot`: marks the groups before it on its chain
-__device__ __forceinline__ void dok_mark_passed(const DevTable &t, const ChainKey &kh, ll_t slot) {
+// a key was placed or found in `slot`: marks the groups before it on its chain that the walk saw without the mark (bit k of
+// `missing`: the chain's group k; 31: some group from there on)
+__device__ __forceinline__ void dok_mark_passed(const DevTable &t, const ChainKey &kh, ll_t slot, unsigned missing) {
   if (!dok_has_passed_bits(t)) return;
   const unsigned placed = (unsigned)slot / (unsigned)t.spg, n_groups = (unsigned)t.n_groups;
   unsigned group = (unsigned)dok_start_group(kh, t), word = dok_chain_word(kh, t);
   while (group != placed) {
+    const unsigned step = min(word >> 6, 31u);
     ull_t *first = (ull_t *)(t.slots + (ull_t)group * 128u + 8u);       // (no slot with such a value is wider than a line)
-    if (!(__ldcg(first) & DOK_PASSED)) atomicOr(first, DOK_PASSED);
+    if (((missing >> step) & 1u) && (step < 31 || !(__ldcg(first) & DOK_PASSED))) atomicOr(first, DOK_PASSED);
     if (!dok_next_group<unsigned>(group, word, n_groups)) break;
   }
 }
@@ -433,7 +437,7 @@ __device__ __forceinline__ Located dok_locate_serial(const DevTable &t, const Ke
 // No-op hit handler for walks that only need the slot.
 template <bool FEW>
 struct NoEmit {
-  static constexpr bool L1 = false, ENDS = false, WORD = false, BOTH = FEW;
+  static constexpr bool L1 = false, ENDS = false, WORD = false, BOTH = FEW, MARKS = false;
   template <int LW>
   __device__ __forceinline__ void operator()(ll_t, int, const ull_t (&)[LW]) const {}
 };
@@ -448,7 +452,7 @@ __device__ __forceinline__ ulonglong2 dok_load_pair(const char *slot) {
 // A lookup that only needs the slot.
 template <bool FEW>
 struct Probe {
-  static constexpr bool L1 = true, ENDS = false, WORD = false, BOTH = FEW;
+  static constexpr bool L1 = true, ENDS = false, WORD = false, BOTH = FEW, MARKS = false;
   template <int LW>
   __device__ __forceinline__ void operator()(ll_t, int, const ull_t (&)[LW]) const {}
 };
@@ -456,7 +460,15 @@ struct Probe {
 // A walk whose owner lanes get the value word of the slot that was found, or of the empty one (of 32-byte slots).
 template <bool FEW>
 struct NeedsWord {
-  static constexpr bool L1 = false, ENDS = false, WORD = true, BOTH = FEW;
+  static constexpr bool L1 = false, ENDS = false, WORD = true, BOTH = FEW, MARKS = false;
+  template <int LW>
+  __device__ __forceinline__ void operator()(ll_t, int, const ull_t (&)[LW]) const {}
+};
+
+// A walk of 64- or 128-byte slots that ends with dok_mark_passed: Located::word has its `missing`.  Lane 1 of the quad, whose part of the line has no tag, reads the word with the mark.
+template <bool FEW>
+struct Marks {
+  static constexpr bool L1 = false, ENDS = false, WORD = false, BOTH = FEW, MARKS = true;
   template <int LW>
   __device__ __forceinline__ void operator()(ll_t, int, const ull_t (&)[LW]) const {}
 };
@@ -513,7 +525,9 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
   const unsigned my_slot = (32u * l) / SB;            // slot (within the group) the chunk belongs to
   const ll_t e_quad = e - l;                          // batch element of the quad's first lane (elements are consecutive)
   const unsigned n_groups = (unsigned)t.n_groups;     // < 2^32 (checked on the host)
-  const char *my_base = t.slots + 32 * l;
+  static_assert(!Emit::MARKS || (SB >= 64 && LW == 1));
+  const char *my_base = t.slots + (Emit::MARKS && l == 1 ? 8 : 32 * l);
+  constexpr unsigned SLOTS = Emit::MARKS ? (1u << SPG) - 1u : 0xfu, UNMARKED = 8u;
   ull_t word_of = 0;
   // results as 32-bit group-relative codes until the end: slot = group * SPG + position
   unsigned found = NONE, empty = NONE, tomb = NONE;
@@ -529,7 +543,8 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
   // what the owner lane does with the outcome of one inspected group: m / me / tb = match, match-or-empty and
   // tombstone bits by slot
   auto advance = [&](unsigned m, unsigned me, unsigned tb) {
-    const int pos = me ? __ffs(me) - 1 : -1;
+    const int pos = (me & SLOTS) ? __ffs(me & SLOTS) - 1 : -1;
+    if (Emit::MARKS && pos < 0 && (m & UNMARKED)) word_of |= 1u << min(word >> 6, 31u);
     const unsigned first_slot = group * SPG;
     if (probes) walked++;
     if (TOMB && tomb == NONE) {
@@ -563,6 +578,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
         if constexpr (Emit::ENDS) bits |= ends(w[r]) << (8u * r);
         if (TOMB) tbits |= (unsigned)(tag == DOK_REMOVED) << (4u * r + my_slot);
       }
+      if constexpr (Emit::MARKS) if (l == 1 && g[r] != NONE && !(w[r][0] & DOK_PASSED)) bits |= UNMARKED << (8u * r);
     }
     bits |= __shfl_xor_sync(FULL, bits, 1);
     bits |= __shfl_xor_sync(FULL, bits, 2);
@@ -605,6 +621,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
     unsigned bits = ((unsigned)(tag == uuid_r) | ((unsigned)(tag == DOK_EMPTY) << 4) |
                      (TOMB ? (unsigned)(tag == DOK_REMOVED) << 8 : 0u)) << my_slot;
     if constexpr (Emit::ENDS) if (g_r != NONE) bits |= ends(wl);
+    if constexpr (Emit::MARKS) if (l == 1 && g_r != NONE && !(wl[0] & DOK_PASSED)) bits |= UNMARKED;
     bits |= __shfl_xor_sync(FULL, bits, 1);
     bits |= __shfl_xor_sync(FULL, bits, 2);
     const unsigned m = bits & 0xfu, me = (bits | (bits >> 4)) & 0xfu;
@@ -650,7 +667,7 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
 // most 8 bytes, one word behind the tag, LW = 4 the whole of a 32-byte slot.
 template <int SB, int LW, bool PASSED>
 struct EmitValue {
-  static constexpr bool L1 = true, ENDS = PASSED, WORD = false, BOTH = false;
+  static constexpr bool L1 = true, ENDS = PASSED, WORD = false, BOTH = false, MARKS = false;
   const DevTable &t;
   char *out_values;
   __device__ __forceinline__ void operator()(ll_t e_r, int pos, const ull_t (&w)[LW]) const {
@@ -703,14 +720,12 @@ enum { DOK_OUT_FOUND = 0, DOK_OUT_CLAIMED_EMPTY = 1, DOK_OUT_REUSED = 2, DOK_OUT
 // so each lost CAS is a slot taken.  In a table that fills up that is no exception -- the rows that are on their way at a time
 // see the same first places -- and a lane that went on by itself, slot by slot, held its warp up: sets of a fifth new rows,
 // 300 k rows of 32-byte slots 60 -> 54 us, 1 M 113 -> 107, 30 k rows of 64-byte slots 59 -> 48.  Every lane of the warp must call.
-template <int SB, bool FEW = false>
-__device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHash &key, bool active, int *outcome) {
-  // (mixed once where the walk is followed by dok_mark_passed; kept in registers elsewhere it cost an insert of 32-byte slots
-  // a fifth)
-  const auto kh = [&] { if constexpr (SB >= 64) return dok_chain(key, t); else return key; }();
+// MARKS: the table may be one with marks.
+template <int SB, bool FEW = false, bool MARKS = (SB >= 64)>
+__device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHash &kh, bool active, int *outcome) {
   ll_t slot = -1;
   do {
-    const Located loc = dok_locate<SB, 1, true>(t, kh, 0, active, nullptr, NoEmit<FEW>());   // the tags are all a claim needs
+    const Located loc = dok_locate<SB, 1, true>(t, kh, 0, active, nullptr, std::conditional_t<MARKS, Marks<FEW>, NoEmit<FEW>>());
     if (active) {
       active = false;
       slot = loc.found;
@@ -721,15 +736,15 @@ __device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHa
         if (slot < 0) {
           *outcome = DOK_OUT_FAILED;                     // no match, no tombstone, no empty slot: the table is full
         } else {
-          const ll_t old = dok_cas_tag(t, slot, expect, key.uuid);
+          const ll_t old = dok_cas_tag(t, slot, expect, kh.uuid);
           if (old == expect) {
             *outcome = expect == DOK_EMPTY ? DOK_OUT_CLAIMED_EMPTY : DOK_OUT_REUSED;
           } else {
-            active = old != key.uuid;
+            active = old != kh.uuid;
           }
         }
       }
-      if constexpr (SB >= 64) if (!active && slot >= 0) dok_mark_passed(t, kh, slot);
+      if constexpr (MARKS) if (loc.word && !active && slot >= 0) dok_mark_passed(t, dok_chain(kh, t), slot, (unsigned)loc.word);
     }
   } while (__any_sync(0xffffffffu, active));
   return slot;

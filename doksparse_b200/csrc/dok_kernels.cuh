@@ -147,6 +147,11 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, De
     default: { constexpr int SB = 0; CALL; break; }     \
   }
 
+// ... with MARKS (dok_find_or_claim): a walk that looks for them takes 2 % longer
+#define DOK_DISPATCH_MARKS(t, CALL)                                                            \
+  if (dok_has_passed_bits(t)) DOK_DISPATCH_SB(t, { constexpr bool MARKS = SB >= 64; CALL; })   \
+  else DOK_DISPATCH_SB(t, { constexpr bool MARKS = false; CALL; })
+
 // launch grid of a batch: one thread per row; sliced batches put the slice in gridDim.y
 inline dim3 dok_grid(const RowKeys &k) {
   if (k.slice_rows == 0) return dim3((unsigned)((k.n + DOK_TPB - 1) / DOK_TPB));
@@ -244,8 +249,8 @@ __device__ __forceinline__ void dok_write_row(const DevTable &t, const DevHash &
 }
 
 // One kernel, for batches whose rows have pairwise different uuids.
-template <int SB, class Keys, class Values>
-__global__ void __launch_bounds__(DOK_TPB, 4) k_set_unique(DevTable t, DevHash hp, Keys keys, Values values,
+template <int SB, bool MARKS, class Keys, class Values>
+__global__ void __launch_bounds__(DOK_TPB, 6) k_set_unique(DevTable t, DevHash hp, Keys keys, Values values,
                                                         uint8_t *__restrict__ out_stored, ll_t *counters) {
   __shared__ BlockTally tally;
   if (keys.idle()) return;
@@ -256,7 +261,7 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_set_unique(DevTable t, DevHash h
   if (active) kh = keys.hash(hp, e);
   active = dok_in_window(t, kh, active);
   int outcome = -1;
-  const ll_t slot = dok_find_or_claim<SB>(t, kh, active, &outcome);
+  const ll_t slot = dok_find_or_claim<SB, false, MARKS>(t, kh, active, &outcome);
   if (active) {
     if (slot >= 0) dok_write_row(t, hp, keys, values, e, slot, outcome != DOK_OUT_FOUND || hp.dtype >= DOK_F16);
     if (out_stored) out_stored[e] = (uint8_t)(slot >= 0);
@@ -355,8 +360,8 @@ __device__ __forceinline__ Twins dok_find_twins(BlockTwins &b, const KeyHash &kh
 // for a batch without equal uuids that is all there is to do.  A row that finds the slot already stamped in
 // this epoch sets the conflict bit and counts a duplicate (in slot_out[n], zeroed by the host before the
 // launch); the second kernel then lets the slot's last row rewrite it.
-template <int SB, bool FEW, class Keys, class Values>
-__global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp, Keys keys, Values values,
+template <int SB, bool FEW, bool MARKS, class Keys, class Values>
+__global__ void __launch_bounds__(DOK_TPB, FEW ? 4 : 6) k_set_claim(DevTable t, DevHash hp, Keys keys, Values values,
                                                        ll_t *__restrict__ slot_out, unsigned *filter, ll_t epoch, int mark_fresh,
                                                        uint8_t *__restrict__ out_stored, ll_t *counters) {
   __shared__ BlockTally tally;
@@ -377,7 +382,7 @@ __global__ void __launch_bounds__(DOK_TPB, 6) k_set_claim(DevTable t, DevHash hp
   const Twins same = dok_find_twins(twins, kh, active, any_twins);
   const bool last = active && same.last == (int)threadIdx.x;
   int outcome = -1, conflict = 0, dup = 0;
-  ll_t slot = dok_find_or_claim<SB, FEW>(t, kh, last, &outcome);
+  ll_t slot = dok_find_or_claim<SB, FEW, MARKS>(t, kh, last, &outcome);
   if (last) {
     const bool fresh = outcome == DOK_OUT_CLAIMED_EMPTY || outcome == DOK_OUT_REUSED;
     slot_out[e] = mark_fresh && fresh ? slot | DOK_ROW_FRESH : slot;
@@ -592,7 +597,7 @@ inline int launch_set_general(const DevTable &t, const DevHash &hp, const Keys &
   if (cudaMemsetAsync(slot_scratch + keys.n, 0, zeroed, st) != cudaSuccess) return dok_check_launch();
   const dim3 grid = dok_grid(keys);
   int rc = DOK_OK;
-  DOK_DISPATCH_SB(t, DOK_BY_SIZE(grid.x * grid.y, DOK_FOR_WINDOWS(t, rc, (k_set_claim<SB, FEW><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, (ll_t *)slot_scratch, filter,
+  DOK_DISPATCH_MARKS(t, DOK_BY_SIZE(grid.x * grid.y, DOK_FOR_WINDOWS(t, rc, (k_set_claim<SB, FEW, MARKS><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, values, (ll_t *)slot_scratch, filter,
                                                                                        (ll_t)epoch, more != nullptr, out_stored, (ll_t *)counters)))));
   if (rc != DOK_OK) return rc;
   dim3 few = grid;
@@ -614,7 +619,7 @@ inline int launch_set_unique(const DevTable &t, const DevHash &hp, const RowKeys
   RowValues rv{values};
   const dim3 grid = dok_grid(keys);
   int rc = DOK_OK;
-  DOK_DISPATCH_SB(t, DOK_FOR_WINDOWS(t, rc, (k_set_unique<SB><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, rv, out_stored, (ll_t *)counters))));
+  DOK_DISPATCH_MARKS(t, DOK_FOR_WINDOWS(t, rc, (k_set_unique<SB, MARKS><<<grid, DOK_TPB, 0, st>>>(wt, hp, keys, rv, out_stored, (ll_t *)counters))));
   return rc;
 }
 
