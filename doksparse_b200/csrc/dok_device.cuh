@@ -664,15 +664,27 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
 
 // Hit handler of `get` (PASSED: of a table whose groups remember that a key went past them): the lane that holds the slot
 // writes the value straight from its registers, so a hit needs no second access to the table.  LW = 2 serves values of at
-// most 8 bytes, one word behind the tag, LW = 4 the whole of a 32-byte slot.
+// most 8 bytes, one word behind the tag, LW = 4 whole slots, each lane of the quad with its part of the value.
 template <int SB, int LW, bool PASSED>
 struct EmitValue {
   static constexpr bool L1 = true, ENDS = PASSED, WORD = false, BOTH = false, MARKS = false;
   const DevTable &t;
   char *out_values;
   __device__ __forceinline__ void operator()(ll_t e_r, int pos, const ull_t (&w)[LW]) const {
-    if ((int)(threadIdx.x & 3u) != pos * (SB / 32)) return;
     char *dst = out_values + e_r * (ll_t)t.vb;
+    if constexpr (LW == 4 && SB != 32) {
+      const int start = pos * SB + 8 - 32 * (int)(threadIdx.x & 3u);      // of the value, from this lane's part of the line
+      const int align = (t.vb & 7) ? t.vb & -t.vb : 8;
+#pragma unroll
+      for (int j = 0; j < LW; j++) {
+        const int at = 8 * j - start;
+        if ((unsigned)at >= (unsigned)t.vb) continue;
+        if (align == 8) *(ull_t *)(dst + at) = w[j];
+        else dok_store_word(dst + at, w[j], t.vb - at < 8 ? t.vb - at : 8, align);
+      }
+      return;
+    }
+    if ((int)(threadIdx.x & 3u) != pos * (SB / 32)) return;
     if constexpr (LW == 2) {
       if (t.vb == 8) *(ull_t *)dst = w[1];
       else dok_store_word(dst, w[1], t.vb, (t.vb & -t.vb));

@@ -16,12 +16,12 @@
 // get
 // ---------------------------------------------------------------------------------------------------------
 // One row per thread: for 32-byte slots with values of at most 8 bytes, whose walk fits 32 registers, so that 64 warps are
-// resident (8.4 M lookups at load 0.6: 251 us; the form below, with half the instructions but 32 warps: 291), for wider
-// values of all other slots, and for batches that dok_get_by_rows names.
+// resident (8.4 M lookups at load 0.6: 251 us; the form below, with half the instructions but 32 warps: 291), for slots wider
+// than a line, and for batches that dok_get_by_rows names.
 // For values of more than 8 bytes the walk reads the tags alone, so that 64 warps are resident here too, and the row's own
 // lane reads the value where it was found -- from L1, as its sector has just come in, and further sectors of the line from
-// L2.  Against whole lines in the registers of 24 warps: 40-byte values, 8 M lookups at load 0.6 499 -> 443 us, 1 M 69 -> 52,
-// 300 k 52 -> 36; 16-byte values, 200 k 24 -> 18, 3000 15 -> 11.  (8 M of those in 32-byte slots: 290 -> 326, so they stay below.)
+// L2.  Against whole lines in the registers of 24 warps: 40-byte values, 300 k lookups of a 64 MB table 33 -> 25 us, 8 M
+// 323 -> 291; 16-byte values, 200 k 24 -> 18, 3000 15 -> 11.
 // Lines through cp.async and shared memory, 40 warps: 445, 62 and 50 for 40-byte values, 292 for 16-byte ones, and 2053
 // instead of 1800 for the churn's, whose popular lines are then not in L1.
 template <int SB, int LW, bool PASSED, bool FEW, class Keys>
@@ -62,8 +62,8 @@ __global__ void __launch_bounds__(DOK_TPB, SB == 0 ? 1 : SB != 32 && LW == 2 ? 6
 // misses in 64-byte slots at load 0.69 750 -> 595, selections of 32-byte slots 153 -> 141.
 // Values of at most 8 bytes lie behind the tag in the word pair that a lane has loaded: the key's own lane fetches it from
 // the lane of the slot that matched, and stores value (or fallback) and flag of its row -- one store for 32 rows of which
-// most are neighbours.  16-byte values of 32-byte slots (dok_get_by_rows) are written by the lane that holds the slot.  Either
-// way a hit needs no second access to the table.
+// most are neighbours.  16-byte values are written by the lane that holds the slot, others by the lanes of the quad.  Either way
+// a hit needs no second access to the table.
 template <int SB, int LW, bool PASSED, class Keys>
 __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, DevHash hp, Keys keys, char *__restrict__ out_values,
                                                                   uint8_t *__restrict__ out_found, Fallback fb, ll_t *counters,
@@ -103,8 +103,8 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, De
         const unsigned row_r = __shfl_sync(FULL, lr.row, base + r);
         const unsigned m_r = (match[r] >> base) & 0xfu, me_r = m_r | ((empty[r] >> base) & 0xfu);
         if (me_r) {
-          const int pos = __ffs(me_r) - 1;
-          if ((m_r >> pos) & 1u) emit(keys.elem(share.first + row_r), pos, f.w[r]);
+          const int lane = __ffs(me_r) - 1;
+          if ((m_r >> lane) & 1u) emit(keys.elem(share.first + row_r), lane * 32 / SB, f.w[r]);
         }
       }
     }
@@ -180,16 +180,29 @@ inline dim3 dok_stream_grid(const Keys &keys) {
 // Which batches of key rows go to k_get_row.  Values of at most 8 bytes in 64- and 128-byte slots: with less than two rows for
 // each lane of k_get there are too few chains for a lane to take up when its own ends (k_get_row's time over k_get's, means
 // over hits, Zipf-distributed hits and misses at loads of 0.3 to 0.85: 30 k rows 0.99, 60 k 0.94, 100 k 0.91, 200 k 0.81,
-// 300 k 0.94, 500 k 1.00, 1 M 1.13), and below a block per SM they stay with k_get.  Wider values of 32-byte slots, where
-// k_get_row looks at the slot a second time: that costs nothing while address translation covers the table (a second access
-// to a sector just read is free in 256 MB, and in 4 GB it costs as much as a line), or the batch is all latency.  16-byte
-// values, k_get / k_get_row, us: 1 M rows, load 0.6, table of 32 MB 42 / 32, 256 MB 50 / 42, 512 MB 52 / 48, 2 GB 54 / 56; 8 M
-// rows 216 / 153, 259 / 200, 271 / 280, 290 / 357; 300 k rows 24..28 / 17..24.  Of 9 to 15 bytes, which no single store
-// takes, 8 M rows 273 / 159 ... 325 / 339, and misses at 0.8 527 / 484.  Selections of a tensor, whose index arithmetic a
-// share does for 32 rows at a time, differ by a tenth either way and stay with k_get.
+// 300 k 0.94, 500 k 1.00, 1 M 1.13), and below a block per SM they stay with k_get.
+// Wider values: k_get_row looks at the slot a second time.  That costs nothing where the batch is all latency or address
+// translation covers the table; beyond, every sector of it costs.  k_get_row / k_get, us, hits at load 0.6 | 30 % hits at 0.8:
+//                                  300 k rows         1 M                8 M
+//   9 to 15 bytes, 32-byte slots   512 MB             47/53   83/90      289/285 430/490
+//                                    2 GB 23/31 43/51 56/55   86/102     375/303 469/514    (2 M: 102/90 140/152)
+//   16 bytes, 32-byte slots        256 MB 20/25 37/47 41/47   77/82      186/240 395/408
+//                                  512 MB 21/25 40/47 49/49   83/83      304/253 430/432
+//   24 bytes, 64-byte slots          2 GB 30/37 64/90 66/81   125/152    408/399 715/731
+//   40 bytes, 64-byte slots        256 MB 29/33 60/74 59/66   115/129    309/352 643/664
+//                                  512 MB 33/35 57/76 72/66   125/133    440/367 686/692
+//   32 bytes, 128-byte slots       256 MB 33/45 92/121 73/80  178/184    387/441 1002/924
+//                                    2 GB 45/47 95/126 96/87  197/201    608/465 1118/1049
+//   64 bytes, 128-byte slots        64 MB 37/41 64/98 88/76   152/164    569/430 887/870
+// So a table's size decides where the value leaves the 32 bytes of its tag, and its own width where it fills three of those.
+// Selections of a tensor, whose index arithmetic a share does for 32 rows at a time, differ by a tenth either way and stay with
+// k_get in 32-byte slots; their values end in the tag's 32 bytes.
 inline bool dok_get_by_rows(const DevTable &t, ll_t n) {
   if (t.vb <= 8) return n >= 148LL * DOK_TPB && n < 148LL * DOK_TPB * 4 * 2;
-  return t.vb < 16 || n < 900000 || t.n_slots * t.sb <= 512LL << 20;
+  if (n < 400000 || (t.sb > 32 && t.vb <= 24)) return true;
+  const ll_t mb = t.n_slots * t.sb >> 20;
+  if (t.vb > 24) return t.vb <= 56 && mb <= 256;
+  return t.vb < 16 ? mb <= 512 || n < 1200000 : mb <= 256 || n < 900000;
 }
 
 template <class Keys>
@@ -209,7 +222,7 @@ inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, vo
   const auto launch = [&](auto slot_bytes, auto words, auto passed) {
     constexpr int SB = decltype(slot_bytes)::value, LW = decltype(words)::value;
     constexpr bool PASSED = decltype(passed)::value, ROWS = std::is_same<Keys, RowKeys>::value;
-    constexpr bool ONLY_ROWS = SB == 0 || (LW == 4 && SB != 32) || (ROWS && SB == 32 && LW == 2);
+    constexpr bool ONLY_ROWS = SB == 0 || (!ROWS && LW == 4 && SB != 32) || (ROWS && SB == 32 && LW == 2);
     if constexpr (ROWS || ONLY_ROWS)
       if (ONLY_ROWS || dok_get_by_rows(t, n)) {
         DOK_BY_SIZE(grid.x * grid.y, DOK_FOR_WINDOWS(t, rc, (k_get_row<SB, LW, PASSED, FEW && LW == 4 && SB != 0, Keys>

@@ -417,6 +417,29 @@ def test_lookups_into_outputs_that_are_only_8_byte_aligned(value_cols, offset):
     assert found.all() and torch.equal(out, stored) and out.data_ptr() == values.data_ptr()
 
 
+@pytest.mark.parametrize("key_size", [1, 2, 3, 4, 6])
+@pytest.mark.parametrize("dtype,cols", [(torch.uint8, 27), (torch.float16, 13), (torch.float32, 3), (torch.float32, 7), (torch.int64, 2), (torch.int64, 5), (torch.int64, 8)])
+@pytest.mark.parametrize("n", [399999, 400001, 900001])                        # on either side of the rule for wide values
+@pytest.mark.parametrize("n_buckets", [1 << 17, (1 << 23) + 77])
+def test_lookups_of_wide_values(key_size, dtype, cols, n, n_buckets):
+    """Hits and misses of values that end in the first, second and third 32 bytes of their slot, tombstones among them."""
+    from doksparse_b200 import CudaClosedHashmap
+    if n_buckets > 1 << 17 and (key_size not in (1, 2, 6) or n == 399999):
+        pytest.skip("the larger table once per width of slots")
+    np.random.seed(1)
+    table = CudaClosedHashmap(n_buckets=n_buckets, rehash_threshold=0.95, tombstone_threshold=None)
+    stored = n_buckets * 4 // 5 if n_buckets == 1 << 17 else 200001
+    keys = lambda c: c[:, None] * torch.arange(3, 3 + key_size, device="cuda") + torch.arange(key_size, device="cuda")
+    values = torch.randint(0, 100, (stored, cols), device="cuda").to(dtype)
+    table.set(keys(torch.arange(stored, device="cuda")), values, assume_unique=True)
+    assert table.remove_rows(keys(torch.arange(0, stored, 5, device="cuda"))).all()
+    asked = torch.randint(0, 2 * stored, (n,), device="cuda")
+    expected = (asked < stored) & (asked % 5 != 0)
+    got, found = table.get(keys(asked), torch.full((cols,), 7, device="cuda", dtype=dtype))
+    assert torch.equal(found, expected)
+    assert torch.equal(got, torch.where(expected[:, None], values[asked.clamp(max=stored - 1)], 7))
+
+
 def _looked_at(numel, elem_bytes):
     """Positions of the sample that decides whether the non-zeros of a dense tensor are listed."""
     each, piece = 16 // elem_bytes, np.arange(1024, dtype=np.uint64)
