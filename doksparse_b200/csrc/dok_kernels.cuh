@@ -232,8 +232,9 @@ inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, vo
     if constexpr (!ONLY_ROWS) DOK_STREAM(t, rc, st, keys, (k_get<SB, LW, PASSED, Keys>), hp, keys, values, out_found, fb, cnt, count_probes);
   };
   const auto by_width = [&](auto slot_bytes) {
-    if (dok_has_passed_bits(t)) launch(slot_bytes, std::integral_constant<int, 2>(), std::true_type());
-    else if (narrow) launch(slot_bytes, std::integral_constant<int, 2>(), std::false_type());
+    if constexpr (decltype(slot_bytes)::value != 32)         // (four slots per group have no marks)
+      if (dok_has_passed_bits(t)) return launch(slot_bytes, std::integral_constant<int, 2>(), std::true_type());
+    if (narrow) launch(slot_bytes, std::integral_constant<int, 2>(), std::false_type());
     else launch(slot_bytes, std::integral_constant<int, 4>(), std::false_type());
   };
   switch (t.sb) {
