@@ -183,7 +183,7 @@ struct Marks {
   long long numbered;          // largest number of a row that shares its value's word with it
   long long renumbered;        // ... that sets in graphs use again and again
   cudaStream_t stream;         // of the numbered sets so far
-  bool any, several;           // there were some; on more than one stream, or in a graph
+  bool any, several;           // there were some; on more than one stream
 };
 
 void marks_dealloc(Marks *self) {
@@ -229,9 +229,8 @@ bool start_over(const Plan *p, Marks *m, cudaStream_t stream) {
     if (dok_launch_count() != launched) continue;            // another thread had the interpreter meanwhile
     if (dok_map_clear_numbers(&p->table, stream) != DOK_OK) return false;
     C10_CUDA_CHECK(cudaStreamSynchronize(stream));
-    m->numbered = m->renumbered;
-    m->any = false;
-    m->several = m->renumbered > 0;
+    m->numbered = 0;
+    m->any = m->several = false;
     return true;
   }
   return false;
@@ -245,12 +244,11 @@ bool take_numbers(const Plan *p, Marks *m, int64_t n, cudaStream_t stream, int64
   if (capturing != cudaStreamCaptureStatusNone) {
     m->renumbered = std::max<long long>(m->renumbered, n);
     m->numbered = std::max(m->numbered, m->renumbered);
-    m->several = true;
     *base = DOK_RENUMBER;
     return true;
   }
-  if (m->numbered > DOK_MAX_NUMBER - n && (m->renumbered > DOK_MAX_NUMBER - n || !start_over(p, m, stream) || m->numbered > DOK_MAX_NUMBER - n))
-    return false;
+  // (sets in graphs are replayed without anybody asking here, so with them no moment is quiet for certain)
+  if (m->numbered > DOK_MAX_NUMBER - n && (m->renumbered > 0 || !start_over(p, m, stream))) return false;
   m->several = m->several || (m->any && m->stream != stream);
   m->any = true;
   m->stream = stream;

@@ -152,10 +152,11 @@ def test_replayed_sets_among_others(n, dtype):
         if i % 2:
             _both_set(table, oracle, *batch(n // 3))
         if i == 2:
-            table._marks.numbered = 0x7ffffff0                 # the next one starts the numbers over
+            table._marks.numbered = 0x7ffffff0                 # none left, and a replay may be on its way at any time: stamps
         gone = np.unique(rng.integers(0, 2 * n, n // 5))[:, None]
         np.testing.assert_array_equal(host(table.remove(dev(gone))), oracle.remove(gone))
         _same(table, oracle, everything)
+    assert table._marks.numbered == 0x7ffffff0 and table._marks.epoch == 2
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
