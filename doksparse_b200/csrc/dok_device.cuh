@@ -672,7 +672,7 @@ struct EmitValue {
   char *out_values;
   __device__ __forceinline__ void operator()(ll_t e_r, int pos, const ull_t (&w)[LW]) const {
     char *dst = out_values + e_r * (ll_t)t.vb;
-    if constexpr (LW == 4 && SB != 32) {
+    if constexpr (LW == 4 && SB != 32) {                   // (128-byte slots of values that fill more than half of them)
       const int start = pos * SB + 8 - 32 * (int)(threadIdx.x & 3u);      // of the value, from this lane's part of the line
       const int align = (t.vb & 7) ? t.vb & -t.vb : 8;
 #pragma unroll
@@ -782,24 +782,37 @@ __device__ __forceinline__ void dok_store_value(const DevTable &t, ll_t slot, co
 }
 
 // slot -> value row
-template <bool L1, class T>
-__device__ __forceinline__ T dok_load_as(const T *p) {
-  return L1 ? __ldca(p) : __ldcg(p);
-}
-template <bool L1 = false>
 __device__ __forceinline__ void dok_load_value(const DevTable &t, ll_t slot, char *dst) {
   const ull_t *src = (const ull_t *)dok_value_ptr(t, slot);
-  if (t.vb == 8) { *(ull_t *)dst = dok_load_as<L1>(src); return; }
-  if (t.vb == 4) { *(unsigned *)dst = dok_load_as<L1>((const unsigned *)src); return; }
+  if (t.vb == 8) { *(ull_t *)dst = __ldcg(src); return; }
+  if (t.vb == 4) { *(unsigned *)dst = __ldcg((const unsigned *)src); return; }
   if ((t.vb & 7) == 0) {
-    for (int w = 0; w < t.vwords; w++) ((ull_t *)dst)[w] = dok_load_as<L1>(src + w);
+    for (int w = 0; w < t.vwords; w++) ((ull_t *)dst)[w] = __ldcg(src + w);
   } else if ((t.vb & 3) == 0) {
-    for (int w = 0; w < (t.vb >> 2); w++) ((unsigned *)dst)[w] = dok_load_as<L1>((const unsigned *)src + w);
+    for (int w = 0; w < (t.vb >> 2); w++) ((unsigned *)dst)[w] = __ldcg((const unsigned *)src + w);
   } else if ((t.vb & 1) == 0) {
-    for (int w = 0; w < (t.vb >> 1); w++) ((unsigned short *)dst)[w] = dok_load_as<L1>((const unsigned short *)src + w);
+    for (int w = 0; w < (t.vb >> 1); w++) ((unsigned short *)dst)[w] = __ldcg((const unsigned short *)src + w);
   } else {
-    for (int w = 0; w < t.vb; w++) dst[w] = dok_load_as<L1>((const char *)src + w);
+    for (int w = 0; w < t.vb; w++) dst[w] = __ldcg((const char *)src + w);
   }
+}
+// ... of more than 8 bytes, for slots found at random: through L1, up to eight pieces on their way together
+template <class T>
+__device__ __forceinline__ void dok_fetch_pieces(const T *src, T *dst, int n) {
+  for (int i = 0; i < n; i += 8) {
+    T v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) if (i + k < n) v[k] = __ldca(src + i + k);
+#pragma unroll
+    for (int k = 0; k < 8; k++) if (i + k < n) dst[i + k] = v[k];
+  }
+}
+__device__ __forceinline__ void dok_fetch_value(const DevTable &t, ll_t slot, char *dst) {
+  const char *src = (const char *)dok_value_ptr(t, slot);
+  if ((t.vb & 7) == 0) dok_fetch_pieces((const ull_t *)src, (ull_t *)dst, t.vwords);
+  else if ((t.vb & 3) == 0) dok_fetch_pieces((const unsigned *)src, (unsigned *)dst, t.vb >> 2);
+  else if ((t.vb & 1) == 0) dok_fetch_pieces((const unsigned short *)src, (unsigned short *)dst, t.vb >> 1);
+  else dok_fetch_pieces((const unsigned char *)src, (unsigned char *)dst, t.vb);
 }
 
 struct Fallback { ull_t w[DOK_MAX_VALUE_BYTES / 8]; };   // miss fill, passed by value

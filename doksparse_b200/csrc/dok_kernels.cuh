@@ -20,10 +20,12 @@
 // than a line, and for batches that dok_get_by_rows names.
 // For values of more than 8 bytes the walk reads the tags alone, so that 64 warps are resident here too, and the row's own
 // lane reads the value where it was found -- from L1, as its sector has just come in, and further sectors of the line from
-// L2.  Against whole lines in the registers of 24 warps: 40-byte values, 300 k lookups of a 64 MB table 33 -> 25 us, 8 M
-// 323 -> 291; 16-byte values, 200 k 24 -> 18, 3000 15 -> 11.
+// L2, up to eight pieces at a time (one after the other: 33.5 M hits of 40-byte values in 8 GB 2294 -> 2050 us, of 28 bytes
+// 2339 -> 2052, 1 M of a 128 MB table 53 -> 49).  Against whole lines in the registers of 24 warps: 40-byte values, 300 k lookups
+// of a 128 MB table 31 -> 25 us, 8 M 367 -> 263; 16-byte values, 200 k 24 -> 18, 3000 15 -> 11.
 // Lines through cp.async and shared memory, 40 warps: 445, 62 and 50 for 40-byte values, 292 for 16-byte ones, and 2053
-// instead of 1800 for the churn's, whose popular lines are then not in L1.
+// instead of 1800 for the churn's, whose popular lines are then not in L1.  Values read and stored by the quad as soon as their
+// tag is found, when the line is in L1 for certain: 33.5 M hits 1852, but misses 1405 -> 1480 and 8 M of a 256 MB table 300 -> 343.
 template <int SB, int LW, bool PASSED, bool FEW, class Keys>
 __global__ void __launch_bounds__(DOK_TPB, SB == 0 ? 1 : SB != 32 && LW == 2 ? 6 : 8)
     k_get_row(DevTable t, DevHash hp, Keys keys, char *__restrict__ out_values, uint8_t *__restrict__ out_found, Fallback fb, ll_t *counters,
@@ -45,7 +47,10 @@ __global__ void __launch_bounds__(DOK_TPB, SB == 0 ? 1 : SB != 32 && LW == 2 ? 6
   const int hit = active && loc.found >= 0;
   if (active) {
     char *dst = out_values + e * (ll_t)t.vb;
-    if (AGAIN && hit) dok_load_value<SB != 0>(t, loc.found, dst);
+    if (AGAIN && hit) {
+      if constexpr (SB == 0) dok_load_value(t, loc.found, dst);
+      else dok_fetch_value(t, loc.found, dst);
+    }
     if (!hit) dok_store_fallback(t, fb, dst);
   }
   if (active && out_found) out_found[e] = (uint8_t)hit;
@@ -181,28 +186,27 @@ inline dim3 dok_stream_grid(const Keys &keys) {
 // each lane of k_get there are too few chains for a lane to take up when its own ends (k_get_row's time over k_get's, means
 // over hits, Zipf-distributed hits and misses at loads of 0.3 to 0.85: 30 k rows 0.99, 60 k 0.94, 100 k 0.91, 200 k 0.81,
 // 300 k 0.94, 500 k 1.00, 1 M 1.13), and below a block per SM they stay with k_get.
-// Wider values: k_get_row looks at the slot a second time.  That costs nothing where the batch is all latency or address
-// translation covers the table; beyond, every sector of it costs.  k_get_row / k_get, us, hits at load 0.6 | 30 % hits at 0.8:
-//                                  300 k rows         1 M                8 M
-//   9 to 15 bytes, 32-byte slots   512 MB             47/53   83/90      289/285 430/490
-//                                    2 GB 23/31 43/51 56/55   86/102     375/303 469/514    (2 M: 102/90 140/152)
-//   16 bytes, 32-byte slots        256 MB 20/25 37/47 41/47   77/82      186/240 395/408
-//                                  512 MB 21/25 40/47 49/49   83/83      304/253 430/432
-//   24 bytes, 64-byte slots          2 GB 30/37 64/90 66/81   125/152    408/399 715/731
-//   40 bytes, 64-byte slots        256 MB 29/33 60/74 59/66   115/129    309/352 643/664
-//                                  512 MB 33/35 57/76 72/66   125/133    440/367 686/692
-//   32 bytes, 128-byte slots       256 MB 33/45 92/121 73/80  178/184    387/441 1002/924
-//                                    2 GB 45/47 95/126 96/87  197/201    608/465 1118/1049
-//   64 bytes, 128-byte slots        64 MB 37/41 64/98 88/76   152/164    569/430 887/870
-// So a table's size decides where the value leaves the 32 bytes of its tag, and its own width where it fills three of those.
-// Selections of a tensor, whose index arithmetic a share does for 32 rows at a time, differ by a tenth either way and stay with
-// k_get in 32-byte slots; their values end in the tag's 32 bytes.
+// Wider values: k_get_row looks at the slot a second time, which costs nothing where the batch is all latency or address
+// translation covers the table.  In larger tables a batch of hits pays for it, but one with misses has more from the 64 warps
+// that walk.  k_get / k_get_row, us, 8 M rows, all / half / none of them stored:
+//                                   load 0.5                     load 0.8
+//   12 bytes, 32-byte slots  1 GB   305/287 343/254 285/236      359/340 504/424 512/487
+//                            4 GB   315/320 347/276 303/250      371/377 514/446 567/510
+//   16 bytes, 32-byte slots 256 MB  227/170 258/192 252/192      267/234 373/360 427/428
+//                            1 GB   254/305 281/258 281/236      303/350 426/420 508/486
+//   28 bytes, 64-byte slots  2 GB   469/473 528/371 430/346      573/563 819/666 815/792
+//   40 bytes, 64-byte slots 512 MB  390/371 446/316 421/326      471/446 678/625 752/756
+//                            2 GB   399/472 453/358 437/349      488/564 708/664 820/803
+//   64 bytes, 128-byte slots 256 MB 430/526 527/504 543/494      565/653 899/944 1034/1149
+//                            4 GB   455/727 553/553 569/549      616/862 1002/1061 1295/1305
+// Values that a lane of k_get stores at once (16 bytes of a 32-byte slot) and those that fill three sectors of their line have
+// less from k_get_row; at 300 k rows these take 41/37 49/39 48/43 and 76/62 125/82 121/85, at 1 M 82/110 98/96 106/96 and
+// 139/143 234/191 258/224 in 4 GB.  Selections of a tensor, whose index arithmetic a share does for 32 rows at a time, differ by
+// a tenth either way and stay with k_get in 32-byte slots.
 inline bool dok_get_by_rows(const DevTable &t, ll_t n) {
   if (t.vb <= 8) return n >= 148LL * DOK_TPB && n < 148LL * DOK_TPB * 4 * 2;
-  if (n < 400000 || (t.sb > 32 && t.vb <= 24)) return true;
-  const ll_t mb = t.n_slots * t.sb >> 20;
-  if (t.vb > 24) return t.vb <= 56 && mb <= 256;
-  return t.vb < 16 ? mb <= 512 || n < 1200000 : mb <= 256 || n < 900000;
+  if (t.vb > 56) return n < 1000000;
+  return t.sb > 32 || t.vb < 16 || n < 900000 || t.n_slots * t.sb <= 256LL << 20;
 }
 
 template <class Keys>
@@ -222,7 +226,7 @@ inline int launch_get(const DevTable &t, const DevHash &hp, const Keys &keys, vo
   const auto launch = [&](auto slot_bytes, auto words, auto passed) {
     constexpr int SB = decltype(slot_bytes)::value, LW = decltype(words)::value;
     constexpr bool PASSED = decltype(passed)::value, ROWS = std::is_same<Keys, RowKeys>::value;
-    constexpr bool ONLY_ROWS = SB == 0 || (!ROWS && LW == 4 && SB != 32) || (ROWS && SB == 32 && LW == 2);
+    constexpr bool ONLY_ROWS = SB == 0 || (LW == 4 && (SB == 64 || (SB == 128 && !ROWS))) || (ROWS && SB == 32 && LW == 2);
     if constexpr (ROWS || ONLY_ROWS)
       if (ONLY_ROWS || dok_get_by_rows(t, n)) {
         DOK_BY_SIZE(grid.x * grid.y, DOK_FOR_WINDOWS(t, rc, (k_get_row<SB, LW, PASSED, FEW && LW == 4 && SB != 0, Keys>

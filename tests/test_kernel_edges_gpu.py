@@ -419,7 +419,7 @@ def test_lookups_into_outputs_that_are_only_8_byte_aligned(value_cols, offset):
 
 @pytest.mark.parametrize("key_size", [1, 2, 3, 4, 6])
 @pytest.mark.parametrize("dtype,cols", [(torch.uint8, 27), (torch.float16, 13), (torch.float32, 3), (torch.float32, 7), (torch.int64, 2), (torch.int64, 5), (torch.int64, 8)])
-@pytest.mark.parametrize("n", [399999, 400001, 900001])                        # on either side of the rule for wide values
+@pytest.mark.parametrize("n", [399999, 900001, 1000001])                        # on either side of the rule for wide values
 @pytest.mark.parametrize("n_buckets", [1 << 17, (1 << 23) + 77])
 def test_lookups_of_wide_values(key_size, dtype, cols, n, n_buckets):
     """Hits and misses of values that end in the first, second and third 32 bytes of their slot, tombstones among them."""
