@@ -170,7 +170,8 @@ __device__ __forceinline__ bool dok_next_group(Index &group, unsigned &word, Ind
 // placed from another start (alpha2 = 0 in a column), and a lookup has to get past the groups that this walk went past.
 // 8.4 M lookups of a 4-D selection, nearly all misses: 587 -> 402 us; 4 M lookups at load 0.8, 30 % hits: 335 -> 210.  What it
 // costs: filling a 4-D tensor with 50 M rows 8.02 -> 8.29 ms (8.63 where the groups are read again for their marks), a table of
-// 2 slots per group up to load 0.8 1.60 -> 1.69, of one 2.53 -> 2.71; general sets of stored keys 2 to 3 %.  With 4 slots per
+// 2 slots per group up to load 0.8 1.60 -> 1.69, of one 2.53 -> 2.71, rebuilt 1.87 -> 2.18 and 2.75 -> 3.14; general sets of
+// stored keys 2 to 3 %.  With 4 slots per
 // group fewer keys go past one: at load 0.36 4 M lookups went from 140 to 127 us, but a table that grows to 300 k rows from 880
 // to 910 and a dense tensor's conversion from 348 to 359 (398 where the bit is written without a look), so those stay without.
 #define DOK_PASSED 0x8000000000000000ULL
@@ -725,6 +726,40 @@ __device__ __forceinline__ Located dok_locate(const DevTable &t, const Key &kh, 
 
 enum { DOK_OUT_FOUND = 0, DOK_OUT_CLAIMED_EMPTY = 1, DOK_OUT_REUSED = 2, DOK_OUT_FAILED = 3 };
 
+// Insert-or-find by one lane, slot by slot.  Phase 1 walks the chain: a matching tag is a hit; at the first empty tag the slot
+// is claimed by CAS unless a tombstone was seen.  Phase 2 walks it again and takes the first slot that is free, tombstone or
+// empty.  missing: of dok_mark_passed.
+template <bool MARKS>
+static __device__ __forceinline__ ll_t dok_find_or_claim_serial(const DevTable &t, const KeyHash &kh, int *outcome, unsigned *missing) {
+  const ll_t uuid = kh.uuid;
+  bool reuse = false;                                    // a tombstone was seen
+  for (int phase = 0; phase < 2; phase++) {
+    ll_t group = dok_start_group(kh, t);
+    unsigned word = dok_chain_word(kh, t);
+    *missing = 0;
+    bool more = true;
+    while (more) {
+      for (int i = 0; i < t.spg && more; i++) {
+        const ll_t slot = group * t.spg + i;
+        ll_t tag = dok_load_tag(t, slot);
+        if (tag == DOK_REMOVED && phase == 0) reuse = true;
+        if (tag == DOK_EMPTY && phase == 0 && reuse) { more = false; break; }
+        if (tag == DOK_EMPTY || (tag == DOK_REMOVED && phase == 1)) {
+          const ll_t old = dok_cas_tag(t, slot, tag, uuid);
+          if (old == tag) { *outcome = tag == DOK_EMPTY ? DOK_OUT_CLAIMED_EMPTY : DOK_OUT_REUSED; return slot; }
+          tag = old;
+        }
+        if (tag == uuid) { *outcome = DOK_OUT_FOUND; return slot; }
+      }
+      if (MARKS && more && !(__ldcg((const ull_t *)(t.slots + (ull_t)group * 128u + 8u)) & DOK_PASSED)) *missing |= 1u << min(word >> 6, 31u);
+      more = more && dok_next_group<ll_t>(group, word, t.n_groups);
+    }
+    if (!reuse) break;
+  }
+  *outcome = DOK_OUT_FAILED;
+  return -1;
+}
+
 // Insert-or-find for the 32 keys of a warp (ClosedHashmap::set, closed_hashmap_impl_class.cu:368-427, without the row
 // stores): one cooperative walk tells every owner lane where its uuid is or where the chain offers a place (first tombstone,
 // else first empty slot); the owner claims that place with one CAS.  Losing the CAS to the same uuid means a twin row of the
@@ -732,8 +767,10 @@ enum { DOK_OUT_FOUND = 0, DOK_OUT_CLAIMED_EMPTY = 1, DOK_OUT_REUSED = 2, DOK_OUT
 // so each lost CAS is a slot taken.  In a table that fills up that is no exception -- the rows that are on their way at a time
 // see the same first places -- and a lane that went on by itself, slot by slot, held its warp up: sets of a fifth new rows,
 // 300 k rows of 32-byte slots 60 -> 54 us, 1 M 113 -> 107, 30 k rows of 64-byte slots 59 -> 48.  Every lane of the warp must call.
+// ORDERED: keys in the order of the table, whose lanes compete for the places of their group on every walk: those that lose go
+// on by themselves (rebuild of 11.7 M rows in 32-byte slots 1535 -> 1430 us, in 64-byte slots 2020 -> 1904).
 // MARKS: the table may be one with marks.
-template <int SB, bool FEW = false, bool MARKS = (SB >= 64)>
+template <int SB, bool FEW = false, bool MARKS = (SB >= 64), bool ORDERED = false>
 __device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHash &kh, bool active, int *outcome) {
   ll_t slot = -1;
   do {
@@ -742,6 +779,7 @@ __device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHa
       active = false;
       slot = loc.found;
       *outcome = DOK_OUT_FOUND;
+      unsigned missing = (unsigned)loc.word;
       if (slot < 0) {
         slot = loc.tomb >= 0 ? loc.tomb : loc.empty;
         const ll_t expect = loc.tomb >= 0 ? DOK_REMOVED : DOK_EMPTY;
@@ -753,10 +791,15 @@ __device__ __forceinline__ ll_t dok_find_or_claim(const DevTable &t, const KeyHa
             *outcome = expect == DOK_EMPTY ? DOK_OUT_CLAIMED_EMPTY : DOK_OUT_REUSED;
           } else {
             active = old != kh.uuid;
+            if constexpr (ORDERED)
+              if (active) {
+                slot = dok_find_or_claim_serial<MARKS>(t, kh, outcome, &missing);
+                active = false;
+              }
           }
         }
       }
-      if constexpr (MARKS) if (loc.word && !active && slot >= 0) dok_mark_passed(t, dok_chain(kh, t), slot, (unsigned)loc.word);
+      if constexpr (MARKS) if (missing && !active && slot >= 0) dok_mark_passed(t, dok_chain(kh, t), slot, missing);
     }
   } while (__any_sync(0xffffffffu, active));
   return slot;

@@ -723,8 +723,8 @@ __global__ void __launch_bounds__(DOK_TPB) k_count_new(DevTable t, DevHash hp, K
 // the reference's rehash = two boolean-mask gathers plus a full `set` with its pre-get and unique
 // (cuda_closed_hashmap.py:456-468) and this library's own compaction + insert.  Live keys are pairwise different,
 // so every row claims a fresh slot; tombstones stay behind.
-template <int SB, bool FEW>
-__global__ void __launch_bounds__(DOK_TPB) k_reinsert(DevTable src, DevTable dst, DevHash hp, ll_t *counters) {
+template <int SB, bool FEW, bool MARKS>
+__global__ void __launch_bounds__(DOK_TPB, FEW ? 4 : 5) k_reinsert(DevTable src, DevTable dst, DevHash hp, ll_t *counters) {
   const ll_t stride = (ll_t)gridDim.x * DOK_TPB;
   int claimed = 0, failed = 0, found = 0;
   for (ll_t base = (ll_t)blockIdx.x * DOK_TPB; base < src.nb; base += stride) {       // uniform over the block
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(DOK_TPB) k_reinsert(DevTable src, DevTable dst
     }
     active = dok_in_window(dst, kh, active);
     int outcome = -1;
-    const ll_t slot = dok_find_or_claim<SB, FEW>(dst, kh, active, &outcome);
+    const ll_t slot = dok_find_or_claim<SB, FEW, MARKS, true>(dst, kh, active, &outcome);
     if (active && slot >= 0) {
       char *drow = dok_key_row(dst, slot);
       if ((dst.kb & 7) == 0) for (int i = 0; i < (dst.kb >> 3); i++) ((ull_t *)drow)[i] = ((const ull_t *)krow)[i];

@@ -275,7 +275,7 @@ int dok_map_reinsert(const dok_table *src, const dok_table *dst, const dok_hash_
   if (blocks > 148 * 8) blocks = 148 * 8;            // 8 resident blocks of 256 threads per SM, grid-stride over the slots
   if (blocks < 1) blocks = 1;
   int rc = DOK_OK;
-  DOK_DISPATCH_SB(dt, DOK_BY_SIZE(blocks, DOK_FOR_WINDOWS(dt, rc, (k_reinsert<SB, FEW><<<(unsigned)blocks, DOK_TPB, 0, (cudaStream_t)stream>>>(
+  DOK_DISPATCH_MARKS(dt, DOK_BY_SIZE(blocks, DOK_FOR_WINDOWS(dt, rc, (k_reinsert<SB, FEW, MARKS><<<(unsigned)blocks, DOK_TPB, 0, (cudaStream_t)stream>>>(
                                                   st_, wt, dh, (ll_t *)counters)))));
   return rc;
 }

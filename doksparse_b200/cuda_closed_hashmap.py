@@ -936,10 +936,6 @@ class CudaClosedHashmap:
         source.value_bytes, source.key_bytes = self._value_bytes, self._key_bytes
         fresh = torch.empty(self._layout.total_bytes, device=self.device, dtype=torch.uint8)     # may raise: nothing changed yet
         state = old_state.clone()
-        # the sizes are those of before; only the tombstones are gone: reused = removed
-        gone = state[_BY_REMOVE + L.CNT_HITS] - state[L.CNT_REUSED_REMOVED]
-        state[L.CNT_CLAIMED_EMPTY] -= gone
-        state[L.CNT_REUSED_REMOVED] += gone
         known = self._shared.known
         self._slots, self._counters_of_table, self._marks, self._shared = fresh, state, L.native().Marks(), _Shared(self._shared.bound)
         self._shared.known = known
@@ -949,6 +945,10 @@ class CudaClosedHashmap:
             L.check(L.lib().dok_map_init(self._c_table(), st), "dok_map_init")
             L.check(L.lib().dok_map_reinsert(ctypes.byref(source), self._c_table(), self._c_hash(), None, st),
                     "dok_map_reinsert")
+        # the sizes are those of before; only the tombstones are gone: reused = removed
+        gone = state[_BY_REMOVE + L.CNT_HITS] - state[L.CNT_REUSED_REMOVED]
+        state[L.CNT_CLAIMED_EMPTY] -= gone
+        state[L.CNT_REUSED_REMOVED] += gone
         for old in (old_slots, old_state):
             old.record_stream(torch.cuda.current_stream(self.device))
         self._tombstone_host_bound = 0
