@@ -183,9 +183,10 @@ inline dim3 dok_stream_grid(const Keys &keys) {
   DOK_FOR_WINDOWS(t, rc, (KERNEL<<<dok_stream_grid<KERNEL>(keys), DOK_TPB, 0, st>>>(wt, __VA_ARGS__)))
 
 // Which batches of key rows go to k_get_row.  Values of at most 8 bytes in 64- and 128-byte slots: with less than two rows for
-// each lane of k_get there are too few chains for a lane to take up when its own ends (k_get_row's time over k_get's, means
-// over hits, Zipf-distributed hits and misses at loads of 0.3 to 0.85: 30 k rows 0.99, 60 k 0.94, 100 k 0.91, 200 k 0.81,
-// 300 k 0.94, 500 k 1.00, 1 M 1.13), and below a block per SM they stay with k_get.
+// each lane of k_get there are too few chains for a lane to take up when its own ends.  k_get / k_get_row, us, 4-byte values in
+// 64-byte slots, table of 2^21 slots at load 0.6, all / none of them stored: 64 rows 7.2/6.9 6.9/6.4, 1000 10.2/9.1 8.4/7.8,
+// 8000 11.9/9.8 10.8/8.6, 37 k 13.4/11.2 11.5/9.8 (at 0.85 29.4/22.1 29.1/23.5); of 2^22 slots at load 0.8 500 k 47/47 45/46,
+// 1 M 62/74 63/75, 4 M 166/240 176/247.
 // Wider values: k_get_row looks at the slot a second time, which costs nothing where the batch is all latency or address
 // translation covers the table.  In larger tables a batch of hits pays for it, but one with misses has more from the 64 warps
 // that walk.  k_get / k_get_row, us, 8 M rows, all / half / none of them stored:
@@ -204,7 +205,7 @@ inline dim3 dok_stream_grid(const Keys &keys) {
 // 139/143 234/191 258/224 in 4 GB.  Selections of a tensor, whose index arithmetic a share does for 32 rows at a time, differ by
 // a tenth either way and stay with k_get in 32-byte slots.
 inline bool dok_get_by_rows(const DevTable &t, ll_t n) {
-  if (t.vb <= 8) return n >= 148LL * DOK_TPB && n < 148LL * DOK_TPB * 4 * 2;
+  if (t.vb <= 8) return n < 148LL * DOK_TPB * 4 * 2;
   if (t.vb > 56) return n < 1000000;
   return t.sb > 32 || t.vb < 16 || n < 900000 || t.n_slots * t.sb <= 256LL << 20;
 }
