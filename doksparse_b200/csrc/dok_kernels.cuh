@@ -76,21 +76,25 @@ __global__ void __launch_bounds__(DOK_TPB, LW == 4 ? 3 : 4) k_get(DevTable t, De
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ WarpQueue queues[DOK_WARPS];
   int hits = 0, probes = 0;
-  dok_walk_share<LW, true>(queues[threadIdx.x >> 5], t, hp, keys, [&](LaneRow &lr, const Lines<LW> &f, const WarpShare &share) {
+  dok_walk_share<LW, true, PASSED>(queues[threadIdx.x >> 5], t, hp, keys, [&](LaneRow &lr, const Lines<LW> &f, const WarpShare &share) {
     const unsigned l = threadIdx.x & 3u, base = threadIdx.x & 28u;
     unsigned m, me, match[4], empty[4];
     ull_t value = 0;
     if constexpr (LW == 2) {
-      const unsigned bits = dok_inspect<SB, LW, PASSED>(lr, f);
-      m = dok_matches(bits, l); me = dok_ends(bits, l);
-      const unsigned from = base + (me ? (unsigned)(__ffs(me) - 1) * (SB / 32) : 0u);
+      if constexpr (SB == 32) {
+        const unsigned bits = dok_inspect<SB, LW>(lr, f);
+        m = dok_matches(bits, l); me = dok_ends(bits, l);
+      } else {
+        dok_inspect_votes<SB, LW, PASSED>(lr, f, m, me, match, empty);
+      }
+      const unsigned from = base + (me ? (unsigned)__ffs(me) - 1 : 0u);
 #pragma unroll
       for (unsigned r = 0; r < 4; r++) {
         const ull_t v = __shfl_sync(FULL, f.w[r][1], from);
         if (l == r) value = v;
       }
     } else {
-      dok_inspect_votes<SB, LW>(lr, f, m, me, match, empty);
+      dok_inspect_votes<SB, LW, false>(lr, f, m, me, match, empty);
       const EmitValue<SB, LW, false> emit{t, out_values};
       // 16-byte values: one store
       const bool pairs = t.vb == 16 && ((size_t)out_values & 15) == 0;

@@ -92,35 +92,35 @@ __device__ __forceinline__ bool dok_refill(const WarpQueue &q, WarpShare &s, Lan
 // One group for each lane: four requests, each for the lines of a quad's key in its turn.
 template <int LW>
 struct Lines { ull_t w[4][LW]; };
-template <int LW, bool L1>
+// MARKS (of 64- and 128-byte slots): the last lane, whose part of the line has no tag, reads the group's mark.
+template <int LW, bool L1, bool MARKS>
 __device__ __forceinline__ void dok_request(const DevTable &t, const LaneRow &lr, Lines<LW> &f) {
-  const char *my_base = t.slots + 32 * (threadIdx.x & 3u);
+  const unsigned l = threadIdx.x & 3u;
+  const char *my_base = t.slots + (MARKS && l == 3 ? 0 : 32 * l);
 #pragma unroll
   for (unsigned r = 0; r < 4; r++)
     dok_load_words<LW, L1>(my_base + (ull_t)__shfl_sync(0xffffffffu, lr.group, (threadIdx.x & 28u) + r) * 128u, f.w[r]);
 }
 
-// What the lines of a quad's four keys hold: byte r = key r, bits 0-3 match, 4-7 empty, by slot of the group.  ENDS: a group
-// that no key went past counts as one whose last slot is empty (dok_mark_passed).
-template <int SB, int LW, bool ENDS>
+// What the lines of a quad's four keys hold: byte r = key r, bits 0-3 match, 4-7 empty, by slot of the group.
+template <int SB, int LW>
 __device__ __forceinline__ unsigned dok_inspect(const LaneRow &lr, const Lines<LW> &f) {
   constexpr unsigned FULL = 0xffffffffu;
   const unsigned l = threadIdx.x & 3u, base = threadIdx.x & 28u;
-  const bool has_tag = ((32u * l) % SB) == 0, look = ENDS && l == 0;
+  const bool has_tag = ((32u * l) % SB) == 0;
   unsigned bits = 0;
 #pragma unroll
   for (unsigned r = 0; r < 4; r++) {
     const ll_t uuid_r = __shfl_sync(FULL, lr.uuid, base + r), tag = (ll_t)f.w[r][0];
     if (has_tag) bits |= ((unsigned)(tag == uuid_r) | ((unsigned)(tag == DOK_EMPTY) << 4)) << (8u * r + 32u * l / SB);
-    if constexpr (ENDS) if (look && !(f.w[r][1] & DOK_PASSED)) bits |= 1u << (8u * r + 3u + 128u / SB);
   }
   bits |= __shfl_xor_sync(FULL, bits, 1);
   bits |= __shfl_xor_sync(FULL, bits, 2);
   return bits;
 }
-// The same by votes, bits by LANE of the quad (the slot at lane p is p * 32 / SB): for whole lines, whose values the quad
-// stores key by key from the votes (1 M lookups of 40-byte values: 69 us, 72 with the bits of a byte per key).
-template <int SB, int LW>
+// The same by votes, bits by LANE of the quad (the slot at lane p is p * 32 / SB).  MARKS: a group that no key went past counts
+// as one with an empty slot at the last lane (dok_mark_passed).
+template <int SB, int LW, bool MARKS>
 __device__ __forceinline__ void dok_inspect_votes(const LaneRow &lr, const Lines<LW> &f, unsigned &m, unsigned &me, unsigned (&match)[4],
                                                   unsigned (&empty)[4]) {
   constexpr unsigned FULL = 0xffffffffu;
@@ -131,7 +131,7 @@ __device__ __forceinline__ void dok_inspect_votes(const LaneRow &lr, const Lines
   for (unsigned r = 0; r < 4; r++) {
     const ll_t uuid_r = __shfl_sync(FULL, lr.uuid, base + r), tag = (ll_t)f.w[r][0];
     match[r] = __ballot_sync(FULL, has_tag && tag == uuid_r);
-    empty[r] = __ballot_sync(FULL, has_tag && tag == DOK_EMPTY);
+    empty[r] = __ballot_sync(FULL, (has_tag && tag == DOK_EMPTY) || (MARKS && l == 3 && !(f.w[r][LW > 1 ? 1 : 0] & DOK_PASSED)));
     if (l == r) { own_m = match[r]; own_e = empty[r]; }
   }
   m = (own_m >> base) & 0xfu;
@@ -142,7 +142,7 @@ __device__ __forceinline__ unsigned dok_ends(unsigned bits, unsigned r) { return
 
 // The loop.  `step(lane's row, lines, share)` inspects the lines, lets the row go to its next group (dok_next_group) or ends
 // it (done()).
-template <int LW, bool L1, class Keys, class Step>
+template <int LW, bool L1, bool MARKS, class Keys, class Step>
 __device__ __forceinline__ void dok_walk_share(WarpQueue &queue, WarpShare share, const DevTable &t, const DevHash &hp, const Keys &keys,
                                                const Step &step) {
   LaneRow lr = DOK_IDLE_LANE;
@@ -150,12 +150,12 @@ __device__ __forceinline__ void dok_walk_share(WarpQueue &queue, WarpShare share
   for (;;) {
     dok_fill_queue(queue, share, t, hp, keys);
     if (!dok_refill(queue, share, lr, t)) break;
-    dok_request<LW, L1>(t, lr, lines);
+    dok_request<LW, L1, MARKS>(t, lr, lines);
     step(lr, lines, share);
   }
 }
 // ... of the warp's part of the whole batch
-template <int LW, bool L1, class Keys, class Step>
+template <int LW, bool L1, bool MARKS, class Keys, class Step>
 __device__ __forceinline__ void dok_walk_share(WarpQueue &queue, const DevTable &t, const DevHash &hp, const Keys &keys, const Step &step) {
-  dok_walk_share<LW, L1>(queue, dok_share(keys.total()), t, hp, keys, step);
+  dok_walk_share<LW, L1, MARKS>(queue, dok_share(keys.total()), t, hp, keys, step);
 }

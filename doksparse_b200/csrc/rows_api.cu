@@ -763,9 +763,9 @@ __global__ void __launch_bounds__(DOK_TPB, 4) k_remove_unique(DevTable t, DevHas
     }
   } else {
     const unsigned first = total * warp / DOK_WARPS, last = total * (warp + 1) / DOK_WARPS;
-    dok_walk_share<1, false>(queues[warp], WarpShare{first, last - first, 0, 0, 0}, t, hp, HeadKeys{keys, head_row},
+    dok_walk_share<1, false, false>(queues[warp], WarpShare{first, last - first, 0, 0, 0}, t, hp, HeadKeys{keys, head_row},
                       [&](LaneRow &lr, const Lines<1> &f, const WarpShare &share) {
-      const unsigned bits = dok_inspect<SB, 1, false>(lr, f), m = dok_matches(bits, tid & 3), me = dok_ends(bits, tid & 3);
+      const unsigned bits = dok_inspect<SB, 1>(lr, f), m = dok_matches(bits, tid & 3), me = dok_ends(bits, tid & 3);
       if (!lr.busy()) return;
       const unsigned pos = me ? (unsigned)__ffs(me) - 1 : 0;
       const unsigned slot = lr.group * (128 / SB) + pos;
