@@ -171,9 +171,9 @@ __device__ __forceinline__ bool dok_next_group(Index &group, unsigned &word, Ind
 // 8.4 M lookups of a 4-D selection, nearly all misses: 587 -> 402 us; 4 M lookups at load 0.8, 30 % hits: 335 -> 210.  What it
 // costs: filling a 4-D tensor with 50 M rows 8.02 -> 8.29 ms (8.63 where the groups are read again for their marks), a table of
 // 2 slots per group up to load 0.8 1.60 -> 1.69, of one 2.53 -> 2.71, rebuilt 1.87 -> 2.18 and 2.75 -> 3.14; general sets of
-// stored keys 2 to 3 %.  With 4 slots per
-// group fewer keys go past one: at load 0.36 4 M lookups went from 140 to 127 us, but a table that grows to 300 k rows from 880
-// to 910 and a dense tensor's conversion from 348 to 359 (398 where the bit is written without a look), so those stay without.
+// stored keys 2 to 3 %.  With 4 slots per group fewer keys go past one: at load 0.36 4 M lookups went from 140 to 127 us, but a
+// table that grows to 300 k rows from 880 to 910 and a dense tensor's conversion from 348 to 359 (398 where the bit is written
+// without a look), so those stay without.
 #define DOK_PASSED 0x8000000000000000ULL
 __host__ __device__ __forceinline__ bool dok_has_passed_bits(const DevTable &t) { return t.vb < 8 && t.spg <= 2; }
 // a key was placed or found in `slot`: marks the groups before it on its chain that the walk saw without the mark (bit k of
@@ -639,8 +639,8 @@ __device__ __forceinline__ Located dok_locate_quad(const DevTable &t, const Key 
 
   // Keys whose chain runs into further groups.  A large batch, which keeps the memory busy, has the fewest instructions with
   // one key per quad and iteration.  A small one waits for the iterations: all of the quad's keys at once while a quad has
-  // more than one (sets of 30 k rows of 64-byte slots at load 0.65 55 -> 49 us, lookups 31 -> 27, a table that grows to 300 k
-  // rows 803 -> 767; no difference at 300 k rows; sets of 33.5 M rows 2694 -> 2713).
+  // more than one (sets of 30 k rows of 64-byte slots at load 0.65 55 -> 49 us, lookups 31 -> 27; no difference at 300 k rows;
+  // sets of 33.5 M rows 2694 -> 2713).
   if constexpr (Emit::BOTH) {
     unsigned pend = FULL;
     for (bool all = true;;) {

@@ -34,7 +34,6 @@ _PARAM_NAMES = ("prime1", "prime2", "alpha1", "alpha2", "beta1", "beta2")
 _STATE_WORDS = 32
 _BY_SET, _BY_REMOVE, _BY_ROWS, _BY_BULK = 0, 8, 16, 24      # set | remove | distinct new rows of float keys | bulk inserts
 _ADJUST = 7              # what n_elements differs by from the slots in use (the reference's DOK assignments over-count)
-_SEQUENCE = 18           # (three words that are free: row numbers are handed out by the host, see _native.Marks)
 _COUNTED_NEW = 23        # result of the exact count of a set that may have to grow the table
 
 
